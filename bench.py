@@ -55,21 +55,21 @@ ALGO_BYTES_PER_CELL_UPDATE = 5 * 40 + 3 * 40 + 3 * 22 * 8          # 848
 # Per-launch compulsory bytes per node of each structured kernel (every
 # input and output element once).
 KERNEL_BYTES_PER_NODE = {
-    "prep": (5 + 9 + 1 + 5 + 5 + 15 + 2) * 8,          # prims, metrics, det -> Q, U_j, F/E/G, sqrt(rho), H
-    "viscous": (5 + 9 + 1 + 4 + 15 + 1) * 8,           # U_j, metrics, det, prims -> Fv/Ev/Gv, mu
+    "prep": (5 + 9 + 1 + 5 + 5 + 15 + 5) * 8,          # prims, metrics, det -> Q, U_j, F/E/G, sqrt(rho) and products
+    "viscous": (5 + 9 + 1 + 1 + 4 + 15 + 1) * 8,       # U_j, metrics, det, width, prims -> Fv/Ev/Gv, mu
     "mu_only": (5 + 1) * 8,
-    "face_i": (5 + 3 + 2 + 3 + 1 + 5 + 5) * 8,         # Q, u/v/w, sqrt(rho)/H, face metric, face det, F -> Fh
-    "face_j": (5 + 3 + 2 + 3 + 1 + 5 + 5) * 8,
-    "face_k": (5 + 3 + 2 + 3 + 1 + 5 + 5) * 8,
+    "face_base": (5 + 3 * (3 + 12)) * 8,               # sqrt(rho) and products, normals -> Roe scalars (3 faces)
+    "face_char": (5 + 3 * (12 + 3 + 10)) * 8,          # Q, Roe scalars, normals -> characteristic values
+    "face_back": (15 + 3 * (8 + 3 + 10 + 20)) * 8,     # F/E/G, scalars, values -> face states, correction terms
+    "face_flux": 3 * (10 + 4 + 10 + 5) * 8,            # face states, face metric and det, terms -> Fh
     "update": (15 + 15 + 10 + 1 + 5 + 8) * 8,          # Fh, Fv/Ev/Gv, two U, det -> U, 8 FLOW fields
 }
-# FP64 operations per face of the FP64 face kernels, from ncu's FP64
-# instruction counters on the 64^3 Taylor-Green case (per face: 818 DFMA,
-# 784 DMUL, 575 DADD; FMA = 2), and the DRAM bytes the same capture measured
-# per face (dram__bytes_read.sum + dram__bytes_write.sum over 262,144 faces;
-# scaled by the face count of a launch for other sizes).
-FP64_FLOP_PER_NODE = {"face_i": 2995, "face_j": 2995, "face_k": 2995}
-DRAM_BYTES_PER_NODE = {"face_i": 153, "face_j": 155, "face_k": 155}
+# FP64-pipe instructions per node of the face pass's characteristic kernel
+# (three faces of five fields; the reference's products, quotients and roots
+# run on the integer pipe) and its DRAM bytes, from ncu's counters on the
+# 64^3 Taylor-Green case.
+FP64_INST_PER_NODE = {"face_char": 1}
+DRAM_BYTES_PER_NODE = {"face_char": 1}
 
 
 # The precision forms (cfd_precision_t) and how each one's arithmetic reads.
@@ -394,11 +394,11 @@ def gpu_arm(args):
     fp64_peak = ctx.probe_flops(True)
     fp32_peak = ctx.probe_flops(False)
     fp64_roof = None
-    if dom in FP64_FLOP_PER_NODE:
-        f = FP64_FLOP_PER_NODE[dom] * N / (table[dom] * 1e-3)
-        fp64_roof = {"kernel": dom, "achieved": f / 1e12, "peak": fp64_peak / 1e12, "unit": "TFLOP/s",
-                     "frac": f / fp64_peak, "peak_source": "FP64 FMA probe of this run",
-                     "note": "DMUL/DADD count one FLOP but take a full FP64 issue slot"}
+    if dom in FP64_INST_PER_NODE:
+        f = FP64_INST_PER_NODE[dom] * N / (table[dom] * 1e-3)
+        fp64_roof = {"kernel": dom, "achieved": f / 1e12, "peak": 0.5 * fp64_peak / 1e12, "unit": "T FP64 instructions/s",
+                     "frac": f / (0.5 * fp64_peak), "peak_source": "FP64 FMA probe of this run (2 FLOP each)",
+                     "note": "the reference's sums; its products, quotients and roots run on the integer pipe"}
     traffic = DRAM_BYTES_PER_NODE[dom] * N if dom in DRAM_BYTES_PER_NODE else None
 
     line = {

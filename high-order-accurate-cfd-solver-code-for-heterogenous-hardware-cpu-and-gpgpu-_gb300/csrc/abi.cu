@@ -86,6 +86,11 @@ Phys make_phys(const cfd_params_t *p)
     P.viscous = p->viscous;
     P.les = p->les;
     P.cs = p->smagorinsky_cs;
+    P.c_temp = 1.4 * P.mach * P.mach * 0.4;
+    P.st = 110.4 / P.t_inf;
+    P.st1 = 1.0 + P.st;
+    P.pr_re = P.prandtl * P.reynolds;
+    P.ck = 1.0 / (1.4 * 0.4 * P.mach * P.mach);
     return P;
 }
 

@@ -355,7 +355,7 @@ std::vector<std::pair<void *, size_t>> mutable_arrays(const BatchInst &I, int pr
     } else {
         v.push_back({I.view.Q, 5 * N * 8});
         v.push_back({I.view.FEG, 15 * N * 8});
-        v.push_back({I.view.sh, 2 * N * 8});
+        v.push_back({I.view.sh, 5 * N * 8});
     }
     return v;
 }
@@ -595,7 +595,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         v.idet64 = idet64;
     } else {
         if ((st = ialloc(b, I, 5 * Nz, &v.Q)) || (st = ialloc(b, I, 15 * Nz, &v.FEG)) || (st = ialloc(b, I, 15 * Nz, &v.V))
-            || (st = ialloc(b, I, 2 * Nz, &v.sh)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))) {
+            || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))) {
             free_instance(I);
             return st;
         }

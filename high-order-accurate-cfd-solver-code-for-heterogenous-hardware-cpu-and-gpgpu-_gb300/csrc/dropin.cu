@@ -180,14 +180,12 @@ __global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restric
     const double D = det[gid];
     const double *fr = flow + 9 * (size_t)gid;
     const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
-    double Fn[5], En[5], Gn[5];
-    ex::node_flux(prim, m, D, Fn, En, Gn);
+    double Fn[5], En[5], Gn[5], Qn[5], H;
+    ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
     double Fvn[5], Evn[5], Gvn[5];
     double mu;
     {
-        double dU[3][5];
-#pragma unroll 1
-        for (int d = 0; d < 3; ++d) {
+        auto dU = [&](int d, double (&out)[5]) {
             int L[7];
 #pragma unroll
             for (int o = 0; o < 7; ++o) L[o] = grid_loc(grid, idx[d][o]);
@@ -196,9 +194,9 @@ __global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restric
                 double f[7];
 #pragma unroll
                 for (int o = 0; o < 7; ++o) f[o] = U[5 * (size_t)idx[d][o] + c];
-                dU[d][c] = visc_deriv_ref(f, L);
+                out[c] = visc_deriv_ref(f, L);
             }
-        }
+        };
         double Ui[5];
 #pragma unroll
         for (int c = 0; c < 5; ++c) Ui[c] = U[5 * (size_t)gid + c];
@@ -207,10 +205,9 @@ __global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restric
         for (int d = 0; d < 3; ++d) {
             const int c = d + 1;
             const double *um = U + 5 * (size_t)idx[d][2], *up = U + 5 * (size_t)idx[d][4];
-            KS[d] = ex::ks(Ui[c], Ui[0], um[c], um[0], up[c], up[0]);
+            KS[d] = ex::ks_root(Ui[c], Ui[0], um[c], um[0], up[c], up[0]);
         }
-        const ex::Visc V{P.mach, P.reynolds, P.prandtl, P.t_inf, P.les, P.cs};
-        ex::viscous_node(dU, Ui, m, D, prim, KS, V, Fvn, Evn, Gvn, mu);
+        ex::viscous_node(dU, Ui, m, D, ex::filter_width(D), prim, KS, P, Fvn, Evn, Gvn, mu);
     }
     double *o;
 #pragma unroll

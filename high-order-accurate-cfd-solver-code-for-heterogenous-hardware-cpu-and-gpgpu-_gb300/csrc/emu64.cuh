@@ -26,6 +26,8 @@
 
 #include <cuda_runtime.h>
 
+#include "exact_int.cuh"
+
 namespace cfd {
 namespace emu {
 
@@ -166,38 +168,8 @@ __device__ __forceinline__ double add(double a, double b)
 
 __device__ __forceinline__ double sub(double a, double b) { return add(a, f64(u64(b) ^ kSign)); }
 
-// a * b.  The 53-bit significands multiply exactly into 106 bits from four
-// 32 x 32 -> 64 products; with the leading bit at 105 (top = 1) or 104 the
-// result is the product shifted right by 52 + top, the next bit down is the
-// round bit and everything below it the sticky flag; then rounding to
-// nearest even as in add.  An operand that is zero, subnormal, infinite or
-// NaN, or an exponent ea + eb - 1023 (+ top) outside [1, 2046] -- a
-// subnormal result or an overflow before rounding -- takes the FP64
-// multiply.
-__device__ __forceinline__ double mul(double a, double b)
-{
-    const uint64_t ua = u64(a), ub = u64(b);
-    const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
-    const uint32_t la = (uint32_t)ua, lb = (uint32_t)ub;
-    const unsigned ea = (ha >> 20) & 0x7ffu, eb = (hb >> 20) & 0x7ffu;
-    const int e = (int)ea + (int)eb - 1023;
-    if (__builtin_expect(ea - 1u >= 0x7feu || eb - 1u >= 0x7feu || (unsigned)e > 2045u, 0)) return fp64_mul(a, b);
-    const uint32_t ah = (ha & 0xfffffu) | 0x100000u, bh = (hb & 0xfffffu) | 0x100000u;
-    const uint64_t p0 = (uint64_t)la * lb;
-    const uint64_t mid = (uint64_t)ah * lb + (uint64_t)la * bh;
-    const uint64_t lo = p0 + (mid << 32);
-    const uint64_t hi = (uint64_t)ah * bh + (mid >> 32) + (lo < p0);   // product = hi * 2^64 + lo
-    const unsigned top = (unsigned)(hi >> 41);
-    const uint64_t M0 = (hi << 12) | (lo >> 52);   // product >> 52
-    const uint64_t G = lo << 12;                   // product bits 51..0 at the top
-    const uint64_t M = M0 >> top;
-    const unsigned rnd = top ? (unsigned)M0 & 1u : (unsigned)(G >> 63);
-    const unsigned stk = top ? (G != 0) : ((G << 1) != 0);
-    const uint64_t up = rnd & (stk | ((unsigned)M & 1u));
-    const int er = e + (int)top;
-    if (__builtin_expect(er < 1, 0)) return fp64_mul(a, b);
-    return f64(((ua ^ ub) & kSign) | ((((uint64_t)(er - 1)) << 52) + M + up));
-}
+// a * b (exact_int.cuh).
+__device__ __forceinline__ double mul(double a, double b) { return xi::mul(a, b); }
 
 // A binary64 value whose +, - and * run on the integer pipe (the routines
 // above; the same bits as the FP64 instructions).  An expression over Dbl

@@ -35,6 +35,8 @@ struct LatView {
     double *U0, *U1, *U2;
     // FP64 stage intermediates
     double *Q, *FEG, *V, *sh, *Fh;
+    const double *kn;          // [9][N] unit normals of the faces
+    const double *del;         // [N] 1 / det^(1/3) (null: evaluated where it is used)
     // FP32 stage intermediates (mixed form)
     float *Q32, *R32, *FEG32, *V32, *Fh32;
     unsigned *flags;           // error word of this lattice
@@ -57,6 +59,14 @@ struct LatView {
     const unsigned char *locflag;
     const int *row_of;         // node n -> reference row (null: row n + 1)
 };
+
+// Scratch of the FP64 face kernels for the faces of nodes n0 .. n0 + ld - 1:
+// [direction][element][ld] (lattice_fp64.cuh, FS_*).
+struct FaceScratch {
+    double *p;
+    int n0, ld;
+};
+constexpr int kFaceScratch = 42;   // doubles per node and direction
 
 __device__ __forceinline__ bool lat_locdir(const LatView &g, int d) { return g.loc8 && ((g.locdirs >> d) & 1); }
 

@@ -20,33 +20,37 @@ __device__ __forceinline__ void prep_values(const LatView &g, int n, int q, doub
 {
     const int N = g.N;
     const double D = g.det[n];
-    const double ke = xdiv::scale2<-1>(rho) * (u * u + v * v + w * w);   // 0.5 rho on the integer pipe, same bits
-    const double E = dv(p, 0.4) + ke;
-    double *Uq = lat_U(g, q);
-    g.Q[0 * N + n] = rho;
-    g.Q[1 * N + n] = rho * u;
-    g.Q[2 * N + n] = rho * v;
-    g.Q[3 * N + n] = rho * w;
-    g.Q[4 * N + n] = E;
-    Uq[0 * N + n] = D * rho;
-    Uq[1 * N + n] = D * rho * u;
-    Uq[2 * N + n] = D * rho * v;
-    Uq[3 * N + n] = D * rho * w;
-    Uq[4 * N + n] = D * E;
     double m[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) m[c] = g.m9[c * N + n];
     const double prim[5] = {rho, u, v, w, p};
-    double F[5], Ec[5], G[5];
-    node_flux(prim, m, D, F, Ec, G);
+    double F[5], Ec[5], G[5], Q[5], H;
+    node_flux(prim, m, D, F, Ec, G, Q, H);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
+        g.Q[c * N + n] = Q[c];
         g.FEG[(0 * 5 + c) * N + n] = F[c];
         g.FEG[(1 * 5 + c) * N + n] = Ec[c];
         g.FEG[(2 * 5 + c) * N + n] = G[c];
     }
-    g.sh[n] = sqrt(rho);
-    g.sh[N + n] = enthalpy(rho, u, v, w, p);
+    double *Uq = lat_U(g, q);
+    {
+        const double re[2] = {rho, Q[4]}, vel[3] = {u, v, w};
+        double d[2], du[3];
+        scaled(D, re, d);
+        scaled(d[0], vel, du);
+        Uq[0 * N + n] = d[0];
+        Uq[1 * N + n] = du[0];
+        Uq[2 * N + n] = du[1];
+        Uq[3 * N + n] = du[2];
+        Uq[4 * N + n] = d[1];
+    }
+    const double s = xi::root(rho), x[4] = {u, v, w, H};
+    double sx[4];
+    scaled(s, x, sx);
+    g.sh[n] = s;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) g.sh[(1 + c) * N + n] = sx[c];
 }
 
 __device__ __forceinline__ void prep_node(const LatView &g, int n, int q)
@@ -76,24 +80,21 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
     const double *Uj = lat_U(g, q);
     int i, j, k;
     lat_ijk(g, n, i, j, k);
-    double dU[3][5], KS[3], Ui[5];
+    double KS[3], Ui[5];
     const bool ghost = lat_ghost(g, n);
     // nodes outside the loc-code band take the central branch (the same
     // expression as the reference's central branch: the same bits)
     const unsigned lflag = g.locflag ? g.locflag[n] : 7u;
 #pragma unroll
     for (int c = 0; c < 5; ++c) Ui[c] = Uj[c * N + n];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int m2 = lat_step(g, i, j, k, d, -2), m1 = lat_step(g, i, j, k, d, -1), p1 = lat_step(g, i, j, k, d, 1),
-                  p2 = lat_step(g, i, j, k, d, 2);
+    auto dU = [&](int d, double (&out)[5]) {
         if (ghost) {
 #pragma unroll
-            for (int c = 0; c < 5; ++c) dU[d][c] = 0.0;
+            for (int c = 0; c < 5; ++c) out[c] = 0.0;
         } else if (!lat_locdir(g, d) || !((lflag >> d) & 1u)) {
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                dU[d][c] = central4(Uj[c * N + m2], Uj[c * N + m1], Uj[c * N + p1], Uj[c * N + p2]);
+            const int at[5] = {lat_step(g, i, j, k, d, -2), lat_step(g, i, j, k, d, -1), n, lat_step(g, i, j, k, d, 1),
+                               lat_step(g, i, j, k, d, 2)};
+            central4([&](int o, int c) { return Uj[c * N + at[o + 2]]; }, out);
         } else {
             int s[7], L[7];
             loc_line(g, i, j, k, d, s, L);
@@ -102,11 +103,14 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
                 double f[7];
 #pragma unroll
                 for (int o = 0; o < 7; ++o) f[o] = Uj[c * N + s[o]];
-                dU[d][c] = visc_deriv_ref(f, L);
+                out[c] = visc_deriv_ref(f, L);
             }
         }
-        const int c = d + 1;
-        KS[d] = ks(Ui[c], Ui[0], Uj[c * N + m1], Uj[m1], Uj[c * N + p1], Uj[p1]);
+    };
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int m1 = lat_step(g, i, j, k, d, -1), p1 = lat_step(g, i, j, k, d, 1), c = d + 1;
+        KS[d] = g.P.les && g.P.les != 2 ? ks_root(Ui[c], Ui[0], Uj[c * N + m1], Uj[m1], Uj[c * N + p1], Uj[p1]) : 0.0;
     }
     double m[9];
 #pragma unroll
@@ -114,8 +118,8 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
     const double prim[5] = {g.prim9[LF_RHO * N + n], g.prim9[LF_U * N + n], g.prim9[LF_V * N + n],
                             g.prim9[LF_W * N + n], g.prim9[LF_P * N + n]};
     double Fv[5], Ev[5], Gv[5], mu;
-    const Visc Vp{g.P.mach, g.P.reynolds, g.P.prandtl, g.P.t_inf, g.P.les, g.P.cs};
-    viscous_node(dU, Ui, m, g.det[n], prim, KS, Vp, Fv, Ev, Gv, mu);
+    const double D = g.det[n];
+    viscous_node(dU, Ui, m, D, g.del ? g.del[n] : filter_width(D), prim, KS, g.P, Fv, Ev, Gv, mu);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         g.V[(0 * 5 + c) * N + n] = Fv[c];
@@ -131,7 +135,7 @@ __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
     const int N = g.N;
     const double *Uj = lat_U(g, q);
     const double Ui[5] = {Uj[n], Uj[N + n], Uj[2 * N + n], Uj[3 * N + n], Uj[4 * N + n]};
-    g.prim9[LF_MU * N + n] = mu_of(Ui, g.P.mach, g.P.t_inf);
+    g.prim9[LF_MU * N + n] = mu_of(Ui, g.P);
 }
 
 // Face n+1/2 along D: Roe average of the two nodes, LLF face flux and the
@@ -155,8 +159,11 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     double r[5];
     {
         const int l = s[2], rr = s[3];   // node (left) and its +D neighbour
-        roe<SD>(g.sh[rr], g.prim9[LF_U * N + rr], g.prim9[LF_V * N + rr], g.prim9[LF_W * N + rr], g.sh[N + rr],
-                g.sh[l], g.prim9[LF_U * N + l], g.prim9[LF_V * N + l], g.prim9[LF_W * N + l], g.sh[N + l], r);
+        const double sb = g.sh[rr], si = g.sh[l];
+        r[4] = sb * si;
+        const Over<SD> den(sb + si);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) r[c] = den(g.sh[(1 + c) * N + rr] + g.sh[(1 + c) * N + l]);
     }
     double Fhat[5];
     face_flux<SD>(pts, g.fm[(D * 3 + 0) * N + n], g.fm[(D * 3 + 1) * N + n], g.fm[(D * 3 + 2) * N + n], g.fdet[D * N + n],
@@ -169,6 +176,127 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
         for (int o = 0; o < 6; ++o) f[o] = NF[c * N + s[o]];
         g.Fh[(D * 5 + c) * N + n] = corrected(Fhat[c], f);
     }
+}
+
+// Face n+1/2 along d in four kernels (physics_exact.cuh), over the faces of
+// a range of nodes: the Roe average and its scalars (base_node), one thread
+// per characteristic field and correction component (char_node), one per
+// component of the face states (back_node), two lanes per face for the LLF
+// flux (flux_node).  What they hand on stays in a scratch of kFaceScratch
+// doubles per face and direction.
+enum { FS_BASE = 0, FS_POS = FB_N, FS_NEG = FS_POS + 5, FS_CA = FS_NEG + 5, FS_CB = FS_CA + 5, FS_QP = FS_CB + 5,
+       FS_QN = FS_QP + 5, FS_N = FS_QN + 5 };
+
+// the scratch column of node n, direction d: element s at [s * ld]
+__device__ __forceinline__ double *face_column(const FaceScratch &fs, int n, int d)
+{
+    return fs.p + (size_t)d * FS_N * fs.ld + (n - fs.n0);
+}
+
+__device__ __forceinline__ bool face_at(const LatView &g, int n, int d, int &i, int &j, int &k)
+{
+    lat_ijk(g, n, i, j, k);
+    return lat_face_needed(g, i, j, k, d);
+}
+
+__device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &fs, int n, int d)
+{
+    const int N = g.N;
+    int i, j, k;
+    if (!face_at(g, n, d, i, j, k)) return;
+    const int rr = lat_step(g, i, j, k, d, 1);
+    // sqrt(rho) and its products with u, v, w, H: left and right node
+    const double sb = g.sh[rr], si = g.sh[n];
+    double r[5], x[4];
+    r[4] = sb * si;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) x[c] = g.sh[(1 + c) * N + rr] + g.sh[(1 + c) * N + n];
+    Over<true>(sb + si).all(x);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) r[c] = x[c];
+    const double kn[3] = {g.kn[(d * 3 + 0) * N + n], g.kn[(d * 3 + 1) * N + n], g.kn[(d * 3 + 2) * N + n]};
+    double B[FB_N], *col = face_column(fs, n, d);
+    face_base(r, kn, B);
+#pragma unroll
+    for (int s = 0; s < FB_N; ++s) col[(size_t)(FS_BASE + s) * fs.ld] = B[s];
+}
+
+__device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q)
+{
+    const int N = g.N;
+    int i, j, k;
+    if (!face_at(g, n, d, i, j, k)) return;
+    double *col = face_column(fs, n, d);
+    const double *kn = g.kn + (size_t)d * 3 * N + n;
+    const size_t ld = fs.ld;
+    double L[5];
+    left_row(q, [&](int s) { return col[(FS_BASE + s) * ld]; }, [&](int c) { return kn[(size_t)c * N]; }, L);
+    double pos, neg;
+    int s[6];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, d, o - 2);
+    char_pair(L, [&](int o, int c) { return g.Q[c * N + s[o]]; }, g.P.eps, pos, neg);
+    col[(FS_POS + q) * ld] = pos;
+    col[(FS_NEG + q) * ld] = neg;
+}
+
+__device__ __forceinline__ void back_node(const LatView &g, const FaceScratch &fs, int n, int d, int q)
+{
+    const int N = g.N;
+    int i, j, k;
+    if (!face_at(g, n, d, i, j, k)) return;
+    double *col = face_column(fs, n, d);
+    const double *kn = g.kn + (size_t)d * 3 * N + n;
+    const size_t ld = fs.ld;
+    double qp, qn;
+    back_pair(q, [&](int s) { return col[(FS_BASE + s) * ld]; }, [&](int c) { return kn[(size_t)c * N]; },
+              [&](int s) { return col[(FS_POS + s) * ld]; }, [&](int s) { return col[(FS_NEG + s) * ld]; }, qp, qn);
+    col[(FS_QP + q) * ld] = qp;
+    col[(FS_QN + q) * ld] = qn;
+    const double *NF = g.FEG + (size_t)(d * 5 + q) * N;
+    double f[6], ca, cb;
+#pragma unroll
+    for (int o = 0; o < 6; ++o) f[o] = NF[lat_step(g, i, j, k, d, o - 2)];
+    correction_terms(f, ca, cb);
+    col[(FS_CA + q) * ld] = ca;
+    col[(FS_CB + q) * ld] = cb;
+}
+
+// lanes 2m and 2m + 1 of a warp: the pos and neg side of one face; lanes
+// without a face take part with a face they do not store
+__device__ __forceinline__ void flux_node(const LatView &g, const FaceScratch &fs, int n, int d, bool active)
+{
+    const int N = g.N;
+    int i, j, k;
+    const bool face = active && face_at(g, n, d, i, j, k);
+    const int side = threadIdx.x & 1;
+    const double *col = face_column(fs, n, d);
+    const size_t ld = fs.ld;
+    double q[5] = {1.0, 0.0, 0.0, 0.0, 2.5}, m[3] = {1.0, 0.0, 0.0}, det = 1.0, Fhat[5];
+    if (face) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c) q[c] = col[(FS_QP + 5 * side + c) * ld];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[c] = g.fm[(d * 3 + c) * N + n];
+        det = g.fdet[d * N + n];
+    }
+    llf_lanes(q, m[0], m[1], m[2], det, Fhat);
+    if (!face) return;
+#pragma unroll
+    for (int c = 0; c < 5; ++c)   // components 0..2 on the even lane, 3..4 on the odd one
+        if ((c >= 3) == (side != 0)) g.Fh[(d * 5 + c) * N + n] = Fhat[c] - col[(FS_CA + c) * ld] + col[(FS_CB + c) * ld];
+}
+
+// What the face and viscous kernels take from the geometry alone, once per
+// solver: the unit normals of the faces along d and the filter width.
+__device__ __forceinline__ void geometry_node(const LatView &g, double *kn, double *del, int n, int d)
+{
+    const int N = g.N;
+    if (d == 0) del[n] = filter_width(g.det[n]);
+    double k[3];
+    face_normal(g.fm[(d * 3 + 0) * N + n], g.fm[(d * 3 + 1) * N + n], g.fm[(d * 3 + 2) * N + n], k);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) kn[(size_t)(d * 3 + c) * N + n] = k[c];
 }
 
 // Weno.cl:3060-3135 at one owned node (ghosts are the boundary routine's):
@@ -209,8 +337,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst, bo
         } else if (g.P.viscous) {
             const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
             const double *Vd = g.V + (size_t)d * 5 * N;
-#pragma unroll
-            for (int c = 0; c < 5; ++c) dvis[d][c] = central4(Vd[c * N + m2], Vd[c * N + m1], Vd[c * N + p1], Vd[c * N + p2]);
+            const int at[5] = {m2, m1, n, p1, p2};
+            central4([&](int o, int c) { return Vd[c * N + at[o + 2]]; }, dvis[d]);
         } else {
 #pragma unroll
             for (int c = 0; c < 5; ++c) dvis[d][c] = 0.0;

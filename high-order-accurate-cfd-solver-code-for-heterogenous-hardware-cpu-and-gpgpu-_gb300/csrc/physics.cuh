@@ -162,6 +162,9 @@ struct Phys {
     double mach, reynolds, prandtl, t_inf, eps;
     int viscous, les;   // les: 0 none, 1 mixed time scale, 2 Smagorinsky
     double cs;          // Smagorinsky C_s
+    // constants of the viscous terms, in the reference's own operations
+    // (make_phys): 1.4 M^2 0.4, 110.4 / T_inf, 1 + that, Pr Re, 1 / (0.56 M^2)
+    double c_temp, st, st1, pr_re, ck;
 };
 
 // Viscous and SGS fluxes at one node from the derivatives of U along the

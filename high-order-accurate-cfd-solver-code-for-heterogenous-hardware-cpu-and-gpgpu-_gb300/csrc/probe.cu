@@ -72,7 +72,8 @@ __device__ __forceinline__ bool same32(float x, float y)
 // mismatches of f2d, d2f (and the hi/lo split), add/sub, mul and the
 // division from a shared reciprocal (xdiv::quotient_int_v, both ways of
 // forming its first quotient, where it accepts the operands; xdiv::div) and
-// the reciprocal (rcp_int and rcp_int_i, rcp, divide)
+// the reciprocal (rcp_int and rcp_int_i, rcp, divide), with the grouped
+// quotients and square roots of exact_int.cuh
 __global__ void k_emu_check(int cls, uint64_t seed, int per, unsigned long long *bad)
 {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,6 +94,16 @@ __global__ void k_emu_check(int cls, uint64_t seed, int per, unsigned long long 
         }
         nb[2] += !same64(emu::add(a, b), __dadd_rn(a, b)) + !same64(emu::sub(a, b), __dsub_rn(a, b));
         nb[3] += !same64(emu::mul(a, b), __dmul_rn(a, b));
+        {   // groups: products, quotients and roots that share one test (exact_int.cuh)
+            const xi::Fac u[3] = {xi::fac(a), xi::fac(b), xi::fac(a)}, v[3] = {xi::fac(b), xi::fac(b), xi::fac(a)};
+            double p[3], q[2] = {a, 1.0}, r[2] = {fabs(a), b};
+            xi::mul_n(u, v, p);
+            nb[3] += !same64(p[0], __dmul_rn(a, b)) + !same64(p[1], __dmul_rn(b, b)) + !same64(p[2], __dmul_rn(a, a));
+            xi::quot_n(q, xi::divisor(b));
+            nb[4] += !same64(q[0], a / b) + !same64(q[1], 1.0 / b) + !same64(xi::divide(b, a), b / a);
+            xi::sqrt_n(r);
+            nb[4] += !same64(r[0], __dsqrt_rn(fabs(a))) + !same64(r[1], __dsqrt_rn(b));
+        }
         {
             const double y = 1.0 / b;
             bool ok;

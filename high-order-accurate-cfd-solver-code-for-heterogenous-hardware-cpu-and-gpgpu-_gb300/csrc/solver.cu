@@ -57,7 +57,6 @@ struct cfd_solver {
     cfd::LatticeMap map;        // lattice path: rows <-> nodes
     cfd::BcDevice bc;           // boundary routine after every stage
     bool has_bc = false;
-    int fp64_tune = -1;         // FP64 lattice: stages before the face passes' budgets are timed (-1: none)
 };
 
 namespace {
@@ -113,7 +112,6 @@ cfd_status_t create_gather(cfd_solver *s, const cfd_geometry_t *g)
 }
 
 cfd_status_t tune_face_tiles(cfd_solver *s);
-cfd_status_t tune_fp64_faces(cfd_solver *s, int j);
 
 cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
 {
@@ -154,9 +152,12 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
             return st;
         cudaMemsetAsync(S.V32, 0, 15 * N * sizeof(float), S.stream);
     } else {          // FP64 stage intermediates
+        const size_t fs_ld = N < kFaceRound ? N : kFaceRound;
         if ((st = dalloc_t(s, 5 * N, &S.Q)) || (st = dalloc_t(s, 15 * N, &S.FEG)) || (st = dalloc_t(s, 15 * N, &S.V))
-            || (st = dalloc_t(s, 2 * N, &S.sh)) || (st = dalloc_t(s, 15 * N, &S.Fh)))
+            || (st = dalloc_t(s, 5 * N, &S.sh)) || (st = dalloc_t(s, 15 * N, &S.Fh))
+            || (st = dalloc_t(s, 9 * N, &S.kn)) || (st = dalloc_t(s, N, &S.del)) || (st = dalloc_t(s, 3 * (size_t)kFaceScratch * fs_ld, &S.fs)))
             return st;
+        S.fs_ld = (int)fs_ld;
         cudaMemsetAsync(S.V, 0, 15 * N * sizeof(double), S.stream);
     }
     for (int q = 0; q < 3; ++q) cudaMemsetAsync(S.U[q], 0, 5 * N * sizeof(double), S.stream);
@@ -213,6 +214,10 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
             S.locflag = locflag;
         }
     }
+    if (!s->mixed) {
+        fp64_geometry(S);
+        s->ctx->launches += 1;
+    }
     if (s->mixed) {
         if (s->form == CFD_PREC_SPLIT) {
             split_geometry(S);
@@ -233,7 +238,6 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
     cudaError_t e = cudaStreamSynchronize(S.stream);   // host vectors go out of scope
     if (e != cudaSuccess) return cuda_fail(s->ctx, e, "solver create sync");
     if (s->mixed) return tune_face_tiles(s);
-    s->fp64_tune = 1;   // on the second stage's real inputs (tune_fp64_faces)
     return CFD_OK;
 }
 
@@ -303,72 +307,6 @@ cfd_status_t tune_face_tiles(cfd_solver *s)
     return CFD_OK;
 }
 
-// Register budgets of the FP64 face passes (2, 3 or 4 blocks of 128 per
-// SM, per direction), timed once per lattice shape in this process, at the
-// solver's second stage: that stage's prep runs first (it runs again in the
-// stage itself, writing the same values), then each budget's face pass on
-// the real inputs (their output, the face fluxes, is rewritten by the
-// stage).  A uniform state does not do: the exact divisions take data-
-// dependent paths, and budgets timed on one mispredicted the NACA0012 and
-// shocked-slab lattices by 10 %.  Nor does the first stage of an impulsive
-// start, whose state is still exactly uniform (zeros and ones everywhere)
-// where every later stage carries rounding-level differences.  The best
-// budget depends on the shape; every budget gives the same bits.
-std::mutex g_fp64_face_mutex;
-std::map<std::array<int, 6>, std::array<int, 3>> g_fp64_face_cache;
-
-std::array<int, 6> fp64_face_key(const cfd_solver *s)
-{
-    const StructuredLaunch &S = s->S;
-    return {S.ni, S.nj, S.nk, S.per, S.loc8 ? 1 : 0, s->ctx->device};
-}
-
-cfd_status_t tune_fp64_faces(cfd_solver *s, int j)
-{
-    s->fp64_tune = -1;
-    StructuredLaunch &S = s->S;
-    const std::array<int, 6> key = fp64_face_key(s);
-    {
-        std::lock_guard<std::mutex> lock(g_fp64_face_mutex);
-        auto it = g_fp64_face_cache.find(key);
-        if (it != g_fp64_face_cache.end()) {
-            for (int d = 0; d < 3; ++d) S.face_mb[d] = it->second[d];
-            return CFD_OK;
-        }
-    }
-    cudaStream_t st = s->ctx->stream;
-    fp64_prep_pass(S, j);
-    s->ctx->launches += 1;
-    cudaEvent_t t0 = nullptr, t1 = nullptr;
-    if (cudaEventCreate(&t0) != cudaSuccess || cudaEventCreate(&t1) != cudaSuccess) {
-        const cudaError_t ce = cudaGetLastError();
-        if (t0) cudaEventDestroy(t0);
-        return cuda_fail(s->ctx, ce, "FP64 face tuner events");
-    }
-    std::array<int, 3> pick = {S.face_mb[0], S.face_mb[1], S.face_mb[2]};
-    for (int d = 0; d < 3; ++d) {
-        float best = 1e30f;
-        for (int mb : {2, 3, 4}) {
-            fp64_face_pass(S, d, mb, st);   // warm-up
-            cudaEventRecord(t0, st);
-            for (int r = 0; r < 2; ++r) fp64_face_pass(S, d, mb, st);
-            cudaEventRecord(t1, st);
-            float ms = 1e30f;
-            if (cudaEventSynchronize(t1) == cudaSuccess) cudaEventElapsedTime(&ms, t0, t1);
-            s->ctx->launches += 3;
-            if (ms < best) best = ms, pick[d] = mb;
-        }
-    }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(s->ctx, e, "FP64 face tuner");
-    for (int d = 0; d < 3; ++d) S.face_mb[d] = pick[d];
-    std::lock_guard<std::mutex> lock(g_fp64_face_mutex);
-    g_fp64_face_cache[key] = pick;
-    return CFD_OK;
-}
-
 // where stage j's U_Q comes from (mixed form; the FP64 form always preps)
 int prep_source(const cfd_solver *s, int j)
 {
@@ -382,12 +320,6 @@ cfd_status_t run_stage(cfd_solver *s, int j, double dt, bool want_L)
     cfd_ctx *ctx = s->ctx;
     s->S.stream = ctx->stream;   // the context's stream may have been replaced
     if (s->path == CFD_PATH_STRUCTURED) {
-        if (s->fp64_tune == 0) {
-            const cfd_status_t st = tune_fp64_faces(s, j);
-            if (st != CFD_OK) return st;
-        } else if (s->fp64_tune > 0) {
-            --s->fp64_tune;
-        }
         ctx->launches += structured_stage(s->S, j, dt, want_L ? s->Lsoa : nullptr, nullptr, nullptr, prep_source(s, j));
         if (s->mixed) s->cur_slot = s->prep_ready = j == 2 ? 0 : j + 1;
         if (s->has_bc) {
@@ -582,7 +514,6 @@ cfd_status_t cfd_solver_set_face_blocks(cfd_solver_t *s, int32_t blocks_i, int32
     cudaStreamSynchronize(s->ctx->stream);
     for (int d = 0; d < 3; ++d)
         if (b[d]) s->S.face_mb[d] = b[d];
-    s->fp64_tune = -1;   // the caller's choice stands
     return CFD_OK;
 }
 
@@ -692,10 +623,6 @@ cfd_status_t cfd_solver_profile_stage(cfd_solver_t *s, int32_t j, double del_t, 
     for (auto &e : ev) cudaEventCreate(&e);
     const char *snames[kMaxStageLaunches + 1] = {};
     int nk = 3;
-    if (s->path == CFD_PATH_STRUCTURED && s->fp64_tune >= 0 && (st = tune_fp64_faces(s, j)) != CFD_OK) {
-        for (auto &e : ev) cudaEventDestroy(e);
-        return st;
-    }
     if (s->path == CFD_PATH_STRUCTURED) {
         nk = structured_stage(s->S, j, del_t, nullptr, ev.data(), snames, prep_source(s, j));
         if (s->mixed) s->cur_slot = s->prep_ready = j == 2 ? 0 : j + 1;

@@ -33,7 +33,7 @@ namespace {
 //   geometry SoA 22 (9 node metrics, det, 3x3 face metrics, 3 face dets),
 //   FLOW 9, U0/U1/U2 15, Q 5, node fluxes 15, viscous fluxes 15,
 //   sqrt(rho) and H 2, face fluxes 15, L 5
-constexpr size_t kPerNode = 22 + 9 + 15 + 5 + 15 + 15 + 2 + 15 + 5;   // 103
+constexpr size_t kPerNode = 22 + 9 + 15 + 5 + 15 + 15 + 5 + 9 + 1 + 3 * kFaceScratch + 15 + 5;   // 242
 constexpr size_t kFlagDoubles = 32;                                    // 256 B for the error word
 constexpr size_t kScratchDoubles = (size_t)CFD_STATIC_MAX_NODES * kPerNode + kFlagDoubles;
 
@@ -141,7 +141,11 @@ extern "C" cfd_status_t cfd_lattice_stage_static(void *cuda_stream, int32_t ni, 
     S.Q = take(5);
     S.FEG = take(15);
     S.V = take(15);
-    S.sh = take(2);
+    S.sh = take(5);
+    S.kn = take(9);
+    S.del = take(1);
+    S.fs = take(3 * kFaceScratch);
+    S.fs_ld = (int)N;
     S.Fh = take(15);
     double *Lsoa = take(5);
     S.flags = (unsigned *)(base + (size_t)CFD_STATIC_MAX_NODES * kPerNode);
@@ -163,6 +167,7 @@ extern "C" cfd_status_t cfd_lattice_stage_static(void *cuda_stream, int32_t ni, 
     to_soa(st, (const double *)U1, 5, 0, 5, N, S.U[1]);
     to_soa(st, (const double *)U2, 5, 0, 5, N, S.U[2]);
 
+    fp64_geometry(S);
     structured_stage(S, j, del_t, L_out ? Lsoa : nullptr);
 
     // results back into the caller's buffers: FLOW, U_j (U_Q's output),

@@ -13,9 +13,9 @@
 //   k_prep    pointwise: Q, U_j = det*Q (U_Q.cl), contravariant node fluxes
 //             F,E,G (Viscous.cl:560-631), sqrt(rho) and H for the Roe average
 //   k_visc    radius-2 star: viscous + MTS SGS fluxes Fv,Ev,Gv and mu
-//   k_face<d, mb> one thread per face i+1/2 along d (face_fp64.cuh, at the
-//     register budget the solver's tuner picked): Roe eigenvectors, WENO5,
-//             LLF, 6th-order correction -> corrected face flux
+//   k_face_*  the faces i+1/2 along each direction (faces_fp64.cu): Roe
+//             eigenvectors, WENO5, LLF, 6th-order correction -> corrected
+//             face flux
 //   k_update  pointwise + radius-2: L = -(flux differences + viscous
 //             divergence), SSP-RK3 stage j, primitive recovery
 // Layout: every field is [component][N] with n = i + ni*(j + nj*k).
@@ -34,13 +34,18 @@ namespace {
 
 __device__ __forceinline__ int node_id() { return blockIdx.x * blockDim.x + threadIdx.x; }
 
-__global__ void __launch_bounds__(128) k_prep(LatView g, int q)
+// Blocks of 128 per SM (registers 80, 128, 72): the integer chains of the
+// products want warps, the spills cost less.  TGV 128^3: prep 0.31 ms at 4
+// to 6 blocks, 0.34 at 8; viscous 1.54 ms at 4, 1.87 at 3, 2.10 at 5;
+// update 0.58, 0.54, 0.53, 0.52 ms at 5, 6, 7, 8.  With the products on the
+// FP64 pipe they took 0.59, 1.89 and 0.66 ms.
+__global__ void __launch_bounds__(128, 6) k_prep(LatView g, int q)
 {
     const int n = node_id();
     if (n < g.N) ex::prep_node(g, n, q);
 }
 
-__global__ void __launch_bounds__(128) k_visc(LatView g, int q)
+__global__ void __launch_bounds__(128, 4) k_visc(LatView g, int q)
 {
     const int n = node_id();
     if (n < g.N) ex::visc_node(g, n, q);
@@ -53,7 +58,7 @@ __global__ void __launch_bounds__(128) k_mu_only(LatView g, int q)
 }
 
 
-__global__ void __launch_bounds__(128) k_update(LatView g, int jst)
+__global__ void __launch_bounds__(128, 7) k_update(LatView g, int jst)
 {
     const int n = node_id();
     if (n < g.N) ex::update_node(g, n, jst, false);
@@ -92,52 +97,24 @@ int structured_stage(const StructuredLaunch &S, int jst, double dt, double *Lout
     const LatView g = make_view(S, dt, Lout);
     const unsigned nb = blocks_for(g.N, 128);
     cudaStream_t st = S.stream;
-    int e = 0;
-    auto mark = [&]() {
-        if (ev) cudaEventRecord(ev[e++], st);
+    int e = 0, k = 0, entries = 0;
+    auto mark = [&](const char *name) {
+        if (names) names[entries] = name;
+        ++entries;
+        if (ev) cudaEventRecord(ev[++e], st);
     };
-    static const char *fp64_names[6] = {"prep", "viscous", "face_i", "face_j", "face_k", "update"};
-    if (names)
-        for (int i = 0; i < 6; ++i) names[i] = fp64_names[i];
-    if (names && !S.P.viscous) names[1] = "mu_only";
-    mark();
+    if (ev) cudaEventRecord(ev[0], st);
     k_prep<<<nb, 128, 0, st>>>(g, jst);
-    mark();
+    mark("prep");
     if (S.P.viscous)
         k_visc<<<nb, 128, 0, st>>>(g, jst);
     else
         k_mu_only<<<nb, 128, 0, st>>>(g, jst);
-    mark();
-    fp64_face_pass(g, 0, S.face_mb[0], st);
-    mark();
-    fp64_face_pass(g, 1, S.face_mb[1], st);
-    mark();
-    fp64_face_pass(g, 2, S.face_mb[2], st);
-    mark();
+    mark(S.P.viscous ? "viscous" : "mu_only");
+    k = 3 + fp64_faces(S, g, st, mark);
     k_update<<<nb, 128, 0, st>>>(g, jst);
-    mark();
-    return 6;
-}
-
-void fp64_face_pass(const LatView &g, int d, int mb, cudaStream_t st)
-{
-    if (mb == 2)
-        fp64_face_pass_mb2(g, d, st);
-    else if (mb == 4)
-        fp64_face_pass_mb4(g, d, st);
-    else
-        fp64_face_pass_mb3(g, d, st);
-}
-
-void fp64_face_pass(const StructuredLaunch &S, int d, int mb, cudaStream_t st)
-{
-    fp64_face_pass(make_view(S, 0.0, nullptr), d, mb, st);
-}
-
-void fp64_prep_pass(const StructuredLaunch &S, int jst)
-{
-    const LatView g = make_view(S, 0.0, nullptr);
-    k_prep<<<blocks_for(g.N, 128), 128, 0, S.stream>>>(g, jst);
+    mark("update");
+    return ev ? entries : k;
 }
 
 void aos_to_soa(cudaStream_t st, const double *aos, int stride, int ncomp, long long N, double *soa, const int *row_of)

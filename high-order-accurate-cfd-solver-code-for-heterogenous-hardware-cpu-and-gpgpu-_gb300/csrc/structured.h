@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
+
 #include "lattice.cuh"
 #include "physics.cuh"
 
@@ -23,7 +25,11 @@ struct StructuredLaunch {
     double *Q;                 // [5][N]
     double *FEG;               // [3][5][N] contravariant node fluxes
     double *V;                 // [3][5][N] viscous fluxes
-    double *sh;                // [2][N]   sqrt(rho), H
+    double *sh;                // [5][N]   sqrt(rho) and its products with u, v, w, H
+    double *kn;                // [9][N]   unit normals of the faces (fp64_geometry)
+    double *del;               // [N]      1 / det^(1/3) (fp64_geometry)
+    double *fs;                // [3][kFaceScratch][fs_ld] scratch of the face kernels (FaceScratch)
+    int fs_ld;                 // nodes whose faces one round of them takes
     double *Fh;                // [3][5][N] corrected face fluxes
     unsigned *flags;
     // mixed-precision form (FP32 stage intermediates, mixed.cu)
@@ -50,9 +56,9 @@ struct StructuredLaunch {
     // face-tile widths of the mixed and split face passes: faces along i
     // (32, 64 or 128) and along j and k (8, 16 or 32) per block of 128
     int tile_i = 64, tile_jk = 16;
-    // FP64 form: blocks of 128 per SM the face passes along i, j, k request
-    // (2, 3 or 4: their register budget; the solver's tuner picks)
-    int face_mb[3] = {3, 3, 2};
+    // FP64 form: register budget of the face pass's characteristic kernel
+    // along i, j, k (2, 3 or 4: 4, 6 or 8 blocks of 128 per SM)
+    int face_mb[3] = {4, 4, 4};
     int per = 7;
     const unsigned char *loc8 = nullptr;
     int locdirs = 0;
@@ -126,6 +132,8 @@ inline LatView make_view(const StructuredLaunch &S, double dt, double *Lout)
     g.FEG = S.FEG;
     g.V = S.V;
     g.sh = S.sh;
+    g.kn = S.kn;
+    g.del = S.del;
     g.Fh = S.Fh;
     g.Q32 = S.Q32;
     g.R32 = S.R32;
@@ -147,21 +155,25 @@ inline LatView make_view(const StructuredLaunch &S, double dt, double *Lout)
 // kMaxStageLaunches+1 entries) receives events bracketing every launch and
 // names (optional) the launch names.  prep_from as for mixed_stage (the FP64
 // form always runs its own prep from FLOW).
-constexpr int kMaxStageLaunches = 6;
+constexpr int kMaxStageLaunches = 7;
+// Nodes whose faces one round of the FP64 face kernels takes at most (2.1 GB
+// of scratch; more nodes run in rounds, each large enough to fill the part).
+constexpr size_t kFaceRound = 1u << 21;
 int structured_stage(const StructuredLaunch &S, int j, double dt, double *Lout, cudaEvent_t *ev = nullptr,
                      const char **names = nullptr, int prep_from = kPrepFromFlow);
+
+// FP64 form: the geometry's part of the face and viscous kernels (once,
+// after upload; one launch), and the face pass (faces_fp64.cu) in rounds of
+// S.fs_ld nodes; mark is called after each timed entry.  Returns the
+// launches.
+void fp64_geometry(const StructuredLaunch &S);
+void fp64_geometry(const LatView &g, double *kn, double *del, cudaStream_t st);
+int fp64_faces(const StructuredLaunch &S, const LatView &g, cudaStream_t st,
+               const std::function<void(const char *)> &mark);
 
 // One face pass along d with face tiles of width `tile` (the tuner's
 // candidates, mixed.cu / split.cu), and a uniform state in the FP32 face
 // inputs (Q32, R32, FEG32) for timing them before any state exists.
-// The FP64 face pass along d at `mb` blocks per SM (face_fp64_mb*.cu), and
-// stage jst's prep alone (the face passes' inputs, for the tuner).
-void fp64_face_pass_mb2(const LatView &g, int d, cudaStream_t st);
-void fp64_face_pass_mb3(const LatView &g, int d, cudaStream_t st);
-void fp64_face_pass_mb4(const LatView &g, int d, cudaStream_t st);
-void fp64_face_pass(const LatView &g, int d, int mb, cudaStream_t st);
-void fp64_face_pass(const StructuredLaunch &S, int d, int mb, cudaStream_t st);
-void fp64_prep_pass(const StructuredLaunch &S, int jst);
 void mixed_face_pass(const StructuredLaunch &S, int d, int tile, cudaStream_t st);
 void split_face_pass(const StructuredLaunch &S, int d, int tile, cudaStream_t st);
 void reduced_uniform_inputs(const StructuredLaunch &S, cudaStream_t st);
