@@ -15,20 +15,22 @@
 // Weno evaluates both faces of each direction at every row, so every
 // interior face is computed twice from identical inputs (as row n's +1/2
 // face and as row n+1's -1/2 face).  With a scratch buffer the launch is
-// split: k_weno_plus computes each row's +1/2 face once and, where its plus
-// neighbour p has this row as its minus neighbour and every input of p's
-// -1/2 face is bit-identical (then so are the stencil rows; face metric,
-// face det and Roe state are compared), also stores it as p's -1/2 face,
-// stamped with the call's generation; k_weno_minus computes the -1/2 faces
-// left unstamped (box edges, loc codes, inconsistent tables), and
-// k_weno<true> reads both faces from the scratch, which keeps the FP64 face
-// code and its registers out of it.  The results are the same bits either
-// way.
-// The drop-in's face kernel runs at 2 blocks of 128 per SM: too few warps
-// to hide the integer product's latency, so the divisions' first quotient
-// comes from the FP64 multiply (exact_div.cuh, CFD_XDIV_QPROD; the same bits
-// either way).
-#define CFD_XDIV_QPROD 0
+// split: the k_row_* kernels compute each row's +1/2 face once and, where
+// its plus neighbour p has this row as its minus neighbour and every input
+// of p's -1/2 face is bit-identical (then so are the stencil rows; face
+// metric, face det and Roe state are compared), also store it as p's -1/2
+// face, stamped with the call's generation; k_weno_minus computes the -1/2
+// faces left unstamped (box edges, loc codes, inconsistent tables), and
+// k_weno<true> reads both faces from the scratch.  The results are the same
+// bits either way.
+//
+// The k_row_* kernels are the lattice face pass (faces_fp64.cu: the FP64
+// pipe runs the sums, the integer pipe the products, quotients and roots,
+// so many small threads) on rows: one thread per face, characteristic
+// field, component and side, in rounds of kRowRound rows.  The first also
+// notes the six stencil rows, so that the neighbour chain (five loads that
+// wait for one another) is walked once per face instead of ten times.  TGV
+// 96^3: cfd_weno 8.9 -> 4.8 ms.
 #include <algorithm>
 
 #include "internal.h"
@@ -65,21 +67,49 @@ __device__ __forceinline__ bool gather_star(const int *grid, int gid, int n_rows
     return true;
 }
 
+// The seven rows of direction d of a star that gather_star has checked.
+__device__ __forceinline__ void star_line(const int *grid, int gid, int d, int s[7])
+{
+    s[3] = gid;
+#pragma unroll
+    for (int o = 1; o <= 3; ++o) {
+        s[3 + o] = grid_nb(grid, s[2 + o], plus_slot(d));
+        s[3 - o] = grid_nb(grid, s[4 - o], minus_slot(d));
+    }
+}
+
+// The derivative of branch b (physics.cuh) from seven rows of one component
+// (stride 5), out of line: rows next to ghosts take it, the others the
+// central form.
+static __device__ __noinline__ double row_deriv(const double *x, int i0, int i1, int i2, int i3, int i4, int i5, int i6,
+                                                int b)
+{
+    const double f[7] = {x[5 * (size_t)i0], x[5 * (size_t)i1], x[5 * (size_t)i2], x[5 * (size_t)i3],
+                         x[5 * (size_t)i4], x[5 * (size_t)i5], x[5 * (size_t)i6]};
+    return branch_deriv<double>(b, f);
+}
+
 // FLOW field offsets inside the 9-double row
 enum { FU = 0, FV = 1, FW = 2, FP = 3, FT = 4, FRHO = 5, FMU = 6, FA = 7, FE = 8 };
 
 // ------------------------------------------------------------------ U_Q --
-// sqrt(rho) and total enthalpy of every row (U_Q.cl:60-65), once per row:
-// sh[2*row], sh[2*row + 1].  k_uq<true> reads them for the row and its six
-// neighbours instead of evaluating them seven times.
+// sqrt(rho) of every row and its products with u, v, w and the total
+// enthalpy (U_Q.cl:60-65), once per row: sh[5*row ..].  k_uq<true> reads
+// them for the row and its six neighbours instead of evaluating them seven
+// times.
 __global__ void __launch_bounds__(128) k_uq_node(const double *__restrict__ flow, int n_rows, double *__restrict__ sh)
 {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n_rows) return;
     const double *f = flow + 9 * (size_t)row;
-    const double rho = f[FRHO];
-    sh[2 * (size_t)row] = sqrt(rho);
-    sh[2 * (size_t)row + 1] = ex::enthalpy(rho, f[FU], f[FV], f[FW], f[FP]);
+    const double rho = f[FRHO], u = f[FU], v = f[FV], w = f[FW];
+    const double s = xi::root(rho), x[4] = {u, v, w, ex::enthalpy(rho, u, v, w, f[FP])};
+    double sx[4];
+    ex::scaled(s, x, sx);
+    double *o = sh + 5 * (size_t)row;
+    o[0] = s;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[1 + c] = sx[c];
 }
 
 // U_Q.cl:36-125.
@@ -102,8 +132,8 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
     }
     const double *fi = flow + 9 * (size_t)gid;
     const double rho = fi[FRHO], u = fi[FU], v = fi[FV], w = fi[FW], p = fi[FP];
-    const double si = SH ? sh[2 * (size_t)gid] : sqrt(rho);
-    const double hi = SH ? sh[2 * (size_t)gid + 1] : ex::enthalpy(rho, u, v, w, p);
+    const double si = SH ? sh[5 * (size_t)gid] : sqrt(rho);
+    const double hi = SH ? 0.0 : ex::enthalpy(rho, u, v, w, p);
     // ROE block order ip, jp, kp, im, jm, km: block d is the +d face
     // (neighbour slot plus_slot(d)), block d + 3 the -d face (minus_slot(d)).
     //
@@ -122,12 +152,20 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
         const bool plus = b < 3;
         const int nr = nb[plus ? plus_slot(d) : minus_slot(d)];
         if (SH && !plus && nr < n_items && grid_nb(grid, nr, plus_slot(d)) == gid) continue;
-        const double *fn = flow + 9 * (size_t)nr;
-        const double rb = fn[FRHO], ub = fn[FU], vb = fn[FV], wb = fn[FW], pb = fn[FP];
-        const double sb = SH ? sh[2 * (size_t)nr] : sqrt(rb);
-        const double hb = SH ? sh[2 * (size_t)nr + 1] : ex::enthalpy(rb, ub, vb, wb, pb);
         double ra[5];
-        ex::roe(sb, ub, vb, wb, hb, si, u, v, w, hi, ra);
+        if (SH) {   // the same sums of products over the same sum
+            const double *sn = sh + 5 * (size_t)nr, *sg = sh + 5 * (size_t)gid;
+            const double sb = sn[0];
+            double x[4] = {sn[1] + sg[1], sn[2] + sg[2], sn[3] + sg[3], sn[4] + sg[4]};
+            ex::Over<true>(sb + si).all(x);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ra[c] = x[c];
+            ra[4] = xi::mul(sb, si);
+        } else {
+            const double *fn = flow + 9 * (size_t)nr;
+            const double rb = fn[FRHO], ub = fn[FU], vb = fn[FV], wb = fn[FW];
+            ex::roe(sqrt(rb), ub, vb, wb, ex::enthalpy(rb, ub, vb, wb, fn[FP]), si, u, v, w, hi, ra);
+        }
         r[6 * b + 0] = ra[0];
         r[6 * b + 1] = ra[1];
         r[6 * b + 2] = ra[2];
@@ -143,36 +181,77 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
         }
     }
     const double D = det[gid];
-    const double ke = xdiv::scale2<-1>(rho) * (u * u + v * v + w * w);   // 0.5 rho, same bits
+    double s[3] = {u, v, w}, q[3], du[3], d2[2];
+    const double vel[3] = {u, v, w};
+    xi::sq_n(s);
+    const double E = ex::dv(p, 0.4) + xi::mul(xdiv::scale2<-1>(rho), s[0] + s[1] + s[2]);   // 0.5 rho: same bits
+    const double re[2] = {rho, E};
+    ex::scaled(rho, vel, q);
+    ex::scaled(D, re, d2);
+    ex::scaled(d2[0], vel, du);
     double *Ur = U + 5 * (size_t)gid, *Qr = Q + 5 * (size_t)gid;
-    Ur[0] = D * rho;
-    Ur[1] = D * rho * u;
-    Ur[2] = D * rho * v;
-    Ur[3] = D * rho * w;
-    const double E = ex::dv(p, 0.4) + ke;
-    Ur[4] = D * E;
+    Ur[0] = d2[0];
+    Ur[1] = du[0];
+    Ur[2] = du[1];
+    Ur[3] = du[2];
+    Ur[4] = d2[1];
     Qr[0] = rho;
-    Qr[1] = rho * u;
-    Qr[2] = rho * v;
-    Qr[3] = rho * w;
+    Qr[1] = q[0];
+    Qr[2] = q[1];
+    Qr[3] = q[2];
     Qr[4] = E;
 }
 
 // -------------------------------------------------------------- Viscous --
 // Viscous.cl:23-643.
-__global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
+// The inviscid node fluxes and the filter width of every row (their own
+// kernel: beside the viscous fluxes they would spill).
+__global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, double *__restrict__ E,
+                                                      double *__restrict__ G, const double *__restrict__ metric,
+                                                      const double *__restrict__ det, const double *__restrict__ flow,
+                                                      int n_items, int les, double *__restrict__ width)
+{
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= n_items) return;
+    const double D = det[gid];
+    double m[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[k] = metric[63 * (size_t)gid + k];
+    const double *fr = flow + 9 * (size_t)gid;
+    const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
+    double Fn[5], En[5], Gn[5], Qn[5], H;
+    ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+        F[5 * (size_t)gid + c] = Fn[c];
+        E[5 * (size_t)gid + c] = En[c];
+        G[5 * (size_t)gid + c] = Gn[c];
+    }
+    if (les) width[gid] = ex::filter_width(D);
+}
+
+// NODE = false: the inviscid node fluxes and the filter width come from
+// k_node_flux (width: one double per row); true: all in one kernel, for
+// callers without the scratch.  TGV 96^3, both kernels: 1.00 ms at 3 or 4
+// blocks per SM, 1.19 at 5; in one kernel 1.17 at 3, 1.38 at 4 (3 KB of spill
+// loads per thread).
+template <bool NODE>
+__global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
                                                  double *__restrict__ E, double *__restrict__ G,
                                                  double *__restrict__ Fv, double *__restrict__ Ev,
                                                  double *__restrict__ Gv, const int *__restrict__ grid,
                                                  const double *__restrict__ metric, const double *__restrict__ det,
-                                                 double *__restrict__ flow, int n_items, int n_rows, unsigned *flags)
+                                                 double *__restrict__ flow, int n_items, int n_rows, unsigned *flags,
+                                                 const double *__restrict__ width)
 {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= n_items) return;
-    int idx[3][7];
-    if (!gather_star(grid, gid, n_rows, idx)) {
-        atomicOr(flags, CFD_FLAG_BAD_INDEX);
-        return;
+    {
+        int idx[3][7];
+        if (!gather_star(grid, gid, n_rows, idx)) {
+            atomicOr(flags, CFD_FLAG_BAD_INDEX);
+            return;
+        }
     }
     double m[9];
 #pragma unroll
@@ -180,22 +259,33 @@ __global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restric
     const double D = det[gid];
     const double *fr = flow + 9 * (size_t)gid;
     const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
-    double Fn[5], En[5], Gn[5], Qn[5], H;
-    ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
+    if (NODE) {
+        double Fn[5], En[5], Gn[5], Qn[5], H;
+        ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            F[5 * (size_t)gid + c] = Fn[c];
+            E[5 * (size_t)gid + c] = En[c];
+            G[5 * (size_t)gid + c] = Gn[c];
+        }
+    }
     double Fvn[5], Evn[5], Gvn[5];
     double mu;
     {
+        // the star is walked again for each direction (it is cached by now):
+        // its 18 rows would not fit the registers beside the fluxes
         auto dU = [&](int d, double (&out)[5]) {
-            int L[7];
+            int s[7], L[7];
+            star_line(grid, gid, d, s);
 #pragma unroll
-            for (int o = 0; o < 7; ++o) L[o] = grid_loc(grid, idx[d][o]);
-#pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                double f[7];
-#pragma unroll
-                for (int o = 0; o < 7; ++o) f[o] = U[5 * (size_t)idx[d][o] + c];
-                out[c] = visc_deriv_ref(f, L);
+            for (int o = 0; o < 7; ++o) L[o] = grid_loc(grid, s[o]);
+            const int b = visc_branch(L);
+            if (b == 5) {
+                ex::central4([&](int o, int c) { return U[5 * (size_t)s[o + 3] + c]; }, out);
+                return;
             }
+#pragma unroll
+            for (int c = 0; c < 5; ++c) out[c] = row_deriv(U + c, s[0], s[1], s[2], s[3], s[4], s[5], s[6], b);
         };
         double Ui[5];
 #pragma unroll
@@ -204,17 +294,15 @@ __global__ void __launch_bounds__(128) k_viscous(Phys P, const double *__restric
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int c = d + 1;
-            const double *um = U + 5 * (size_t)idx[d][2], *up = U + 5 * (size_t)idx[d][4];
-            KS[d] = ex::ks_root(Ui[c], Ui[0], um[c], um[0], up[c], up[0]);
+            const double *um = U + 5 * (size_t)grid_nb(grid, gid, minus_slot(d)),
+                         *up = U + 5 * (size_t)grid_nb(grid, gid, plus_slot(d));
+            KS[d] = P.les && P.les != 2 ? ex::ks_root(Ui[c], Ui[0], um[c], um[0], up[c], up[0]) : 0.0;
         }
-        ex::viscous_node(dU, Ui, m, D, ex::filter_width(D), prim, KS, P, Fvn, Evn, Gvn, mu);
+        ex::viscous_node(dU, Ui, m, D, NODE ? ex::filter_width(D) : width[gid], prim, KS, P, Fvn, Evn, Gvn, mu);
     }
     double *o;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        o = F + 5 * (size_t)gid; o[c] = Fn[c];
-        o = E + 5 * (size_t)gid; o[c] = En[c];
-        o = G + 5 * (size_t)gid; o[c] = Gn[c];
         o = Fv + 5 * (size_t)gid; o[c] = P.viscous ? Fvn[c] : 0.0;
         o = Ev + 5 * (size_t)gid; o[c] = P.viscous ? Evn[c] : 0.0;
         o = Gv + 5 * (size_t)gid; o[c] = P.viscous ? Gvn[c] : 0.0;
@@ -273,46 +361,148 @@ __device__ __forceinline__ bool plus_line(const int *grid, int n, int n_rows, in
 
 __device__ __forceinline__ bool same_bits(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
 
-// +1/2 face of every row gid < n_items along d = blockIdx.y whose stencil
-// stays in the table: Fp[(d*5 + c)*ld + gid]; also p's -1/2 face
-// Fm[(d*5 + c)*ld + p] with stamp[d*ld + p] = gen for the plus neighbour p
-// whose minus neighbour is gid, when p's face data are gid's bit for bit.
-// blocks per SM the +1/2-face kernel's register budget allows: 2 (GB300,
-// TGV 128^3: drop-in 2.89e7 cell-updates/s against 2.85e7 at 3)
-#ifndef CFD_WENO_PLUS_MIN_BLOCKS
-#define CFD_WENO_PLUS_MIN_BLOCKS 2
-#endif
-__global__ void __launch_bounds__(128, CFD_WENO_PLUS_MIN_BLOCKS) k_weno_plus(Phys P, const double *__restrict__ deter,
-                                                       const int *__restrict__ grid, const double *__restrict__ Q,
-                                                       const double *__restrict__ metric,
-                                                       const double *__restrict__ roe, const double *__restrict__ F,
-                                                       const double *__restrict__ E, const double *__restrict__ G,
-                                                       int n_items, int n_rows, double *__restrict__ Fp,
-                                                       double *__restrict__ Fm, unsigned *__restrict__ stamp,
-                                                       unsigned gen, long long ld)
+// Scratch of one face of the k_row_* kernels, element s of column (row -
+// first row, direction) at [s * ld]: the Roe scalars, the unit normal, the
+// characteristic values, the correction terms, the face states, and the six
+// stencil rows (two per double; the first is -1 when the chain leaves the
+// table).
+enum { RF_BASE = 0, RF_KN = ex::FB_N, RF_POS = RF_KN + 3, RF_NEG = RF_POS + 5, RF_CA = RF_NEG + 5, RF_CB = RF_CA + 5,
+       RF_QP = RF_CB + 5, RF_QN = RF_QP + 5, RF_ROWS = RF_QN + 5, RF_N = RF_ROWS + 3 };
+static_assert(RF_N == kRowFace, "scratch of a row's face");
+
+struct RowRound {
+    double *p;      // [3][RF_N][ld]
+    int r0, r1;     // rows of this round
+    int ld;
+};
+
+__device__ __forceinline__ double *row_column(const RowRound &R, int gid, int d)
 {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int d = blockIdx.y;
-    if (gid >= n_items) return;
-    int st[6];
-    if (!plus_line(grid, gid, n_rows, d, st)) return;
-    double Fh[5];
-    face_side(P, gid, d, 0, st, deter, Q, metric, roe, d == 0 ? F : (d == 1 ? E : G), Fh);
+    return R.p + (size_t)d * RF_N * R.ld + (gid - R.r0);
+}
+
+__device__ __forceinline__ void stencil_rows(const double *col, size_t ld, int st[6])
+{
 #pragma unroll
-    for (int c = 0; c < 5; ++c) Fp[(d * 5 + c) * ld + gid] = Fh[c];
-    const int p = st[3];
-    if ((unsigned)p >= (unsigned)n_items || grid_nb(grid, p, minus_slot(d)) != gid) return;
-    // p's -1/2 face reads metric block 2+2d, DETERM 2d+1 and ROE block d+3 of p
-    const double *fg = metric + 63 * (size_t)gid + 9 * (1 + 2 * d) + 3 * d;
-    const double *fp = metric + 63 * (size_t)p + 9 * (2 + 2 * d) + 3 * d;
-    const double *rg = roe + 36 * (size_t)gid + 6 * d, *rp = roe + 36 * (size_t)p + 6 * (d + 3);
-    if (same_bits(fg[0], fp[0]) && same_bits(fg[1], fp[1]) && same_bits(fg[2], fp[2])
-        && same_bits(deter[6 * (size_t)gid + 2 * d], deter[6 * (size_t)p + 2 * d + 1]) && same_bits(rg[0], rp[0])
-        && same_bits(rg[1], rp[1]) && same_bits(rg[2], rp[2]) && same_bits(rg[4], rp[4]) && same_bits(rg[5], rp[5])) {
-#pragma unroll
-        for (int c = 0; c < 5; ++c) Fm[(d * 5 + c) * ld + p] = Fh[c];
-        stamp[d * ld + p] = gen;
+    for (int k = 0; k < 3; ++k) {
+        const double w = col[(RF_ROWS + k) * ld];
+        st[2 * k] = (int)xi::hi32(w);
+        st[2 * k + 1] = (int)xi::lo32(w);
     }
+}
+
+__global__ void __launch_bounds__(128, 6) k_row_base(const int *__restrict__ grid, const double *__restrict__ metric,
+                                                     const double *__restrict__ roe, int n_rows, RowRound R)
+{
+    const int gid = R.r0 + blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
+    if (gid >= R.r1) return;
+    double *col = row_column(R, gid, d);
+    const size_t ld = R.ld;
+    int st[6];
+    if (!plus_line(grid, gid, n_rows, d, st)) {
+        col[RF_ROWS * ld] = xi::words(0xffffffffu, 0u);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) col[(RF_ROWS + k) * ld] = xi::words((uint32_t)st[2 * k], (uint32_t)st[2 * k + 1]);
+    const double *fm = metric + 63 * (size_t)gid + 9 * (1 + 2 * d) + 3 * d;
+    const double *ra = roe + 36 * (size_t)gid + 6 * d;
+    const double r[5] = {ra[0], ra[1], ra[2], ra[4], ra[5]};
+    double kn[3], B[ex::FB_N];
+    ex::face_normal(fm[0], fm[1], fm[2], kn);
+    ex::face_base(r, kn, B);
+#pragma unroll
+    for (int s = 0; s < ex::FB_N; ++s) col[(RF_BASE + s) * ld] = B[s];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) col[(RF_KN + c) * ld] = kn[c];
+}
+
+__global__ void __launch_bounds__(128, 8) k_row_char(const double *__restrict__ Q, double eps, RowRound R)
+{
+    const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;
+    if (gid >= R.r1) return;
+    double *col = row_column(R, gid, d);
+    const size_t ld = R.ld;
+    int st[6];
+    stencil_rows(col, ld, st);
+    if (st[0] < 0) return;
+    double L[5], pos, neg;
+    ex::left_row(q, [&](int s) { return col[(RF_BASE + s) * ld]; }, [&](int c) { return col[(RF_KN + c) * ld]; }, L);
+    ex::char_pair(L, [&](int o, int c) { return Q[5 * (size_t)st[o] + c]; }, eps, pos, neg);
+    col[(RF_POS + q) * ld] = pos;
+    col[(RF_NEG + q) * ld] = neg;
+}
+
+__global__ void __launch_bounds__(128, 6) k_row_back(const double *__restrict__ F, const double *__restrict__ E,
+                                                     const double *__restrict__ G, RowRound R)
+{
+    const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;
+    if (gid >= R.r1) return;
+    double *col = row_column(R, gid, d);
+    const size_t ld = R.ld;
+    int st[6];
+    stencil_rows(col, ld, st);
+    if (st[0] < 0) return;
+    double qp, qn, f[6], ca, cb;
+    ex::back_pair(q, [&](int s) { return col[(RF_BASE + s) * ld]; }, [&](int c) { return col[(RF_KN + c) * ld]; },
+                  [&](int s) { return col[(RF_POS + s) * ld]; }, [&](int s) { return col[(RF_NEG + s) * ld]; }, qp, qn);
+    col[(RF_QP + q) * ld] = qp;
+    col[(RF_QN + q) * ld] = qn;
+    const double *NF = (d == 0 ? F : (d == 1 ? E : G)) + q;
+#pragma unroll
+    for (int o = 0; o < 6; ++o) f[o] = NF[5 * (size_t)st[o]];
+    ex::correction_terms(f, ca, cb);
+    col[(RF_CA + q) * ld] = ca;
+    col[(RF_CB + q) * ld] = cb;
+}
+
+// Two lanes per face: Fp[(d*5 + c)*n_all + gid]; also p's -1/2 face
+// Fm[(d*5 + c)*n_all + p] with stamp[d*n_all + p] = gen for the plus
+// neighbour p whose minus neighbour is gid, when p's face data are gid's
+// bit for bit.
+__global__ void __launch_bounds__(128, 4) k_row_flux(const double *__restrict__ deter, const int *__restrict__ grid,
+                                                     const double *__restrict__ metric, const double *__restrict__ roe,
+                                                     int n_items, int n_rows, double *__restrict__ Fp,
+                                                     double *__restrict__ Fm, unsigned *__restrict__ stamp,
+                                                     unsigned gen, long long n_all, RowRound R)
+{
+    const int t = R.r0 + (blockIdx.x * blockDim.x + threadIdx.x) / 2, d = blockIdx.y, side = threadIdx.x & 1;
+    const bool in = t < R.r1;
+    const int gid = in ? t : R.r0;
+    const double *col = row_column(R, gid, d);
+    const size_t ld = R.ld;
+    int st[6];
+    stencil_rows(col, ld, st);
+    const bool face = in && st[0] >= 0;   // the other lanes take part with a face they do not store
+    const double *fm = metric + 63 * (size_t)gid + 9 * (1 + 2 * d) + 3 * d;
+    double q[5] = {1.0, 0.0, 0.0, 0.0, 2.5}, m[3] = {1.0, 0.0, 0.0}, det = 1.0, Fh[5];
+    if (face) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c) q[c] = col[(RF_QP + 5 * side + c) * ld];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[c] = fm[c];
+        det = deter[6 * (size_t)gid + 2 * d];
+    }
+    ex::llf_lanes(q, m[0], m[1], m[2], det, Fh);
+    if (!face) return;
+    const int p = st[3];
+    bool shared = (unsigned)p < (unsigned)n_items && grid_nb(grid, p, minus_slot(d)) == gid;
+    if (shared) {   // p's -1/2 face reads metric block 2+2d, DETERM 2d+1 and ROE block d+3 of p
+        const double *mp = metric + 63 * (size_t)p + 9 * (2 + 2 * d) + 3 * d;
+        const double *rg = roe + 36 * (size_t)gid + 6 * d, *rp = roe + 36 * (size_t)p + 6 * (d + 3);
+        shared = same_bits(m[0], mp[0]) && same_bits(m[1], mp[1]) && same_bits(m[2], mp[2])
+                 && same_bits(det, deter[6 * (size_t)p + 2 * d + 1]) && same_bits(rg[0], rp[0])
+                 && same_bits(rg[1], rp[1]) && same_bits(rg[2], rp[2]) && same_bits(rg[4], rp[4])
+                 && same_bits(rg[5], rp[5]);
+    }
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+        if ((c >= 3) != (side != 0)) continue;   // components 0..2 on the even lane, 3..4 on the odd one
+        const double f = Fh[c] - col[(RF_CA + c) * ld] + col[(RF_CB + c) * ld];
+        Fp[(d * 5 + c) * n_all + gid] = f;
+        if (shared) Fm[(d * 5 + c) * n_all + p] = f;
+    }
+    if (shared && side == 0) stamp[d * n_all + p] = gen;
 }
 
 // Rows of offsets -3..2 of row n along d; false if the chain leaves
@@ -335,7 +525,7 @@ __device__ __forceinline__ bool minus_line(const int *grid, int n, int n_rows, i
     return true;
 }
 
-// The -1/2 face of every row gid < n_items along each d that k_weno_plus
+// The -1/2 face of every row gid < n_items along each d that the k_row_* kernels
 // did not stamp, from the row's own face data (metric block 2+2d, DETERM
 // 2d+1, ROE block d+3): Fm and stamp = gen.  A grid-stride scan of the
 // rows, direction by direction, with a resident-sized grid: on a periodic
@@ -365,11 +555,11 @@ __global__ void __launch_bounds__(128, 2) k_weno_minus(Phys P, const double *__r
 
 // Weno.cl:36-3137: per row, both faces of each direction from the row's own
 // face data (metric blocks, DETERM, ROE_AVERAGING), as the reference does.
-// REUSE: the +1/2 faces come from k_weno_plus (Fp), the -1/2 faces from Fm
-// (k_weno_plus or k_weno_minus; every row whose stencil stays in the table
+// REUSE: the +1/2 faces come from the k_row_* kernels (Fp), the -1/2 faces from Fm
+// (the k_row_* kernels or k_weno_minus; every row whose stencil stays in the table
 // is stamped with this call's generation).
 template <bool REUSE>
-__global__ void __launch_bounds__(128) k_weno(Phys P, int j, double mach, double dt, const double *__restrict__ deter,
+__global__ void __launch_bounds__(128, REUSE ? 5 : 1) k_weno(Phys P, int j, double mach, double dt, const double *__restrict__ deter,
                                               const double *__restrict__ det, double *__restrict__ U0,
                                               double *__restrict__ U1, double *__restrict__ U2,
                                               const int *__restrict__ grid, const double *__restrict__ Q,
@@ -418,10 +608,15 @@ __global__ void __launch_bounds__(128) k_weno(Phys P, int j, double mach, double
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
             dflux[d][c] = Fh[0][c] - Fh[1][c];
-            double f[7];
+        }
+        const int b = weno_visc_branch(Lc);
+        if (b == 5) {
+            ex::central4([&](int o, int c) { return VF[5 * (size_t)idx[d][o + 3] + c]; }, dvis[d]);
+        } else {
 #pragma unroll
-            for (int o = 0; o < 7; ++o) f[o] = VF[5 * (size_t)idx[d][o] + c];
-            dvis[d][c] = weno_visc_deriv_ref(f, Lc);
+            for (int c = 0; c < 5; ++c)
+                dvis[d][c] = row_deriv(VF + c, idx[d][0], idx[d][1], idx[d][2], idx[d][3], idx[d][4], idx[d][5],
+                                       idx[d][6], b);
         }
     };
     if (REUSE) {
@@ -470,7 +665,7 @@ __global__ void __launch_bounds__(128) k_weno(Phys P, int j, double mach, double
 int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
               double *roe, int n_items, int n_rows, unsigned *flags, double *node_scratch, long long scratch_rows)
 {
-    if (node_scratch && scratch_rows >= n_rows) {   // 2 of the 15 doubles per row
+    if (node_scratch && scratch_rows >= n_rows) {   // 5 of the 30 doubles per row
         k_uq_node<<<blocks_for(n_rows, 128), 128, 0, st>>>(flow, n_rows, node_scratch);
         k_uq<true><<<blocks_for(n_items, 128), 128, 0, st>>>(U, Q, grid, det, flow, roe, n_items, n_rows, flags,
                                                              node_scratch);
@@ -480,12 +675,20 @@ int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const doub
     return 1;
 }
 
-void launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
+int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
                     double *Ev, double *Gv, const int *grid, const double *metric, const double *det, double *flow,
-                    int n_items, int n_rows, unsigned *flags)
+                    int n_items, int n_rows, unsigned *flags, double *scratch, long long scratch_rows)
 {
-    k_viscous<<<blocks_for(n_items, 128), 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items,
-                                                        n_rows, flags);
+    const unsigned nb = blocks_for(n_items, 128);
+    if (scratch && scratch_rows >= n_items) {
+        k_node_flux<<<nb, 128, 0, st>>>(F, E, G, metric, det, flow, n_items, P.les, scratch);
+        k_viscous<false><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
+                                             scratch);
+        return 2;
+    }
+    k_viscous<true><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
+                                        nullptr);
+    return 1;
 }
 
 // Grid of k_weno_minus: two resident blocks of 128 per SM, at most one
@@ -513,8 +716,16 @@ void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, 
         const long long ld = scratch_rows;
         double *Fp = face_scratch, *Fm = face_scratch + 15 * ld;
         unsigned *stamp = face_stamps(face_scratch, ld);
-        k_weno_plus<<<dim3(nb, 3), 128, 0, st>>>(P, deter, grid, Q, metric, roe, F, E, G, n_items, n_rows, Fp, Fm,
-                                                 stamp, gen, ld);
+        const int round = (int)row_round(ld);
+        for (int r0 = 0; r0 < n_items; r0 += round) {
+            const RowRound R{face_scratch + 30 * ld, r0, std::min(n_items, r0 + round), round};
+            const unsigned n = blocks_for(R.r1 - r0, 128);
+            k_row_base<<<dim3(n, 3), 128, 0, st>>>(grid, metric, roe, n_rows, R);
+            k_row_char<<<dim3(5 * n, 3), 128, 0, st>>>(Q, P.eps, R);
+            k_row_back<<<dim3(5 * n, 3), 128, 0, st>>>(F, E, G, R);
+            k_row_flux<<<dim3(blocks_for(2LL * (R.r1 - r0), 128), 3), 128, 0, st>>>(
+                deter, grid, metric, roe, n_items, n_rows, Fp, Fm, stamp, gen, ld, R);
+        }
         k_weno_minus<<<minus_blocks(n_items), 128, 0, st>>>(P, deter, grid, Q, metric, roe, F, E, G, n_items, n_rows,
                                                              Fm, stamp, gen, ld);
         k_weno<true><<<nb, 128, 0, st>>>(P, j, mach, dt, deter, det, U0, U1, U2, grid, Q, metric, roe, Fv, Ev, Gv, F, E,

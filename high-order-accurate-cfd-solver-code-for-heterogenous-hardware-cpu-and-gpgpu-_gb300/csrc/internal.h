@@ -31,7 +31,7 @@ struct cfd_ctx {
     unsigned *h_flags = nullptr;   // pinned mirror
     uint64_t launches = 0;
     std::string last_error;
-    // cfd_weno's face scratch (15 doubles per row, allocated by
+    // cfd_weno's face scratch (30 doubles per row and one round's, allocated by
     // cfd_ctx_set_rows; null: each row evaluates both faces itself)
     double *d_face = nullptr;   // face_scratch_bytes(face_rows)
     long long face_rows = 0;
@@ -78,35 +78,49 @@ cfd_status_t stage_in(cfd_ctx *ctx, BufArg *a, int n, const char *who);
 cfd_status_t stage_out(cfd_ctx *ctx, const BufArg *a, int n, cfd_status_t launch_status);
 
 // Drop-in kernel launchers (dropin.cu).  All pointers are device pointers.
-// U_Q; with a scratch of >= n_rows rows (15 doubles each, cfd_weno's face
-// scratch) it first computes sqrt(rho) and H once per row.  Returns the
+// U_Q; with a scratch of >= n_rows rows (30 doubles each, cfd_weno's face
+// scratch) it first computes sqrt(rho) and its products once per row.  Returns the
 // kernels launched (2 or 1).
 int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
               double *roe, int n_items, int n_rows, unsigned *flags, double *node_scratch, long long scratch_rows);
-void launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
+// Viscous; the scratch as for launch_uq.  Returns the kernels launched.
+int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
                     double *Ev, double *Gv, const int *grid, const double *metric, const double *det, double *flow,
-                    int n_items, int n_rows, unsigned *flags);
+                    int n_items, int n_rows, unsigned *flags, double *scratch, long long scratch_rows);
 void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, const double *deter,
                  const double *det, double *U0, double *U1, double *U2, const int *grid, const double *Q,
                  const double *metric, const double *roe, const double *Fv, const double *Ev, const double *Gv,
                  const double *F, const double *E, const double *G, double *flow, int n_items, int n_rows,
                  unsigned *flags, double *L_out, double *face_scratch, long long scratch_rows, unsigned gen);
 // Face scratch of launch_weno for `rows` rows: +1/2 faces [3][5][rows] and
-// -1/2 faces [3][5][rows] (doubles), then generation stamps [3][rows]
-// (unsigned, zero when allocated).  gen: a value new to the scratch on every
-// call (next_face_gen).
-inline size_t face_scratch_bytes(long long rows) { return (size_t)rows * (30 * sizeof(double) + 3 * sizeof(unsigned)); }
-inline unsigned *face_stamps(double *scratch, long long rows) { return reinterpret_cast<unsigned *>(scratch + 30 * rows); }
+// -1/2 faces [3][5][rows] (doubles), the face kernels' own scratch for one
+// round of rows, then generation stamps [3][rows] (unsigned, zero when
+// allocated).  gen: a value new to the scratch on every call
+// (next_face_gen).
+constexpr long long kRowRound = 1 << 18;   // rows of one round of the face kernels: 302 MB, some 25 waves of blocks
+constexpr int kRowFace = 48;               // doubles of one row's face along one direction
+inline long long row_round(long long rows) { return rows < kRowRound ? rows : kRowRound; }
+inline size_t face_scratch_doubles(long long rows) { return (size_t)rows * 30 + (size_t)row_round(rows) * 3 * kRowFace; }
+inline size_t face_scratch_bytes(long long rows)
+{
+    return face_scratch_doubles(rows) * sizeof(double) + (size_t)rows * 3 * sizeof(unsigned);
+}
+inline unsigned *face_stamps(double *scratch, long long rows)
+{
+    return reinterpret_cast<unsigned *>(scratch + face_scratch_doubles(rows));
+}
 inline unsigned next_face_gen(unsigned &g)
 {
     g = g + 1 == 0 ? 1 : g + 1;
     return g;
 }
-// Kernels one launch_weno issues: 2 with a face scratch of >= n_items rows,
-// else 1.
+// Kernels one launch_weno issues: four face kernels per round, the unstamped
+// faces and the update with a face scratch of >= n_items rows, else 1.
 inline int weno_launches(const double *face_scratch, long long scratch_rows, int n_items)
 {
-    return face_scratch && scratch_rows >= n_items ? 3 : 1;
+    if (!face_scratch || scratch_rows < n_items) return 1;
+    const long long round = row_round(scratch_rows);
+    return (int)(4 * ((n_items + round - 1) / round) + 2);
 }
 
 }  // namespace cfd
