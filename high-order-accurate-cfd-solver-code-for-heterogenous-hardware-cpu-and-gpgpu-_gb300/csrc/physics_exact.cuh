@@ -343,15 +343,15 @@ struct WenoConst {
 __device__ __forceinline__ WenoConst weno_const(double cm2, double cm1, double c0, double c1, double c2, double c3)
 {
     WenoConst w;
-    uint32_t h[8], l[8], any = 0u;
-    any |= xi::small_words<3, 0>(c0, h[0], l[0]);
-    any |= xi::small_words<15, -3>(c0, h[1], l[1]);
-    any |= xi::small_words<3, 0>(c1, h[2], l[2]);
-    any |= xi::small_words<15, -3>(c1, h[3], l[3]);
-    any |= xi::small_words<5, -2>(c2, h[4], l[4]);
-    any |= xi::small_words<3, -3>(c3, h[5], l[5]);
-    any |= xi::small_words<5, -2>(cm1, h[6], l[6]);
-    any |= xi::small_words<3, -3>(cm2, h[7], l[7]);
+    uint32_t h[8], l[8], k[8];
+    k[0] = xi::small_words<3, 0>(c0, h[0], l[0]);
+    k[1] = xi::small_words<15, -3>(c0, h[1], l[1]);
+    k[2] = xi::small_words<3, 0>(c1, h[2], l[2]);
+    k[3] = xi::small_words<15, -3>(c1, h[3], l[3]);
+    k[4] = xi::small_words<5, -2>(c2, h[4], l[4]);
+    k[5] = xi::small_words<3, -3>(c3, h[5], l[5]);
+    k[6] = xi::small_words<5, -2>(cm1, h[6], l[6]);
+    k[7] = xi::small_words<3, -3>(cm2, h[7], l[7]);
     w.b0 = xi::words(h[0], l[0]);
     w.q0 = xi::words(h[0] - (2u << 20), l[0]);
     w.h0 = xi::words(h[0] - (3u << 20), l[0]);
@@ -364,19 +364,19 @@ __device__ __forceinline__ WenoConst weno_const(double cm2, double cm1, double c
     w.h3 = xi::words(h[5], l[5]);
     w.vm1 = xi::words(h[6], l[6]);
     w.hm2 = xi::words(h[7], l[7]);
-    if (__builtin_expect(any != 0u, 0)) {
-        w.b0 = 3.0 * c0;
-        w.q0 = (3.0 / 4.0) * c0;
-        w.h0 = (3.0 / 8.0) * c0;
-        w.f0 = (15.0 / 8.0) * c0;
-        w.b1 = 3.0 * c1;
-        w.q1 = (3.0 / 4.0) * c1;
-        w.h1 = (3.0 / 8.0) * c1;
-        w.f1 = (15.0 / 8.0) * c1;
-        w.v2 = (5.0 / 4.0) * c2;
-        w.h3 = (3.0 / 8.0) * c3;
-        w.vm1 = (5.0 / 4.0) * cm1;
-        w.hm2 = (3.0 / 8.0) * cm2;
+    if (__builtin_expect((k[0] | k[2] | k[4] | k[5] | k[6] | k[7]) != 0u, 0)) {
+        w.b0 = xi::small_or(k[0], h[0], l[0], c0, 3.0);
+        w.q0 = xi::small_or(k[0], h[0] - (2u << 20), l[0], c0, 3.0 / 4.0);
+        w.h0 = xi::small_or(k[0], h[0] - (3u << 20), l[0], c0, 3.0 / 8.0);
+        w.f0 = xi::small_or(k[1], h[1], l[1], c0, 15.0 / 8.0);
+        w.b1 = xi::small_or(k[2], h[2], l[2], c1, 3.0);
+        w.q1 = xi::small_or(k[2], h[2] - (2u << 20), l[2], c1, 3.0 / 4.0);
+        w.h1 = xi::small_or(k[2], h[2] - (3u << 20), l[2], c1, 3.0 / 8.0);
+        w.f1 = xi::small_or(k[3], h[3], l[3], c1, 15.0 / 8.0);
+        w.v2 = xi::small_or(k[4], h[4], l[4], c2, 5.0 / 4.0);
+        w.h3 = xi::small_or(k[5], h[5], l[5], c3, 3.0 / 8.0);
+        w.vm1 = xi::small_or(k[6], h[6], l[6], cm1, 5.0 / 4.0);
+        w.hm2 = xi::small_or(k[7], h[7], l[7], cm2, 3.0 / 8.0);
     }
     return w;
 }
@@ -625,26 +625,22 @@ __device__ __forceinline__ void llf_lanes(const double q[5], double mx, double m
 __device__ __forceinline__ void correction_terms(const double f[6], double &a, double &b)
 {
     double p[8];   // 5 f0, 39 f1, 34 f2, 34 f3, 39 f4, 5 f5, 3 f1, 3 f4
-    uint32_t h[8], l[8], any = 0u;
-    any |= xi::small_words<5, 0>(f[0], h[0], l[0]);
-    any |= xi::small_words<39, 0>(f[1], h[1], l[1]);
-    any |= xi::small_words<17, 1>(f[2], h[2], l[2]);
-    any |= xi::small_words<17, 1>(f[3], h[3], l[3]);
-    any |= xi::small_words<39, 0>(f[4], h[4], l[4]);
-    any |= xi::small_words<5, 0>(f[5], h[5], l[5]);
-    any |= xi::small_words<3, 0>(f[1], h[6], l[6]);
-    any |= xi::small_words<3, 0>(f[4], h[7], l[7]);
+    uint32_t h[8], l[8], k[8];
+    k[0] = xi::small_words<5, 0>(f[0], h[0], l[0]);
+    k[1] = xi::small_words<39, 0>(f[1], h[1], l[1]);
+    k[2] = xi::small_words<17, 1>(f[2], h[2], l[2]);
+    k[3] = xi::small_words<17, 1>(f[3], h[3], l[3]);
+    k[4] = xi::small_words<39, 0>(f[4], h[4], l[4]);
+    k[5] = xi::small_words<5, 0>(f[5], h[5], l[5]);
+    k[6] = xi::small_words<3, 0>(f[1], h[6], l[6]);
+    k[7] = xi::small_words<3, 0>(f[4], h[7], l[7]);
 #pragma unroll
     for (int i = 0; i < 8; ++i) p[i] = xi::words(h[i], l[i]);
-    if (__builtin_expect(any != 0u, 0)) {
-        p[0] = 5.0 * f[0];
-        p[1] = 39.0 * f[1];
-        p[2] = 34.0 * f[2];
-        p[3] = 34.0 * f[3];
-        p[4] = 39.0 * f[4];
-        p[5] = 5.0 * f[5];
-        p[6] = 3.0 * f[1];
-        p[7] = 3.0 * f[4];
+    if (__builtin_expect((k[0] | k[1] | k[2] | k[3] | k[4] | k[5]) != 0u, 0)) {
+        const double x[8] = {f[0], f[1], f[2], f[3], f[4], f[5], f[1], f[4]};
+        const double c[8] = {5.0, 39.0, 34.0, 34.0, 39.0, 5.0, 3.0, 3.0};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p[i] = xi::small_or(k[i], h[i], l[i], x[i], c[i]);
     }
     const double s2 = -p[0] + p[1] - p[2] - p[3] + p[4] - p[5];
     const double d4 = xdiv::scale2<-1>(f[0] - p[6] + xdiv::scale2<1>(f[2]) + xdiv::scale2<1>(f[3]) - p[7] + f[5]);
