@@ -59,6 +59,9 @@ struct cfd_batch {
     BatchItem *d_items = nullptr;
     size_t items_cap = 0;
     int nitems = 0;
+    double *d_scratch = nullptr;          // FP64 form: face scratch of round_tiles tiles
+    size_t scratch_cap = 0;               // doubles
+    int round_tiles = 0;
     int n_views = 0;
     unsigned *d_words = nullptr;          // [0..1] barrier, [2] batch flags, [3] phase-A work counter, [4..] per-slot flags
     int threads = 128;
@@ -90,7 +93,7 @@ uint64_t instance_bytes(int precision, int64_t N)
     // split: FP32 face metrics (9), node geometry (11), prim32 (9), Q32/R32/FEG32/V32 (40) and the hi/lo
     // state copy (10); FP64 1/det and Fh (16)
     if (precision == CFD_PREC_SPLIT) return (doubles + 16 * (uint64_t)N) * 8 + (9 + 11 + 9 + 40 + 10) * (uint64_t)N * 4;
-    return (doubles + 52 * (uint64_t)N) * 8;
+    return (doubles + 65 * (uint64_t)N) * 8;   // stage intermediates (55), unit normals (9), filter width
 }
 
 void drop_graph(cfd_batch *b)
@@ -232,9 +235,36 @@ cfd_status_t rebuild(cfd_batch *b)
         if (e != cudaSuccess) return cuda_fail(b->ctx, e, "batch item table upload");
         b->nitems = (int)items.size();
     }
+    if (b->precision == CFD_PREC_FP64 && b->ntiles > 0) {
+        // scratch for one round of tiles: kBatchRound nodes, or as many as
+        // there is memory for
+        int round = std::min(b->ntiles, std::max(1, kBatchRound / T));
+        for (;; round = (round + 1) / 2) {
+            const size_t need = 3 * (size_t)kFaceScratch * (size_t)round * (size_t)T;
+            if (need <= b->scratch_cap) break;
+            if (b->d_scratch) cudaFree(b->d_scratch);
+            b->d_scratch = nullptr;
+            b->scratch_cap = 0;
+            e = cudaMalloc(&b->d_scratch, need * sizeof(double));
+            if (e == cudaSuccess) {
+                b->scratch_cap = need;
+                break;
+            }
+            b->d_scratch = nullptr;
+            if (e != cudaErrorMemoryAllocation || round == 1) return cuda_fail(b->ctx, e, "batch face scratch");
+            cudaGetLastError();
+        }
+        b->round_tiles = round;
+    }
     drop_graph(b);
     b->dirty = false;
     return CFD_OK;
+}
+
+// Kernel launches of one RK step.
+int step_launches(const cfd_batch *b)
+{
+    return 3 * (b->precision == CFD_PREC_FP64 ? batch_launches_fp64(b->ntiles, b->round_tiles) : 1);
 }
 
 BatchLaunch launch_of(cfd_batch *b)
@@ -248,6 +278,8 @@ BatchLaunch launch_of(cfd_batch *b)
     L.tiled = b->nitems > 0 ? 1 : 0;
     L.items = b->d_items;
     L.nitems = b->nitems;
+    L.scratch = b->d_scratch;
+    L.round_tiles = b->round_tiles;
     L.bar = bar_words(b);
     L.gflags = batch_flags(b);
     // generous deadline for the barrier: 5 s + 50 ns per node of the batch
@@ -403,6 +435,7 @@ cfd_status_t cfd_batch_destroy(cfd_batch_t *b)
     if (b->d_views) cudaFree(b->d_views);
     if (b->d_tiles) cudaFree(b->d_tiles);
     if (b->d_items) cudaFree(b->d_items);
+    if (b->d_scratch) cudaFree(b->d_scratch);
     if (b->d_words) cudaFree(b->d_words);
     delete b;
     return CFD_OK;
@@ -565,6 +598,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     v.U2 = U2;
     v.flags = slot_flags(b, slot);
     v.Lout = nullptr;
+    double *kn = nullptr, *del = nullptr;
     if (b->precision == CFD_PREC_MIXED) {
         float *fm32, *fdet32, *node32, *idet32;
         if ((st = ialloc(b, I, 9 * Nz, &fm32)) || (st = ialloc(b, I, 3 * Nz, &fdet32))
@@ -595,10 +629,13 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         v.idet64 = idet64;
     } else {
         if ((st = ialloc(b, I, 5 * Nz, &v.Q)) || (st = ialloc(b, I, 15 * Nz, &v.FEG)) || (st = ialloc(b, I, 15 * Nz, &v.V))
-            || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))) {
+            || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))
+            || (st = ialloc(b, I, 9 * Nz, &kn)) || (st = ialloc(b, I, Nz, &del))) {
             free_instance(I);
             return st;
         }
+        v.kn = kn;
+        v.del = del;
     }
     cudaStream_t sm = ctx->stream;
     cudaError_t e = cudaMemcpyAsync(m9, host_ptr(S->m9), 9 * Nz * 8, cudaMemcpyHostToDevice, sm);
@@ -650,11 +687,12 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         split_geometry(S);
         batch_prep_split(v, sm);
     } else {
+        fp64_geometry(v, kn, del, sm);
         batch_prep_fp64(v, sm);
     }
     ctx->launches += b->precision == CFD_PREC_MIXED   ? 2 + kMixedGeometryLaunches
                      : b->precision == CFD_PREC_SPLIT ? 2 + kSplitGeometryLaunches
-                                                      : 2;
+                                                      : 3;
     e = cudaStreamSynchronize(sm);   // host geometry vectors go out of scope
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -713,7 +751,7 @@ cfd_status_t enqueue_steps(cfd_batch_t *b, int32_t nsteps)
     for (int s = 0; s < nsteps; ++s) {
         cudaError_t e = b->graph_ok ? cudaGraphLaunch(b->gexec, sm) : launch_step(b);
         if (e != cudaSuccess) return cuda_fail(b->ctx, e, "batch step launch");
-        b->ctx->launches += 3;
+        b->ctx->launches += step_launches(b);
     }
     return CFD_OK;
 }
@@ -907,7 +945,7 @@ cfd_status_t cfd_batch_tune(cfd_batch_t *b, int32_t steps_per_trial)
         bool ok = true;
         for (int s = 0; s < steps_per_trial && ok; ++s) ok = one() == cudaSuccess;
         cudaEventRecord(t1, sm);
-        b->ctx->launches += 3 * (steps_per_trial + 1);
+        b->ctx->launches += step_launches(b) * (steps_per_trial + 1);
         if (!ok || cudaEventSynchronize(t1) != cudaSuccess) { cudaGetLastError(); continue; }
         float ms = 0;
         cudaEventElapsedTime(&ms, t0, t1);

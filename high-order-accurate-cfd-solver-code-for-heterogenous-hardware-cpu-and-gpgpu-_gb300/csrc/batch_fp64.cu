@@ -1,9 +1,18 @@
-// batch_fp64.cu -- the batched persistent stage kernel instantiated with the
-// per-node operations of the exact FP64 evaluation order (compiled with --fmad=false) form.
-// The batched stage runs 8 warps per SM: too few to hide the integer
-// product's latency, so the divisions' first quotient comes from the FP64
-// multiply (exact_div.cuh, CFD_XDIV_QPROD; the same bits either way).
-#define CFD_XDIV_QPROD 0
+// batch_fp64.cu -- the batched stage in the FP64 form (compiled with
+// --fmad=false, reference evaluation order).
+//
+// The FP64 pipe bounds it, so it runs as the single lattice does
+// (faces_fp64.cu): the viscous fluxes and the face pass as kernels of their
+// own over the tile table of all instances, each at the registers its part
+// needs, and only the last one -- the LLF fluxes, the grid barrier, then the
+// update with the next stage's U_Q -- as a persistent cooperative launch.
+// One persistent launch for the whole stage needed 250 registers (8 warps
+// per SM), too few to hide the integer chains of the products and quotients.
+// The face scratch is the batch's, kept between steps, for at most
+// kBatchRound nodes; a larger batch runs its faces in rounds of tiles.
+// 8 vortices (24^3-48^3, 384,631 nodes), one step with FLOW in and out:
+// 13.9 ms as one persistent launch per stage, 11.8 with the integer products
+// in it, 8.7 ms here.
 #include "batch_kernel.cuh"
 #include "batch_ops.h"
 #include "internal.h"
@@ -12,34 +21,105 @@
 namespace cfd {
 namespace {
 
-// 1: shared reciprocals in the face flux (exact_div.cuh), as in the
-// single-lattice kernels; 0: a division per quotient.  Same bits either
-// way; with the quotients' rounding on the integer pipe the shared form is
-// the faster here too (64 vortices: 2.30e7 against 2.15e7 cell-updates/s).
-#ifndef CFD_FBATCH_SHARED_DIV
-#define CFD_FBATCH_SHARED_DIV 1
-#endif
-
 struct Ops {
-    static constexpr int kMinBlocks = 1;
     static __device__ __forceinline__ void prep(const LatView &g, int n, int q) { ex::prep_node(g, n, q); }
-    static __device__ __forceinline__ void visc(const LatView &g, int n, int q) { ex::visc_node(g, n, q); }
-    static __device__ __forceinline__ void mu(const LatView &g, int n, int q) { ex::mu_node(g, n, q); }
-    template <int D>
-    static __device__ __forceinline__ void face(const LatView &g, int n)
-    {
-        ex::face_node<D, CFD_FBATCH_SHARED_DIV != 0>(g, n);
-    }
-    static __device__ __forceinline__ void update(const LatView &g, int n, int j) { ex::update_node(g, n, j, true); }
 };
+
+__global__ void __launch_bounds__(256, 2) k_batch_visc(const LatView *__restrict__ views,
+                                                       const BatchTile *__restrict__ tiles, int jst)
+{
+    const BatchTile t = tiles[blockIdx.x];
+    if ((int)threadIdx.x >= t.count) return;
+    const LatView &g = views[t.inst];
+    if (g.P.viscous) ex::visc_node(g, t.n0 + threadIdx.x, jst);
+    else ex::mu_node(g, t.n0 + threadIdx.x, jst);
+}
+
+// Scratch columns of tile w of a round: the round's tiles back to back.
+__device__ __forceinline__ FaceScratch tile_scratch(double *p, const BatchTile &t, int w, int ld)
+{
+    return {p, t.n0 - w * (int)blockDim.x, ld};
+}
+
+// Tiles t0 + w of the round that starts at t0; blockIdx.y the direction,
+// neighbouring blocks the fields or components of one tile.
+__global__ void __launch_bounds__(256, 4) k_batch_base(const LatView *__restrict__ views,
+                                                       const BatchTile *__restrict__ tiles, int t0, double *p, int ld)
+{
+    const int w = blockIdx.x;
+    const BatchTile t = tiles[t0 + w];
+    if ((int)threadIdx.x < t.count)
+        ex::base_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(256, 4) k_batch_char(const LatView *__restrict__ views,
+                                                       const BatchTile *__restrict__ tiles, int t0, double *p, int ld)
+{
+    const int w = blockIdx.x / 5u;
+    const BatchTile t = tiles[t0 + w];
+    if ((int)threadIdx.x < t.count)
+        ex::char_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u);
+}
+
+__global__ void __launch_bounds__(256, 3) k_batch_back(const LatView *__restrict__ views,
+                                                       const BatchTile *__restrict__ tiles, int t0, double *p, int ld)
+{
+    const int w = blockIdx.x / 5u;
+    const BatchTile t = tiles[t0 + w];
+    if ((int)threadIdx.x < t.count)
+        ex::back_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u);
+}
+
+// Half h of tile w's faces along d, two lanes per face.
+__device__ __forceinline__ void flux_half(const LatView *__restrict__ views, const BatchTile *__restrict__ tiles,
+                                          int t0, int w, int d, int h, double *p, int ld)
+{
+    const BatchTile t = tiles[t0 + w];
+    const int k = h * (int)(blockDim.x / 2) + (int)(threadIdx.x / 2);
+    const bool in = k < t.count;
+    ex::flux_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + (in ? k : 0), d, in);
+}
+
+__global__ void __launch_bounds__(256, 2) k_batch_flux(const LatView *__restrict__ views,
+                                                       const BatchTile *__restrict__ tiles, int t0, double *p, int ld)
+{
+    flux_half(views, tiles, t0, blockIdx.x / 2u, blockIdx.y, blockIdx.x % 2u, p, ld);
+}
+
+// The last round's fluxes, the grid barrier, and the update of every tile.
+__global__ void __launch_bounds__(256, 2)
+k_batch_close(const LatView *__restrict__ views, const BatchTile *__restrict__ tiles, int ntiles, int t0, int jst,
+              double *p, int ld, unsigned *bar, unsigned *gflags, unsigned long long limit_ns)
+{
+    const int items = 6 * (ntiles - t0);
+    for (int w = next_item(bar); w < items; w = next_item(bar)) flux_half(views, tiles, t0, w / 6, (w % 6) >> 1, w & 1, p, ld);
+    if (!grid_barrier(bar, gridDim.x, limit_ns, gflags)) return;
+    for (int w = blockIdx.x; w < ntiles; w += gridDim.x) {
+        const BatchTile t = tiles[w];
+        if ((int)threadIdx.x < t.count) ex::update_node(views[t.inst], t.n0 + threadIdx.x, jst, true);
+    }
+}
 
 }  // namespace
 
 cudaError_t batch_stage_fp64(const BatchLaunch &b, int j)
 {
+    const int T = b.threads, ld = b.round_tiles * T;
+    k_batch_visc<<<b.ntiles, T, 0, b.stream>>>(b.views, b.tiles, j);
+    int t0 = 0;
+    for (;; t0 += b.round_tiles) {
+        const int nt = b.ntiles - t0 < b.round_tiles ? b.ntiles - t0 : b.round_tiles;
+        k_batch_base<<<dim3(nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+        k_batch_char<<<dim3(5 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+        k_batch_back<<<dim3(5 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+        if (t0 + nt == b.ntiles) break;   // the closing launch takes this round's fluxes
+        k_batch_flux<<<dim3(2 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+    }
+    const cudaError_t e = cudaPeekAtLastError();
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(b.blocks);
-    cfg.blockDim = dim3(b.threads);
+    cfg.blockDim = dim3(T);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = b.stream;
     cudaLaunchAttribute attr[1];
@@ -47,7 +127,14 @@ cudaError_t batch_stage_fp64(const BatchLaunch &b, int j)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_batch_stage<Ops>, b.views, b.tiles, b.ntiles, j, b.bar, b.gflags, b.limit_ns);
+    return cudaLaunchKernelEx(&cfg, k_batch_close, b.views, b.tiles, b.ntiles, t0, j, b.scratch, ld, b.bar, b.gflags,
+                              b.limit_ns);
+}
+
+int batch_launches_fp64(int ntiles, int round_tiles)
+{
+    const int rounds = (ntiles + round_tiles - 1) / round_tiles;
+    return 1 + 4 * rounds;   // viscous; base, char, back and the fluxes or the closing launch
 }
 
 void batch_prep_fp64(const LatView &g, cudaStream_t st)
@@ -58,7 +145,7 @@ void batch_prep_fp64(const LatView &g, cudaStream_t st)
 int batch_occupancy_fp64(int threads)
 {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_stage<Ops>, threads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_close, threads, 0) != cudaSuccess) return 0;
     return nb;
 }
 

@@ -1,5 +1,5 @@
-// batch_ops.h -- host-side launch interface of the batched persistent kernel
-// for the two precision forms (batch_fp64.cu, batch_mixed.cu).
+// batch_ops.h -- host-side launch interface of the batched stage for the
+// precision forms (batch_fp64.cu, batch_mixed.cu, batch_split.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,12 +32,23 @@ struct BatchLaunch {
     const BatchItem *items = nullptr;
     int nitems = 0;
     int tiled = 0;
+    // FP64 form: the face kernels' scratch, [3][kFaceScratch] columns of
+    // round_tiles tiles
+    double *scratch = nullptr;
+    int round_tiles = 0;
 };
 
-// One RK stage j (cooperative launch).  Returns the launch error.
+// Nodes whose faces one round of the FP64 form's face kernels takes at most
+// (1.06 GB of scratch).
+constexpr int kBatchRound = 1 << 20;
+
+// One RK stage j (its last or only launch cooperative).  Returns the launch
+// error.
 cudaError_t batch_stage_fp64(const BatchLaunch &b, int j);
 cudaError_t batch_stage_mixed(const BatchLaunch &b, int j);
 cudaError_t batch_stage_split(const BatchLaunch &b, int j);
+// Launches of one FP64 stage (the reduced forms: 1).
+int batch_launches_fp64(int ntiles, int round_tiles);
 // Stage-0 prep of one lattice.
 void batch_prep_fp64(const LatView &g, cudaStream_t st);
 void batch_prep_mixed(const LatView &g, cudaStream_t st);
