@@ -140,7 +140,7 @@ __device__ __forceinline__ void tile_stencil(const float *sQ, const float *sR, i
 #pragma unroll
         for (int q = 0; q < 5; ++q) P[o][q] = make_float2(sQ[q * S + T::at(t + o, a)], sQ[q * S + T::at(t + 5 - o, a)]);
     const int er = T::at(t + 3, a), el = T::at(t + 2, a);
-    roe_average<float>(sR[3 * S + er], sR[er], sR[S + er], sR[2 * S + er], sR[4 * S + er], sR[3 * S + el], sR[el],
+    roe_average(sR[3 * S + er], sR[er], sR[S + er], sR[2 * S + er], sR[4 * S + er], sR[3 * S + el], sR[el],
                        sR[S + el], sR[2 * S + el], sR[4 * S + el], r);
 }
 

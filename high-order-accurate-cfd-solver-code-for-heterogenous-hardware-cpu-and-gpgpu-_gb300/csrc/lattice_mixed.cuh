@@ -66,14 +66,14 @@ __device__ __forceinline__ dfl df_mul(dfl x, dfl c)
 // x * c rounded once to FP32
 __device__ __forceinline__ float df_mul_f(dfl x, dfl c)
 {
-    return fmaf(x.h, c.h, fmaf(x.h, c.l, x.l * c.h));
+    return fmaf(x.h, c.h, fmaf(x.h, c.l, __fmul_rn(x.l, c.h)));
 }
 
 // a / b rounded to FP32 (within about one ulp), r an approximation of 1/b.h
 __device__ __forceinline__ float df_div_f(dfl a, dfl b, float r)
 {
     const float q = a.h * r;
-    const float rem = fmaf(-q, b.h, a.h) + (a.l - q * b.l);
+    const float rem = fmaf(-q, b.h, a.h) + fmaf(-q, b.l, a.l);
     return fmaf(rem, r, q);
 }
 
@@ -84,8 +84,8 @@ __device__ __forceinline__ dfl df_div(dfl a, dfl b, float r)
     const float p = q * b.h;
     const float pe = fmaf(q, b.h, -p);
     // remainder a - q*b, then one correction step
-    const float rem = ((a.h - p) - pe) + (a.l - q * b.l);
-    return quick_two_sum(q, rem * r);
+    const float rem = ((a.h - p) - pe) + fmaf(-q, b.l, a.l);
+    return quick_two_sum(q, __fmul_rn(rem, r));
 }
 
 // 1/3 and 2/3 as hi + lo
@@ -124,16 +124,16 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
 {
     const int N = g.N;
     const dfl idet = {g.idet32[n], g.idet32[N + n]};
-    const float r0 = 1.0f / Un[0].h;
+    const float r0 = frcp(Un[0].h);
     const float rho = df_mul_f(Un[0], idet);
     const float u = df_div_f(Un[1], Un[0], r0), v = df_div_f(Un[2], Un[0], r0), w = df_div_f(Un[3], Un[0], r0);
-    const float ke = 0.5f * (u * u + v * v + w * w);
+    const float ke = __fmul_rn(0.5f, dot3(u, u, v, v, w, w));
     const dfl q4 = df_div(Un[4], Un[0], r0);   // E / rho
     const dfl e2 = df_add(q4, {-ke, 0.0f});      // internal energy e
     const dfl rho2 = df_mul(Un[0], idet);
     const float p = df_mul_f(df_mul(rho2, e2), {kGm1H, kGm1L});
-    const float irho = 1.0f / rho;
-    const float pr = p * irho;
+    const float irho = frcp(rho);
+    const float pr = __fmul_rn(p, irho);
     g.prim32[LF_P * N + n] = p;
     if (!(isfinite(rho) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(p))) atomicOr(g.flags, 2u);
     const float E = df_mul_f(Un[4], idet);
@@ -145,14 +145,14 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
     g.R32[0 * N + n] = u;
     g.R32[1 * N + n] = v;
     g.R32[2 * N + n] = w;
-    g.R32[3 * N + n] = sqrtf(rho);
+    g.R32[3 * N + n] = fsqrt(rho);
     g.R32[4 * N + n] = q4.h + (q4.l + pr);     // H = E/rho + p/rho
     float m[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
     const float prim[5] = {rho, u, v, w, p};
     float Fx[5], Ex[5], Gx[5];
-    node_inviscid_flux<float>(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
+    node_inviscid_flux(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         g.FEG32[(0 * 5 + c) * N + n] = Fx[c];
@@ -221,10 +221,12 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
     int i, j, k;
     lat_ijk(g, n, i, j, k);
     float dU[3][5], KS[3], Ui[5];
+    auto filtered = [](float a, float b, float c) { return fmaf(0.25f, a + c, __fmul_rn(0.5f, b)); };
     const bool ghost = LOC && lat_ghost(g, n);
     const unsigned lflag = (LOC && g.locflag) ? g.locflag[n] : 7u;
 #pragma unroll
     for (int c = 0; c < 5; ++c) Ui[c] = W[c * N + n];
+    const float r0 = frcp(Ui[0]);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int m2 = lat_step(g, i, j, k, d, -2), m1 = lat_step(g, i, j, k, d, -1), p1 = lat_step(g, i, j, k, d, 1),
@@ -239,7 +241,7 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
                 const float *H = W + c * N, *L = W + (5 + c) * N;
                 const float d1 = (__ldg(H + p1) - __ldg(H + m1)) + (__ldg(L + p1) - __ldg(L + m1));
                 const float d2 = (__ldg(H + p2) - __ldg(H + m2)) + (__ldg(L + p2) - __ldg(L + m2));
-                dU[d][c] = (1.0f / 12.0f) * (8.0f * d1 - d2);
+                dU[d][c] = __fmul_rn(1.0f / 12.0f, fmaf(8.0f, d1, -d2));
             }
         } else {
             int s[7], L7[7];
@@ -261,15 +263,15 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
         const int c = d + 1;
         const float um = __ldg(W + c * N + m1), up = __ldg(W + c * N + p1);
         const float rm = __ldg(W + m1), rp = __ldg(W + p1);
-        const float dlt = qdiv(Ui[c], Ui[0]) - qdiv(0.25f * um + 0.5f * Ui[c] + 0.25f * up, 0.25f * rm + 0.5f * Ui[0] + 0.25f * rp);
-        KS[d] = dlt * dlt;
+        const float dlt = fmaf(Ui[c], r0, -qdiv(filtered(um, Ui[c], up), filtered(rm, Ui[0], rp)));
+        KS[d] = fabsf(dlt);
     }
     float m[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
     const float prim[5] = {g.Q32[n], g.R32[n], g.R32[N + n], g.R32[2 * N + n], g.prim32[LF_P * N + n]};
     float Fv[5], Ev[5], Gv[5], mu;
-    viscous_node_flux<float>(dU, Ui, m, g.node32[9 * N + n], g.node32[10 * N + n], prim, KS, g.P, Fv, Ev, Gv, mu);
+    viscous_node_flux(dU, Ui, m, g.node32[9 * N + n], g.node32[10 * N + n], prim, KS, g.P, Fv, Ev, Gv, mu);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         g.V32[(0 * 5 + c) * N + n] = Fv[c];
@@ -287,7 +289,7 @@ __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
     const float uu = W[N + n] * iU0, vv = W[2 * N + n] * iU0, ww = W[3 * N + n] * iU0;
     const float mach = (float)g.P.mach;
     const float d_temp = 1.4f * mach * mach * 0.4f * (W[4 * N + n] * iU0 - 0.5f * (uu * uu + vv * vv + ww * ww));
-    const float sd = sqrtf(d_temp);
+    const float sd = fsqrt(d_temp);
     const float S = 110.4f / (float)g.P.t_inf;
     g.prim32[LF_MU * N + n] = (sd * sd * sd) * qdiv(1.0f + S, d_temp + S);
 }
@@ -312,7 +314,7 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     {
         const int l = s[2], rr = s[3];
         const float *R = g.R32;
-        roe_average<float>(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
+        roe_average(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
                            R[N + l], R[2 * N + l], R[4 * N + l], r);
     }
     float Fhat[5];
@@ -324,7 +326,7 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
         float f[6];
 #pragma unroll
         for (int o = 0; o < 6; ++o) f[o] = NF[c * N + s[o]];
-        g.Fh32[(D * 5 + c) * N + n] = Fhat[c] + x2::face_correction_sym(f);
+        g.Fh32[(D * 5 + c) * N + n] = __fadd_rn(Fhat[c], x2::face_correction_sym(f));
     }
 }
 
@@ -352,7 +354,7 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
     for (int q = 0; q < 5; ++q) {
         float f[6];
         tile_node_fluxes<T>(sF, q, t, a, f);
-        g.Fh32[(D * 5 + q) * N + n] = Fhat[q] + x2::face_correction_sym(f);
+        g.Fh32[(D * 5 + q) * N + n] = __fadd_rn(Fhat[q], x2::face_correction_sym(f));
     }
 }
 
@@ -415,8 +417,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
             for (int c = 0; c < 5; ++c)
-                Lf[c] += (1.0f / 12.0f) * (8.0f * (ld(Vd + c * N + p1) - ld(Vd + c * N + m1))
-                                           - (ld(Vd + c * N + p2) - ld(Vd + c * N + m2)));
+                Lf[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ld(Vd + c * N + p1) - ld(Vd + c * N + m1),
+                                                -(ld(Vd + c * N + p2) - ld(Vd + c * N + m2))), Lf[c]);
         }
     }
     if (g.Lout) {

@@ -67,9 +67,9 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const double Un[
 #pragma unroll
     for (int c = 0; c < 5; ++c) q[c] = emu::d2f(emu::mul(Un[c], id));
     const float rho = q[0];
-    const float ir = 1.0f / rho;
-    const float u = q[1] * ir, v = q[2] * ir, w = q[3] * ir;
-    const float p = 0.4f * (q[4] - 0.5f * (q[1] * u + q[2] * v + q[3] * w));
+    const float ir = frcp(rho);
+    const float u = __fmul_rn(q[1], ir), v = __fmul_rn(q[2], ir), w = __fmul_rn(q[3], ir);
+    const float p = __fmul_rn(0.4f, fmaf(-0.5f, dot3(q[1], u, q[2], v, q[3], w), q[4]));
     g.prim32[LF_P * N + n] = p;
     if (!(isfinite(rho) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(p))) atomicOr(g.flags, 2u);
 #pragma unroll
@@ -77,14 +77,14 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const double Un[
     g.R32[0 * N + n] = u;
     g.R32[1 * N + n] = v;
     g.R32[2 * N + n] = w;
-    g.R32[3 * N + n] = sqrtf(rho);
-    g.R32[4 * N + n] = (q[4] + p) * ir;   // H = (E + p) / rho
+    g.R32[3 * N + n] = fsqrt(rho);
+    g.R32[4 * N + n] = __fmul_rn(q[4] + p, ir);   // H = (E + p) / rho
     float m[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
     const float prim[5] = {rho, u, v, w, p};
     float Fx[5], Ex[5], Gx[5];
-    node_inviscid_flux<float>(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
+    node_inviscid_flux(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         g.FEG32[(0 * 5 + c) * N + n] = Fx[c];
@@ -166,7 +166,7 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     {
         const int l = s[2], rr = s[3];
         const float *R = g.R32;
-        roe_average<float>(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
+        roe_average(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
                            R[N + l], R[2 * N + l], R[4 * N + l], r);
     }
     const float *NF = g.FEG32 + (size_t)D * 5 * N;
@@ -270,8 +270,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
             for (int c = 0; c < 5; ++c)
-                Lv[c] += (1.0f / 12.0f) * (8.0f * (ldf(Vd + c * N + p1) - ldf(Vd + c * N + m1))
-                                           - (ldf(Vd + c * N + p2) - ldf(Vd + c * N + m2)));
+                Lv[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ldf(Vd + c * N + p1) - ldf(Vd + c * N + m1),
+                                                -(ldf(Vd + c * N + p2) - ldf(Vd + c * N + m2))), Lv[c]);
         }
     }
 #pragma unroll

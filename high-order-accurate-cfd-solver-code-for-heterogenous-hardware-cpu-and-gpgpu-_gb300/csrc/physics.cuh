@@ -13,89 +13,121 @@
 
 namespace cfd {
 
-// Quotient and reciprocal square root.  The float forms use the hardware
-// approximations (__fdividef: about 2 ulp for |b| < 2^126; rsqrtf); other
-// types compute them exactly.
+// Quotient, square root and its reciprocal.  The float forms are the
+// hardware approximations (about 2 ulp) with subnormal operands and results
+// taken as zero: the forms that keep subnormals scale their operand into
+// range and the result back, four instructions more at each of a face's 54
+// (physics_x2.cuh; a face direction of the split TGV 128^3 0.118 -> 0.107 ms).  Their operands here are
+// densities, sums with the WENO epsilon, sound speeds and metrics, none
+// within 2^-60 of that range.  Other types compute exactly.
+__device__ __forceinline__ float frcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float fsqrt(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float frsqrt(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 template <class T> __device__ __forceinline__ T qdiv(T a, T b) { return a / b; }
-template <> __device__ __forceinline__ float qdiv<float>(float a, float b) { return __fdividef(a, b); }
-template <class T> __device__ __forceinline__ T qrsqrt(T x) { return T(1) / sqrt(x); }
-template <> __device__ __forceinline__ float qrsqrt<float>(float x) { return rsqrtf(x); }
+template <> __device__ __forceinline__ float qdiv<float>(float a, float b) { return a * frcp(b); }
+template <class T> __device__ __forceinline__ T qsqrt(T x) { return sqrt(x); }
+template <> __device__ __forceinline__ float qsqrt<float>(float x) { return fsqrt(x); }
+
+// Sums of products with their contraction written out, so that every kernel
+// that evaluates a face (tiles of any shape, the batched stage) rounds it
+// alike: a b + c d, a b - c d, a b + c d + e f.
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float det2(float a, float b, float c, float d) { return fmaf(a, b, -__fmul_rn(c, d)); }
+__device__ __forceinline__ float dot3(float a, float b, float c, float d, float e, float f)
+{
+    return fmaf(a, b, dot2(c, d, e, f));
+}
 
 // Roe-averaged face state from the two adjacent nodes (U_Q.cl:60-109):
 // out = {u, v, w, h, rho}.  sb/hb belong to the neighbour, si/hi to the node.
-template <class T>
-__device__ __forceinline__ void roe_average(T sb, T ub, T vb, T wb, T hb, T si, T ui, T vi, T wi, T hi,
-                                            T out[5])
+__device__ __forceinline__ void roe_average(float sb, float ub, float vb, float wb, float hb, float si, float ui,
+                                            float vi, float wi, float hi, float out[5])
 {
-    const T iden = qdiv(T(1.0), sb + si);
-    out[4] = sb * si;
-    out[0] = (sb * ub + si * ui) * iden;
-    out[1] = (sb * vb + si * vi) * iden;
-    out[2] = (sb * wb + si * wi) * iden;
-    out[3] = (sb * hb + si * hi) * iden;
+    const float iden = frcp(sb + si);
+    out[4] = __fmul_rn(sb, si);
+    out[0] = __fmul_rn(dot2(sb, ub, si, ui), iden);
+    out[1] = __fmul_rn(dot2(sb, vb, si, vi), iden);
+    out[2] = __fmul_rn(dot2(sb, wb, si, wi), iden);
+    out[3] = __fmul_rn(dot2(sb, hb, si, hi), iden);
 }
 
 // Roe eigen-system of one face (Weno.cl:337-413): k_bar = grad(zeta)/|grad(zeta)|
 // from the face metric, sound speed from the Roe state, left (Lm) and right
 // (R) eigenvector matrices of the Euler flux Jacobian along k_bar.
-template <class T>
 struct FaceEigen {
-    T kx, ky, kz, a, alpha, beta, theta, phi, ru, rv, rw, rr, irr, ia2;
+    float kx, ky, kz, a, alpha, beta, theta, phi, ru, rv, rw, rr, irr, ia2;
 
-    __device__ __forceinline__ void init(T mx, T my, T mz, const T roe[5])
+    __device__ __forceinline__ void init(float mx, float my, float mz, const float roe[5])
     {
         ru = roe[0];
         rv = roe[1];
         rw = roe[2];
-        const T rh = roe[3];
+        const float rh = roe[3];
         rr = roe[4];
-        const T ikk = qrsqrt(mx * mx + my * my + mz * mz);
-        a = sqrt(T(0.4) * (rh - T(0.5) * (ru * ru + rv * rv + rw * rw)));
-        kx = mx * ikk;
-        ky = my * ikk;
-        kz = mz * ikk;
-        theta = kx * ru + ky * rv + kz * rw;
-        phi = T(0.5) * T(0.4) * (ru * ru + rv * rv + rw * rw);
-        const T is2 = T(0.70710678118654752);  // 1/sqrt(2.0)
-        const T ia = qdiv(T(1.0), a);
-        irr = qdiv(T(1.0), rr);
-        ia2 = ia * ia;
-        alpha = rr * ia * is2;
-        beta = irr * ia * is2;
+        const float ikk = frsqrt(dot3(mx, mx, my, my, mz, mz));
+        const float q2 = dot3(ru, ru, rv, rv, rw, rw);
+        a = fsqrt(__fmul_rn(0.4f, fmaf(-0.5f, q2, rh)));
+        kx = __fmul_rn(mx, ikk);
+        ky = __fmul_rn(my, ikk);
+        kz = __fmul_rn(mz, ikk);
+        theta = dot3(kx, ru, ky, rv, kz, rw);
+        phi = __fmul_rn(0.2f, q2);
+        const float is2 = 0.70710678118654752f;  // 1/sqrt(2.0)
+        const float ia = __fmul_rn(frcp(a), is2);
+        irr = frcp(rr);
+        ia2 = __fmul_rn(__fmul_rn(ia, ia), 2.0f);
+        alpha = __fmul_rn(rr, ia);
+        beta = __fmul_rn(irr, ia);
     }
 
     // Left eigenvectors, rows of l_eigen_Q (Weno.cl:384-412).
-    __device__ __forceinline__ void left(T Lm[5][5]) const
+    __device__ __forceinline__ void left(float Lm[5][5]) const
     {
-        const T ph = phi * ia2;
-        const T g2 = T(0.4) * ia2;
-        Lm[0][0] = kx * (T(1.0) - ph) - ((kz * rv - ky * rw) * irr);
-        Lm[0][1] = kx * g2 * ru;
-        Lm[0][2] = (kx * g2 * rv) + (kz * irr);
-        Lm[0][3] = (kx * g2 * rw) - (ky * irr);
-        Lm[0][4] = -kx * g2;
-        Lm[1][0] = ky * (T(1.0) - ph) - ((kx * rw - kz * ru) * irr);
-        Lm[1][1] = (ky * g2 * ru) - kz * irr;
-        Lm[1][2] = ky * g2 * rv;
-        Lm[1][3] = (ky * g2 * rw) + (kx * irr);
-        Lm[1][4] = -ky * g2;
-        Lm[2][0] = kz * (T(1.0) - ph) - ((ky * ru - kx * rv) * irr);
-        Lm[2][1] = kz * g2 * ru + (ky * irr);
-        Lm[2][2] = kz * g2 * rv - (kx * irr);
-        Lm[2][3] = kz * g2 * rw;
-        Lm[2][4] = -kz * g2;
-        Lm[3][0] = beta * (phi - theta * a);
-        Lm[3][1] = -beta * (T(0.4) * ru - kx * a);
-        Lm[3][2] = -beta * (T(0.4) * rv - ky * a);
-        Lm[3][3] = -beta * (T(0.4) * rw - kz * a);
-        Lm[3][4] = beta * T(0.4);
-        Lm[4][0] = beta * (phi + theta * a);
-        Lm[4][1] = -beta * (T(0.4) * ru + kx * a);
-        Lm[4][2] = -beta * (T(0.4) * rv + ky * a);
-        Lm[4][3] = -beta * (T(0.4) * rw + kz * a);
-        Lm[4][4] = beta * T(0.4);
+        const float g2 = __fmul_rn(0.4f, ia2), omf = fmaf(-phi, ia2, 1.0f);
+        const float gx = __fmul_rn(kx, g2), gy = __fmul_rn(ky, g2), gz = __fmul_rn(kz, g2);
+        const float ix = __fmul_rn(kx, irr), iy = __fmul_rn(ky, irr), iz = __fmul_rn(kz, irr);
+        Lm[0][0] = fmaf(kx, omf, -det2(iz, rv, iy, rw));
+        Lm[0][1] = __fmul_rn(gx, ru);
+        Lm[0][2] = fmaf(gx, rv, iz);
+        Lm[0][3] = fmaf(gx, rw, -iy);
+        Lm[0][4] = -gx;
+        Lm[1][0] = fmaf(ky, omf, -det2(ix, rw, iz, ru));
+        Lm[1][1] = fmaf(gy, ru, -iz);
+        Lm[1][2] = __fmul_rn(gy, rv);
+        Lm[1][3] = fmaf(gy, rw, ix);
+        Lm[1][4] = -gy;
+        Lm[2][0] = fmaf(kz, omf, -det2(iy, ru, ix, rv));
+        Lm[2][1] = fmaf(gz, ru, iy);
+        Lm[2][2] = fmaf(gz, rv, -ix);
+        Lm[2][3] = __fmul_rn(gz, rw);
+        Lm[2][4] = -gz;
+        const float b4 = __fmul_rn(0.4f, beta), ba = __fmul_rn(beta, a), bp = __fmul_rn(beta, phi);
+        Lm[3][0] = fmaf(-ba, theta, bp);
+        Lm[3][1] = fmaf(-b4, ru, __fmul_rn(ba, kx));
+        Lm[3][2] = fmaf(-b4, rv, __fmul_rn(ba, ky));
+        Lm[3][3] = fmaf(-b4, rw, __fmul_rn(ba, kz));
+        Lm[3][4] = b4;
+        Lm[4][0] = fmaf(ba, theta, bp);
+        Lm[4][1] = fmaf(-b4, ru, -__fmul_rn(ba, kx));
+        Lm[4][2] = fmaf(-b4, rv, -__fmul_rn(ba, ky));
+        Lm[4][3] = fmaf(-b4, rw, -__fmul_rn(ba, kz));
+        Lm[4][4] = b4;
     }
-
 };
 
 // Branch selection of the location-code-driven first derivative of the
@@ -168,127 +200,117 @@ struct Phys {
 };
 
 // Viscous and SGS fluxes at one node from the derivatives of U along the
-// three directions (Viscous.cl:439-631), FMA-friendly rewrite for the
-// mixed-precision form (T = float there).  dU[d][c]: derivative of U_c along
-// direction d; Ui: U at the node; m: node metrics (9); det: node det;
-// DEL: the filter width det^(-1/3); prim: rho,u,v,w,p of FLOW at the node;
-// KS: the three MTS test-filter velocity-difference squares.  Writes
-// contravariant Fv/Ev/Gv (x det) and mu.
-template <class T>
-__device__ __forceinline__ void viscous_node_flux(const T dU[3][5], const T Ui[5], const T m[9], T det, T DEL,
-                                                  const T prim[5], const T KS[3], const Phys &P, T Fv[5], T Ev[5],
-                                                  T Gv[5], T &mu_out)
+// three directions (Viscous.cl:439-631) in FP32, contraction written out
+// (as for the face).  dU[d][c]: derivative of U_c along direction d; Ui: U
+// at the node; m: node metrics (9); det: node det; DEL: the filter width
+// det^(-1/3); prim: rho,u,v,w,p of FLOW at the node; KS: the magnitudes of
+// the three MTS test-filter velocity differences (the roots of the
+// reference's KS).  Writes contravariant Fv/Ev/Gv (x det) and mu.
+__device__ __forceinline__ void viscous_node_flux(const float dU[3][5], const float Ui[5], const float m[9], float det,
+                                                  float DEL, const float prim[5], const float KS[3], const Phys &P,
+                                                  float Fv[5], float Ev[5], float Gv[5], float &mu_out)
 {
-    const T Mach = (T)P.mach, Reyl = (T)P.reynolds, Pr = (T)P.prandtl, Free_t = (T)P.t_inf;
-    const T U0 = Ui[0], U1 = Ui[1], U2 = Ui[2], U3 = Ui[3], U4 = Ui[4];
-    const T iU0 = qdiv(T(1.0), U0);
-    const T iU00 = iU0 * iU0;
-    T uc[3], vc[3], wc[3], tc[3];
+    auto mul = [](float a, float b) { return __fmul_rn(a, b); };
+    const float Mach = (float)P.mach, Reyl = (float)P.reynolds, Pr = (float)P.prandtl, Free_t = (float)P.t_inf;
+    const float iU0 = frcp(Ui[0]);
+    const float uu = mul(Ui[1], iU0), vv = mul(Ui[2], iU0), ww = mul(Ui[3], iU0), ee = mul(Ui[4], iU0);
+    float uc[3], vc[3], wc[3], tc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        uc[d] = iU0 * dU[d][1] - (U1 * iU00) * dU[d][0];
-        vc[d] = iU0 * dU[d][2] - (U2 * iU00) * dU[d][0];
-        wc[d] = iU0 * dU[d][3] - (U3 * iU00) * dU[d][0];
+        uc[d] = mul(iU0, fmaf(-uu, dU[d][0], dU[d][1]));
+        vc[d] = mul(iU0, fmaf(-vv, dU[d][0], dU[d][2]));
+        wc[d] = mul(iU0, fmaf(-ww, dU[d][0], dU[d][3]));
+        tc[d] = fmaf(iU0, fmaf(-ee, dU[d][0], dU[d][4]), -dot3(uu, uc[d], vv, vc[d], ww, wc[d]));
     }
-    const T uu = U1 * iU0, vv = U2 * iU0, ww = U3 * iU0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-        tc[d] = iU0 * dU[d][4] - (U4 * iU00) * dU[d][0] - uu * uc[d] - vv * vc[d] - ww * wc[d];
-
     // Sutherland's law with T = gamma M^2 (gamma-1) e (Viscous.cl:451-458)
-    const T d_temp = (T(1.4) * Mach * Mach * T(0.4) * ((U4 * iU0) - T(0.5) * (uu * uu + vv * vv + ww * ww)));
-    const T sd = sqrt(d_temp);
-    const T S = T(110.4) / Free_t;
-    const T mu = (sd * sd * sd) * qdiv(T(1.0) + S, d_temp + S);
+    const float d_temp = mul(1.4f * 0.4f * Mach * Mach, fmaf(-0.5f, dot3(uu, uu, vv, vv, ww, ww), ee));
+    const float sd = fsqrt(d_temp);
+    const float S = qdiv(110.4f, Free_t);
+    const float mu = mul(mul(mul(sd, sd), sd), qdiv(1.0f + S, d_temp + S));
     mu_out = mu;
-
-    const T zx = m[0], zy = m[1], zz = m[2], ex = m[3], ey = m[4], ez = m[5], xx = m[6], xy = m[7], xz = m[8];
-    const T dudx = uc[0] * zx + uc[1] * ex + uc[2] * xx, dudy = uc[0] * zy + uc[1] * ey + uc[2] * xy,
-            dudz = uc[0] * zz + uc[1] * ez + uc[2] * xz;
-    const T dvdx = vc[0] * zx + vc[1] * ex + vc[2] * xx, dvdy = vc[0] * zy + vc[1] * ey + vc[2] * xy,
-            dvdz = vc[0] * zz + vc[1] * ez + vc[2] * xz;
-    const T dwdx = wc[0] * zx + wc[1] * ex + wc[2] * xx, dwdy = wc[0] * zy + wc[1] * ey + wc[2] * xy,
-            dwdz = wc[0] * zz + wc[1] * ez + wc[2] * xz;
-    const T dtdx = tc[0] * zx + tc[1] * ex + tc[2] * xx, dtdy = tc[0] * zy + tc[1] * ey + tc[2] * xy,
-            dtdz = tc[0] * zz + tc[1] * ez + tc[2] * xz;
-
-    const T kq = -(mu * T(1.4) * qdiv(T(1.0), Pr * Reyl));
-    const T qx_ = kq * dtdx, qy_ = kq * dtdy, qz_ = kq * dtdz;   // Viscous.cl:461-463
-    const T mr = mu * qdiv(T(1.0), Reyl);                                       // Viscous.cl:466-476
-    const T txx = mr * (T(4.0 / 3.0) * dudx - T(2.0 / 3.0) * dvdy - T(2.0 / 3.0) * dwdz);
-    const T tyy = mr * (T(4.0 / 3.0) * dvdy - T(2.0 / 3.0) * dudx - T(2.0 / 3.0) * dwdz);
-    const T tzz = mr * (T(4.0 / 3.0) * dwdz - T(2.0 / 3.0) * dudx - T(2.0 / 3.0) * dvdy);
-    const T sxy = dudy + dvdx, sxz = dudz + dwdx, syz = dvdz + dwdy;
-    const T txy = mr * sxy, txz = mr * sxz, tyz = mr * syz;
-
-    T TXY = 0, TYZ = 0, TXZ = 0, TXX = 0, TYY = 0, TZZ = 0, HX = 0, HY = 0, HZ = 0, DX = 0, DY = 0, DZ = 0;
+    float gu[3], gv[3], gw[3], gt[3];   // gradients along x, y, z
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        gu[x] = dot3(uc[0], m[x], uc[1], m[3 + x], uc[2], m[6 + x]);
+        gv[x] = dot3(vc[0], m[x], vc[1], m[3 + x], vc[2], m[6 + x]);
+        gw[x] = dot3(wc[0], m[x], wc[1], m[3 + x], wc[2], m[6 + x]);
+        gt[x] = dot3(tc[0], m[x], tc[1], m[3 + x], tc[2], m[6 + x]);
+    }
+    const float sxy = gu[1] + gv[0], sxz = gu[2] + gw[0], syz = gv[2] + gw[1];
+    const float kq = -mul(mul(mu, 1.4f), qdiv(1.0f, Pr * Reyl));   // Viscous.cl:461-463
+    const float mr = mul(mu, qdiv(1.0f, Reyl));                    // Viscous.cl:466-476
+    const float trace = mul(-2.0f / 3.0f, gu[0] + gv[1] + gw[2]);
+    // stress and heat flux, the molecular part; the SGS part is added below
+    float txx = -mul(mr, fmaf(2.0f, gu[0], trace)), tyy = -mul(mr, fmaf(2.0f, gv[1], trace)),
+          tzz = -mul(mr, fmaf(2.0f, gw[2], trace));
+    float txy = -mul(mr, sxy), txz = -mul(mr, sxz), tyz = -mul(mr, syz);
+    const float u = prim[1], v = prim[2], w = prim[3];
+    float ex = fmaf(kq, gt[0], dot3(u, txx, v, txy, w, txz)), ey = fmaf(kq, gt[1], dot3(u, txy, v, tyy, w, tyz)),
+          ez = fmaf(kq, gt[2], dot3(u, txz, v, tyz, w, tzz));
     if (P.les) {  // SGS model: mixed time scale (Viscous.cl:490-558) or Smagorinsky
-        const T C_MTS = T(0.03), C_T = T(10.0);
-        const T s_xy = T(0.5) * sxy, s_yz = T(0.5) * syz, s_xz = T(0.5) * sxz;
-        T ed[3];
+        const float C_MTS = 0.03f, iC_T = 0.1f;
+        const float off = mul(0.25f, dot3(sxy, sxy, syz, syz, sxz, sxz));   // sum of (s_ij / 2)^2
+        const float dia = dot3(gu[0], gu[0], gv[1], gv[1], gw[2], gw[2]);
+        float ed[3];
         if (P.les == 2) {   // (C_s Delta)^2 |S|, |S| = sqrt(2 S_ij S_ij), Delta = det^(1/3) = 1/DEL
-            const T S = sqrt(T(2.0) * (dudx * dudx + dvdy * dvdy + dwdz * dwdz)
-                             + T(4.0) * (s_xy * s_xy + s_yz * s_yz + s_xz * s_xz));
-            const T ls = qdiv(T(P.cs), DEL);
-            ed[0] = ed[1] = ed[2] = (ls * ls) * S;
+            const float ls = qdiv((float)P.cs, DEL);
+            ed[0] = ed[1] = ed[2] = mul(mul(ls, ls), fsqrt(dot2(2.0f, dia, 4.0f, off)));
         } else {
-            const T mod = sqrt(T(2.0) * ((s_xy * s_xy + s_yz * s_yz + s_xz * s_xz)
-                                         + T(2.0 / 3.0) * (dudx * dudx + dvdy * dvdy + dwdz * dwdz)));
+            const float mod = fsqrt(mul(2.0f, fmaf(2.0f / 3.0f, dia, off)));
+            const float dm = mul(DEL, mod), cd = mul(C_MTS, DEL);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                const T sk = sqrt(KS[d]);
-                if (mod != T(0.0)) {
-                    const T R = qdiv(DEL * mod, sk);
-                    ed[d] = qdiv(C_MTS, T(1.0) + R * (T(1.0) / C_T)) * DEL * sk;
-                } else {
-                    ed[d] = C_MTS * DEL * sk;
-                }
+                const float sk = KS[d];
+                const float e0 = mul(cd, sk);
+                ed[d] = mod != 0.0f ? mul(frcp(fmaf(qdiv(dm, sk), iC_T, 1.0f)), e0) : e0;
             }
         }
-        const T r2 = T(-2.0) * U0;
-        TXY = r2 * ed[0] * s_xy;
-        TYZ = r2 * ed[1] * s_yz;
-        TXZ = r2 * ed[2] * s_xz;
-        TXX = r2 * ed[0] * dudx;
-        TYY = r2 * ed[1] * dvdy;
-        TZZ = r2 * ed[2] * dwdz;
-        const T kQ = -qdiv(T(1.0), T(1.4) * T(0.4) * Mach * Mach);
-        const T Qx = kQ * ed[0] * dtdx, Qy = kQ * ed[1] * dtdy, Qz = kQ * ed[2] * dtdz;
-        HX = Qx + (TXX + TXY + TXZ) * prim[1];
-        HY = Qy + (TXY + TYY + TYZ) * prim[2];
-        HZ = Qz + (TXZ + TYZ + TZZ) * prim[3];
-        DX = T(0.4) * Qx;
-        DY = T(0.4) * Qy;
-        DZ = T(0.4) * Qz;
+        const float r2 = mul(-2.0f, Ui[0]);
+        const float r0 = mul(r2, ed[0]), r1 = mul(r2, ed[1]), rz = mul(r2, ed[2]);
+        const float TXY = mul(r0, mul(0.5f, sxy)), TYZ = mul(r1, mul(0.5f, syz)), TXZ = mul(rz, mul(0.5f, sxz));
+        const float TXX = mul(r0, gu[0]), TYY = mul(r1, gv[1]), TZZ = mul(rz, gw[2]);
+        const float kQ = mul(-1.4f, qdiv(1.0f, 1.4f * 0.4f * Mach * Mach));   // Q and its 0.4 Q share
+        ex += fmaf(mul(kQ, ed[0]), gt[0], mul(TXX + TXY + TXZ, u));
+        ey += fmaf(mul(kQ, ed[1]), gt[1], mul(TXY + TYY + TYZ, v));
+        ez += fmaf(mul(kQ, ed[2]), gt[2], mul(TXZ + TYZ + TZZ, w));
+        txx += TXX;
+        tyy += TYY;
+        tzz += TZZ;
+        txy += TXY;
+        txz += TXZ;
+        tyz += TYZ;
     }
-    const T u = prim[1], v = prim[2], w = prim[3];
-    // Cartesian viscous fluxes, Viscous.cl:580-596
-    const T tFv[5] = {T(0), -txx + TXX, -txy + TXY, -txz + TXZ, ((-u * txx - v * txy - w * txz) + qx_ + HX + DX)};
-    const T tEv[5] = {T(0), -txy + TXY, -tyy + TYY, -tyz + TYZ, ((-u * txy - v * tyy - w * tyz) + qy_ + HY + DY)};
-    const T tGv[5] = {T(0), -txz + TXZ, -tyz + TYZ, -tzz + TZZ, ((-u * txz - v * tyz - w * tzz) + qz_ + HZ + DZ)};
+    // Cartesian viscous fluxes, Viscous.cl:580-596, through the metrics
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        Fv[c] = det * (zx * tFv[c] + zy * tEv[c] + zz * tGv[c]);
-        Ev[c] = det * (ex * tFv[c] + ey * tEv[c] + ez * tGv[c]);
-        Gv[c] = det * (xx * tFv[c] + xy * tEv[c] + xz * tGv[c]);
+    for (int d = 0; d < 3; ++d) {
+        float *o = d == 0 ? Fv : (d == 1 ? Ev : Gv);
+        const float mx = mul(det, m[3 * d]), my = mul(det, m[3 * d + 1]), mz = mul(det, m[3 * d + 2]);
+        o[0] = 0.0f;
+        o[1] = dot3(mx, txx, my, txy, mz, txz);
+        o[2] = dot3(mx, txy, my, tyy, mz, tyz);
+        o[3] = dot3(mx, txz, my, tyz, mz, tzz);
+        o[4] = dot3(mx, ex, my, ey, mz, ez);
     }
 }
 
 // Contravariant node inviscid fluxes F, E, G (x det) from the primitives,
-// Viscous.cl:560-578 and 615-631 (FMA-friendly, mixed form).
-template <class T>
-__device__ __forceinline__ void node_inviscid_flux(const T prim[5], const T m[9], T det, T F[5], T E[5], T G[5])
+// Viscous.cl:560-578 and 615-631, in FP32: det (m_d . U) q + p det m_d.
+__device__ __forceinline__ void node_inviscid_flux(const float prim[5], const float m[9], float det, float F[5],
+                                                   float E[5], float G[5])
 {
-    const T rho = prim[0], u = prim[1], v = prim[2], w = prim[3], p = prim[4];
-    const T Et = (p * T(2.5) + T(0.5) * rho * (u * u + v * v + w * w)) + p;
-    const T tF[5] = {rho * u, rho * u * u + p, rho * v * u, rho * u * w, Et * u};
-    const T tE[5] = {rho * v, rho * v * u, rho * v * v + p, rho * v * w, Et * v};
-    const T tG[5] = {rho * w, rho * u * w, rho * v * w, rho * w * w + p, Et * w};
+    const float rho = prim[0], u = prim[1], v = prim[2], w = prim[3], p = prim[4];
+    const float ke = __fmul_rn(__fmul_rn(0.5f, rho), dot3(u, u, v, v, w, w));
+    const float Et = fmaf(p, 3.5f, ke);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        F[c] = det * (m[0] * tF[c] + m[1] * tE[c] + m[2] * tG[c]);
-        E[c] = det * (m[3] * tF[c] + m[4] * tE[c] + m[5] * tG[c]);
-        G[c] = det * (m[6] * tF[c] + m[7] * tE[c] + m[8] * tG[c]);
+    for (int d = 0; d < 3; ++d) {
+        float *o = d == 0 ? F : (d == 1 ? E : G);
+        const float mx = __fmul_rn(det, m[3 * d]), my = __fmul_rn(det, m[3 * d + 1]), mz = __fmul_rn(det, m[3 * d + 2]);
+        const float un = dot3(mx, u, my, v, mz, w), ru = __fmul_rn(rho, un);
+        o[0] = ru;
+        o[1] = dot2(ru, u, mx, p);
+        o[2] = dot2(ru, v, my, p);
+        o[3] = dot2(ru, w, mz, p);
+        o[4] = __fmul_rn(Et, un);
     }
 }
 

@@ -26,7 +26,7 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, b2(-1.0f), a); }
 __device__ __forceinline__ float2 swap2(float2 a) { return make_float2(a.y, a.x); }
-__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(frcp(a.x), frcp(a.y)); }
 
 // Jiang-Shu smoothness indicator of a three-point stencil from its two
 // differences t (second) and u (first-derivative form): 13/12 t^2 + 1/4 u^2
@@ -56,24 +56,23 @@ __device__ __forceinline__ float2 weno5_pos2(const float2 c[6], float eps)
 }
 
 // q = R c on both lanes (R: right eigenvectors of the face, Weno.cl:349-380)
-__device__ __forceinline__ void right_times2(const FaceEigen<float> &eg, const float2 c[5], float2 q[5])
+__device__ __forceinline__ void right_times2(const FaceEigen &eg, const float2 c[5], float2 q[5])
 {
     const float kx = eg.kx, ky = eg.ky, kz = eg.kz, al = eg.alpha, a = eg.a, ru = eg.ru, rv = eg.rv, rw = eg.rw,
                 rr = eg.rr, th = eg.theta;
-    const float e0 = (eg.phi + a * a) * 2.5f, ph5 = eg.phi * 2.5f;
+    const float ph5 = __fmul_rn(eg.phi, 2.5f), e0 = fmaf(__fmul_rn(a, a), 2.5f, ph5), ala = __fmul_rn(al, a);
+    const float nx = __fmul_rn(kx, rr), ny = __fmul_rn(ky, rr), nz = __fmul_rn(kz, rr);
     const float2 s34 = add2(c[3], c[4]), d34 = sub2(c[3], c[4]);
+    auto row = [&](float r0, float r1, float r2, float rs, float rd) {
+        return fma2(b2(r0), c[0], fma2(b2(r1), c[1], fma2(b2(r2), c[2], fma2(b2(rs), s34, mul2(b2(rd), d34)))));
+    };
     q[0] = fma2(b2(kx), c[0], fma2(b2(ky), c[1], fma2(b2(kz), c[2], mul2(b2(al), s34))));
     // alpha (ru + kx a) c3 + alpha (ru - kx a) c4 = alpha ru (c3 + c4) + alpha kx a (c3 - c4)
-    q[1] = fma2(b2(kx * ru), c[0], fma2(b2(ky * ru - kz * rr), c[1], fma2(b2(kz * ru + ky * rr), c[2],
-                fma2(b2(al * ru), s34, mul2(b2(al * kx * a), d34)))));
-    q[2] = fma2(b2(kx * rv + kz * rr), c[0], fma2(b2(ky * rv), c[1], fma2(b2(kz * rv - kx * rr), c[2],
-                fma2(b2(al * rv), s34, mul2(b2(al * ky * a), d34)))));
-    q[3] = fma2(b2(kx * rw - ky * rr), c[0], fma2(b2(ky * rw + kx * rr), c[1], fma2(b2(kz * rw), c[2],
-                fma2(b2(al * rw), s34, mul2(b2(al * kz * a), d34)))));
-    q[4] = fma2(b2(kx * ph5 + rr * (kz * rv - ky * rw)), c[0],
-                fma2(b2(ky * ph5 + rr * (kx * rw - kz * ru)), c[1],
-                     fma2(b2(kz * ph5 + rr * (ky * ru - kx * rv)), c[2],
-                          fma2(b2(al * e0), s34, mul2(b2(al * th * a), d34)))));
+    q[1] = row(__fmul_rn(kx, ru), fmaf(ky, ru, -nz), fmaf(kz, ru, ny), __fmul_rn(al, ru), __fmul_rn(ala, kx));
+    q[2] = row(fmaf(kx, rv, nz), __fmul_rn(ky, rv), fmaf(kz, rv, -nx), __fmul_rn(al, rv), __fmul_rn(ala, ky));
+    q[3] = row(fmaf(kx, rw, -ny), fmaf(ky, rw, nx), __fmul_rn(kz, rw), __fmul_rn(al, rw), __fmul_rn(ala, kz));
+    q[4] = row(fmaf(kx, ph5, det2(nz, rv, ny, rw)), fmaf(ky, ph5, det2(nx, rw, nz, ru)),
+               fmaf(kz, ph5, det2(ny, ru, nx, rv)), __fmul_rn(al, e0), __fmul_rn(ala, th));
 }
 
 // Contravariant Euler flux of the face states on both lanes through the face
@@ -92,8 +91,8 @@ __device__ __forceinline__ float2 contravariant_flux2(const float2 q[5], float m
     f[3] = fma2(q[3], un, mul2(b2(mz), pr));
     f[4] = mul2(hq, un);
     const float2 e = fma2(q[4], ir, mul2(b2(-0.5f), fma2(u, u, fma2(v, v, mul2(w, w)))));
-    const float2 c2k = mul2(b2(1.4f * 0.4f * (mx * mx + my * my + mz * mz)), e);
-    return add2(un, make_float2(sqrtf(c2k.x), sqrtf(c2k.y)));
+    const float2 c2k = mul2(b2(__fmul_rn(1.4f * 0.4f, dot3(mx, mx, my, my, mz, mz))), e);
+    return add2(un, make_float2(fsqrt(c2k.x), fsqrt(c2k.y)));
 }
 
 // Reconstructed face states of one face on the two lanes, (pos, neg):
@@ -111,7 +110,7 @@ template <bool DEV = false>
 __device__ __forceinline__ void reconstruct_face2(const float2 P[3][5], float mx, float my, float mz,
                                                   const float roe[5], float eps, const float *ref, float2 q[5])
 {
-    FaceEigen<float> eg;
+    FaceEigen eg;
     eg.init(mx, my, mz, roe);
     float2 C[5];   // (pos, neg) of each characteristic variable
     {
@@ -150,10 +149,11 @@ __device__ __forceinline__ void llf_face_flux2(const float2 P[3][5], float mx, f
     const float2 lam = contravariant_flux2(q, mx, my, mz, f);
     const float alpha = fmaxf(fabsf(lam.x), fabsf(lam.y));
     const float2 sa = make_float2(-alpha, alpha);
+    const float hd = 0.5f * det_f;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         const float2 t = fma2(sa, q[c], f[c]);
-        Fhat[c] = (0.5f * det_f) * (t.x + t.y);
+        Fhat[c] = __fmul_rn(hd, t.x + t.y);
     }
 }
 
@@ -185,8 +185,8 @@ __device__ __forceinline__ void llf_face_flux2_split(const float2 P[3][5], float
     // lambda_5 = U.m + c |m| in FP32 (the LLF speed)
     const float2 un32 = fma2(b2(mx), u, fma2(b2(my), v, mul2(b2(mz), w)));
     const float2 e = fma2(q[4], ir, mul2(b2(-0.5f), fma2(u, u, fma2(v, v, mul2(w, w)))));
-    const float2 c2k = mul2(b2(1.4f * 0.4f * (mx * mx + my * my + mz * mz)), e);
-    const float2 lam = add2(un32, make_float2(sqrtf(c2k.x), sqrtf(c2k.y)));
+    const float2 c2k = mul2(b2(__fmul_rn(1.4f * 0.4f, dot3(mx, mx, my, my, mz, mz))), e);
+    const float2 lam = add2(un32, make_float2(fsqrt(c2k.x), fsqrt(c2k.y)));
     const float alpha = fmaxf(fabsf(lam.x), fabsf(lam.y));
     const double hd = 0.5 * det_f;
     const float hd32 = emu::d2f(hd);
@@ -198,7 +198,7 @@ __device__ __forceinline__ void llf_face_flux2_split(const float2 P[3][5], float
     for (int c = 0; c < 5; ++c) {
         const float qp = c == 4 ? q[4].x + pr.x : q[c].x, qn = c == 4 ? q[4].y + pr.y : q[c].y;
         qs[c] = qp + qn;
-        x[c] = fmaf(hd32, fmaf(0.5f * (qp - qn), dun, -alpha * (q[c].x - q[c].y)), extra[c]);
+        x[c] = fmaf(hd32, fmaf(__fmul_rn(0.5f, qp - qn), dun, -__fmul_rn(alpha, q[c].x - q[c].y)), extra[c]);
     }
     // FP64: the metric products of the sum term and of the pressure (the
     // FP32 -> FP64 conversions on the integer pipe, emu::f2d: exact)

@@ -57,8 +57,9 @@ __global__ void __launch_bounds__(256) k_mu_s(LatView g)
     if (n < g.N) mx::mu_node(g, n, 0);
 }
 
+// 64 registers: a direction at 128^3 0.102-0.107 ms, 0.105-0.109 at 80.
 #ifndef CFD_SFACE_MIN_BLOCKS
-#define CFD_SFACE_MIN_BLOCKS 6
+#define CFD_SFACE_MIN_BLOCKS 8
 #endif
 // One instance per candidate tile width (face_tile.cuh): faces along i of
 // 32, 64 or 128, along j or k of 8, 16 or 32; the solver times them when it
