@@ -22,7 +22,7 @@ namespace cfd {
 namespace {
 
 struct Ops {
-    static __device__ __forceinline__ void prep(const LatView &g, int n, int q) { ex::prep_node(g, n, q); }
+    static __device__ __forceinline__ void prep(const LatView &g, int n, int q) { ex::prep_node<true>(g, n, q); }
 };
 
 __global__ void __launch_bounds__(256, 2) k_batch_visc(const LatView *__restrict__ views,
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_visc(const LatView *__restrict
     const BatchTile t = tiles[blockIdx.x];
     if ((int)threadIdx.x >= t.count) return;
     const LatView &g = views[t.inst];
-    if (g.P.viscous) ex::visc_node(g, t.n0 + threadIdx.x, jst);
+    if (g.P.viscous) ex::visc_node<true>(g, t.n0 + threadIdx.x, jst);
     else ex::mu_node(g, t.n0 + threadIdx.x, jst);
 }
 
@@ -96,7 +96,7 @@ k_batch_close(const LatView *__restrict__ views, const BatchTile *__restrict__ t
     if (!grid_barrier(bar, gridDim.x, limit_ns, gflags)) return;
     for (int w = blockIdx.x; w < ntiles; w += gridDim.x) {
         const BatchTile t = tiles[w];
-        if ((int)threadIdx.x < t.count) ex::update_node(views[t.inst], t.n0 + threadIdx.x, jst, true);
+        if ((int)threadIdx.x < t.count) ex::update_node<true>(views[t.inst], t.n0 + threadIdx.x, jst, true);
     }
 }
 

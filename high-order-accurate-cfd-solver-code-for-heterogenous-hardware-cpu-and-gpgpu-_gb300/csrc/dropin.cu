@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) k_uq_node(const double *__restrict__ flow
     const double rho = f[FRHO], u = f[FU], v = f[FV], w = f[FW];
     const double s = xi::root(rho), x[4] = {u, v, w, ex::enthalpy(rho, u, v, w, f[FP])};
     double sx[4];
-    ex::scaled(s, x, sx);
+    ex::scaled<true>(s, x, sx);
     double *o = sh + 5 * (size_t)row;
     o[0] = s;
 #pragma unroll
@@ -186,9 +186,9 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
     xi::sq_n(s);
     const double E = ex::dv(p, 0.4) + xi::mul(xdiv::scale2<-1>(rho), s[0] + s[1] + s[2]);   // 0.5 rho: same bits
     const double re[2] = {rho, E};
-    ex::scaled(rho, vel, q);
-    ex::scaled(D, re, d2);
-    ex::scaled(d2[0], vel, du);
+    ex::scaled<true>(rho, vel, q);
+    ex::scaled<true>(D, re, d2);
+    ex::scaled<true>(d2[0], vel, du);
     double *Ur = U + 5 * (size_t)gid, *Qr = Q + 5 * (size_t)gid;
     Ur[0] = d2[0];
     Ur[1] = du[0];
@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
 // Viscous.cl:23-643.
 // The inviscid node fluxes and the filter width of every row (their own
 // kernel: beside the viscous fluxes they would spill).
+template <bool I>
 __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, double *__restrict__ E,
                                                       double *__restrict__ G, const double *__restrict__ metric,
                                                       const double *__restrict__ det, const double *__restrict__ flow,
@@ -214,19 +215,12 @@ __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, do
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= n_items) return;
     const double D = det[gid];
-    double m[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) m[k] = metric[63 * (size_t)gid + k];
+    const double *m = metric + 63 * (size_t)gid;
     const double *fr = flow + 9 * (size_t)gid;
     const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
-    double Fn[5], En[5], Gn[5], Qn[5], H;
-    ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        F[5 * (size_t)gid + c] = Fn[c];
-        E[5 * (size_t)gid + c] = En[c];
-        G[5 * (size_t)gid + c] = Gn[c];
-    }
+    double Qn[5], H;
+    ex::node_flux<I>(prim, [&](int k) { return m[k]; }, D,
+                  [&](int e, int c, double f) { (e == 0 ? F : (e == 1 ? E : G))[5 * (size_t)gid + c] = f; }, Qn, H);
     if (les) width[gid] = ex::filter_width(D);
 }
 
@@ -235,7 +229,7 @@ __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, do
 // callers without the scratch.  TGV 96^3, both kernels: 1.00 ms at 3 or 4
 // blocks per SM, 1.19 at 5; in one kernel 1.17 at 3, 1.38 at 4 (3 KB of spill
 // loads per thread).
-template <bool NODE>
+template <bool NODE, bool I>
 __global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
                                                  double *__restrict__ E, double *__restrict__ G,
                                                  double *__restrict__ Fv, double *__restrict__ Ev,
@@ -253,23 +247,16 @@ __global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__rest
             return;
         }
     }
-    double m[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) m[k] = metric[63 * (size_t)gid + k];
+    const double *m = metric + 63 * (size_t)gid;
     const double D = det[gid];
     const double *fr = flow + 9 * (size_t)gid;
     const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
+    auto metric_at = [&](int k) { return m[k]; };
     if (NODE) {
-        double Fn[5], En[5], Gn[5], Qn[5], H;
-        ex::node_flux(prim, m, D, Fn, En, Gn, Qn, H);
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            F[5 * (size_t)gid + c] = Fn[c];
-            E[5 * (size_t)gid + c] = En[c];
-            G[5 * (size_t)gid + c] = Gn[c];
-        }
+        double Qn[5], H;
+        ex::node_flux<I>(prim, metric_at, D,
+                      [&](int e, int c, double f) { (e == 0 ? F : (e == 1 ? E : G))[5 * (size_t)gid + c] = f; }, Qn, H);
     }
-    double Fvn[5], Evn[5], Gvn[5];
     double mu;
     {
         // the star is walked again for each direction (it is cached by now):
@@ -281,7 +268,7 @@ __global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__rest
             for (int o = 0; o < 7; ++o) L[o] = grid_loc(grid, s[o]);
             const int b = visc_branch(L);
             if (b == 5) {
-                ex::central4([&](int o, int c) { return U[5 * (size_t)s[o + 3] + c]; }, out);
+                ex::central4<I>([&](int o, int c) { return U[5 * (size_t)s[o + 3] + c]; }, out);
                 return;
             }
 #pragma unroll
@@ -298,14 +285,11 @@ __global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__rest
                          *up = U + 5 * (size_t)grid_nb(grid, gid, plus_slot(d));
             KS[d] = P.les && P.les != 2 ? ex::ks_root(Ui[c], Ui[0], um[c], um[0], up[c], up[0]) : 0.0;
         }
-        ex::viscous_node(dU, Ui, m, D, NODE ? ex::filter_width(D) : width[gid], prim, KS, P, Fvn, Evn, Gvn, mu);
-    }
-    double *o;
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        o = Fv + 5 * (size_t)gid; o[c] = P.viscous ? Fvn[c] : 0.0;
-        o = Ev + 5 * (size_t)gid; o[c] = P.viscous ? Evn[c] : 0.0;
-        o = Gv + 5 * (size_t)gid; o[c] = P.viscous ? Gvn[c] : 0.0;
+        ex::viscous_node<I>(dU, Ui, metric_at, D, NODE ? ex::filter_width(D) : width[gid], prim, KS, P,
+                         [&](int e, int c, double f) {
+                             (e == 0 ? Fv : (e == 1 ? Ev : Gv))[5 * (size_t)gid + c] = P.viscous ? f : 0.0;
+                         },
+                         mu);
     }
     flow[9 * (size_t)gid + FMU] = mu;
 }
@@ -611,7 +595,7 @@ __global__ void __launch_bounds__(128, REUSE ? 5 : 1) k_weno(Phys P, int j, doub
         }
         const int b = weno_visc_branch(Lc);
         if (b == 5) {
-            ex::central4([&](int o, int c) { return VF[5 * (size_t)idx[d][o + 3] + c]; }, dvis[d]);
+            ex::central4<true>([&](int o, int c) { return VF[5 * (size_t)idx[d][o + 3] + c]; }, dvis[d]);
         } else {
 #pragma unroll
             for (int c = 0; c < 5; ++c)
@@ -645,7 +629,7 @@ __global__ void __launch_bounds__(128, REUSE ? 5 : 1) k_weno(Phys P, int j, doub
 #pragma unroll
     for (int c = 0; c < 5; ++c) { u0[c] = U0[r5 + c]; u1[c] = U1[r5 + c]; u2[c] = U2[r5 + c]; }
     double rho, u, v, w, e, p, t, a;
-    ex::rk_and_primitives(j, dt, mach, det[gid], u0, u1, u2, L, Un, rho, u, v, w, e, p, t, a);
+    ex::rk_and_primitives<true>(j, dt, mach, det[gid], u0, u1, u2, L, Un, rho, u, v, w, e, p, t, a);
     double *Uo = j == 0 ? U1 : (j == 1 ? U2 : U0);
 #pragma unroll
     for (int c = 0; c < 5; ++c) Uo[r5 + c] = Un[c];
@@ -681,12 +665,13 @@ int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, d
 {
     const unsigned nb = blocks_for(n_items, 128);
     if (scratch && scratch_rows >= n_items) {
-        k_node_flux<<<nb, 128, 0, st>>>(F, E, G, metric, det, flow, n_items, P.les, scratch);
-        k_viscous<false><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
+        const bool fp = n_items <= kPlainNodes;
+        (fp ? k_node_flux<false> : k_node_flux<true>)<<<nb, 128, 0, st>>>(F, E, G, metric, det, flow, n_items, P.les, scratch);
+        (fp ? k_viscous<false, false> : k_viscous<false, true>)<<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
                                              scratch);
         return 2;
     }
-    k_viscous<true><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
+    k_viscous<true, false><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
                                         nullptr);
     return 1;
 }

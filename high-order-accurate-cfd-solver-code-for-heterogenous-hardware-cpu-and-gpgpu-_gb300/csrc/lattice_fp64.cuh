@@ -15,30 +15,24 @@ namespace ex {
 
 // U_Q.cl for one node from primitives in registers: U_q = det*Q, Q, the
 // contravariant node fluxes (Viscous.cl:560-631), sqrt(rho) and H.
+template <bool I>
 __device__ __forceinline__ void prep_values(const LatView &g, int n, int q, double rho, double u, double v, double w,
                                             double p)
 {
     const int N = g.N;
     const double D = g.det[n];
-    double m[9];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = g.m9[c * N + n];
     const double prim[5] = {rho, u, v, w, p};
-    double F[5], Ec[5], G[5], Q[5], H;
-    node_flux(prim, m, D, F, Ec, G, Q, H);
+    double Q[5], H;
+    node_flux<I>(prim, [&](int c) { return g.m9[c * N + n]; }, D,
+              [&](int d, int c, double f) { g.FEG[(d * 5 + c) * N + n] = f; }, Q, H);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        g.Q[c * N + n] = Q[c];
-        g.FEG[(0 * 5 + c) * N + n] = F[c];
-        g.FEG[(1 * 5 + c) * N + n] = Ec[c];
-        g.FEG[(2 * 5 + c) * N + n] = G[c];
-    }
+    for (int c = 0; c < 5; ++c) g.Q[c * N + n] = Q[c];
     double *Uq = lat_U(g, q);
     {
         const double re[2] = {rho, Q[4]}, vel[3] = {u, v, w};
         double d[2], du[3];
-        scaled(D, re, d);
-        scaled(d[0], vel, du);
+        scaled<I>(D, re, d);
+        scaled<I>(d[0], vel, du);
         Uq[0 * N + n] = d[0];
         Uq[1 * N + n] = du[0];
         Uq[2 * N + n] = du[1];
@@ -47,16 +41,17 @@ __device__ __forceinline__ void prep_values(const LatView &g, int n, int q, doub
     }
     const double s = xi::root(rho), x[4] = {u, v, w, H};
     double sx[4];
-    scaled(s, x, sx);
+    scaled<I>(s, x, sx);
     g.sh[n] = s;
 #pragma unroll
     for (int c = 0; c < 4; ++c) g.sh[(1 + c) * N + n] = sx[c];
 }
 
+template <bool I = true>
 __device__ __forceinline__ void prep_node(const LatView &g, int n, int q)
 {
     const int N = g.N;
-    prep_values(g, n, q, g.prim9[LF_RHO * N + n], g.prim9[LF_U * N + n], g.prim9[LF_V * N + n],
+    prep_values<I>(g, n, q, g.prim9[LF_RHO * N + n], g.prim9[LF_U * N + n], g.prim9[LF_V * N + n],
                 g.prim9[LF_W * N + n], g.prim9[LF_P * N + n]);
 }
 
@@ -74,6 +69,7 @@ __device__ __forceinline__ void loc_line(const LatView &g, int i, int j, int k, 
 // periodic lattice, where every node has loc 0; the loc-code branches of
 // Viscous.cl:285-332 on a lattice with loc codes; zero at ghosts, which no
 // branch covers), viscous + MTS SGS fluxes, mu.
+template <bool I>
 __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
 {
     const int N = g.N;
@@ -94,7 +90,7 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
         } else if (!lat_locdir(g, d) || !((lflag >> d) & 1u)) {
             const int at[5] = {lat_step(g, i, j, k, d, -2), lat_step(g, i, j, k, d, -1), n, lat_step(g, i, j, k, d, 1),
                                lat_step(g, i, j, k, d, 2)};
-            central4([&](int o, int c) { return Uj[c * N + at[o + 2]]; }, out);
+            central4<I>([&](int o, int c) { return Uj[c * N + at[o + 2]]; }, out);
         } else {
             int s[7], L[7];
             loc_line(g, i, j, k, d, s, L);
@@ -107,25 +103,17 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
             }
         }
     };
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < 3; ++d) {
         const int m1 = lat_step(g, i, j, k, d, -1), p1 = lat_step(g, i, j, k, d, 1), c = d + 1;
-        KS[d] = g.P.les && g.P.les != 2 ? ks_root(Ui[c], Ui[0], Uj[c * N + m1], Uj[m1], Uj[c * N + p1], Uj[p1]) : 0.0;
+        KS[d] = g.P.les && g.P.les != 2 ? ks_root(Uj[c * N + n], Ui[0], Uj[c * N + m1], Uj[m1], Uj[c * N + p1], Uj[p1]) : 0.0;
     }
-    double m[9];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = g.m9[c * N + n];
     const double prim[5] = {g.prim9[LF_RHO * N + n], g.prim9[LF_U * N + n], g.prim9[LF_V * N + n],
                             g.prim9[LF_W * N + n], g.prim9[LF_P * N + n]};
-    double Fv[5], Ev[5], Gv[5], mu;
+    double mu;
     const double D = g.det[n];
-    viscous_node(dU, Ui, m, D, g.del ? g.del[n] : filter_width(D), prim, KS, g.P, Fv, Ev, Gv, mu);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        g.V[(0 * 5 + c) * N + n] = Fv[c];
-        g.V[(1 * 5 + c) * N + n] = Ev[c];
-        g.V[(2 * 5 + c) * N + n] = Gv[c];
-    }
+    viscous_node<I>(dU, Ui, [&](int c) { return g.m9[c * N + n]; }, D, g.del ? g.del[n] : filter_width(D), prim, KS, g.P,
+                 [&](int d, int c, double f) { g.V[(d * 5 + c) * N + n] = f; }, mu);
     g.prim9[LF_MU * N + n] = mu;
 }
 
@@ -135,7 +123,7 @@ __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
     const int N = g.N;
     const double *Uj = lat_U(g, q);
     const double Ui[5] = {Uj[n], Uj[N + n], Uj[2 * N + n], Uj[3 * N + n], Uj[4 * N + n]};
-    g.prim9[LF_MU * N + n] = mu_of(Ui, g.P);
+    g.prim9[LF_MU * N + n] = mu_of<true>(Ui, g.P);
 }
 
 // Face n+1/2 along D: Roe average of the two nodes, LLF face flux and the
@@ -304,6 +292,7 @@ __device__ __forceinline__ void geometry_node(const LatView &g, double *kn, doub
 // of Weno.cl:2732-2856 on a lattice with loc codes), SSP-RK3 stage jst,
 // primitives.  With fuse_next the node then runs the next stage's prep on
 // the new primitives.
+template <bool I>
 __device__ __forceinline__ void update_node(const LatView &g, int n, int jst, bool fuse_next)
 {
     const int N = g.N;
@@ -316,38 +305,43 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst, bo
     }
     int i, j, k;
     lat_ijk(g, n, i, j, k);
-    double dflux[3][5], dvis[3][5];
+    // the sum in the reference's order: the flux differences of the three
+    // directions, then the viscous ones (loops: see viscous_node)
+    double L[5];
     const unsigned lflag = g.locflag ? g.locflag[n] : 7u;   // as in visc_node
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < 3; ++d) {
         const int m1 = lat_step(g, i, j, k, d, -1);
 #pragma unroll
-        for (int c = 0; c < 5; ++c) dflux[d][c] = g.Fh[(d * 5 + c) * N + n] - g.Fh[(d * 5 + c) * N + m1];
+        for (int c = 0; c < 5; ++c) {
+            const double df = g.Fh[(d * 5 + c) * N + n] - g.Fh[(d * 5 + c) * N + m1];
+            L[c] = d == 0 ? df : L[c] + df;
+        }
+    }
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) {
+        double dvis[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const double *Vd = g.V + (size_t)d * 5 * N;
         if (g.P.viscous && lat_locdir(g, d) && ((lflag >> d) & 1u)) {
-            int s[7], L[7];
-            loc_line(g, i, j, k, d, s, L);
-            const double *Vd = g.V + (size_t)d * 5 * N;
+            int s[7], B[7];
+            loc_line(g, i, j, k, d, s, B);
 #pragma unroll
             for (int c = 0; c < 5; ++c) {
                 double f[7];
 #pragma unroll
                 for (int o = 0; o < 7; ++o) f[o] = Vd[c * N + s[o]];
-                dvis[d][c] = weno_visc_deriv_ref(f, L);
+                dvis[c] = weno_visc_deriv_ref(f, B);
             }
         } else if (g.P.viscous) {
-            const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
-            const double *Vd = g.V + (size_t)d * 5 * N;
-            const int at[5] = {m2, m1, n, p1, p2};
-            central4([&](int o, int c) { return Vd[c * N + at[o + 2]]; }, dvis[d]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 5; ++c) dvis[d][c] = 0.0;
+            const int at[5] = {lat_step(g, i, j, k, d, -2), lat_step(g, i, j, k, d, -1), n, lat_step(g, i, j, k, d, 1),
+                               lat_step(g, i, j, k, d, 2)};
+            central4<I>([&](int o, int c) { return Vd[c * N + at[o + 2]]; }, dvis);
         }
-    }
-    double L[5];
 #pragma unroll
-    for (int c = 0; c < 5; ++c)
-        L[c] = (-1.0) * (dflux[0][c] + dflux[1][c] + dflux[2][c] + dvis[0][c] + dvis[1][c] + dvis[2][c]);
+        for (int c = 0; c < 5; ++c) L[c] = L[c] + dvis[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 5; ++c) L[c] = (-1.0) * L[c];
     if (g.Lout) {
 #pragma unroll
         for (int c = 0; c < 5; ++c) g.Lout[c * N + n] = L[c];
@@ -356,7 +350,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst, bo
 #pragma unroll
     for (int c = 0; c < 5; ++c) { u0[c] = g.U0[c * N + n]; u1[c] = g.U1[c * N + n]; u2[c] = g.U2[c * N + n]; }
     double rho, u, v, w, e, p, t, a;
-    rk_and_primitives(jst, g.dt, g.P.mach, g.det[n], u0, u1, u2, L, Un, rho, u, v, w, e, p, t, a);
+    rk_and_primitives<I>(jst, g.dt, g.P.mach, g.det[n], u0, u1, u2, L, Un, rho, u, v, w, e, p, t, a);
     double *Uo = jst == 0 ? g.U1 : (jst == 1 ? g.U2 : g.U0);
 #pragma unroll
     for (int c = 0; c < 5; ++c) Uo[c * N + n] = Un[c];
@@ -369,7 +363,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst, bo
     g.prim9[LF_T * N + n] = t;
     g.prim9[LF_A * N + n] = a;
     if (!(isfinite(rho) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(p))) atomicOr(g.flags, 2u);
-    if (fuse_next) prep_values(g, n, jst == 2 ? 0 : jst + 1, rho, u, v, w, p);
+    if (fuse_next) prep_values<I>(g, n, jst == 2 ? 0 : jst + 1, rho, u, v, w, p);
 }
 
 }  // namespace ex

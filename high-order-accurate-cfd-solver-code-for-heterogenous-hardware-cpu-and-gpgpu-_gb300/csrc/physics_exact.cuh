@@ -660,41 +660,63 @@ __device__ __forceinline__ double corrected(double Fhat, const double f[6])
     return Fhat - (1.0 / 24.0) * d2 + (7.0 / 5760.0) * d4;
 }
 
-// r[i] = a[i] b[i] on the integer pipe.
-template <int N>
+// r[i] = a[i] b[i], r[i] = k b[i], x[i] = x[i]^2, a b: on the integer pipe
+// (I), or on the FP64 pipe with the same bits.  The per-node kernels are
+// built both ways: a few blocks per SM cannot keep the FP64 pipe busy, and
+// there the integer form's seven times longer code costs more to fetch than
+// it saves (kPlainNodes, internal.h).
+template <bool I, int N>
 __device__ __forceinline__ void products(const double (&a)[N], const double (&b)[N], double (&r)[N])
 {
-    xi::Fac fa[N], fb[N];
+    if (I) {
+        xi::Fac fa[N], fb[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        fa[i] = xi::fac(a[i]);
-        fb[i] = xi::fac(b[i]);
+        for (int i = 0; i < N; ++i) {
+            fa[i] = xi::fac(a[i]);
+            fb[i] = xi::fac(b[i]);
+        }
+        xi::mul_n(fa, fb, r);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) r[i] = a[i] * b[i];
     }
-    xi::mul_n(fa, fb, r);
 }
 
-// r[i] = k b[i]
-template <int N>
+template <bool I, int N>
 __device__ __forceinline__ void scaled(double k, const double (&b)[N], double (&r)[N])
 {
-    xi::Fac fa[N], fb[N];
+    double a[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        fa[i] = xi::fac(k);
-        fb[i] = xi::fac(b[i]);
+    for (int i = 0; i < N; ++i) a[i] = k;
+    products<I>(a, b, r);
+}
+
+template <bool I, int N>
+__device__ __forceinline__ void squares(double (&x)[N])
+{
+    if (I) {
+        xi::sq_n(x);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = x[i] * x[i];
     }
-    xi::mul_n(fa, fb, r);
+}
+
+template <bool I>
+__device__ __forceinline__ double product(double a, double b)
+{
+    return I ? xi::mul(a, b) : a * b;
 }
 
 // Fourth-order central first derivatives (Viscous.cl:325-332 and the loc==0
 // branch of Weno.cl:2771-2778) of five values; f(o, c): value c at offset o.
-template <class F>
+template <bool I, class F>
 __device__ __forceinline__ void central4(const F &f, double *out)
 {
     double b[5], r[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) b[c] = xdiv::scale2<3>(f(1, c) - f(-1, c)) - (f(2, c) - f(-2, c));   // 8 (...): the exponent moved
-    scaled(1.0 / 12.0, b, r);
+    scaled<I>(1.0 / 12.0, b, r);
 #pragma unroll
     for (int c = 0; c < 5; ++c) out[c] = r[c];
 }
@@ -714,117 +736,127 @@ __device__ __forceinline__ double zero_dot(double mx, double my, double mz, doub
 // 1 / det^(1/3), the filter width the SGS terms take (Viscous.cl:490).
 __device__ __forceinline__ double filter_width(double det) { return dv(1.0, cbrt(det)); }
 
-// Cartesian flux vectors tF, tE, tG (components c0 .. 4 in [N]) through the
-// node metrics m[9], x det: out[d][c] = det (m_d . (tF, tE, tG)[c]).
-template <int N>
-__device__ __forceinline__ void through_metrics(const double m[9], double det, const double (&tF)[N],
-                                                const double (&tE)[N], const double (&tG)[N], double *F, double *E,
-                                                double *G)
+// Cartesian flux vectors tF, tE, tG ([N] components) through the node
+// metrics (m(k), k = 0..8), x det: store(d, c, det (m_d . (tF, tE, tG)[c])).
+// A loop over the directions: the instruction cache holds it once.
+template <bool I, int N, class Metric, class Store>
+__device__ __forceinline__ void through_metrics(const Metric &m, double det, const double (&tF)[N],
+                                                const double (&tE)[N], const double (&tG)[N], const Store &store)
 {
-#pragma unroll
+#pragma unroll 1
     for (int d = 0; d < 3; ++d) {
-        const xi::Fac fx = xi::fac(m[3 * d]), fy = xi::fac(m[3 * d + 1]), fz = xi::fac(m[3 * d + 2]);
+        const double mx = m(3 * d), my = m(3 * d + 1), mz = m(3 * d + 2);
         double s[N], r[N];
 #pragma unroll
         for (int c = 0; c < N; ++c) {
-            const xi::Fac a[3] = {fx, fy, fz}, b[3] = {xi::fac(tF[c]), xi::fac(tE[c]), xi::fac(tG[c])};
+            const double a[3] = {mx, my, mz}, b[3] = {tF[c], tE[c], tG[c]};
             double q[3];
-            xi::mul_n(a, b, q);
+            products<I>(a, b, q);
             s[c] = q[0] + q[1] + q[2];
         }
-        scaled(det, s, r);
-        double *out = d == 0 ? F : (d == 1 ? E : G);
+        scaled<I>(det, s, r);
 #pragma unroll
-        for (int c = 0; c < N; ++c) out[c] = r[c];
+        for (int c = 0; c < N; ++c) store(d, c, r[c]);
     }
 }
 
 // Viscous.cl:439-631 at one node, in the reference's order.  dU(d, out):
-// the derivatives of U along d; Ui[5], node metrics m[9], det, filter width DEL, FLOW primitives
-// (rho,u,v,w,p), the three MTS test-filter differences K (roots of the
-// reference's KS).  Writes the contravariant viscous fluxes Fv,Ev,Gv and mu
+// the derivatives of U along d; Ui[5], node metrics m(k), det, filter width
+// DEL, FLOW primitives (rho,u,v,w,p), the three MTS test-filter differences
+// K (roots of the reference's KS).  store(d, c, value) takes the
+// contravariant viscous fluxes Fv, Ev, Gv (d = 0, 1, 2); mu_out the viscosity
 // (the inviscid node fluxes come from node_flux).  The products run on the
-// integer pipe in groups, the sums on the FP64 pipe.
-template <class Deriv>
-__device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5], const double m[9], double DET_I,
+// integer pipe in groups, the sums on the FP64 pipe.  Directions, gradients
+// and flux rows are loops with their small arrays in local memory: unrolled,
+// one node's 10,000 instructions (160 KB) outgrew the instruction cache
+// (TGV 128^3 1.54 -> 1.45 ms; 4,913 nodes 82 -> 61 us, and 32 us with the
+// products on the FP64 pipe).
+template <bool I, class Deriv, class Metric, class Store>
+__device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5], const Metric &m, double DET_I,
                                              double DEL, const double prim[5], const double K[3], const Phys &P,
-                                             double Fv[5], double Ev[5], double Gv[5], double &mu_out)
+                                             const Store &store, double &mu_out)
 {
     using xdiv::scale2;   // products by powers of two: the exponent moved
-    double uc[3], vc[3], wc[3], tc[3], d_temp;
+    double g[4][3], d_temp;   // derivatives of u, v, w and of the energy term along the directions
     {
         double s[4] = {Ui[0], Ui[1], Ui[2], Ui[3]};
-        xi::sq_n(s);
+        squares<I>(s);
         double x[5] = {1.0, Ui[1], Ui[2], Ui[3], Ui[4]}, y[7] = {Ui[1], Ui[2], Ui[3], Ui[4], s[1], s[2], s[3]};
         Over<true>(Ui[0]).all(x);   // r0, v1, v2, v3, U4 / U0
         Over<true>(s[0]).all(y);    // a1 .. a4, U1^2, U2^2, U3^2 over U0^2
-        d_temp = xi::mul(P.c_temp, x[4] - scale2<-1>(y[4] + y[5] + y[6]));
-        const xi::Fac r0 = xi::fac(x[0]), a1 = xi::fac(y[0]), a2 = xi::fac(y[1]), a3 = xi::fac(y[2]), a4 = xi::fac(y[3]);
-        const xi::Fac v1 = xi::fac(x[1]), v2 = xi::fac(x[2]), v3 = xi::fac(x[3]);
-#pragma unroll
+        d_temp = product<I>(P.c_temp, x[4] - scale2<-1>(y[4] + y[5] + y[6]));
+#pragma unroll 1
         for (int d = 0; d < 3; ++d) {
             double du[5];
             dU(d, du);
-            const xi::Fac d0 = xi::fac(du[0]);
-            const xi::Fac f[8] = {r0, a1, r0, a2, r0, a3, r0, a4};
-            const xi::Fac g[8] = {xi::fac(du[1]), d0, xi::fac(du[2]), d0, xi::fac(du[3]), d0, xi::fac(du[4]), d0};
+            const double f[8] = {x[0], y[0], x[0], y[1], x[0], y[2], x[0], y[3]};
+            const double e[8] = {du[1], du[0], du[2], du[0], du[3], du[0], du[4], du[0]};
             double r[8], t[3];
-            xi::mul_n(f, g, r);
-            uc[d] = r[0] - r[1];
-            vc[d] = r[2] - r[3];
-            wc[d] = r[4] - r[5];
-            const xi::Fac fv[3] = {v1, v2, v3}, gv[3] = {xi::fac(uc[d]), xi::fac(vc[d]), xi::fac(wc[d])};
-            xi::mul_n(fv, gv, t);
-            tc[d] = r[6] - r[7] - t[0] - t[1] - t[2];
+            products<I>(f, e, r);
+            const double u = r[0] - r[1], v = r[2] - r[3], w = r[4] - r[5];
+            const double fv[3] = {x[1], x[2], x[3]}, gv[3] = {u, v, w};
+            products<I>(fv, gv, t);
+            g[0][d] = u;
+            g[1][d] = v;
+            g[2][d] = w;
+            g[3][d] = r[6] - r[7] - t[0] - t[1] - t[2];
         }
     }
     double mr, kq;
     {
         const double sd = xi::root(d_temp);
-        const double mu = xi::mul(xi::mul(xi::mul(sd, sd), sd), dv(P.st1, d_temp + P.st));
+        const double mu = product<I>(product<I>(product<I>(sd, sd), sd), dv(P.st1, d_temp + P.st));
         mu_out = mu;
-        double q[2] = {xi::mul(mu, 1.4), mu};
+        double q[2] = {product<I>(mu, 1.4), mu};
         const double by[2] = {P.pr_re, P.reynolds};
         xi::div_n(q, by);
         kq = q[0];
         mr = q[1];
     }
-    // gradients: along x, y, z (columns of m) of one variable's derivatives,
-    // and the mixed sums in the reference's order
+    // gradients along x, y, z of one variable's derivatives (heat x, y, z; ux,
+    // vy, wz), and the mixed sums s_xy, s_xz, s_yz (s_zx: s_xz the other way
+    // round) in the reference's order.  Pass i takes variable p along x and
+    // q along y.
     double gt[3], ux, vy, wz, s_xy, s_xz, s_yz, s_zx;
     {
-        auto six = [&](const double (&p)[3], int x, const double (&q)[3], int y, double (&r)[6]) {
-            const double a[6] = {p[0], p[1], p[2], q[0], q[1], q[2]};
-            const double b[6] = {m[x], m[3 + x], m[6 + x], m[y], m[3 + y], m[6 + y]};
-            products(a, b, r);
-        };
-        double r[6];
-        six(tc, 0, tc, 1, r);
-        gt[0] = r[0] + r[1] + r[2];
-        gt[1] = r[3] + r[4] + r[5];
-        six(tc, 2, uc, 0, r);
-        gt[2] = r[0] + r[1] + r[2];
-        ux = r[3] + r[4] + r[5];
-        six(vc, 1, wc, 2, r);
-        vy = r[0] + r[1] + r[2];
-        wz = r[3] + r[4] + r[5];
-        six(uc, 1, vc, 0, r);
-        s_xy = r[0] + r[1] + r[2] + r[3] + r[4] + r[5];
-        six(uc, 2, wc, 0, r);
-        s_xz = r[0] + r[1] + r[2] + r[3] + r[4] + r[5];
-        s_zx = r[3] + r[4] + r[5] + r[0] + r[1] + r[2];
-        six(vc, 2, wc, 1, r);
-        s_yz = r[0] + r[1] + r[2] + r[3] + r[4] + r[5];
+        double sums[6][2], s_back = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < 6; ++i) {
+            const int p = (0x100133 >> (4 * i)) & 15, x = (0x221120 >> (4 * i)) & 15;
+            const int q = (0x221203 >> (4 * i)) & 15, y = (0x100201 >> (4 * i)) & 15;
+            const double a[6] = {g[p][0], g[p][1], g[p][2], g[q][0], g[q][1], g[q][2]};
+            const double b[6] = {m(x), m(3 + x), m(6 + x), m(y), m(3 + y), m(6 + y)};
+            double r[6];
+            products<I>(a, b, r);
+            const double s1 = r[0] + r[1] + r[2];
+            if (i < 3) {
+                sums[i][1] = r[3] + r[4] + r[5];
+                sums[i][0] = s1;
+            } else {
+                sums[i][0] = s1 + r[3] + r[4] + r[5];
+            }
+            if (i == 4) s_back = r[3] + r[4] + r[5] + r[0] + r[1] + r[2];
+        }
+        gt[0] = sums[0][0];
+        gt[1] = sums[0][1];
+        gt[2] = sums[1][0];
+        ux = sums[1][1];
+        vy = sums[2][0];
+        wz = sums[2][1];
+        s_xy = sums[3][0];
+        s_xz = sums[4][0];
+        s_yz = sums[5][0];
+        s_zx = s_back;
     }
     double qz, qe, qx, tauzz, tauee, tauxx, tauze, tauzx, tauex;
     {
         const double g[3] = {ux, vy, wz};
         double t[3], r[6], h[3];
-        scaled(2.0 / 3.0, g, t);   // 4/3 x is twice 2/3 x
+        scaled<I>(2.0 / 3.0, g, t);   // 4/3 x is twice 2/3 x
         const double b[6] = {scale2<1>(t[0]) - t[1] - t[2], scale2<1>(t[1]) - t[0] - t[2],
                              scale2<1>(t[2]) - t[0] - t[1], s_xy, s_xz, s_yz};
-        scaled(mr, b, r);
-        scaled(-kq, gt, h);
+        scaled<I>(mr, b, r);
+        scaled<I>(-kq, gt, h);
         qz = h[0];
         qe = h[1];
         qx = h[2];
@@ -843,7 +875,7 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
         const double yz = scale2<-1>(s_yz), xy = scale2<-1>(s_xy);
         const double xz = scale2<-1>(s_zx);
         double s[6] = {xy, yz, xz, ux, vy, wz};
-        xi::sq_n(s);
+        squares<I>(s);
         double E[3];
         if (P.les == 2) {
             // Smagorinsky (no counterpart in the reference): (C_s Delta)^2 |S|,
@@ -853,10 +885,10 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
             const double ls = P.cs * cbrt(DET_I);
             E[0] = E[1] = E[2] = (ls * ls) * S;
         } else {
-            const double mod = xi::root(scale2<1>((s[0] + s[1] + s[2]) + xi::mul(2.0 / 3.0, s[3] + s[4] + s[5])));
+            const double mod = xi::root(scale2<1>((s[0] + s[1] + s[2]) + product<I>(2.0 / 3.0, s[3] + s[4] + s[5])));
             double c[3] = {C_MTS, C_MTS, C_MTS}, e[3];
             if (mod != 0.0) {
-                const double dm = xi::mul(DEL, mod);
+                const double dm = product<I>(DEL, mod);
                 double R[3] = {dm, dm, dm};
                 const double by[3] = {K[0], K[1], K[2]};
                 xi::div_n(R, by);
@@ -864,17 +896,17 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
                 const double one[3] = {1.0 + R[0], 1.0 + R[1], 1.0 + R[2]};
                 xi::div_n(c, one);
             }
-            scaled(DEL, c, e);
+            scaled<I>(DEL, c, e);
             const double k[3] = {K[0], K[1], K[2]};
-            products(e, k, E);
+            products<I>(e, k, E);
         }
         double r[3], g[3], tau[6], Q[3];
-        scaled(-scale2<1>(Ui[0]), E, r);   // -2.0 * U0_I
-        scaled(-P.ck, E, g);
+        scaled<I>(-scale2<1>(Ui[0]), E, r);   // -2.0 * U0_I
+        scaled<I>(-P.ck, E, g);
         {
             const double a[6] = {r[0], r[1], r[2], r[0], r[1], r[2]}, b[6] = {xy, yz, xz, ux, vy, wz};
-            products(a, b, tau);
-            products(g, gt, Q);
+            products<I>(a, b, tau);
+            products<I>(g, gt, Q);
         }
         TAU_XY = tau[0];
         TAU_YZ = tau[1];
@@ -885,11 +917,11 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
         const double a[9] = {TAU_XX, TAU_XY, TAU_XZ, TAU_XY, TAU_YY, TAU_YZ, TAU_XZ, TAU_YZ, TAU_ZZ};
         const double b[9] = {u, u, u, v, v, v, w, w, w};
         double h[9], D[3];
-        products(a, b, h);
+        products<I>(a, b, h);
         H_X = Q[0] + (h[0] + h[1] + h[2]);
         H_Y = Q[1] + (h[3] + h[4] + h[5]);
         H_Z = Q[2] + (h[6] + h[7] + h[8]);
-        scaled(0.4, Q, D);
+        scaled<I>(0.4, Q, D);
         D_X = D[0];
         D_Y = D[1];
         D_Z = D[2];
@@ -899,7 +931,7 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
         const double a[9] = {-u, v, w, -u, v, w, -u, v, w};
         const double b[9] = {tauzz, tauze, tauzx, tauze, tauee, tauex, tauzx, tauex, tauxx};
         double r[9];
-        products(a, b, r);
+        products<I>(a, b, r);
         e[0] = (r[0] - r[1] - r[2]) + qz + H_X + D_X;
         e[1] = (r[3] - r[4] - r[5]) + qe + H_Y + D_Y;
         e[2] = (r[6] - r[7] - r[8]) + qx + H_Z + D_Z;
@@ -907,24 +939,24 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
     const double tF[4] = {-tauzz + TAU_XX, -tauze + TAU_XY, -tauzx + TAU_XZ, e[0]};
     const double tE[4] = {-tauze + TAU_XY, -tauee + TAU_YY, -tauex + TAU_YZ, e[1]};
     const double tG[4] = {-tauzx + TAU_XZ, -tauex + TAU_YZ, -tauxx + TAU_ZZ, e[2]};
-    Fv[0] = zero_dot(m[0], m[1], m[2], DET_I);
-    Ev[0] = zero_dot(m[3], m[4], m[5], DET_I);
-    Gv[0] = zero_dot(m[6], m[7], m[8], DET_I);
-    through_metrics(m, DET_I, tF, tE, tG, Fv + 1, Ev + 1, Gv + 1);
+#pragma unroll 1
+    for (int d = 0; d < 3; ++d) store(d, 0, zero_dot(m(3 * d), m(3 * d + 1), m(3 * d + 2), DET_I));
+    through_metrics<I>(m, DET_I, tF, tE, tG, [&](int d, int c, double v) { store(d, c + 1, v); });
 }
 
-// Contravariant inviscid node fluxes F, E, G (x det) from the primitives
-// (rho,u,v,w,p), Viscous.cl:560-578 and 615-631, with the values U_Q shares
+// Contravariant inviscid node fluxes F, E, G (x det; store(d, c, value)) from
+// the primitives (rho,u,v,w,p), Viscous.cl:560-578 and 615-631, with the values U_Q shares
 // (U_Q.cl:60-122): Q = {rho, rho u, rho v, rho w, E} and the total enthalpy H.
-__device__ __forceinline__ void node_flux(const double prim[5], const double m[9], double DET_I, double F[5],
-                                          double E[5], double G[5], double Q[5], double &H)
+template <bool I, class Metric, class Store>
+__device__ __forceinline__ void node_flux(const double prim[5], const Metric &m, double DET_I, const Store &store,
+                                          double Q[5], double &H)
 {
     const double rho = prim[0], u = prim[1], v = prim[2], w = prim[3], p = prim[4];
     double s[3] = {u, v, w}, r[3], t[9];
     const double vel[3] = {u, v, w};
-    xi::sq_n(s);
-    scaled(rho, vel, r);   // rho u, rho v, rho w
-    const double en = dv(p, 0.4) + xi::mul(xdiv::scale2<-1>(rho), s[0] + s[1] + s[2]);
+    squares<I>(s);
+    scaled<I>(rho, vel, r);   // rho u, rho v, rho w
+    const double en = dv(p, 0.4) + product<I>(xdiv::scale2<-1>(rho), s[0] + s[1] + s[2]);
     const double Et = en + p;
     H = dv(Et, rho);
     Q[0] = rho;
@@ -935,12 +967,12 @@ __device__ __forceinline__ void node_flux(const double prim[5], const double m[9
     {
         // rho u u, rho v u, rho u w, rho v v, rho v w, rho w w, Et u, Et v, Et w
         const double a[9] = {r[0], r[1], r[0], r[1], r[1], r[2], Et, Et, Et}, b[9] = {u, u, w, v, w, w, u, v, w};
-        products(a, b, t);
+        products<I>(a, b, t);
     }
     const double tF[5] = {r[0], t[0] + p, t[1], t[2], t[6]};
     const double tE[5] = {r[1], t[1], t[3] + p, t[4], t[7]};
     const double tG[5] = {r[2], t[2], t[4], t[5] + p, t[8]};
-    through_metrics(m, DET_I, tF, tE, tG, F, E, G);
+    through_metrics<I>(m, DET_I, tF, tE, tG, store);
 }
 
 // Root of the MTS test filter's velocity-difference square
@@ -960,20 +992,22 @@ __device__ __forceinline__ double ks_root(double Uc_i, double U0_i, double Uc_m,
 }
 
 // Sutherland viscosity from U only (Viscous.cl:451-458).
+template <bool I>
 __device__ __forceinline__ double mu_of(const double Ui[5], const Phys &P)
 {
     double s[4] = {Ui[0], Ui[1], Ui[2], Ui[3]};
-    xi::sq_n(s);
+    squares<I>(s);
     double y[3] = {s[1], s[2], s[3]};
     Over<true>(s[0]).all(y);
-    const double d_temp = xi::mul(P.c_temp, dv(Ui[4], Ui[0]) - xdiv::scale2<-1>(y[0] + y[1] + y[2]));
+    const double d_temp = product<I>(P.c_temp, dv(Ui[4], Ui[0]) - xdiv::scale2<-1>(y[0] + y[1] + y[2]));
     const double sd = xi::root(d_temp);
-    return xi::mul(xi::mul(xi::mul(sd, sd), sd), dv(P.st1, d_temp + P.st));
+    return product<I>(product<I>(product<I>(sd, sd), sd), dv(P.st1, d_temp + P.st));
 }
 
 // SSP-RK3 stage j and primitive recovery (Weno.cl:3084-3135).  Returns the
 // new U in Un and writes FLOW fields rho,u,v,w,e,p,t,a into fo[9]
 // (u,v,w,p,t,rho,mu,a,e order; mu untouched).
+template <bool I>
 __device__ __forceinline__ void rk_and_primitives(int j, double del_t, double mach, double det, const double U0[5],
                                                   const double U1[5], const double U2[5], const double L[5],
                                                   double Un[5], double &rho, double &u, double &v, double &w,
@@ -982,30 +1016,30 @@ __device__ __forceinline__ void rk_and_primitives(int j, double del_t, double ma
     const double l5[5] = {L[0], L[1], L[2], L[3], L[4]};
     if (j == 0) {
         double t[5];
-        scaled(del_t, l5, t);
+        scaled<I>(del_t, l5, t);
 #pragma unroll
         for (int c = 0; c < 5; ++c) Un[c] = U0[c] + t[c];
     } else if (j == 1) {
         const double z[5] = {U0[0], U0[1], U0[2], U0[3], U0[4]};
         double s[5], t[5];
-        scaled(3.0 / 4.0, z, s);
-        scaled(0.25 * del_t, l5, t);
+        scaled<I>(3.0 / 4.0, z, s);
+        scaled<I>(0.25 * del_t, l5, t);
 #pragma unroll
         for (int c = 0; c < 5; ++c) Un[c] = s[c] + xdiv::scale2<-2>(U1[c]) + t[c];
     } else {
         double t[5], s[5], r[5], z[5] = {U0[0], U0[1], U0[2], U0[3], U0[4]};
         const double y[5] = {U2[0], U2[1], U2[2], U2[3], U2[4]};
         Over<true>(3.0).all(z);
-        scaled(del_t, l5, t);
-        scaled(2.0 / 3.0, y, s);
-        scaled(2.0 / 3.0, t, r);
+        scaled<I>(del_t, l5, t);
+        scaled<I>(2.0 / 3.0, y, s);
+        scaled<I>(2.0 / 3.0, t, r);
 #pragma unroll
         for (int c = 0; c < 5; ++c) Un[c] = z[c] + s[c] + r[c];
     }
     double fu[5];
     {
         const double un[5] = {Un[0], Un[1], Un[2], Un[3], Un[4]};
-        scaled(dv(1.0, det), un, fu);
+        scaled<I>(dv(1.0, det), un, fu);
     }
     rho = fu[0];
     const Over<true> d0(fu[0]);   // u, v, w, e, p / rho and 1.4 p / rho share the divisor
@@ -1015,12 +1049,12 @@ __device__ __forceinline__ void rk_and_primitives(int j, double del_t, double ma
     v = q[1];
     w = q[2];
     double s[3] = {u, v, w};
-    xi::sq_n(s);
+    squares<I>(s);
     e = q[3] - xdiv::scale2<-1>(s[0] + s[1] + s[2]);
-    p = xi::mul(xi::mul(e, rho), 0.4);
-    double r[2] = {p, xi::mul(1.4, p)};
+    p = product<I>(product<I>(e, rho), 0.4);
+    double r[2] = {p, product<I>(1.4, p)};
     d0.all(r);
-    t = xi::mul(1.4 * mach * mach, r[0]);
+    t = product<I>(1.4 * mach * mach, r[0]);
     a_ = xi::root(r[1]);
 }
 

@@ -39,16 +39,18 @@ __device__ __forceinline__ int node_id() { return blockIdx.x * blockDim.x + thre
 // to 6 blocks, 0.34 at 8; viscous 1.54 ms at 4, 1.87 at 3, 2.10 at 5;
 // update 0.58, 0.54, 0.53, 0.52 ms at 5, 6, 7, 8.  With the products on the
 // FP64 pipe they took 0.59, 1.89 and 0.66 ms.
+template <bool I>
 __global__ void __launch_bounds__(128, 6) k_prep(LatView g, int q)
 {
     const int n = node_id();
-    if (n < g.N) ex::prep_node(g, n, q);
+    if (n < g.N) ex::prep_node<I>(g, n, q);
 }
 
+template <bool I>
 __global__ void __launch_bounds__(128, 4) k_visc(LatView g, int q)
 {
     const int n = node_id();
-    if (n < g.N) ex::visc_node(g, n, q);
+    if (n < g.N) ex::visc_node<I>(g, n, q);
 }
 
 __global__ void __launch_bounds__(128) k_mu_only(LatView g, int q)
@@ -58,10 +60,11 @@ __global__ void __launch_bounds__(128) k_mu_only(LatView g, int q)
 }
 
 
-__global__ void __launch_bounds__(128, 7) k_update(LatView g, int jst)
+template <bool I>
+__global__ void __launch_bounds__(128, I ? 7 : 4) k_update(LatView g, int jst)
 {
     const int n = node_id();
-    if (n < g.N) ex::update_node(g, n, jst, false);
+    if (n < g.N) ex::update_node<I>(g, n, jst, false);
 }
 
 // AoS reference rows (row stride `stride` doubles) <-> SoA [comp][N].
@@ -104,15 +107,16 @@ int structured_stage(const StructuredLaunch &S, int jst, double dt, double *Lout
         if (ev) cudaEventRecord(ev[++e], st);
     };
     if (ev) cudaEventRecord(ev[0], st);
-    k_prep<<<nb, 128, 0, st>>>(g, jst);
+    const bool fp = g.N <= kPlainNodes;   // products of the per-node kernels on the FP64 pipe
+    (fp ? k_prep<false> : k_prep<true>)<<<nb, 128, 0, st>>>(g, jst);
     mark("prep");
     if (S.P.viscous)
-        k_visc<<<nb, 128, 0, st>>>(g, jst);
+        (fp ? k_visc<false> : k_visc<true>)<<<nb, 128, 0, st>>>(g, jst);
     else
         k_mu_only<<<nb, 128, 0, st>>>(g, jst);
     mark(S.P.viscous ? "viscous" : "mu_only");
     k = 3 + fp64_faces(S, g, st, mark);
-    k_update<<<nb, 128, 0, st>>>(g, jst);
+    (fp ? k_update<false> : k_update<true>)<<<nb, 128, 0, st>>>(g, jst);
     mark("update");
     return ev ? entries : k;
 }

@@ -38,3 +38,42 @@ def test_rounds_of_the_face_scratch_equal_the_gather_path(ctx):
         got.append(s.get_u0()[1:])   # row 0 is the layout's dummy row, not a node
         s.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("shape", [(36, 37, 37), (37, 37, 37)])
+def test_product_forms_have_the_same_bits(ctx, shape):
+    """49,284 and 50,653 nodes: either side of the line up to which the
+    solver's and the drop-in's per-node kernels take their products on the
+    FP64 pipe; the batch takes them on the integer pipe at every size.  FLOW
+    is compared: the batch's U0 is already the next stage's."""
+    from cfd_gb300 import cases, runtime
+    c = cases.taylor_green(shape=shape)
+    b = runtime.Batch(ctx, 0)
+    slot = b.add(c)
+    b.step(2)
+    want = b.get_flow(slot)[1:c.sd_node + 1]
+    b.close()
+    for path in (1, 0):
+        s = runtime.Solver(ctx, c, force_path=path)
+        s.set_flow(c.arrays["flow"])
+        s.step(c.dt, 2)
+        assert np.array_equal(s.get_flow()[1:c.sd_node + 1], want)
+        s.close()
+
+
+def test_batch_rounds_equal_the_solver(ctx):
+    """Five instances of 216,000 nodes: two rounds of the batch's face
+    scratch (2^20 nodes each), the last instance in the second."""
+    from cfd_gb300 import cases, runtime
+    c = cases.taylor_green(n=60)
+    s = runtime.Solver(ctx, c)
+    s.set_flow(c.arrays["flow"])
+    s.step(c.dt, 1)
+    want = s.get_flow()[1:c.sd_node + 1]
+    s.close()
+    b = runtime.Batch(ctx, 0)
+    slots = [b.add(c) for _ in range(5)]
+    b.step(1)
+    for slot in slots:
+        assert np.array_equal(b.get_flow(slot)[1:c.sd_node + 1], want)
+    b.close()
