@@ -88,11 +88,11 @@ unsigned *slot_flags(cfd_batch *b, int slot) { return b->d_words + 4 + slot; }
 uint64_t instance_bytes(int precision, int64_t N)
 {
     const uint64_t doubles = (22 + 9 + 15) * (uint64_t)N + 14 * (uint64_t)(N + 1);
-    // mixed: FP32 face/node geometry (12 + 10 + 2), prim32 (9), stage intermediates (55)
-    if (precision == CFD_PREC_MIXED) return doubles * 8 + (12 + 11 + 2 + 9 + 55) * (uint64_t)N * 4;
-    // split: FP32 face metrics (9), node geometry (11), prim32 (9), Q32/R32/FEG32/V32 (40) and the hi/lo
+    // mixed: FP32 face/node geometry (12 + 10 + 2), prim32 (9), stage intermediates (40)
+    if (precision == CFD_PREC_MIXED) return doubles * 8 + (12 + 11 + 2 + 9 + 40) * (uint64_t)N * 4;
+    // split: FP32 face metrics (9), node geometry (11), prim32 (9), Q32/R32/V32 (25) and the hi/lo
     // state copy (10); FP64 1/det and Fh (16)
-    if (precision == CFD_PREC_SPLIT) return (doubles + 16 * (uint64_t)N) * 8 + (9 + 11 + 9 + 40 + 10) * (uint64_t)N * 4;
+    if (precision == CFD_PREC_SPLIT) return (doubles + 16 * (uint64_t)N) * 8 + (9 + 11 + 9 + 25 + 10) * (uint64_t)N * 4;
     return (doubles + 65 * (uint64_t)N) * 8;   // stage intermediates (55), unit normals (9), filter width
 }
 
@@ -383,7 +383,6 @@ std::vector<std::pair<void *, size_t>> mutable_arrays(const BatchInst &I, int pr
         v.push_back({I.view.prim32, 9 * N * 4});
         v.push_back({I.view.Q32, 5 * N * 4});
         v.push_back({I.view.R32, 5 * N * 4});
-        v.push_back({I.view.FEG32, 15 * N * 4});
     } else {
         v.push_back({I.view.Q, 5 * N * 8});
         v.push_back({I.view.FEG, 15 * N * 8});
@@ -604,7 +603,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         if ((st = ialloc(b, I, 9 * Nz, &fm32)) || (st = ialloc(b, I, 3 * Nz, &fdet32))
             || (st = ialloc(b, I, 11 * Nz, &node32)) || (st = ialloc(b, I, 2 * Nz, &idet32))
             || (st = ialloc(b, I, 9 * Nz, &v.prim32)) || (st = ialloc(b, I, 5 * Nz, &v.Q32))
-            || (st = ialloc(b, I, 5 * Nz, &v.R32)) || (st = ialloc(b, I, 15 * Nz, &v.FEG32))
+            || (st = ialloc(b, I, 5 * Nz, &v.R32))
             || (st = ialloc(b, I, 15 * Nz, &v.V32)) || (st = ialloc(b, I, 15 * Nz, &v.Fh32))) {
             free_instance(I);
             return st;
@@ -618,7 +617,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         double *idet64;
         if ((st = ialloc(b, I, 9 * Nz, &fm32)) || (st = ialloc(b, I, 11 * Nz, &node32)) || (st = ialloc(b, I, Nz, &idet64))
             || (st = ialloc(b, I, 9 * Nz, &v.prim32)) || (st = ialloc(b, I, 5 * Nz, &v.Q32))
-            || (st = ialloc(b, I, 5 * Nz, &v.R32)) || (st = ialloc(b, I, 15 * Nz, &v.FEG32))
+            || (st = ialloc(b, I, 5 * Nz, &v.R32))
             || (st = ialloc(b, I, 15 * Nz, &v.V32)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))
             || (st = ialloc(b, I, 10 * Nz, &v.Whl))) {
             free_instance(I);

@@ -80,6 +80,22 @@ __device__ __forceinline__ TileAt tile_of_block()
     return {(int)blockIdx.x * T::kTile, (int)blockIdx.y * T::kWide, (int)blockIdx.z};
 }
 
+// The node flux along D of a node from the state that derive left: rho from
+// Q, velocities from the Roe inputs, the pressure.  Forming it where it is
+// read (at most 1.6 times per face) takes 15 loads and 15 stores per node
+// out of the update and 60 bytes per node out of memory.
+template <int D, bool RO>
+__device__ __forceinline__ void lat_node_flux(const LatView &g, int node, float o[5])
+{
+    auto ld = [](const float *p) { return RO ? __ldg(p) : *p; };
+    const int N = g.N;
+    const float prim[5] = {ld(g.Q32 + node), ld(g.R32 + node), ld(g.R32 + N + node), ld(g.R32 + 2 * N + node),
+                           ld(g.prim32 + LF_P * N + node)};
+    const float m[3] = {__ldg(g.node32 + 3 * D * N + node), __ldg(g.node32 + (3 * D + 1) * N + node),
+                        __ldg(g.node32 + (3 * D + 2) * N + node)};
+    node_inviscid_flux(prim, m, __ldg(g.node32 + 9 * N + node), o);
+}
+
 // Stages the block's stencil lines of Q, the Roe inputs and the node fluxes
 // along D (read-only in the face pass: non-coherent loads, unless RO is
 // false because the same launch wrote them) into sQ/sR/sF, each
@@ -91,7 +107,6 @@ __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, fl
     auto ld = [](const float *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
     const int nA = lat_extent(g, T::A);
-    const float *NF = g.FEG32 + (size_t)D * 5 * N;
     for (int m = threadIdx.x; m < S; m += blockDim.x) {
         int b, a;
         T::staged(m, b, a);
@@ -101,11 +116,13 @@ __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, fl
         c[T::B] = at.cB;
         const int node = c[0] + g.ni * (c[1] + g.nj * c[2]);
         const int e = T::at(b, a);
+        float f[5];
+        lat_node_flux<D, RO>(g, node, f);
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
             sQ[q * S + e] = ld(g.Q32 + q * N + node);
             sR[q * S + e] = ld(g.R32 + q * N + node);
-            sF[q * S + e] = ld(NF + q * N + node);
+            sF[q * S + e] = f[q];
         }
     }
     __syncthreads();

@@ -16,7 +16,7 @@ namespace cfd {
 // two FP32 numbers (hi + lo, about 48 significant bits) in the same bytes as
 // the FP64 form's [5][N] doubles: hi at [c][N], lo at [5 + c][N].  Split
 // form: U0/U1/U2 are the FP64 form's doubles, the stage intermediates FP32
-// (Q32, R32, FEG32, V32) except the face fluxes Fh (FP64).
+// (Q32, R32, V32) except the face fluxes Fh (FP64).
 struct LatView {
     int ni, nj, nk, N;
     Phys P;
@@ -38,7 +38,7 @@ struct LatView {
     const double *kn;          // [9][N] unit normals of the faces
     const double *del;         // [N] 1 / det^(1/3) (null: evaluated where it is used)
     // FP32 stage intermediates (mixed form)
-    float *Q32, *R32, *FEG32, *V32, *Fh32;
+    float *Q32, *R32, *V32, *Fh32;
     unsigned *flags;           // error word of this lattice
     double *Lout;              // optional [5][N] right-hand side output
     // Non-periodic directions: bit d of `per` set = direction d periodic.

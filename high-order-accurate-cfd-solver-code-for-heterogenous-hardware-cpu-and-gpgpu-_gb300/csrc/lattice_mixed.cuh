@@ -117,9 +117,9 @@ __device__ __forceinline__ void store_state(const LatView &g, int q, int n, cons
 }
 
 // U_Q of the next stage from the state Un (= det * Q): the inputs of the
-// face stage -- Q, the Roe inputs (u, v, w, sqrt(rho), H), the contravariant
-// node fluxes -- and the pressure (prim32); the viscous pass takes rho from
-// Q and u, v, w from the Roe inputs, and FLOW leaves through flow_out_node.
+// face stage -- Q, the Roe inputs (u, v, w, sqrt(rho), H) and the pressure
+// (prim32); the viscous pass takes rho from Q and u, v, w from the Roe
+// inputs, and FLOW leaves through flow_out_node.
 __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
 {
     const int N = g.N;
@@ -147,18 +147,6 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
     g.R32[2 * N + n] = w;
     g.R32[3 * N + n] = fsqrt(rho);
     g.R32[4 * N + n] = q4.h + (q4.l + pr);     // H = E/rho + p/rho
-    float m[9];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
-    const float prim[5] = {rho, u, v, w, p};
-    float Fx[5], Ex[5], Gx[5];
-    node_inviscid_flux(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        g.FEG32[(0 * 5 + c) * N + n] = Fx[c];
-        g.FEG32[(1 * 5 + c) * N + n] = Ex[c];
-        g.FEG32[(2 * 5 + c) * N + n] = Gx[c];
-    }
 }
 
 // U_Q from the FP64 FLOW (after an upload): U = det * Q(FLOW) in FP64, split
@@ -273,7 +261,7 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
     float Fv[5], Ev[5], Gv[5], mu;
     viscous_node_flux(dU, Ui, m, g.node32[9 * N + n], g.node32[10 * N + n], prim, KS, g.P, Fv, Ev, Gv, mu);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
+    for (int c = 1; c < 5; ++c) {   // mass has no viscous flux: component 0 stays as it was zeroed
         g.V32[(0 * 5 + c) * N + n] = Fv[c];
         g.V32[(1 * 5 + c) * N + n] = Ev[c];
         g.V32[(2 * 5 + c) * N + n] = Gv[c];
@@ -320,12 +308,12 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     float Fhat[5];
     x2::llf_face_flux2(P, g.fm32[(D * 3 + 0) * N + n], g.fm32[(D * 3 + 1) * N + n], g.fm32[(D * 3 + 2) * N + n],
                        g.fdet32[D * N + n], r, (float)g.P.eps, Fhat);
-    const float *NF = g.FEG32 + (size_t)D * 5 * N;
+    float NF[6][5];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) lat_node_flux<D, false>(g, s[o], NF[o]);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        float f[6];
-#pragma unroll
-        for (int o = 0; o < 6; ++o) f[o] = NF[c * N + s[o]];
+        const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
         g.Fh32[(D * 5 + c) * N + n] = __fadd_rn(Fhat[c], x2::face_correction_sym(f));
     }
 }
@@ -406,7 +394,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const int b = weno_visc_branch(L7);
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) {
+            for (int c = 1; c < 5; ++c) {
                 float f[7];
 #pragma unroll
                 for (int o = 0; o < 7; ++o) f[o] = ld(Vd + c * N + s[o]);
@@ -416,7 +404,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 0; c < 5; ++c)
+            for (int c = 1; c < 5; ++c)
                 Lf[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ld(Vd + c * N + p1) - ld(Vd + c * N + m1),
                                                 -(ld(Vd + c * N + p2) - ld(Vd + c * N + m2))), Lf[c]);
         }

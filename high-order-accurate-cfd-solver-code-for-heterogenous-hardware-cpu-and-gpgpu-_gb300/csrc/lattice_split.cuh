@@ -21,6 +21,7 @@
 #pragma once
 
 #include "boundary.h"
+#include "exact_div.cuh"
 #include "lattice.cuh"
 #include "lattice_mixed.cuh"
 #include "physics_x2.cuh"
@@ -45,8 +46,8 @@ __device__ __forceinline__ void store_state(const LatView &g, int q, int n, cons
 }
 
 // U_Q of the next stage from the state Un (= det * Q): Q in FP64, rounded
-// once to FP32 for the face stage; the Roe inputs (u, v, w, sqrt(rho), H),
-// the pressure and the contravariant node fluxes in FP32; and the state as
+// once to FP32 for the face stage; the Roe inputs (u, v, w, sqrt(rho), H)
+// and the pressure in FP32; and the state as
 // hi + lo FP32 pairs in g.Whl ([10][N]), a read copy from which the viscous
 // pass takes its neighbour differences on the FP32 pipe (the differences of
 // hi parts are exact between neighbours within a factor of two).
@@ -79,18 +80,6 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const double Un[
     g.R32[2 * N + n] = w;
     g.R32[3 * N + n] = fsqrt(rho);
     g.R32[4 * N + n] = __fmul_rn(q[4] + p, ir);   // H = (E + p) / rho
-    float m[9];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
-    const float prim[5] = {rho, u, v, w, p};
-    float Fx[5], Ex[5], Gx[5];
-    node_inviscid_flux(prim, m, g.node32[9 * N + n], Fx, Ex, Gx);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        g.FEG32[(0 * 5 + c) * N + n] = Fx[c];
-        g.FEG32[(1 * 5 + c) * N + n] = Ex[c];
-        g.FEG32[(2 * 5 + c) * N + n] = Gx[c];
-    }
 }
 
 // U = det * Q(FLOW) in FP64 (U_Q.cl:112-116) into slot q, then derive.
@@ -169,13 +158,12 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
         roe_average(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
                            R[N + l], R[2 * N + l], R[4 * N + l], r);
     }
-    const float *NF = g.FEG32 + (size_t)D * 5 * N;
-    float corr[5];
+    float NF[6][5], corr[5];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) lat_node_flux<D, false>(g, s[o], NF[o]);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        float f[6];
-#pragma unroll
-        for (int o = 0; o < 6; ++o) f[o] = NF[c * N + s[o]];
+        const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
         corr[c] = x2::face_correction_sym(f);
     }
     double Fh[5];
@@ -238,7 +226,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
     lat_ijk(g, n, i, j, k);
     const unsigned lflag = (LOC && g.locflag) ? g.locflag[n] : 7u;
     double Ld[5];   // sum of flux differences (= -L), started by the i direction's
-    float Lv[5] = {0.f, 0.f, 0.f, 0.f, 0.f};     // viscous divergence
+    float Lv[5] = {0.f, 0.f, 0.f, 0.f, 0.f};     // viscous divergence; mass has none
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int m1 = lat_step(g, i, j, k, d, -1);
@@ -259,7 +247,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const int b = weno_visc_branch(L7);
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) {
+            for (int c = 1; c < 5; ++c) {
                 float f[7];
 #pragma unroll
                 for (int o = 0; o < 7; ++o) f[o] = ldf(Vd + c * N + s[o]);
@@ -269,13 +257,13 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
             const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 0; c < 5; ++c)
+            for (int c = 1; c < 5; ++c)
                 Lv[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ldf(Vd + c * N + p1) - ldf(Vd + c * N + m1),
                                                 -(ldf(Vd + c * N + p2) - ldf(Vd + c * N + m2))), Lv[c]);
         }
     }
 #pragma unroll
-    for (int c = 0; c < 5; ++c) Ld[c] += emu::f2d(Lv[c]);
+    for (int c = 1; c < 5; ++c) Ld[c] += emu::f2d(Lv[c]);
     if (g.Lout) {
 #pragma unroll
         for (int c = 0; c < 5; ++c) g.Lout[c * N + n] = -Ld[c];
@@ -290,13 +278,12 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
         double U1[5];
         load_state(g, 1, n, U1);
 #pragma unroll
-        for (int c = 0; c < 5; ++c) Un[c] = fma(0.75, U0[c], fma(0.25, U1[c], (-0.25 * dt) * Ld[c]));
+        for (int c = 0; c < 5; ++c) Un[c] = xdiv::scale2<-2>(fma(3.0, U0[c], fma(-dt, Ld[c], U1[c])));
     } else {
         double U2[5];
         load_state(g, 2, n, U2);
 #pragma unroll
-        for (int c = 0; c < 5; ++c)
-            Un[c] = fma(1.0 / 3.0, U0[c], fma(2.0 / 3.0, U2[c], (-2.0 / 3.0 * dt) * Ld[c]));
+        for (int c = 0; c < 5; ++c) Un[c] = emu::mul(1.0 / 3.0, fma(2.0, fma(-dt, Ld[c], U2[c]), U0[c]));
     }
     store_state(g, jst == 2 ? 0 : jst + 1, n, Un);
     derive(g, n, Un);

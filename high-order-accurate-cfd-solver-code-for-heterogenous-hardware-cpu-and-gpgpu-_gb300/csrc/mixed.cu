@@ -302,7 +302,7 @@ void mixed_face_pass(const StructuredLaunch &S, int d, int tile, cudaStream_t st
 namespace {
 
 // rho = 1, zero velocity, p = 1: the FP32 face inputs of a uniform state
-__global__ void k_uniform_inputs(float *Q32, float *R32, float *FEG32, long long N)
+__global__ void k_uniform_inputs(float *Q32, float *R32, float *p32, long long N)
 {
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
@@ -312,8 +312,7 @@ __global__ void k_uniform_inputs(float *Q32, float *R32, float *FEG32, long long
         Q32[c * N + n] = q[c];
         R32[c * N + n] = r[c];
     }
-#pragma unroll
-    for (int c = 0; c < 15; ++c) FEG32[c * N + n] = 0.0f;
+    p32[n] = 1.0f;
 }
 
 }  // namespace
@@ -321,7 +320,7 @@ __global__ void k_uniform_inputs(float *Q32, float *R32, float *FEG32, long long
 void reduced_uniform_inputs(const StructuredLaunch &S, cudaStream_t st)
 {
     const long long N = (long long)S.ni * S.nj * S.nk;
-    k_uniform_inputs<<<blocks_for(N, 256), 256, 0, st>>>(S.Q32, S.R32, S.FEG32, N);
+    k_uniform_inputs<<<blocks_for(N, 256), 256, 0, st>>>(S.Q32, S.R32, S.prim32 + LF_P * N, N);
 }
 
 }  // namespace cfd

@@ -293,25 +293,21 @@ __device__ __forceinline__ void viscous_node_flux(const float dU[3][5], const fl
     }
 }
 
-// Contravariant node inviscid fluxes F, E, G (x det) from the primitives,
-// Viscous.cl:560-578 and 615-631, in FP32: det (m_d . U) q + p det m_d.
-__device__ __forceinline__ void node_inviscid_flux(const float prim[5], const float m[9], float det, float F[5],
-                                                   float E[5], float G[5])
+// Contravariant node inviscid flux along one direction (x det) from the
+// primitives, Viscous.cl:560-578 and 615-631, in FP32:
+// det (m . U) q + p det m.
+__device__ __forceinline__ void node_inviscid_flux(const float prim[5], const float m[3], float det, float o[5])
 {
     const float rho = prim[0], u = prim[1], v = prim[2], w = prim[3], p = prim[4];
     const float ke = __fmul_rn(__fmul_rn(0.5f, rho), dot3(u, u, v, v, w, w));
     const float Et = fmaf(p, 3.5f, ke);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        float *o = d == 0 ? F : (d == 1 ? E : G);
-        const float mx = __fmul_rn(det, m[3 * d]), my = __fmul_rn(det, m[3 * d + 1]), mz = __fmul_rn(det, m[3 * d + 2]);
-        const float un = dot3(mx, u, my, v, mz, w), ru = __fmul_rn(rho, un);
-        o[0] = ru;
-        o[1] = dot2(ru, u, mx, p);
-        o[2] = dot2(ru, v, my, p);
-        o[3] = dot2(ru, w, mz, p);
-        o[4] = __fmul_rn(Et, un);
-    }
+    const float mx = __fmul_rn(det, m[0]), my = __fmul_rn(det, m[1]), mz = __fmul_rn(det, m[2]);
+    const float un = dot3(mx, u, my, v, mz, w), ru = __fmul_rn(rho, un);
+    o[0] = ru;
+    o[1] = dot2(ru, u, mx, p);
+    o[2] = dot2(ru, v, my, p);
+    o[3] = dot2(ru, w, mz, p);
+    o[4] = __fmul_rn(Et, un);
 }
 
 }  // namespace cfd

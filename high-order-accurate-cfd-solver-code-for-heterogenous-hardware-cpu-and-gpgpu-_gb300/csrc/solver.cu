@@ -136,7 +136,7 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
     for (int q = 0; q < 3; ++q)
         if ((st = dalloc_t(s, 5 * N, &S.U[q]))) return st;
     if (s->form == CFD_PREC_SPLIT) {   // FP32 stage intermediates, FP64 face fluxes
-        if ((st = dalloc_t(s, 5 * N, &S.Q32)) || (st = dalloc_t(s, 5 * N, &S.R32)) || (st = dalloc_t(s, 15 * N, &S.FEG32))
+        if ((st = dalloc_t(s, 5 * N, &S.Q32)) || (st = dalloc_t(s, 5 * N, &S.R32))
             || (st = dalloc_t(s, 15 * N, &S.V32)) || (st = dalloc_t(s, 15 * N, &S.Fh))
             || (st = dalloc_t(s, 9 * N, &S.fm32)) || (st = dalloc_t(s, 11 * N, &S.node32))
             || (st = dalloc_t(s, N, &S.idet64)) || (st = dalloc_t(s, 9 * N, &S.prim32))
@@ -144,7 +144,7 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
             return st;
         cudaMemsetAsync(S.V32, 0, 15 * N * sizeof(float), S.stream);
     } else if (s->mixed) {   // FP32 stage intermediates
-        if ((st = dalloc_t(s, 5 * N, &S.Q32)) || (st = dalloc_t(s, 5 * N, &S.R32)) || (st = dalloc_t(s, 15 * N, &S.FEG32))
+        if ((st = dalloc_t(s, 5 * N, &S.Q32)) || (st = dalloc_t(s, 5 * N, &S.R32))
             || (st = dalloc_t(s, 15 * N, &S.V32)) || (st = dalloc_t(s, 15 * N, &S.Fh32))
             || (st = dalloc_t(s, 9 * N, &S.fm32)) || (st = dalloc_t(s, 3 * N, &S.fdet32))
             || (st = dalloc_t(s, 11 * N, &S.node32)) || (st = dalloc_t(s, 2 * N, &S.idet32))

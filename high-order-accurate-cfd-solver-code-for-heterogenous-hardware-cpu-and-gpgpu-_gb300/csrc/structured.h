@@ -35,7 +35,6 @@ struct StructuredLaunch {
     // mixed-precision form (FP32 stage intermediates, mixed.cu)
     float *Q32 = nullptr;      // [5][N]
     float *R32 = nullptr;      // [5][N] u, v, w, sqrt(rho), H
-    float *FEG32 = nullptr;    // [3][5][N]
     float *V32 = nullptr;      // [3][5][N]
     float *Fh32 = nullptr;     // [3][5][N]
     float *fm32 = nullptr;     // [3][3][N]
@@ -137,7 +136,6 @@ inline LatView make_view(const StructuredLaunch &S, double dt, double *Lout)
     g.Fh = S.Fh;
     g.Q32 = S.Q32;
     g.R32 = S.R32;
-    g.FEG32 = S.FEG32;
     g.V32 = S.V32;
     g.Fh32 = S.Fh32;
     g.flags = S.flags;
@@ -173,7 +171,7 @@ int fp64_faces(const StructuredLaunch &S, const LatView &g, cudaStream_t st,
 
 // One face pass along d with face tiles of width `tile` (the tuner's
 // candidates, mixed.cu / split.cu), and a uniform state in the FP32 face
-// inputs (Q32, R32, FEG32) for timing them before any state exists.
+// inputs (Q32, R32, pressure) for timing them before any state exists.
 void mixed_face_pass(const StructuredLaunch &S, int d, int tile, cudaStream_t st);
 void split_face_pass(const StructuredLaunch &S, int d, int tile, cudaStream_t st);
 void reduced_uniform_inputs(const StructuredLaunch &S, cudaStream_t st);
