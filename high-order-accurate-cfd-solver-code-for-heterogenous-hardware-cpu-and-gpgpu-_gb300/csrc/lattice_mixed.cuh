@@ -307,10 +307,13 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     }
     float Fhat[5];
     x2::llf_face_flux2(P, g.fm32[(D * 3 + 0) * N + n], g.fm32[(D * 3 + 1) * N + n], g.fm32[(D * 3 + 2) * N + n],
-                       g.fdet32[D * N + n], r, (float)g.P.eps, Fhat);
+                       g.fdet32[D * N + n], r, x2::weno_eps2(g.P), Fhat);
     float NF[6][5];
 #pragma unroll
-    for (int o = 0; o < 6; ++o) lat_node_flux<D, false>(g, s[o], NF[o]);
+    for (int o = 0; o < 6; ++o) {
+        const NodeIn in = lat_node_in<D, false>(g, s[o]);
+        node_inviscid_flux(in.prim, in.m, in.det, NF[o]);
+    }
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
@@ -328,16 +331,22 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
 {
     constexpr int S = T::kStaged;
     float *sQ = smem, *sR = smem + 5 * S, *sF = smem + 10 * S;
-    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
-    int n, t, a;
-    if (!tile_face<T, D>(g, at, n, t, a)) return;
     const int N = g.N;
+    int n, t, a;
+    const bool face = tile_face<T, D>(g, at, n, t, a);
+    float m[3] = {0.f, 0.f, 0.f}, det_f = 0.f;   // loaded while the staging waits
+    if (face) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[c] = __ldg(g.fm32 + (D * 3 + c) * N + n);
+        det_f = __ldg(g.fdet32 + D * N + n);
+    }
+    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
+    if (!face) return;
     float2 P[3][5];
     float r[5];
     tile_stencil<T>(sQ, sR, t, a, P, r);
     float Fhat[5];
-    x2::llf_face_flux2(P, g.fm32[(D * 3 + 0) * N + n], g.fm32[(D * 3 + 1) * N + n], g.fm32[(D * 3 + 2) * N + n],
-                       g.fdet32[D * N + n], r, (float)g.P.eps, Fhat);
+    x2::llf_face_flux2(P, m[0], m[1], m[2], det_f, r, x2::weno_eps2(g.P), Fhat);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         float f[6];

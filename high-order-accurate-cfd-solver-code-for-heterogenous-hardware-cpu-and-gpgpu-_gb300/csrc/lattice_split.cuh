@@ -9,7 +9,7 @@
 // average (Weno.cl:2585-2728, 2913-2947; physics_x2.cuh
 // llf_face_flux2_split), and the flux difference L (Weno.cl:3060-3082).
 // FP32: the Roe average, eigenvectors, characteristic projection, WENO5 (on
-// the stencil's deviation from the face's left node), back-projection, the
+// the stencil's differences), back-projection, the
 // face states' velocities and pressures, lambda_5 and the LLF dissipation
 // alpha (q+ - q-), the viscous and SGS fluxes and their divergence
 // (Viscous.cl:439-631, the mixed form's code on a hi + lo FP32 read copy of
@@ -124,14 +124,28 @@ __host__ __device__ __forceinline__ LatView hilo_view(const LatView &g)
 // The FP64 face flux of face n+1/2 along D from its stencil (P, pairs of
 // points k and 5-k) and Roe state r, plus corr, the FP32 sixth-order
 // correction of each component.
+struct FaceMetric {
+    double m[3], det;
+    float m32[3];
+};
 template <int D>
-__device__ __forceinline__ void face_flux(const LatView &g, int n, const float2 P[3][5], const float r[5],
-                                          const float corr[5], double out[5])
+__device__ __forceinline__ FaceMetric face_metric(const LatView &g, int n)
 {
     const int N = g.N;
-    const double dm[3] = {g.fm[(D * 3 + 0) * N + n], g.fm[(D * 3 + 1) * N + n], g.fm[(D * 3 + 2) * N + n]};
-    x2::llf_face_flux2_split(P, g.fm32[(D * 3 + 0) * N + n], g.fm32[(D * 3 + 1) * N + n],
-                             g.fm32[(D * 3 + 2) * N + n], dm, g.fdet[D * N + n], r, emu::d2f(g.P.eps), corr, out);
+    FaceMetric f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        f.m[c] = __ldg(g.fm + (D * 3 + c) * N + n);
+        f.m32[c] = __ldg(g.fm32 + (D * 3 + c) * N + n);
+    }
+    f.det = __ldg(g.fdet + D * N + n);
+    return f;
+}
+
+__device__ __forceinline__ void face_flux(const LatView &g, const FaceMetric &f, const float2 P[3][5], const float r[5],
+                                          const float corr[5], double out[5])
+{
+    x2::llf_face_flux2_split(P, f.m32[0], f.m32[1], f.m32[2], f.m, f.det, r, x2::weno_eps2(g.P), corr, out);
 }
 
 // Face n+1/2 along D with its stencil read from the lattice (the batched
@@ -160,14 +174,17 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
     }
     float NF[6][5], corr[5];
 #pragma unroll
-    for (int o = 0; o < 6; ++o) lat_node_flux<D, false>(g, s[o], NF[o]);
+    for (int o = 0; o < 6; ++o) {
+        const NodeIn in = lat_node_in<D, false>(g, s[o]);
+        node_inviscid_flux(in.prim, in.m, in.det, NF[o]);
+    }
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
         corr[c] = x2::face_correction_sym(f);
     }
     double Fh[5];
-    face_flux<D>(g, n, P, r, corr, Fh);
+    face_flux(g, face_metric<D>(g, n), P, r, corr, Fh);
 #pragma unroll
     for (int c = 0; c < 5; ++c) g.Fh[(D * 5 + c) * N + n] = Fh[c];
 }
@@ -179,10 +196,10 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
 {
     constexpr int S = T::kStaged;
     float *sQ = smem, *sR = smem + 5 * S, *sF = smem + 10 * S;
-    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
-    int n, t, a;
-    if (!tile_face<T, D>(g, at, n, t, a)) return;
     const int N = g.N;
+    int n, t, a;
+    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
+    if (!tile_face<T, D>(g, at, n, t, a)) return;
     float2 P[3][5];
     float r[5];
     tile_stencil<T>(sQ, sR, t, a, P, r);
@@ -194,7 +211,7 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
         corr[q] = x2::face_correction_sym(f);
     }
     double Fh[5];
-    face_flux<D>(g, n, P, r, corr, Fh);
+    face_flux(g, face_metric<D>(g, n), P, r, corr, Fh);
 #pragma unroll
     for (int q = 0; q < 5; ++q) g.Fh[(D * 5 + q) * N + n] = Fh[q];
 }
