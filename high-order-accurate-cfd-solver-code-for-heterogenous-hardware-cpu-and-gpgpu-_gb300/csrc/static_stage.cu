@@ -32,7 +32,8 @@ namespace {
 // doubles per lattice node held in the scratch array:
 //   geometry SoA 22 (9 node metrics, det, 3x3 face metrics, 3 face dets),
 //   FLOW 9, U0/U1/U2 15, Q 5, node fluxes 15, viscous fluxes 15,
-//   sqrt(rho) and H 2, face fluxes 15, L 5
+//   sqrt(rho) and its products with u, v, w, H 5, unit normals 9, filter
+//   width 1, hand-over between the face kernels 126, face fluxes 15, L 5
 constexpr size_t kPerNode = 22 + 9 + 15 + 5 + 15 + 15 + 5 + 9 + 1 + 3 * kFaceScratch + 15 + 5;   // 242
 constexpr size_t kFlagDoubles = 32;                                    // 256 B for the error word
 constexpr size_t kScratchDoubles = (size_t)CFD_STATIC_MAX_NODES * kPerNode + kFlagDoubles;
@@ -62,36 +63,56 @@ cfd_status_t scratch_address(double **out)
     return CFD_OK;
 }
 
-// rows 1..N of an AoS buffer (row stride `stride` doubles, columns
-// offset..offset+ncomp-1) <-> SoA [ncomp][N]
-__global__ void k_cols_to_soa(const double *__restrict__ aos, int stride, int offset, int ncomp, long long N,
-                              double *__restrict__ soa)
+// The stage's inputs and results in the reference layout, rows 1..N.
+struct Rows {
+    const double *det, *deter, *metric;
+    double *U[3], *flow, *L;
+};
+
+// Reference rows -> SoA in one launch, a thread per node and component, and
+// the error word to zero.  Components of a node, in the order of the scratch
+// array's first 46 rows: det after the 9 node metrics, the 3x3 face
+// metrics, 3 face dets, FLOW, U0, U1, U2.  On a few thousand nodes a launch
+// costs 3 us whatever it moves: twelve of them, a memset and four for the
+// results were 55 of the 222 us of a stage on 17^3 nodes.
+constexpr int kIn = 46;
+__global__ void __launch_bounds__(256) k_rows_to_soa(Rows R, long long N, double *__restrict__ soa, unsigned *flags)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N * ncomp) return;
-    const long long n = t / ncomp;
-    const int c = (int)(t % ncomp);
-    soa[c * N + n] = aos[(n + 1) * stride + offset + c];
+    if (t == 0) *flags = 0;
+    if (t >= N * kIn) return;
+    const long long n = t / kIn, r = n + 1;
+    const int c = (int)(t % kIn);
+    double v;
+    if (c < 9) v = R.metric[r * 63 + c];
+    else if (c == 9) v = R.det[r];
+    else if (c < 19) {
+        const int d = (c - 10) / 3;
+        v = R.metric[r * 63 + 9 * (1 + 2 * d) + (c - 10)];   // row d of the face metric of face d
+    } else if (c < 22) v = R.deter[r * 6 + 2 * (c - 19)];
+    else if (c < 31) v = R.flow[r * 9 + (c - 22)];
+    else {
+        const int q = (c - 31) / 5;
+        v = R.U[q][r * 5 + (c - 31) % 5];
+    }
+    soa[c * N + n] = v;
 }
 
-__global__ void k_soa_to_cols(const double *__restrict__ soa, int stride, int offset, int ncomp, long long N,
-                              double *__restrict__ aos)
+// Results back into the caller's rows: FLOW, U_j (U_Q's output), the U the
+// stage advanced, and L.
+__global__ void __launch_bounds__(256)
+k_soa_to_rows(Rows R, long long N, const double *__restrict__ flow, const double *__restrict__ Uj, int j,
+              const double *__restrict__ Ua, int advanced, const double *__restrict__ L)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N * ncomp) return;
-    const long long n = t / ncomp;
-    const int c = (int)(t % ncomp);
-    aos[(n + 1) * stride + offset + c] = soa[c * N + n];
-}
-
-void to_soa(cudaStream_t st, const double *aos, int stride, int offset, int ncomp, long long N, double *soa)
-{
-    k_cols_to_soa<<<blocks_for(N * ncomp, 256), 256, 0, st>>>(aos, stride, offset, ncomp, N, soa);
-}
-
-void from_soa(cudaStream_t st, const double *soa, int stride, int offset, int ncomp, long long N, double *aos)
-{
-    k_soa_to_cols<<<blocks_for(N * ncomp, 256), 256, 0, st>>>(soa, stride, offset, ncomp, N, aos);
+    if (t >= N * 9) return;
+    const long long n = t / 9, r = n + 1;
+    const int c = (int)(t % 9);
+    R.flow[r * 9 + c] = flow[c * N + n];
+    if (c >= 5) return;
+    R.U[j][r * 5 + c] = Uj[c * N + n];
+    R.U[advanced][r * 5 + c] = Ua[c * N + n];
+    if (R.L) R.L[r * 5 + c] = L[c * N + n];
 }
 
 }  // namespace
@@ -129,11 +150,10 @@ extern "C" cfd_status_t cfd_lattice_stage_static(void *cuda_stream, int32_t ni, 
     S.stream = st;
     S.P = make_phys(params);
     S.mixed = 0;
-    double *m9 = take(9), *dt_ = take(1), *fm = take(9), *fdet = take(3);
-    S.m9 = m9;
-    S.det = dt_;
-    S.fm = fm;
-    S.fdet = fdet;
+    S.m9 = take(9);   // the inputs, in k_rows_to_soa's order
+    S.det = take(1);
+    S.fm = take(9);
+    S.fdet = take(3);
     S.prim9 = take(9);
     S.U[0] = take(5);
     S.U[1] = take(5);
@@ -150,37 +170,19 @@ extern "C" cfd_status_t cfd_lattice_stage_static(void *cuda_stream, int32_t ni, 
     double *Lsoa = take(5);
     S.flags = (unsigned *)(base + (size_t)CFD_STATIC_MAX_NODES * kPerNode);
 
-    // the error word must start at zero; every other region is written
-    // before it is read within this call
-    cudaError_t e = cudaMemsetAsync(S.flags, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return CFD_ECUDA;
-
-    // reference layout (rows 1..N) -> SoA
-    to_soa(st, det, 1, 0, 1, N, dt_);
-    to_soa(st, (const double *)metric, 63, 0, 9, N, m9);
-    for (int d = 0; d < 3; ++d) {
-        to_soa(st, (const double *)metric, 63, 9 * (1 + 2 * d) + 3 * d, 3, N, fm + (size_t)3 * d * N);
-        to_soa(st, (const double *)deter, 6, 2 * d, 1, N, fdet + (size_t)d * N);
-    }
-    to_soa(st, (const double *)FLOW, 9, 0, 9, N, S.prim9);
-    to_soa(st, (const double *)U0, 5, 0, 5, N, S.U[0]);
-    to_soa(st, (const double *)U1, 5, 0, 5, N, S.U[1]);
-    to_soa(st, (const double *)U2, 5, 0, 5, N, S.U[2]);
+    // every region is written before it is read within this call
+    const Rows R{det, (const double *)deter, (const double *)metric,
+                 {(double *)U0, (double *)U1, (double *)U2}, (double *)FLOW, (double *)L_out};
+    k_rows_to_soa<<<blocks_for(N * kIn, 256), 256, 0, st>>>(R, N, base, S.flags);
 
     fp64_geometry(S);
     structured_stage(S, j, del_t, L_out ? Lsoa : nullptr);
 
-    // results back into the caller's buffers: FLOW, U_j (U_Q's output),
-    // the U the stage advanced, and L
-    cfd_column_t *Ucaller[3] = {U0, U1, U2};
     const int advanced = j == 0 ? 1 : (j == 1 ? 2 : 0);
-    from_soa(st, S.prim9, 9, 0, 9, N, (double *)FLOW);
-    from_soa(st, S.U[j], 5, 0, 5, N, (double *)Ucaller[j]);
-    from_soa(st, S.U[advanced], 5, 0, 5, N, (double *)Ucaller[advanced]);
-    if (L_out) from_soa(st, Lsoa, 5, 0, 5, N, (double *)L_out);
+    k_soa_to_rows<<<blocks_for(N * 9, 256), 256, 0, st>>>(R, N, S.prim9, S.U[j], j, S.U[advanced], advanced, Lsoa);
 
     // peek, not get: a failed launch stays readable by the caller's own checks
-    e = cudaPeekAtLastError();
+    cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess) return CFD_ECUDA;
     unsigned flags = 0;
     e = cudaMemcpyAsync(&flags, S.flags, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
