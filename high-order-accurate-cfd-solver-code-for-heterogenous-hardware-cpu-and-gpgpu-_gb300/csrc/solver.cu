@@ -218,6 +218,10 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
         fp64_geometry(S);
         s->ctx->launches += 1;
     }
+    if (cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking) != cudaSuccess
+        || cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming) != cudaSuccess
+        || cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming) != cudaSuccess)
+        return cuda_fail(s->ctx, cudaGetLastError(), "solver side stream");
     if (s->mixed) {
         if (s->form == CFD_PREC_SPLIT) {
             split_geometry(S);
@@ -226,10 +230,6 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
             mixed_geometry(S);
             s->ctx->launches += kMixedGeometryLaunches;
         }
-        if (cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking) != cudaSuccess
-            || cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming) != cudaSuccess
-            || cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming) != cudaSuccess)
-            return cuda_fail(s->ctx, cudaGetLastError(), "solver side stream");
         for (int f = 0; f < 2; ++f)
             if (cudaStreamCreateWithFlags(&S.face_side[f], cudaStreamNonBlocking) != cudaSuccess
                 || cudaEventCreateWithFlags(&S.face_join[f], cudaEventDisableTiming) != cudaSuccess)

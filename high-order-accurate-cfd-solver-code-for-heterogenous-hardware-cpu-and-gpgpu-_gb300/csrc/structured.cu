@@ -110,12 +110,24 @@ int structured_stage(const StructuredLaunch &S, int jst, double dt, double *Lout
     const bool fp = g.N <= kPlainNodes;   // products of the per-node kernels on the FP64 pipe
     (fp ? k_prep<false> : k_prep<true>)<<<nb, 128, 0, st>>>(g, jst);
     mark("prep");
+    // The viscous and the face kernels are independent (the update reads
+    // both): side by side the one's latency hides behind the other's work.
+    // A stage on 17^3 nodes 107 -> 86 us, 24^3 155 -> 134, 46^3 675 -> 645,
+    // 128^3 12.43 -> 12.41 ms.  Not when each launch is timed.
+    const bool side = S.side && !ev;
+    cudaStream_t sv = side ? S.side : st;
+    if (side) {
+        cudaEventRecord(S.fork, st);
+        cudaStreamWaitEvent(sv, S.fork, 0);
+    }
     if (S.P.viscous)
-        (fp ? k_visc<false> : k_visc<true>)<<<nb, 128, 0, st>>>(g, jst);
+        (fp ? k_visc<false> : k_visc<true>)<<<nb, 128, 0, sv>>>(g, jst);
     else
-        k_mu_only<<<nb, 128, 0, st>>>(g, jst);
+        k_mu_only<<<nb, 128, 0, sv>>>(g, jst);
+    if (side) cudaEventRecord(S.join, sv);
     mark(S.P.viscous ? "viscous" : "mu_only");
     k = 3 + fp64_faces(S, g, st, mark);
+    if (side) cudaStreamWaitEvent(st, S.join, 0);
     (fp ? k_update<false> : k_update<true>)<<<nb, 128, 0, st>>>(g, jst);
     mark("update");
     return ev ? entries : k;

@@ -44,7 +44,7 @@ struct StructuredLaunch {
     double *idet64 = nullptr;  // [N] 1/det (split form)
     float *Whl = nullptr;      // [10][N] hi/lo read copy of the stage's state (split form)
     float *prim32 = nullptr;   // [9][N] FP32 pressure (LF_P) and mu (LF_MU) of the stage
-    // mixed form: side stream and fork/join events for the viscous pass,
+    // side stream and fork/join events for the viscous pass,
     // and two more for the j and k face passes (null: everything on `stream`)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
