@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "cfd_rhs.h"
+#include "exact_int.cuh"
 #include "lattice.cuh"
 
 namespace cfd {
@@ -139,56 +140,43 @@ void bc_apply_split(cudaStream_t st, const BcDevice &bc, const LatView &g, int q
 // negated; node rules copy their source (zero velocity on walls and tips);
 // a singular mirror pass writes ghost m from singular-chain node m with the
 // velocity negated.  Outside a group each target depends only on nodes the
-// entry does not write.  St provides prims(n, rho, u, v, w, p, t) and
-// set(n, rho, u, v, w, p).
+// entry does not write.
+// A rule that copies a node takes its state U over, by the quotient of the
+// two Jacobians (U = det Q): rho, u, v, w and p need not be formed, which
+// leaves one quotient (on the integer pipe) and five products where they
+// took eight quotients and some fifty operations of the FP64 pipe: a block
+// of 256 x 64 x 16 with ghost layers 16.4 -> 10.2 us.
+// St provides U(n, U[5]) and put(n, U[5]) (FP64), det(n) and set(n, rho, u,
+// v, w, p).
 template <class St>
 __device__ __forceinline__ void bc_target_rules(const St &S, int type, const BcEntry &e, int m, double mach)
 {
-    const double gm2 = 1.4 * mach * mach;
-    double rho, u, v, w, p, t;
     const int cls = bc_class(e);
-    if (cls == BC_EDGE) {
-        if (m != 0) return;
-        S.prims(e.s[0], rho, u, v, w, p, t);
-        if (bc_no_slip(type)) u = v = w = 0.0;
-        S.set(e.b, gm2 * (p / t), u, v, w, p);
-        return;
-    }
-    if (cls == BC_MIRROR) {
-        if (m == 0) return;
-        const int node = e.g[m - 1];
-        for (int k = m; k < 3; ++k)
-            if (e.g[k] == node) return;
-        S.prims(e.s[m - 1], rho, u, v, w, p, t);
-        S.set(node, rho, -u, -v, -w, p);
-        return;
-    }
+    if (cls == BC_EDGE ? m != 0 : cls == BC_MIRROR && m == 0) return;
     const int node = m == 0 ? e.b : e.g[m - 1];
     // the routine writes the targets in order: when a collapsed chain names a
     // node twice, the later target's write stands
-    for (int k = m; k < 3; ++k)
-        if (e.g[k] == node) return;
-    if (type == BC_INLET || type == BC_OUTLET) {   // node and ghosts alike
-        if (type == BC_INLET) {
-            u = 1.0;
-            v = w = 0.0;
-            p = 1.0 / gm2;
-            t = 1.0;
-        } else {
-            S.prims(e.s[0], rho, u, v, w, p, t);
-        }
-        S.set(node, gm2 * (p / t), u, v, w, p);
+    if (cls != BC_EDGE)
+        for (int k = m; k < 3; ++k)
+            if (e.g[k] == node) return;
+    if (cls == BC_FACE && type == BC_INLET) {   // node and ghosts alike
+        const double gm2 = 1.4 * mach * mach, p = 1.0 / gm2;
+        S.set(node, gm2 * p, 1.0, 0.0, 0.0, p);
         return;
     }
-    // boundary (mirror copy) and wall (no slip): ghost m from inward node m,
-    // the node itself from the first inward node
-    S.prims(e.s[m == 0 ? 0 : m - 1], rho, u, v, w, p, t);
-    if (m == 0 && type == BC_WALL)
-        S.set(node, gm2 * (p / t), 0.0, 0.0, 0.0, p);
-    else if (type == BC_WALL)
-        S.set(node, rho, -u, -v, -w, p);
-    else
-        S.set(node, rho, u, v, w, p);
+    const bool outlet = cls == BC_FACE && type == BC_OUTLET;   // node and ghosts from the first inward node
+    const int src = e.s[m == 0 || outlet ? 0 : m - 1];
+    const bool still = m == 0 && (cls == BC_EDGE ? bc_no_slip(type) : type == BC_WALL);
+    const bool negate = m != 0 && (cls == BC_MIRROR || type == BC_WALL);
+    double U[5];
+    S.U(src, U);
+    const double k = xi::divide(S.det(node), S.det(src)), kv = still ? 0.0 : (negate ? -k : k);
+    if (still) U[4] = fma(-0.5, xi::divide(fma(U[1], U[1], fma(U[2], U[2], U[3] * U[3])), U[0]), U[4]);
+    U[0] *= k;
+    U[4] *= k;
+#pragma unroll
+    for (int c = 1; c < 4; ++c) U[c] *= kv;
+    S.put(node, U);
 }
 
 }  // namespace cfd

@@ -62,8 +62,7 @@ Phys make_phys(const cfd_params_t *p);
 // their products on the FP64 pipe (physics_exact.cuh products).  The three
 // together, on the FP64 pipe against the integer pipe: 24^3 nodes 61 and
 // 75 us, 53,000 with ghost layers 110 and 125, 40^3 128 and 128, 46^3 182
-// and 169, 64^3
-// 400 and 328.
+// and 169, 64^3 400 and 328.
 #ifndef CFD_PLAIN_NODES
 #define CFD_PLAIN_NODES 64000
 #endif

@@ -455,63 +455,39 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 
 // ------------------------------------------------ boundary routine ---
 
-// FP64 primitives of the hi/lo state of node n in slot q.
-__device__ __forceinline__ void state_prims(const LatView &g, int q, int n, double mach, double &rho, double &u,
-                                            double &v, double &w, double &p, double &t)
-{
-    const int N = g.N;
-    const float *W = lat_W(g, q);
-    double fu[5];
-    const double id = 1.0 / g.det[n];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) fu[c] = id * ((double)W[c * N + n] + (double)W[(5 + c) * N + n]);
-    rho = fu[0];
-    u = fu[1] / fu[0];
-    v = fu[2] / fu[0];
-    w = fu[3] / fu[0];
-    const double e = fu[4] / fu[0] - 0.5 * (u * u + v * v + w * w);
-    p = e * rho * 0.4;
-    t = (1.4 * mach * mach) * (p / rho);
-}
-
-// Node n takes the state of primitives (rho, u, v, w, p) in slot q, and the
-// next stage's U_Q outputs.
-__device__ __forceinline__ void set_prims(const LatView &g, int q, int n, double rho, double u, double v, double w,
-                                          double p)
-{
-    const double D = g.det[n];
-    const double E = p / 0.4 + 0.5 * rho * (u * u + v * v + w * w);
-    const double U[5] = {D * rho, D * rho * u, D * rho * v, D * rho * w, D * E};
-    dfl Un[5];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        Un[c].h = (float)U[c];
-        Un[c].l = (float)(U[c] - (double)Un[c].h);
-    }
-    store_state(g, q, n, Un);
-    derive(g, n, Un);
-}
-
 // Target m of one entry of the reference's boundary routine
-// (bc_target_rules) on the hi/lo state in slot q.
+// (bc_target_rules) on the hi/lo state in slot q.  A node that is written
+// takes its state and the next stage's U_Q outputs.
 struct HiLoState {
     const LatView &g;
     int q;
-    double mach;
-    __device__ __forceinline__ void prims(int n, double &rho, double &u, double &v, double &w, double &p,
-                                          double &t) const
+    __device__ __forceinline__ double det(int n) const { return g.det[n]; }
+    __device__ __forceinline__ void U(int n, double U[5]) const
     {
-        state_prims(g, q, n, mach, rho, u, v, w, p, t);
+        const float *W = lat_W(g, q);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) U[c] = emu::f2d(W[c * g.N + n]) + emu::f2d(W[(5 + c) * g.N + n]);
+    }
+    __device__ __forceinline__ void put(int n, const double U[5]) const
+    {
+        dfl Un[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) emu::hi_lo(U[c], Un[c].h, Un[c].l);
+        store_state(g, q, n, Un);
+        derive(g, n, Un);
     }
     __device__ __forceinline__ void set(int n, double rho, double u, double v, double w, double p) const
     {
-        set_prims(g, q, n, rho, u, v, w, p);
+        const double D = g.det[n];
+        const double E = p / 0.4 + 0.5 * rho * (u * u + v * v + w * w);
+        const double U[5] = {D * rho, D * rho * u, D * rho * v, D * rho * w, D * E};
+        put(n, U);
     }
 };
 
 __device__ __forceinline__ void bc_target(const LatView &g, int type, const BcEntry &e, int m, int q, double mach)
 {
-    bc_target_rules(HiLoState{g, q, mach}, type, e, m, mach);
+    bc_target_rules(HiLoState{g, q}, type, e, m, mach);
 }
 
 // FP64 FLOW of the state in slot q (boundary output): the FP64 form's

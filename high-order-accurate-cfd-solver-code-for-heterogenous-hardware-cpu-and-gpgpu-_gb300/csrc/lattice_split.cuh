@@ -330,11 +330,12 @@ __device__ __forceinline__ void state_prims(const LatView &g, int q, int n, doub
 struct F64State {
     const LatView &g;
     int q;
-    double mach;
-    __device__ __forceinline__ void prims(int n, double &rho, double &u, double &v, double &w, double &p,
-                                          double &t) const
+    __device__ __forceinline__ double det(int n) const { return g.det[n]; }
+    __device__ __forceinline__ void U(int n, double U[5]) const { load_state(g, q, n, U); }
+    __device__ __forceinline__ void put(int n, const double U[5]) const
     {
-        state_prims(g, q, n, mach, rho, u, v, w, p, t);
+        store_state(g, q, n, U);
+        derive(g, n, U);
     }
     __device__ __forceinline__ void set(int n, double rho, double u, double v, double w, double p) const
     {
@@ -344,7 +345,7 @@ struct F64State {
 
 __device__ __forceinline__ void bc_target(const LatView &g, int type, const BcEntry &e, int m, int q, double mach)
 {
-    bc_target_rules(F64State{g, q, mach}, type, e, m, mach);
+    bc_target_rules(F64State{g, q}, type, e, m, mach);
 }
 
 // FP64 FLOW of the state in slot q (boundary output); mu from the last

@@ -72,6 +72,41 @@ def test_independent_lists_fill_in_one_launch(ctx, oracle_mod, variant, launches
     assert n == launches
 
 
+@pytest.mark.parametrize("ghost_chain", ["apart", "second_ghost_again", "back_to_the_node", "into_the_interior"])
+def test_entries_with_coinciding_nodes_fill_in_order(ctx, oracle_mod, ghost_chain):
+    """An entry's targets are written side by side only where its node,
+    ghosts and sources all differ; chains that name a node twice (here one
+    wall node's, rewired) give what the routine's own order gives."""
+    from cfd_gb300 import cases, runtime
+    c = cases.channel(ni=16, nj=12, nk=8)
+    a, bc = c.copy().arrays, c.bc
+    a["flow"][1:] = np.random.default_rng(7).uniform(0.5, 1.5, a["flow"][1:].shape)
+    g, b = a["grid"], int(bc.wall[len(bc.wall) // 2])
+    slot = next(f"N{k}" for k in range(6) if int(g[b][f"N{k}"]) > c.sd_node)   # towards the ghosts
+    inward = next(f"N{k}" for k in range(6) if k % 2 == int(slot[1]) % 2 and f"N{k}" != slot
+                  and int(g[b][f"N{k}"]) <= c.sd_node)
+    g1 = int(g[b][slot])
+    if ghost_chain == "second_ghost_again":
+        g2 = int(g[g1][slot])
+        g[slot][g2] = g2
+    elif ghost_chain == "back_to_the_node":
+        g[slot][g1] = b
+    elif ghost_chain == "into_the_interior":
+        g[slot][g1] = int(g[b][inward])
+    bnd = runtime.Boundary(ctx, g, bc)
+    dev = ctx.alloc(a["flow"].nbytes)
+    try:
+        ctx.write(dev, a["flow"])
+        bnd.fill(dev, c.params.mach, 1, c.sd_node)
+        out = np.empty_like(a["flow"])
+        ctx.read(out, dev)
+    finally:
+        ctx.free(dev)
+        bnd.close()
+    oracle_mod.boundary_fill(a, bc, c.params.mach, 1, c.sd_node)
+    assert np.array_equal(out, a["flow"])
+
+
 def test_singular_wall_node_is_unsupported(ctx):
     from cfd_gb300 import abi, runtime
     z, a, bc = golden_inputs()
