@@ -87,7 +87,7 @@ __device__ __forceinline__ void set_prims(const LatView &g, int q, int n, double
                                           double p)
 {
     const double D = g.det[n];
-    const double E = p / 0.4 + 0.5 * rho * (u * u + v * v + w * w);
+    const double E = xi::divide(p, 0.4) + 0.5 * rho * (u * u + v * v + w * w);
     const double Un[5] = {D * rho, D * rho * u, D * rho * v, D * rho * w, D * E};
     store_state(g, q, n, Un);
     derive(g, n, Un);
@@ -97,7 +97,7 @@ __device__ __forceinline__ void set_prims(const LatView &g, int q, int n, double
 __device__ __forceinline__ void init_node(const LatView &g, int n, int q)
 {
     const int N = g.N;
-    g.prim32[LF_MU * N + n] = (float)g.prim9[LF_MU * N + n];
+    g.prim32[LF_MU * N + n] = emu::d2f(g.prim9[LF_MU * N + n]);
     set_prims(g, q, n, g.prim9[LF_RHO * N + n], g.prim9[LF_U * N + n], g.prim9[LF_V * N + n], g.prim9[LF_W * N + n],
               g.prim9[LF_P * N + n]);
 }
@@ -308,25 +308,6 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 
 // ------------------------------------------------ boundary routine ---
 
-// FP64 primitives of the state of node n in slot q.
-__device__ __forceinline__ void state_prims(const LatView &g, int q, int n, double mach, double &rho, double &u,
-                                            double &v, double &w, double &p, double &t)
-{
-    const int N = g.N;
-    const double *U = lat_U(g, q);
-    double fu[5];
-    const double id = 1.0 / g.det[n];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) fu[c] = id * U[c * N + n];
-    rho = fu[0];
-    u = fu[1] / fu[0];
-    v = fu[2] / fu[0];
-    w = fu[3] / fu[0];
-    const double e = fu[4] / fu[0] - 0.5 * (u * u + v * v + w * w);
-    p = e * rho * 0.4;
-    t = (1.4 * mach * mach) * (p / rho);
-}
-
 struct F64State {
     const LatView &g;
     int q;
@@ -348,24 +329,12 @@ __device__ __forceinline__ void bc_target(const LatView &g, int type, const BcEn
     bc_target_rules(F64State{g, q}, type, e, m, mach);
 }
 
-// FP64 FLOW of the state in slot q (boundary output); mu from the last
-// viscous pass.
+// FP64 FLOW of the state in slot q (boundary output).
 __device__ __forceinline__ void flow_out_node(const LatView &g, int n, int q)
 {
-    const int N = g.N;
-    const double mach = g.P.mach;
-    double rho, u, v, w, p, t;
-    state_prims(g, q, n, mach, rho, u, v, w, p, t);
-    double *F = g.prim9;
-    F[LF_RHO * N + n] = rho;
-    F[LF_U * N + n] = u;
-    F[LF_V * N + n] = v;
-    F[LF_W * N + n] = w;
-    F[LF_E * N + n] = p / (0.4 * rho);
-    F[LF_P * N + n] = p;
-    F[LF_T * N + n] = t;
-    F[LF_A * N + n] = sqrt(1.4 * p / rho);
-    F[LF_MU * N + n] = (double)g.prim32[LF_MU * N + n];
+    double U[5];
+    load_state(g, q, n, U);
+    mx::flow_out<true>(g, n, g.idet64[n], U);
 }
 
 }  // namespace sp
