@@ -64,10 +64,10 @@ __global__ void __launch_bounds__(256) k_mu_m(LatView g, int q)
     if (n < g.N) mx::mu_node(g, n, q);
 }
 
-// 79 registers, no spills: a direction at 128^3 0.078 ms; 0.082 at 64
-// registers, 0.080 at 96.
+// 72 registers, no spills: a direction at 128^3 0.070 ms; 0.073 at 64
+// registers, 0.072 at 77, 0.078 at 94.
 #ifndef CFD_MFACE_MIN_BLOCKS
-#define CFD_MFACE_MIN_BLOCKS 6
+#define CFD_MFACE_MIN_BLOCKS 7
 #endif
 
 // Faces per tile along D (a block of 128 threads covers kTile x 128/kTile

@@ -67,66 +67,39 @@ __device__ __forceinline__ void roe_average(float sb, float ub, float vb, float 
 }
 
 // Roe eigen-system of one face (Weno.cl:337-413): k_bar = grad(zeta)/|grad(zeta)|
-// from the face metric, sound speed from the Roe state, left (Lm) and right
-// (R) eigenvector matrices of the Euler flux Jacobian along k_bar.
+// from the face metric, sound speed from the Roe state, and what the left and
+// right eigenvectors of the Euler flux Jacobian along k_bar are made of
+// (physics_x2.cuh left_times, right_times2).
 struct FaceEigen {
-    float kx, ky, kz, a, alpha, beta, theta, phi, ru, rv, rw, rr, irr, ia2;
+    float kx, ky, kz, ru, rv, rw, h2, g2;             // unit normal; Roe velocities, |u|^2/2; 0.4 / a^2
+    float ix, iy, iz, b4, ba, nx, ny, nz, al, ala, ae;
 
     __device__ __forceinline__ void init(float mx, float my, float mz, const float roe[5])
     {
         ru = roe[0];
         rv = roe[1];
         rw = roe[2];
-        const float rh = roe[3];
-        rr = roe[4];
+        const float rh = roe[3], rr = roe[4];
         const float ikk = frsqrt(dot3(mx, mx, my, my, mz, mz));
-        const float q2 = dot3(ru, ru, rv, rv, rw, rw);
-        a = fsqrt(__fmul_rn(0.4f, fmaf(-0.5f, q2, rh)));
         kx = __fmul_rn(mx, ikk);
         ky = __fmul_rn(my, ikk);
         kz = __fmul_rn(mz, ikk);
-        theta = dot3(kx, ru, ky, rv, kz, rw);
-        phi = __fmul_rn(0.2f, q2);
-        const float is2 = 0.70710678118654752f;  // 1/sqrt(2.0)
-        const float ia = __fmul_rn(frcp(a), is2);
-        irr = frcp(rr);
-        ia2 = __fmul_rn(__fmul_rn(ia, ia), 2.0f);
-        alpha = __fmul_rn(rr, ia);
-        beta = __fmul_rn(irr, ia);
-    }
-
-    // Left eigenvectors, rows of l_eigen_Q (Weno.cl:384-412).
-    __device__ __forceinline__ void left(float Lm[5][5]) const
-    {
-        const float g2 = __fmul_rn(0.4f, ia2), omf = fmaf(-phi, ia2, 1.0f);
-        const float gx = __fmul_rn(kx, g2), gy = __fmul_rn(ky, g2), gz = __fmul_rn(kz, g2);
-        const float ix = __fmul_rn(kx, irr), iy = __fmul_rn(ky, irr), iz = __fmul_rn(kz, irr);
-        Lm[0][0] = fmaf(kx, omf, -det2(iz, rv, iy, rw));
-        Lm[0][1] = __fmul_rn(gx, ru);
-        Lm[0][2] = fmaf(gx, rv, iz);
-        Lm[0][3] = fmaf(gx, rw, -iy);
-        Lm[0][4] = -gx;
-        Lm[1][0] = fmaf(ky, omf, -det2(ix, rw, iz, ru));
-        Lm[1][1] = fmaf(gy, ru, -iz);
-        Lm[1][2] = __fmul_rn(gy, rv);
-        Lm[1][3] = fmaf(gy, rw, ix);
-        Lm[1][4] = -gy;
-        Lm[2][0] = fmaf(kz, omf, -det2(iy, ru, ix, rv));
-        Lm[2][1] = fmaf(gz, ru, iy);
-        Lm[2][2] = fmaf(gz, rv, -ix);
-        Lm[2][3] = __fmul_rn(gz, rw);
-        Lm[2][4] = -gz;
-        const float b4 = __fmul_rn(0.4f, beta), ba = __fmul_rn(beta, a), bp = __fmul_rn(beta, phi);
-        Lm[3][0] = fmaf(-ba, theta, bp);
-        Lm[3][1] = fmaf(-b4, ru, __fmul_rn(ba, kx));
-        Lm[3][2] = fmaf(-b4, rv, __fmul_rn(ba, ky));
-        Lm[3][3] = fmaf(-b4, rw, __fmul_rn(ba, kz));
-        Lm[3][4] = b4;
-        Lm[4][0] = fmaf(ba, theta, bp);
-        Lm[4][1] = fmaf(-b4, ru, -__fmul_rn(ba, kx));
-        Lm[4][2] = fmaf(-b4, rv, -__fmul_rn(ba, ky));
-        Lm[4][3] = fmaf(-b4, rw, -__fmul_rn(ba, kz));
-        Lm[4][4] = b4;
+        h2 = __fmul_rn(0.5f, dot3(ru, ru, rv, rv, rw, rw));
+        const float a2 = __fmul_rn(0.4f, __fsub_rn(rh, h2)), a = fsqrt(a2), ia = frcp(a), irr = frcp(rr);
+        constexpr float is2 = 0.70710678118654752f;   // 1 / sqrt(2)
+        const float rs = __fmul_rn(rr, is2), irs = __fmul_rn(irr, is2);
+        g2 = __fmul_rn(0.4f, __fmul_rn(ia, ia));
+        ix = __fmul_rn(kx, irr);
+        iy = __fmul_rn(ky, irr);
+        iz = __fmul_rn(kz, irr);
+        nx = __fmul_rn(kx, rr);
+        ny = __fmul_rn(ky, rr);
+        nz = __fmul_rn(kz, rr);
+        al = __fmul_rn(rs, ia);              // alpha = rho / (sqrt(2) a)
+        ala = rs;                            // alpha a
+        ae = __fmul_rn(__fmul_rn(rs, a), 2.5f);   // alpha a^2 / 0.4
+        b4 = __fmul_rn(__fmul_rn(irs, ia), 0.4f); // 0.4 / (sqrt(2) rho a)
+        ba = irs;                            // beta a
     }
 };
 

@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(256) k_mu_s(LatView g)
     if (n < g.N) mx::mu_node(g, n, 0);
 }
 
-// 64 registers: a direction at 128^3 0.097 ms; 0.097 at 72 but the aerofoil
-// block 1 % slower, 0.106 at 80.
+// 64 registers: a direction at 128^3 0.091 ms, 0.093 at 72 and at 80.
 #ifndef CFD_SFACE_MIN_BLOCKS
 #define CFD_SFACE_MIN_BLOCKS 8
 #endif
