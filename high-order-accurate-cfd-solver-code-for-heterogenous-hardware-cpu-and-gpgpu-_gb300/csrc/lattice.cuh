@@ -4,6 +4,8 @@
 // persistent kernel (batch_*.cu), which holds one LatView per instance.
 #pragma once
 
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "physics.cuh"
@@ -109,6 +111,26 @@ __device__ __forceinline__ int lat_step(const LatView &g, int i, int j, int k, i
     else if (d == 1) j = p ? lwrap(j + o, g.nj) : lclamp(j + o, g.nj);
     else k = p ? lwrap(k + o, g.nk) : lclamp(k + o, g.nk);
     return i + g.ni * (j + g.nj * k);
+}
+
+// p[n] with the node as an unsigned 32-bit byte offset from a base that is
+// the same for the warp: one offset register serves every component, where
+// the index c N + n costs an addition and a widening product per load (a
+// fifth of the reduced forms' viscous and update instructions).
+// RO: through the non-coherent path.
+template <bool RO = true, class T>
+__device__ __forceinline__ T lat_ldg(const T *p, unsigned bytes)
+{
+    const T *a = reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + bytes);
+    return RO ? __ldg(a) : *a;
+}
+
+// Component c of node n of a [components][N] array, addressed the same way.
+template <class T>
+__device__ __forceinline__ T &lat_at(T *p, int c, int N, int n)
+{
+    using B = typename std::conditional<std::is_const<T>::value, const char, char>::type;
+    return *reinterpret_cast<T *>(reinterpret_cast<B *>(p + (size_t)c * N) + (unsigned)sizeof(T) * (unsigned)n);
 }
 
 __device__ __forceinline__ int lat_coord(int i, int j, int k, int d) { return d == 0 ? i : (d == 1 ? j : k); }

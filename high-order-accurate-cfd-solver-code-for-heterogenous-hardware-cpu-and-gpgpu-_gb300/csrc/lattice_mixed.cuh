@@ -88,11 +88,9 @@ __device__ __forceinline__ dfl df_div(dfl a, dfl b, float r)
     return quick_two_sum(q, __fmul_rn(rem, r));
 }
 
-// 1/3 and 2/3 as hi + lo
+// 1/3 as hi + lo
 constexpr float kThirdH = (float)(1.0 / 3.0);
 constexpr float kThirdL = (float)(1.0 / 3.0 - (double)(float)(1.0 / 3.0));
-constexpr float kTwoThirdH = (float)(2.0 / 3.0);
-constexpr float kTwoThirdL = (float)(2.0 / 3.0 - (double)(float)(2.0 / 3.0));
 // gamma - 1 = 0.4 as hi + lo
 constexpr float kGm1H = (float)0.4;
 constexpr float kGm1L = (float)(0.4 - (double)(float)0.4);
@@ -102,7 +100,7 @@ __device__ __forceinline__ void load_state(const LatView &g, int q, int n, dfl U
     const int N = g.N;
     const float *W = lat_W(g, q);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) Un[c] = {W[c * N + n], W[(5 + c) * N + n]};
+    for (int c = 0; c < 5; ++c) Un[c] = {lat_at(W, c, N, n), lat_at(W, 5 + c, N, n)};
 }
 
 __device__ __forceinline__ void store_state(const LatView &g, int q, int n, const dfl Un[5])
@@ -111,8 +109,8 @@ __device__ __forceinline__ void store_state(const LatView &g, int q, int n, cons
     float *W = lat_W(g, q);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        W[c * N + n] = Un[c].h;
-        W[(5 + c) * N + n] = Un[c].l;
+        lat_at(W, c, N, n) = Un[c].h;
+        lat_at(W, 5 + c, N, n) = Un[c].l;
     }
 }
 
@@ -123,7 +121,7 @@ __device__ __forceinline__ void store_state(const LatView &g, int q, int n, cons
 __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
 {
     const int N = g.N;
-    const dfl idet = {g.idet32[n], g.idet32[N + n]};
+    const dfl idet = {lat_at(g.idet32, 0, N, n), lat_at(g.idet32, 1, N, n)};
     const float r0 = frcp(Un[0].h);
     const float rho = df_mul_f(Un[0], idet);
     const float u = df_div_f(Un[1], Un[0], r0), v = df_div_f(Un[2], Un[0], r0), w = df_div_f(Un[3], Un[0], r0);
@@ -134,19 +132,19 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const dfl Un[5])
     const float p = df_mul_f(df_mul(rho2, e2), {kGm1H, kGm1L});
     const float irho = frcp(rho);
     const float pr = __fmul_rn(p, irho);
-    g.prim32[LF_P * N + n] = p;
+    lat_at(g.prim32, LF_P, N, n) = p;
     if (!(isfinite(rho) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(p))) atomicOr(g.flags, 2u);
     const float E = df_mul_f(Un[4], idet);
-    g.Q32[0 * N + n] = rho;
-    g.Q32[1 * N + n] = df_mul_f(Un[1], idet);
-    g.Q32[2 * N + n] = df_mul_f(Un[2], idet);
-    g.Q32[3 * N + n] = df_mul_f(Un[3], idet);
-    g.Q32[4 * N + n] = E;
-    g.R32[0 * N + n] = u;
-    g.R32[1 * N + n] = v;
-    g.R32[2 * N + n] = w;
-    g.R32[3 * N + n] = fsqrt(rho);
-    g.R32[4 * N + n] = q4.h + (q4.l + pr);     // H = E/rho + p/rho
+    lat_at(g.Q32, 0, N, n) = rho;
+    lat_at(g.Q32, 1, N, n) = df_mul_f(Un[1], idet);
+    lat_at(g.Q32, 2, N, n) = df_mul_f(Un[2], idet);
+    lat_at(g.Q32, 3, N, n) = df_mul_f(Un[3], idet);
+    lat_at(g.Q32, 4, N, n) = E;
+    lat_at(g.R32, 0, N, n) = u;
+    lat_at(g.R32, 1, N, n) = v;
+    lat_at(g.R32, 2, N, n) = w;
+    lat_at(g.R32, 3, N, n) = fsqrt(rho);
+    lat_at(g.R32, 4, N, n) = q4.h + (q4.l + pr);     // H = E/rho + p/rho
 }
 
 // U_Q from the FP64 FLOW (after an upload): U = det * Q(FLOW) in FP64, split
@@ -220,12 +218,13 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
 #pragma unroll
             for (int c = 0; c < 5; ++c) dU[d][c] = 0.0f;
         } else if (!LOC || !lat_locdir(g, d) || !((lflag >> d) & 1u)) {
+            const unsigned o2 = 4u * m2, o1 = 4u * m1, q1 = 4u * p1, q2 = 4u * p2;
 #pragma unroll
             for (int c = 0; c < 5; ++c) {
                 // the state slot is read-only in this pass: non-coherent loads
-                const float *H = W + c * N, *L = W + (5 + c) * N;
-                const float d1 = (__ldg(H + p1) - __ldg(H + m1)) + (__ldg(L + p1) - __ldg(L + m1));
-                const float d2 = (__ldg(H + p2) - __ldg(H + m2)) + (__ldg(L + p2) - __ldg(L + m2));
+                const float *H = W + (size_t)c * N, *L = W + (size_t)(5 + c) * N;
+                const float d1 = (lat_ldg(H, q1) - lat_ldg(H, o1)) + (lat_ldg(L, q1) - lat_ldg(L, o1));
+                const float d2 = (lat_ldg(H, q2) - lat_ldg(H, o2)) + (lat_ldg(L, q2) - lat_ldg(L, o2));
                 dU[d][c] = __fmul_rn(1.0f / 12.0f, fmaf(8.0f, d1, -d2));
             }
         } else {
@@ -245,25 +244,27 @@ __device__ __forceinline__ void visc_node(const LatView &g, int n, int q)
                 dU[d][c] = branch_deriv_diff(b, dl);
             }
         }
+        const float *Wd = W + (size_t)(d + 1) * N;
         const int c = d + 1;
-        const float um = __ldg(W + c * N + m1), up = __ldg(W + c * N + p1);
-        const float rm = __ldg(W + m1), rp = __ldg(W + p1);
+        const float um = lat_ldg(Wd, 4u * m1), up = lat_ldg(Wd, 4u * p1);
+        const float rm = lat_ldg(W, 4u * m1), rp = lat_ldg(W, 4u * p1);
         const float dlt = fmaf(Ui[c], r0, -qdiv(filtered(um, Ui[c], up), filtered(rm, Ui[0], rp)));
         KS[d] = fabsf(dlt);
     }
     float m[9];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = g.node32[c * N + n];
-    const float prim[5] = {g.Q32[n], g.R32[n], g.R32[N + n], g.R32[2 * N + n], g.prim32[LF_P * N + n]};
+    for (int c = 0; c < 9; ++c) m[c] = lat_at(g.node32, c, N, n);
+    const float prim[5] = {lat_at(g.Q32, 0, N, n), lat_at(g.R32, 0, N, n), lat_at(g.R32, 1, N, n), lat_at(g.R32, 2, N, n),
+                           lat_at(g.prim32, LF_P, N, n)};
     float Fv[5], Ev[5], Gv[5], mu;
-    viscous_node_flux(dU, Ui, m, g.node32[9 * N + n], g.node32[10 * N + n], prim, KS, g.P, Fv, Ev, Gv, mu);
+    viscous_node_flux(dU, Ui, m, lat_at(g.node32, 9, N, n), lat_at(g.node32, 10, N, n), prim, KS, g.P, Fv, Ev, Gv, mu);
 #pragma unroll
     for (int c = 1; c < 5; ++c) {   // mass has no viscous flux: component 0 stays as it was zeroed
-        g.V32[(0 * 5 + c) * N + n] = Fv[c];
-        g.V32[(1 * 5 + c) * N + n] = Ev[c];
-        g.V32[(2 * 5 + c) * N + n] = Gv[c];
+        lat_at(g.V32, c, N, n) = Fv[c];
+        lat_at(g.V32, 5 + c, N, n) = Ev[c];
+        lat_at(g.V32, 10 + c, N, n) = Gv[c];
     }
-    g.prim32[LF_MU * N + n] = mu;
+    lat_at(g.prim32, LF_MU, N, n) = mu;
 }
 
 __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
@@ -334,8 +335,8 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
     float m[3] = {0.f, 0.f, 0.f}, det_f = 0.f;   // loaded while the staging waits
     if (face) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) m[c] = __ldg(g.fm32 + (D * 3 + c) * N + n);
-        det_f = __ldg(g.fdet32 + D * N + n);
+        for (int c = 0; c < 3; ++c) m[c] = lat_ldg(g.fm32 + (size_t)(D * 3 + c) * N, 4u * n);
+        det_f = lat_ldg(g.fdet32 + (size_t)D * N, 4u * n);
     }
     stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
     if (!face) return;
@@ -348,7 +349,7 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
     for (int q = 0; q < 5; ++q) {
         float f[6];
         tile_node_fluxes<T>(sF, q, t, a, f);
-        g.Fh32[(D * 5 + q) * N + n] = __fadd_rn(Fhat[q], x2::face_correction_sym(f));
+        lat_at(g.Fh32, D * 5 + q, N, n) = __fadd_rn(Fhat[q], x2::face_correction_sym(f));
     }
 }
 
@@ -357,7 +358,7 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
 // factor of two subtract exactly); the RK accumulation is hi/lo:
 //   jst 0: U1 = U0 + dt L
 //   jst 1: U2 = 3/4 U0 + 1/4 U1 + 1/4 dt L
-//   jst 2: U0 = 1/3 U0 + 2/3 U2 + 2/3 dt L
+//   jst 2: U0 = (U0 + 2 (U2 + dt L)) / 3
 // and the new state lands in slot (jst+1) mod 3, which is also the next
 // stage's U_Q slot.  LOC as for visc_node.  RO: the face and viscous
 // fluxes were written by an earlier launch, so they may be read through the
@@ -389,7 +390,10 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
     for (int d = 0; d < 3; ++d) {
         const int m1 = lat_step(g, i, j, k, d, -1);
 #pragma unroll
-        for (int c = 0; c < 5; ++c) Lf[c] += ld(g.Fh32 + (d * 5 + c) * N + n) - ld(g.Fh32 + (d * 5 + c) * N + m1);
+        for (int c = 0; c < 5; ++c) {
+            const float *Fd = g.Fh32 + (size_t)(d * 5 + c) * N;
+            Lf[c] += lat_ldg<RO>(Fd, 4u * n) - lat_ldg<RO>(Fd, 4u * m1);
+        }
         if (LOC && g.P.viscous && lat_locdir(g, d) && ((lflag >> d) & 1u)) {
             int s[7], L7[7];
 #pragma unroll
@@ -408,11 +412,13 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             }
         } else if (g.P.viscous) {
             const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
-            const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 1; c < 5; ++c)
-                Lf[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ld(Vd + c * N + p1) - ld(Vd + c * N + m1),
-                                                -(ld(Vd + c * N + p2) - ld(Vd + c * N + m2))), Lf[c]);
+            for (int c = 1; c < 5; ++c) {
+                const float *V = g.V32 + (size_t)(d * 5 + c) * N;
+                const float d1 = lat_ldg<RO>(V, 4u * p1) - lat_ldg<RO>(V, 4u * m1),
+                            d2 = lat_ldg<RO>(V, 4u * p2) - lat_ldg<RO>(V, 4u * m2);
+                Lf[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, d1, -d2), Lf[c]);
+            }
         }
     }
     if (g.Lout) {
@@ -440,10 +446,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
         load_state(g, 2, n, U2);
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
-            const dfl a = df_mul(U0[c], {kThirdH, kThirdL});
-            const dfl b = df_mul(U2[c], {kTwoThirdH, kTwoThirdL});
-            const dfl t = df_mul(df_mul({-Lf[c], 0.0f}, dt), {kTwoThirdH, kTwoThirdL});
-            Un[c] = df_add(df_add(a, b), t);
+            const dfl a = df_add(U2[c], df_mul({-Lf[c], 0.0f}, dt));   // (U0 + 2 (U2 + dt L)) / 3
+            Un[c] = df_mul(df_add(U0[c], {2.0f * a.h, 2.0f * a.l}), {kThirdH, kThirdL});
         }
     }
     store_state(g, jst == 2 ? 0 : jst + 1, n, Un);

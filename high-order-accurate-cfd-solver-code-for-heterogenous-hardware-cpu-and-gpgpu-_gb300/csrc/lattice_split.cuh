@@ -34,7 +34,7 @@ __device__ __forceinline__ void load_state(const LatView &g, int q, int n, doubl
     const int N = g.N;
     const double *U = lat_U(g, q);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) Un[c] = U[c * N + n];
+    for (int c = 0; c < 5; ++c) Un[c] = lat_at(U, c, N, n);
 }
 
 __device__ __forceinline__ void store_state(const LatView &g, int q, int n, const double Un[5])
@@ -42,7 +42,7 @@ __device__ __forceinline__ void store_state(const LatView &g, int q, int n, cons
     const int N = g.N;
     double *U = lat_U(g, q);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) U[c * N + n] = Un[c];
+    for (int c = 0; c < 5; ++c) lat_at(U, c, N, n) = Un[c];
 }
 
 // U_Q of the next stage from the state Un (= det * Q): Q in FP64, rounded
@@ -60,10 +60,10 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const double Un[
     for (int c = 0; c < 5; ++c) {
         float h, l;
         emu::hi_lo(Un[c], h, l);
-        g.Whl[c * N + n] = h;
-        g.Whl[(5 + c) * N + n] = l;
+        lat_at(g.Whl, c, N, n) = h;
+        lat_at(g.Whl, 5 + c, N, n) = l;
     }
-    const double id = g.idet64[n];
+    const double id = lat_at(g.idet64, 0, N, n);
     float q[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) q[c] = emu::d2f(emu::mul(Un[c], id));
@@ -71,15 +71,15 @@ __device__ __forceinline__ void derive(const LatView &g, int n, const double Un[
     const float ir = frcp(rho);
     const float u = __fmul_rn(q[1], ir), v = __fmul_rn(q[2], ir), w = __fmul_rn(q[3], ir);
     const float p = __fmul_rn(0.4f, fmaf(-0.5f, dot3(q[1], u, q[2], v, q[3], w), q[4]));
-    g.prim32[LF_P * N + n] = p;
+    lat_at(g.prim32, LF_P, N, n) = p;
     if (!(isfinite(rho) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(p))) atomicOr(g.flags, 2u);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) g.Q32[c * N + n] = q[c];
-    g.R32[0 * N + n] = u;
-    g.R32[1 * N + n] = v;
-    g.R32[2 * N + n] = w;
-    g.R32[3 * N + n] = fsqrt(rho);
-    g.R32[4 * N + n] = __fmul_rn(q[4] + p, ir);   // H = (E + p) / rho
+    for (int c = 0; c < 5; ++c) lat_at(g.Q32, c, N, n) = q[c];
+    lat_at(g.R32, 0, N, n) = u;
+    lat_at(g.R32, 1, N, n) = v;
+    lat_at(g.R32, 2, N, n) = w;
+    lat_at(g.R32, 3, N, n) = fsqrt(rho);
+    lat_at(g.R32, 4, N, n) = __fmul_rn(q[4] + p, ir);   // H = (E + p) / rho
 }
 
 // U = det * Q(FLOW) in FP64 (U_Q.cl:112-116) into slot q, then derive.
@@ -135,10 +135,10 @@ __device__ __forceinline__ FaceMetric face_metric(const LatView &g, int n)
     FaceMetric f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        f.m[c] = __ldg(g.fm + (D * 3 + c) * N + n);
-        f.m32[c] = __ldg(g.fm32 + (D * 3 + c) * N + n);
+        f.m[c] = lat_ldg(g.fm + (size_t)(D * 3 + c) * N, 8u * n);
+        f.m32[c] = lat_ldg(g.fm32 + (size_t)(D * 3 + c) * N, 4u * n);
     }
-    f.det = __ldg(g.fdet + D * N + n);
+    f.det = lat_ldg(g.fdet + (size_t)D * N, 8u * n);
     return f;
 }
 
@@ -213,21 +213,20 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
     double Fh[5];
     face_flux(g, face_metric<D>(g, n), P, r, corr, Fh);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) g.Fh[(D * 5 + q) * N + n] = Fh[q];
+    for (int q = 0; q < 5; ++q) lat_at(g.Fh, D * 5 + q, N, n) = Fh[q];
 }
 
 // RHS and SSP-RK3 stage jst: the face-flux difference in FP64, the viscous
 // divergence in FP32 (added in FP64), and the RK accumulation in FP64:
 //   jst 0: U1 = U0 + dt L
-//   jst 1: U2 = 3/4 U0 + 1/4 U1 + 1/4 dt L
-//   jst 2: U0 = 1/3 U0 + 2/3 U2 + 2/3 dt L
+//   jst 1: U2 = (3 U0 + (U1 + dt L)) / 4
+//   jst 2: U0 = (U0 + 2 (U2 + dt L)) / 3
 // The new state lands in slot (jst+1) mod 3, which is also the next stage's
 // U_Q slot.  LOC and RO as for the mixed form's update_node.
 template <bool LOC, bool RO = true>
 __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 {
     auto ldf = [](const float *p) { return RO ? __ldg(p) : *p; };
-    auto ldd = [](const double *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
     if (LOC && lat_ghost(g, n)) {   // ghosts: the state moves on (mixed form's update_node)
         if (g.Lout) {
@@ -251,7 +250,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
         // frees here (TGV 128^3: update 0.23 -> 0.31 ms with one direction)
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
-            const double df = ldd(g.Fh + (d * 5 + c) * N + n) - ldd(g.Fh + (d * 5 + c) * N + m1);
+            const double *Fd = g.Fh + (size_t)(d * 5 + c) * N;
+            const double df = lat_ldg<RO>(Fd, 8u * n) - lat_ldg<RO>(Fd, 8u * m1);
             Ld[c] = d == 0 ? df : Ld[c] + df;
         }
         if (LOC && g.P.viscous && lat_locdir(g, d) && ((lflag >> d) & 1u)) {
@@ -272,11 +272,13 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             }
         } else if (g.P.viscous) {
             const int m2 = lat_step(g, i, j, k, d, -2), p1 = lat_step(g, i, j, k, d, 1), p2 = lat_step(g, i, j, k, d, 2);
-            const float *Vd = g.V32 + (size_t)d * 5 * N;
 #pragma unroll
-            for (int c = 1; c < 5; ++c)
-                Lv[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, ldf(Vd + c * N + p1) - ldf(Vd + c * N + m1),
-                                                -(ldf(Vd + c * N + p2) - ldf(Vd + c * N + m2))), Lv[c]);
+            for (int c = 1; c < 5; ++c) {
+                const float *V = g.V32 + (size_t)(d * 5 + c) * N;
+                const float d1 = lat_ldg<RO>(V, 4u * p1) - lat_ldg<RO>(V, 4u * m1),
+                            d2 = lat_ldg<RO>(V, 4u * p2) - lat_ldg<RO>(V, 4u * m2);
+                Lv[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, d1, -d2), Lv[c]);
+            }
         }
     }
 #pragma unroll

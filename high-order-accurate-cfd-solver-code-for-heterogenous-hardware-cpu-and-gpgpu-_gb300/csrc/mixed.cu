@@ -39,13 +39,13 @@ __global__ void __launch_bounds__(256) k_prep_m(LatView g, int src, int dst)
     if (n < g.N) mx::prep_node(g, n, src, dst);
 }
 
-// Blocks of 256 per SM that the viscous pass's registers must allow: 6 on
-// periodic lattices (40 registers: latency bound, more warps help; 4, 5, 6,
-// 8 measured 0.122, 0.114, 0.112, 0.145 ms on TGV 128^3), 4 with loc codes
-// (64 registers; the branch code spills below that: 0.140 ms against 0.148
-// and 0.175 at 5 and 6 on the NACA0012 O-grid).
+// Blocks of 256 per SM that the viscous pass's registers must allow: 4 (64
+// registers) on periodic lattices, where the loads in flight bound it (128^3
+// 0.096 ms; 0.104 at 5, 0.106 at 3; 0.106 at 6 with an index per component),
+// and with loc codes (the branch code spills below that: 0.140 ms against
+// 0.148 and 0.175 at 5 and 6 on the NACA0012 O-grid).
 #ifndef CFD_MVISC_MIN_BLOCKS
-#define CFD_MVISC_MIN_BLOCKS 6
+#define CFD_MVISC_MIN_BLOCKS 4
 #endif
 #ifndef CFD_MVISC_LOC_MIN_BLOCKS
 #define CFD_MVISC_LOC_MIN_BLOCKS 4
@@ -109,8 +109,12 @@ void launch_face_tile(const LatView &g, cudaStream_t st, int tile)
     }
 }
 
+// 48 registers: at 128^3 0.115 ms, 0.127 at 64, 0.119 at 40
+#ifndef CFD_MUPD_MIN_BLOCKS
+#define CFD_MUPD_MIN_BLOCKS 5
+#endif
 template <bool LOC>
-__global__ void __launch_bounds__(256) k_update_m(LatView g, int jst)
+__global__ void __launch_bounds__(256, CFD_MUPD_MIN_BLOCKS) k_update_m(LatView g, int jst)
 {
     const int n = node_id();
     if (n < g.N) mx::update_node<LOC>(g, n, jst);

@@ -37,8 +37,10 @@ __global__ void __launch_bounds__(256) k_prep_s(LatView g, int src, int dst)
 
 // The viscous pass is the mixed form's (FP32, the same launch bounds) on
 // the hi/lo read copy of the state (sp::hilo_view).
+// 64 registers: at 128^3 0.101 ms, 0.103 at 51, 0.105 at 80 (0.112 at 40 and
+// with an index per component)
 #ifndef CFD_SVISC_MIN_BLOCKS
-#define CFD_SVISC_MIN_BLOCKS 6
+#define CFD_SVISC_MIN_BLOCKS 4
 #endif
 #ifndef CFD_SVISC_LOC_MIN_BLOCKS
 #define CFD_SVISC_LOC_MIN_BLOCKS 4
@@ -57,9 +59,9 @@ __global__ void __launch_bounds__(256) k_mu_s(LatView g)
     if (n < g.N) mx::mu_node(g, n, 0);
 }
 
-// 64 registers: a direction at 128^3 0.091 ms, 0.093 at 72 and at 80.
+// 72 registers: a direction at 128^3 0.093 ms; 0.094 at 64 registers.
 #ifndef CFD_SFACE_MIN_BLOCKS
-#define CFD_SFACE_MIN_BLOCKS 8
+#define CFD_SFACE_MIN_BLOCKS 7
 #endif
 // One instance per candidate tile width (face_tile.cuh): faces along i of
 // 32, 64 or 128, along j or k of 8, 16 or 32; the solver times them when it
@@ -93,8 +95,12 @@ void launch_face_tile_s(const LatView &g, cudaStream_t st, int tile)
     }
 }
 
+// 64 registers: at 128^3 0.190 ms, 0.193 at 48 and 40, 0.221 unbounded
+#ifndef CFD_SUPD_MIN_BLOCKS
+#define CFD_SUPD_MIN_BLOCKS 4
+#endif
 template <bool LOC>
-__global__ void __launch_bounds__(256) k_update_s(LatView g, int jst)
+__global__ void __launch_bounds__(256, CFD_SUPD_MIN_BLOCKS) k_update_s(LatView g, int jst)
 {
     const int n = node_id();
     if (n < g.N) sp::update_node<LOC>(g, n, jst);
