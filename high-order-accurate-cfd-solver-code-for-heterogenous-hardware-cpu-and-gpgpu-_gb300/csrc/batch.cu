@@ -53,9 +53,8 @@ struct cfd_batch {
     BatchTile *d_tiles = nullptr;
     size_t tiles_cap = 0;
     int ntiles = 0;
-    // tiled form (reduced-precision batches): phase A items (viscous ranges
-    // and shared-memory face tiles); d_tiles then holds phase B's 1-D tiles
-    bool face_tiles = false;
+    bool face_tiles = false;              // CFD_BATCH_FACE_TILES asked for: node tiles of kFaceThreads
+    // reduced forms: the viscous ranges and the face tiles of every instance
     BatchItem *d_items = nullptr;
     size_t items_cap = 0;
     int nitems = 0;
@@ -131,44 +130,22 @@ void face_tile_items(const LatView &g, int v, std::vector<BatchItem> &out)
     for (unsigned z = 0; z < gr.z; ++z)
         for (unsigned y = 0; y < gr.y; ++y)
             for (unsigned x = 0; x < gr.x; ++x)
-                out.push_back(BatchItem{v, 1 + D, (int)x * T::kTile, (int)y * T::kWide, (int)z, 0});
+                out.push_back(BatchItem{v, D, (int)x * T::kTile, (int)y * T::kWide, (int)z, 0});
 }
 
-// Phase A items of the tiled form in the order the blocks take them (from
-// the shared counter): kind-major as the 1-D form (CFD_BATCH_KIND_MAJOR),
-// else position w has kind (w % G + w / G) mod 4 while that kind has items
-// left (else the next kind that has), so that the blocks running at one
-// time work on every kind of the same region.
-std::vector<BatchItem> order_items(std::vector<BatchItem> q[4], int G)
+// Nodes per node tile (threads per block of the closing kernel).
+int node_tile(const cfd_batch *b)
 {
-    size_t total = 0, head[4] = {0, 0, 0, 0};
-    for (int k = 0; k < 4; ++k) total += q[k].size();
-    std::vector<BatchItem> out;
-    out.reserve(total);
-    if (CFD_BATCH_KIND_MAJOR) {   // as the 1-D form: i, j, k faces, then the viscous ranges
-        for (int k : {1, 2, 3, 0}) out.insert(out.end(), q[k].begin(), q[k].end());
-        return out;
-    }
-    for (size_t w = 0; w < total; ++w) {
-        const int k0 = (int)(((w % G) + (w / G)) & 3);
-        for (int t = 0; t < 4; ++t) {
-            const int k = (k0 + t) & 3;
-            if (head[k] < q[k].size()) {
-                out.push_back(q[k][head[k]++]);
-                break;
-            }
-        }
-    }
-    return out;
+    return b->face_tiles && b->precision != CFD_PREC_FP64 ? kFaceThreads : b->threads;
 }
 
 cfd_status_t rebuild(cfd_batch *b)
 {
     std::vector<LatView> views;
     std::vector<BatchTile> tiles;
-    std::vector<BatchItem> kinds[4];
-    const bool tiled = b->face_tiles && b->precision != CFD_PREC_FP64;
-    const int T = tiled ? kFaceThreads : b->threads;
+    std::vector<BatchItem> faces[3];
+    const bool reduced = b->precision != CFD_PREC_FP64;
+    const int T = node_tile(b);
     uint64_t nodes = 0;
     for (size_t s = 0; s < b->slots.size(); ++s) {
         BatchInst &I = b->slots[s];
@@ -177,11 +154,10 @@ cfd_status_t rebuild(cfd_batch *b)
         const int v = (int)views.size();
         views.push_back(I.view);
         for (int n0 = 0; n0 < I.N; n0 += T) tiles.push_back(BatchTile{v, n0, std::min(T, I.N - n0), 0});
-        if (tiled) {
-            for (int n0 = 0; n0 < I.N; n0 += T) kinds[0].push_back(BatchItem{v, 0, n0, std::min(T, I.N - n0), 0, 0});
-            face_tile_items<0>(I.view, v, kinds[1]);
-            face_tile_items<1>(I.view, v, kinds[2]);
-            face_tile_items<2>(I.view, v, kinds[3]);
+        if (reduced) {
+            face_tile_items<0>(I.view, v, faces[0]);
+            face_tile_items<1>(I.view, v, faces[1]);
+            face_tile_items<2>(I.view, v, faces[2]);
         }
         nodes += (uint64_t)I.N;
     }
@@ -210,19 +186,22 @@ cfd_status_t rebuild(cfd_batch *b)
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int occ = b->precision == CFD_PREC_MIXED   ? batch_occupancy_mixed(T, tiled)
-                    : b->precision == CFD_PREC_SPLIT ? batch_occupancy_split(T, tiled)
+    const int occ = b->precision == CFD_PREC_MIXED   ? batch_occupancy_mixed(T)
+                    : b->precision == CFD_PREC_SPLIT ? batch_occupancy_split(T)
                                                      : batch_occupancy_fp64(T);
     if (occ <= 0) return fail(b->ctx, CFD_EUNSUPPORTED, "batch: stage kernel does not fit at this tile size");
     int blocks = occ * sms;
     if (b->blocks_override > 0) blocks = std::min(blocks, b->blocks_override);
-    size_t n_a = 4 * (size_t)std::max(b->ntiles, 1);   // phase A items
-    if (tiled) n_a = std::max<size_t>(1, kinds[0].size() + kinds[1].size() + kinds[2].size() + kinds[3].size());
+    const size_t n_a = (reduced ? 1 : 4) * (size_t)std::max(b->ntiles, 1);   // items of the closing launch
     blocks = std::max(1, (int)std::min<size_t>((size_t)blocks, n_a));
     b->blocks = blocks;
     b->nitems = 0;
-    if (tiled) {
-        const std::vector<BatchItem> items = order_items(kinds, blocks);
+    if (reduced) {
+        std::vector<BatchItem> items;
+        for (int v = 0; v < (int)views.size(); ++v)
+            for (int n0 = 0; n0 < views[v].N; n0 += kFaceThreads)
+                items.push_back(BatchItem{v, 3, n0, std::min(kFaceThreads, views[v].N - n0), 0, 0});
+        for (const auto &f : faces) items.insert(items.end(), f.begin(), f.end());
         if (items.size() > b->items_cap) {
             if (b->d_items) cudaFree(b->d_items);
             b->items_cap = std::max<size_t>(items.size(), 2 * b->items_cap);
@@ -264,7 +243,7 @@ cfd_status_t rebuild(cfd_batch *b)
 // Kernel launches of one RK step.
 int step_launches(const cfd_batch *b)
 {
-    return 3 * (b->precision == CFD_PREC_FP64 ? batch_launches_fp64(b->ntiles, b->round_tiles) : 1);
+    return 3 * (b->precision == CFD_PREC_FP64 ? batch_launches_fp64(b->ntiles, b->round_tiles) : 2);
 }
 
 BatchLaunch launch_of(cfd_batch *b)
@@ -273,9 +252,8 @@ BatchLaunch launch_of(cfd_batch *b)
     L.views = b->d_views;
     L.tiles = b->d_tiles;
     L.ntiles = b->ntiles;
-    L.threads = b->threads;
+    L.threads = node_tile(b);
     L.blocks = b->blocks;
-    L.tiled = b->nitems > 0 ? 1 : 0;
     L.items = b->d_items;
     L.nitems = b->nitems;
     L.scratch = b->d_scratch;
@@ -921,20 +899,14 @@ cfd_status_t cfd_batch_tune(cfd_batch_t *b, int32_t steps_per_trial)
         }
     };
     copy_all(true);
-    // 1-D tiles of 32, 64, 128, 256 nodes, and for the reduced forms the
-    // shared-memory face tiles
-    std::vector<int> candidates = {32, 64, 128, 256};
-    if (b->precision != CFD_PREC_FP64) candidates.push_back(CFD_BATCH_FACE_TILES);
-    const int threads0 = b->threads;
-    const bool faces0 = b->face_tiles;
-    int best = faces0 ? CFD_BATCH_FACE_TILES : threads0;
+    int best = node_tile(b);
     float best_ms = 1e30f;
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
-    for (int T : candidates) {
-        b->face_tiles = T == CFD_BATCH_FACE_TILES;
-        if (!b->face_tiles) b->threads = T;
+    b->face_tiles = false;
+    for (int T : {32, 64, 128, 256}) {   // nodes per tile
+        b->threads = T;
         b->dirty = true;
         if ((st = rebuild(b)) != CFD_OK) continue;
         if (b->use_graph) try_capture(b);
@@ -960,8 +932,7 @@ cfd_status_t cfd_batch_tune(cfd_batch_t *b, int32_t steps_per_trial)
     e = cudaStreamSynchronize(sm);
     cudaFree(backup);
     if (e != cudaSuccess) return cuda_fail(b->ctx, e, "cfd_batch_tune restore");
-    b->face_tiles = best == CFD_BATCH_FACE_TILES;
-    b->threads = b->face_tiles ? threads0 : best;
+    b->threads = best;
     b->dirty = true;
     return rebuild(b);
 }
@@ -977,7 +948,7 @@ cfd_status_t cfd_batch_info(const cfd_batch_t *b, cfd_batch_info_t *info)
     }
     info->n_active = n;
     info->n_held = held;
-    info->tile_nodes = b->face_tiles && b->precision != CFD_PREC_FP64 ? kFaceThreads : b->threads;
+    info->tile_nodes = node_tile(b);
     info->face_tiles = b->face_tiles && b->precision != CFD_PREC_FP64 ? 1 : 0;
     info->blocks = b->blocks;
     info->graph = b->graph_ok ? 1 : 0;

@@ -1,23 +1,25 @@
-// batch_kernel.cuh -- one persistent launch per RK stage over many lattices.
+// batch_kernel.cuh -- the batched RK stage over many lattices.
 //
-// Work is described by a tile table: tile t = (instance, first node, node
-// count), tile size = block size, so one thread owns one node of a tile.
-// A stage has two phases separated by a grid-wide barrier:
-//   A  for every tile: viscous fluxes and the three face fluxes (4 work items
-//      per tile, taken in order from a shared counter, so that blocks that
-//      run at the same time share a tile's data and none waits long)
-//   B  for every tile: RHS, RK stage, primitives, and the next stage's prep
-//      (U_Q) on the new primitives
-// The kernel is launched cooperatively (all blocks co-resident) with at most
-// the occupancy limit of blocks; the barrier's wait is bounded by a
-// %globaltimer deadline, after which it sets CFD_FLAG_TIMEOUT and the block
-// returns instead of spinning.
+// Work is described by tables: node tile t = (instance, first node, node
+// count), tile size = block size, so one thread owns one node of a tile; and
+// (reduced forms) face tiles (face_tile.cuh) of every instance.  A reduced
+// form's stage is two launches:
+//   k_batch_fluxes          the viscous fluxes (one block per node range) and
+//                           the three face fluxes (one block per face tile)
+//   k_batch_close_reduced   persistent: the grid-wide barrier, then every
+//                           node tile's RHS, RK stage and next U_Q
+// (batch_fp64.cu has the FP64 form's launches.)  The closing kernel is
+// launched cooperatively (all blocks co-resident) with at most the occupancy
+// limit of blocks; the barrier's wait is bounded by a %globaltimer deadline,
+// after which it sets CFD_FLAG_TIMEOUT and the block returns instead of
+// spinning.
 //
 // Ops supplies the per-node operations of one precision form
-// (lattice_fp64.cuh or lattice_mixed.cuh); this header is included by the
+// (lattice_mixed.cuh, lattice_split.cuh); this header is included by the
 // translation unit compiled with that form's flags.
 #pragma once
 
+#include "batch_ops.h"
 #include "face_tile.cuh"
 #include "lattice.cuh"
 
@@ -40,8 +42,8 @@ __device__ __forceinline__ unsigned long long global_ns()
 // Sense-reversing grid barrier over `nblocks` co-resident blocks.
 // bar[0] = arrival count, bar[1] = generation.  Returns false (and sets the
 // timeout bit) if the generation does not advance before the deadline.
-// The last block to arrive also clears bar[3], the phase-A work counter
-// (every block has stopped taking phase-A items when it arrives), so the
+// The last block to arrive also clears bar[3], the work counter
+// (every block has stopped taking items when it arrives), so the
 // next launch starts from item 0.
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, unsigned long long limit_ns,
                                              unsigned *gflags)
@@ -77,10 +79,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned nblocks, un
     return s_ok != 0;
 }
 
-// Next phase-A item of this block: blocks take items in order from a
+// Next item before the barrier of this block: blocks take items in order from a
 // shared counter (bar[3]), so a block that finishes early takes more and
 // no block idles long at the barrier (with a fixed item-to-block map some
-// blocks ran phase A ~10 % longer than the rest and everyone waited).
+// blocks ran ~10 % longer than the rest and everyone waited).
 __device__ __forceinline__ int next_item(unsigned *bar)
 {
     __shared__ int s_w;
@@ -90,52 +92,53 @@ __device__ __forceinline__ int next_item(unsigned *bar)
     return s_w;
 }
 
-// Phase A's item order: kind-major (1: every tile's i faces, then every
-// tile's j faces, then k, then the viscous items -- the blocks running at
-// one time work on one direction, as the single-lattice passes do) or
-// tile-major (0: the four kinds of a tile one after the other).  64
-// vortices, tuned tiles: mixed 1.33e9 against 1.29e9 cell-updates/s, split
-// 1.02e9 against 9.6e8.
-#ifndef CFD_BATCH_KIND_MAJOR
-#define CFD_BATCH_KIND_MAJOR 1
-#endif
+// Kind 3: the viscous range of b nodes from node a of one lattice; otherwise a
+// face tile along D = kind (a = first face along D, b = first node across,
+// c = line of the third axis; face_tile.cuh).
+struct BatchItem {
+    int inst, kind, a, b, c, pad;
+};
 
-// Blocks of up to 256 threads (the tile sizes 32, 64, 128, 256); Ops::kMinBlocks
-// bounds the registers so that many blocks stay resident (the mixed form is
-// latency bound; the FP64 form keeps its registers).
+// The fluxes of every instance: the viscous ranges first (their chains are
+// the longest), then the face tiles, one direction after the other's (blocks
+// that run at the same time work on one direction's code).  A kernel of its
+// own runs at the registers of the
+// face pass alone (72); in one persistent launch with the viscous and update
+// code it had 80 with spills.  24 vortices of 24^3 to 72^3 (2.7 million
+// nodes), a stage: mixed 0.60 -> 0.50 ms, split 0.81 -> 0.79; one of 24^3,
+// viscous, mixed 17.3 -> 15.8 us (18.1 with the viscous ranges in the closing
+// launch).  Tile widths
+// chosen per instance (8, 16 or 32, the least padding) were slower: 0.50
+// and 0.82.
 template <class Ops>
-__global__ void __launch_bounds__(256, Ops::kMinBlocks)
-k_batch_stage(const LatView *__restrict__ views, const BatchTile *__restrict__ tiles, int ntiles, int jst,
-              unsigned *bar, unsigned *gflags, unsigned long long limit_ns)
+__global__ void __launch_bounds__(kFaceThreads, Ops::kFaceBlocks)
+k_batch_fluxes(const LatView *__restrict__ views, const BatchItem *__restrict__ items, int jst)
 {
-    // Item w: tile w % ntiles of kind w / ntiles (kind-major), or tile w >> 2
-    // of kind w & 3 (the four items of a tile taken one after the other, by
-    // different blocks at about the same time: they share the tile's data in
-    // L2).
-    const int items = 4 * ntiles;
-    for (int w = next_item(bar); w < items; w = next_item(bar)) {
-#if CFD_BATCH_KIND_MAJOR
-        const BatchTile t = tiles[w % ntiles];
-        const int kind = (w / ntiles + 1) & 3;   // i faces, j faces, k faces, then the viscous items
-#else
-        const BatchTile t = tiles[w >> 2];
-        const int kind = w & 3;
-#endif
-        if ((int)threadIdx.x < t.count) {
-            const LatView &g = views[t.inst];
-            const int n = t.n0 + threadIdx.x;
-            if (kind == 0) {
-                if (g.P.viscous) Ops::visc(g, n, jst);
-                else Ops::mu(g, n, jst);
-            } else if (kind == 1) {
-                Ops::template face<0>(g, n);
-            } else if (kind == 2) {
-                Ops::template face<1>(g, n);
-            } else {
-                Ops::template face<2>(g, n);
-            }
-        }
-    }
+    __shared__ float smem[Ops::kTileSmemFloats];
+    const BatchItem it = items[blockIdx.x];
+    const LatView &g = views[it.inst];
+    const TileAt at{it.a, it.b, it.c};
+    if (it.kind == 3) {
+        if ((int)threadIdx.x >= it.b) return;
+        const int n = it.a + threadIdx.x;
+        if (g.P.viscous) Ops::visc(g, n, jst);
+        else Ops::mu(g, n, jst);
+    } else if (it.kind == 0) Ops::template face_tile<0>(g, at, smem);
+    else if (it.kind == 1) Ops::template face_tile<1>(g, at, smem);
+    else Ops::template face_tile<2>(g, at, smem);
+}
+
+// The grid barrier and the update of every node tile, in blocks of up to 256
+// threads (the tile sizes 32, 64, 128, 256) at 64 registers, as the single
+// lattice's update.  The barrier orders nothing here (the fluxes are an
+// earlier launch's); it is the bounded wait that cfd_batch_set_wait_limit
+// sets and that a step reports as CFD_ETIMEOUT when the grid is not
+// co-resident, and costs 2 us.
+template <class Ops>
+__global__ void __launch_bounds__(256, 4)
+k_batch_close_reduced(const LatView *__restrict__ views, const BatchTile *__restrict__ tiles, int ntiles, int jst,
+                      unsigned *bar, unsigned *gflags, unsigned long long limit_ns)
+{
     if (!grid_barrier(bar, gridDim.x, limit_ns, gflags)) return;
     for (int w = blockIdx.x; w < ntiles; w += gridDim.x) {
         const BatchTile t = tiles[w];
@@ -143,48 +146,32 @@ k_batch_stage(const LatView *__restrict__ views, const BatchTile *__restrict__ t
     }
 }
 
-// One work item of phase A of the tiled form (the reduced-precision
-// forms): kind 0 a viscous range of one lattice (a = first node, b = nodes),
-// kind 1 + D a face tile along D (a = first face along D, b = first node
-// across, c = line of the third axis; face_tile.cuh).
-struct BatchItem {
-    int inst, kind, a, b, c, pad;
-};
-
-// The persistent stage over items: phase A's face items stage their stencil
-// lines in shared memory as the single-lattice face passes do (Ops::face_tile)
-// instead of gathering each face's points through L1; phase B updates 1-D
-// tiles (upd) of kFaceThreads nodes.  The item order (built on the host)
-// rotates the kinds across rounds of the grid, as k_batch_stage does.
+// One stage of a reduced form on b.stream.
 template <class Ops>
-__global__ void __launch_bounds__(kFaceThreads, Ops::kMinBlocksTiled)
-k_batch_stage_tiled(const LatView *__restrict__ views, const BatchItem *__restrict__ items, int nitems,
-                    const BatchTile *__restrict__ upd, int nupd, int jst, unsigned *bar, unsigned *gflags,
-                    unsigned long long limit_ns)
+cudaError_t batch_stage_reduced(const BatchLaunch &b, int j)
 {
-    __shared__ float smem[Ops::kTileSmemFloats];
-    for (int w = next_item(bar); w < nitems; w = next_item(bar)) {
-        const BatchItem it = items[w];
-        const LatView &g = views[it.inst];
-        const TileAt at{it.a, it.b, it.c};
-        if (it.kind == 0) {
-            if ((int)threadIdx.x < it.b) {
-                if (g.P.viscous) Ops::visc(g, it.a + threadIdx.x, jst);
-                else Ops::mu(g, it.a + threadIdx.x, jst);
-            }
-        } else if (it.kind == 1) {
-            Ops::template face_tile<0>(g, at, smem);
-        } else if (it.kind == 2) {
-            Ops::template face_tile<1>(g, at, smem);
-        } else {
-            Ops::template face_tile<2>(g, at, smem);
-        }
-    }   // next_item synchronises the block before the next item restages smem
-    if (!grid_barrier(bar, gridDim.x, limit_ns, gflags)) return;
-    for (int w = blockIdx.x; w < nupd; w += gridDim.x) {
-        const BatchTile t = upd[w];
-        if ((int)threadIdx.x < t.count) Ops::update(views[t.inst], t.n0 + threadIdx.x, jst);
-    }
+    k_batch_fluxes<Ops><<<b.nitems, kFaceThreads, 0, b.stream>>>(b.views, b.items, j);
+    const cudaError_t e = cudaPeekAtLastError();
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(b.blocks);
+    cfg.blockDim = dim3(b.threads);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = b.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_batch_close_reduced<Ops>, b.views, b.tiles, b.ntiles, j, b.bar,
+                              b.gflags, b.limit_ns);
+}
+
+template <class Ops>
+int batch_occupancy_reduced(int threads)
+{
+    int nb = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_close_reduced<Ops>, threads, 0) == cudaSuccess ? nb : 0;
 }
 
 // prep (U_Q) of stage 0 for one lattice, before its first stage

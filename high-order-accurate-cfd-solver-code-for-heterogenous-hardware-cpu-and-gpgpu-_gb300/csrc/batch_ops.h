@@ -11,7 +11,7 @@ namespace cfd {
 struct BatchTile;
 struct BatchItem;
 
-// Face-tile shapes of the batched kernel's tiled form: faces along i x
+// Face-tile shapes of the reduced forms' face launch: faces along i x
 // nodes across for i faces, faces along j or k for j and k faces
 // (kFaceThreads faces per tile).  Shorter i tiles than the single-lattice
 // pass: batched lattices are small (edges 32-96).
@@ -28,10 +28,9 @@ struct BatchLaunch {
     unsigned *gflags;          // device error word of the batch
     unsigned long long limit_ns;
     cudaStream_t stream;
-    // tiled form (reduced-precision forms): phase A items, phase B uses tiles
+    // reduced forms: viscous ranges and face tiles
     const BatchItem *items = nullptr;
     int nitems = 0;
-    int tiled = 0;
     // FP64 form: the face kernels' scratch, [3][kFaceScratch] columns of
     // round_tiles tiles
     double *scratch = nullptr;
@@ -47,16 +46,15 @@ constexpr int kBatchRound = 1 << 20;
 cudaError_t batch_stage_fp64(const BatchLaunch &b, int j);
 cudaError_t batch_stage_mixed(const BatchLaunch &b, int j);
 cudaError_t batch_stage_split(const BatchLaunch &b, int j);
-// Launches of one FP64 stage (the reduced forms: 1).
+// Launches of one FP64 stage (the reduced forms: 2).
 int batch_launches_fp64(int ntiles, int round_tiles);
 // Stage-0 prep of one lattice.
 void batch_prep_fp64(const LatView &g, cudaStream_t st);
 void batch_prep_mixed(const LatView &g, cudaStream_t st);
 void batch_prep_split(const LatView &g, cudaStream_t st);
-// Co-resident blocks per SM of the stage kernel at `threads` per block
-// (tiled: the tiled form's kernel, kFaceThreads per block).
+// Co-resident blocks per SM of the closing kernel at `threads` per block.
 int batch_occupancy_fp64(int threads);
-int batch_occupancy_mixed(int threads, bool tiled = false);
-int batch_occupancy_split(int threads, bool tiled = false);
+int batch_occupancy_mixed(int threads);
+int batch_occupancy_split(int threads);
 
 }  // namespace cfd

@@ -87,30 +87,27 @@ __device__ __forceinline__ TileAt tile_of_block()
 struct NodeIn {
     float prim[5], m[3], det;
 };
-template <int D, bool RO>
+template <int D>
 __device__ __forceinline__ NodeIn lat_node_in(const LatView &g, int node)
 {
-    auto ld = [](const float *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
-    return {{ld(g.Q32 + node), ld(g.R32 + node), ld(g.R32 + N + node), ld(g.R32 + 2 * N + node),
-             ld(g.prim32 + LF_P * N + node)},
+    return {{__ldg(g.Q32 + node), __ldg(g.R32 + node), __ldg(g.R32 + N + node), __ldg(g.R32 + 2 * N + node),
+             __ldg(g.prim32 + LF_P * N + node)},
             {__ldg(g.node32 + 3 * D * N + node), __ldg(g.node32 + (3 * D + 1) * N + node),
              __ldg(g.node32 + (3 * D + 2) * N + node)},
             __ldg(g.node32 + 9 * N + node)};
 }
 
 // Stages the block's stencil lines of Q, the Roe inputs and the node fluxes
-// along D (read-only in the face pass: non-coherent loads, unless RO is
-// false because the same launch wrote them) into sQ/sR/sF, each
+// along D (read-only in the face pass: non-coherent loads) into sQ/sR/sF, each
 // [5][T::kStaged]; ends with __syncthreads().  A block stages 1.04 to 1.6
 // nodes per thread: all of a thread's loads are issued before its first
 // store, so that the block waits for memory once (a direction of
 // TGV 128^3, split: 0.100 -> 0.097 ms).
-template <class T, int D, bool RO = true>
+template <class T, int D>
 __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, float *sQ, float *sR, float *sF)
 {
     constexpr int S = T::kStaged, R = (S + kFaceThreads - 1) / kFaceThreads;
-    auto ld = [](const float *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
     const int nA = lat_extent(g, T::A);
     int e[R];
@@ -128,11 +125,11 @@ __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, fl
         c[T::B] = at.cB;
         const int node = c[0] + g.ni * (c[1] + g.nj * c[2]);
         e[k] = T::at(b, a);
-        in[k] = lat_node_in<D, RO>(g, node);
+        in[k] = lat_node_in<D>(g, node);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) q[k][x] = ld(g.Q32 + (x + 1) * N + node);
+        for (int x = 0; x < 4; ++x) q[k][x] = __ldg(g.Q32 + (x + 1) * N + node);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) r[k][x] = ld(g.R32 + (x + 3) * N + node);
+        for (int x = 0; x < 2; ++x) r[k][x] = __ldg(g.R32 + (x + 3) * N + node);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) {

@@ -117,12 +117,10 @@ __device__ __forceinline__ int lat_step(const LatView &g, int i, int j, int k, i
 // the same for the warp: one offset register serves every component, where
 // the index c N + n costs an addition and a widening product per load (a
 // fifth of the reduced forms' viscous and update instructions).
-// RO: through the non-coherent path.
-template <bool RO = true, class T>
+template <class T>
 __device__ __forceinline__ T lat_ldg(const T *p, unsigned bytes)
 {
-    const T *a = reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + bytes);
-    return RO ? __ldg(a) : *a;
+    return __ldg(reinterpret_cast<const T *>(reinterpret_cast<const char *>(p) + bytes));
 }
 
 // Component c of node n of a [components][N] array, addressed the same way.

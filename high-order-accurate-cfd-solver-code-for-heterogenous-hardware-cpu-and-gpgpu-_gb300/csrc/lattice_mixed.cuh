@@ -280,51 +280,11 @@ __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
     g.prim32[LF_MU * N + n] = (sd * sd * sd) * qdiv(1.0f + S, d_temp + S);
 }
 
-// Face n+1/2 along D, all FP32, on paired lanes (physics_x2.cuh).
-template <int D>
-__device__ __forceinline__ void face_node(const LatView &g, int n)
-{
-    const int N = g.N;
-    int i, j, k;
-    lat_ijk(g, n, i, j, k);
-    if (!lat_face_needed(g, i, j, k, D)) return;
-    int s[6];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, D, o - 2);
-    float2 P[3][5];   // (point k, point 5-k)
-#pragma unroll
-    for (int o = 0; o < 3; ++o)
-#pragma unroll
-        for (int c = 0; c < 5; ++c) P[o][c] = make_float2(g.Q32[c * N + s[o]], g.Q32[c * N + s[5 - o]]);
-    float r[5];
-    {
-        const int l = s[2], rr = s[3];
-        const float *R = g.R32;
-        roe_average(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
-                           R[N + l], R[2 * N + l], R[4 * N + l], r);
-    }
-    float Fhat[5];
-    x2::llf_face_flux2(P, g.fm32[(D * 3 + 0) * N + n], g.fm32[(D * 3 + 1) * N + n], g.fm32[(D * 3 + 2) * N + n],
-                       g.fdet32[D * N + n], r, x2::weno_eps2(g.P), Fhat);
-    float NF[6][5];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) {
-        const NodeIn in = lat_node_in<D, false>(g, s[o]);
-        node_inviscid_flux(in.prim, in.m, in.det, NF[o]);
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
-        g.Fh32[(D * 5 + c) * N + n] = __fadd_rn(Fhat[c], x2::face_correction_sym(f));
-    }
-}
-
 // Faces along D of one staged tile (face_tile.cuh): the block of
 // kFaceThreads threads stages the tile's stencil lines into smem
 // (tile_smem_floats<T>() floats) and each thread evaluates its face.  Every
-// thread of the block must call it (it synchronises the block).  RO as in
-// stage_face_lines.
-template <class T, int D, bool RO = true>
+// thread of the block must call it (it synchronises the block).
+template <class T, int D>
 __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *smem)
 {
     constexpr int S = T::kStaged;
@@ -338,7 +298,7 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
         for (int c = 0; c < 3; ++c) m[c] = lat_ldg(g.fm32 + (size_t)(D * 3 + c) * N, 4u * n);
         det_f = lat_ldg(g.fdet32 + (size_t)D * N, 4u * n);
     }
-    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
+    stage_face_lines<T, D>(g, at, sQ, sR, sF);
     if (!face) return;
     float2 P[3][5];
     float r[5];
@@ -360,14 +320,10 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
 //   jst 1: U2 = 3/4 U0 + 1/4 U1 + 1/4 dt L
 //   jst 2: U0 = (U0 + 2 (U2 + dt L)) / 3
 // and the new state lands in slot (jst+1) mod 3, which is also the next
-// stage's U_Q slot.  LOC as for visc_node.  RO: the face and viscous
-// fluxes were written by an earlier launch, so they may be read through the
-// non-coherent path (not in the batched kernel, which writes them in the
-// same launch).
-template <bool LOC, bool RO = true>
+// stage's U_Q slot.  LOC as for visc_node.
+template <bool LOC>
 __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 {
-    auto ld = [](const float *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
     if (LOC && lat_ghost(g, n)) {
         // Ghosts are the boundary routine's, which fills those next to face
@@ -392,7 +348,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
             const float *Fd = g.Fh32 + (size_t)(d * 5 + c) * N;
-            Lf[c] += lat_ldg<RO>(Fd, 4u * n) - lat_ldg<RO>(Fd, 4u * m1);
+            Lf[c] += lat_ldg(Fd, 4u * n) - lat_ldg(Fd, 4u * m1);
         }
         if (LOC && g.P.viscous && lat_locdir(g, d) && ((lflag >> d) & 1u)) {
             int s[7], L7[7];
@@ -407,7 +363,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             for (int c = 1; c < 5; ++c) {
                 float f[7];
 #pragma unroll
-                for (int o = 0; o < 7; ++o) f[o] = ld(Vd + c * N + s[o]);
+                for (int o = 0; o < 7; ++o) f[o] = __ldg(Vd + c * N + s[o]);
                 Lf[c] += branch_deriv<float>(b, f);
             }
         } else if (g.P.viscous) {
@@ -415,8 +371,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 #pragma unroll
             for (int c = 1; c < 5; ++c) {
                 const float *V = g.V32 + (size_t)(d * 5 + c) * N;
-                const float d1 = lat_ldg<RO>(V, 4u * p1) - lat_ldg<RO>(V, 4u * m1),
-                            d2 = lat_ldg<RO>(V, 4u * p2) - lat_ldg<RO>(V, 4u * m2);
+                const float d1 = lat_ldg(V, 4u * p1) - lat_ldg(V, 4u * m1),
+                            d2 = lat_ldg(V, 4u * p2) - lat_ldg(V, 4u * m2);
                 Lf[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, d1, -d2), Lf[c]);
             }
         }

@@ -148,57 +148,16 @@ __device__ __forceinline__ void face_flux(const LatView &g, const FaceMetric &f,
     x2::llf_face_flux2_split(P, f.m32[0], f.m32[1], f.m32[2], f.m, f.det, r, x2::weno_eps2(g.P), corr, out);
 }
 
-// Face n+1/2 along D with its stencil read from the lattice (the batched
-// kernel's face item; the single-lattice pass stages tiles in split.cu).
-template <int D>
-__device__ __forceinline__ void face_node(const LatView &g, int n)
-{
-    const int N = g.N;
-    int i, j, k;
-    lat_ijk(g, n, i, j, k);
-    if (!lat_face_needed(g, i, j, k, D)) return;
-    int s[6];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, D, o - 2);
-    float2 P[3][5];
-#pragma unroll
-    for (int o = 0; o < 3; ++o)
-#pragma unroll
-        for (int c = 0; c < 5; ++c) P[o][c] = make_float2(g.Q32[c * N + s[o]], g.Q32[c * N + s[5 - o]]);
-    float r[5];
-    {
-        const int l = s[2], rr = s[3];
-        const float *R = g.R32;
-        roe_average(R[3 * N + rr], R[rr], R[N + rr], R[2 * N + rr], R[4 * N + rr], R[3 * N + l], R[l],
-                           R[N + l], R[2 * N + l], R[4 * N + l], r);
-    }
-    float NF[6][5], corr[5];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) {
-        const NodeIn in = lat_node_in<D, false>(g, s[o]);
-        node_inviscid_flux(in.prim, in.m, in.det, NF[o]);
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        const float f[6] = {NF[0][c], NF[1][c], NF[2][c], NF[3][c], NF[4][c], NF[5][c]};
-        corr[c] = x2::face_correction_sym(f);
-    }
-    double Fh[5];
-    face_flux(g, face_metric<D>(g, n), P, r, corr, Fh);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) g.Fh[(D * 5 + c) * N + n] = Fh[c];
-}
-
 // Faces along D of one staged tile (mx::face_tile with the FP64 face
 // flux of face_flux written to Fh).
-template <class T, int D, bool RO = true>
+template <class T, int D>
 __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *smem)
 {
     constexpr int S = T::kStaged;
     float *sQ = smem, *sR = smem + 5 * S, *sF = smem + 10 * S;
     const int N = g.N;
     int n, t, a;
-    stage_face_lines<T, D, RO>(g, at, sQ, sR, sF);
+    stage_face_lines<T, D>(g, at, sQ, sR, sF);
     if (!tile_face<T, D>(g, at, n, t, a)) return;
     float2 P[3][5];
     float r[5];
@@ -222,11 +181,10 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
 //   jst 1: U2 = (3 U0 + (U1 + dt L)) / 4
 //   jst 2: U0 = (U0 + 2 (U2 + dt L)) / 3
 // The new state lands in slot (jst+1) mod 3, which is also the next stage's
-// U_Q slot.  LOC and RO as for the mixed form's update_node.
-template <bool LOC, bool RO = true>
+// U_Q slot.  LOC as for the mixed form's update_node.
+template <bool LOC>
 __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 {
-    auto ldf = [](const float *p) { return RO ? __ldg(p) : *p; };
     const int N = g.N;
     if (LOC && lat_ghost(g, n)) {   // ghosts: the state moves on (mixed form's update_node)
         if (g.Lout) {
@@ -251,7 +209,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
             const double *Fd = g.Fh + (size_t)(d * 5 + c) * N;
-            const double df = lat_ldg<RO>(Fd, 8u * n) - lat_ldg<RO>(Fd, 8u * m1);
+            const double df = lat_ldg(Fd, 8u * n) - lat_ldg(Fd, 8u * m1);
             Ld[c] = d == 0 ? df : Ld[c] + df;
         }
         if (LOC && g.P.viscous && lat_locdir(g, d) && ((lflag >> d) & 1u)) {
@@ -267,7 +225,7 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
             for (int c = 1; c < 5; ++c) {
                 float f[7];
 #pragma unroll
-                for (int o = 0; o < 7; ++o) f[o] = ldf(Vd + c * N + s[o]);
+                for (int o = 0; o < 7; ++o) f[o] = __ldg(Vd + c * N + s[o]);
                 Lv[c] += branch_deriv<float>(b, f);
             }
         } else if (g.P.viscous) {
@@ -275,8 +233,8 @@ __device__ __forceinline__ void update_node(const LatView &g, int n, int jst)
 #pragma unroll
             for (int c = 1; c < 5; ++c) {
                 const float *V = g.V32 + (size_t)(d * 5 + c) * N;
-                const float d1 = lat_ldg<RO>(V, 4u * p1) - lat_ldg<RO>(V, 4u * m1),
-                            d2 = lat_ldg<RO>(V, 4u * p2) - lat_ldg<RO>(V, 4u * m2);
+                const float d1 = lat_ldg(V, 4u * p1) - lat_ldg(V, 4u * m1),
+                            d2 = lat_ldg(V, 4u * p2) - lat_ldg(V, 4u * m2);
                 Lv[c] = fmaf(1.0f / 12.0f, fmaf(8.0f, d1, -d2), Lv[c]);
             }
         }
