@@ -37,8 +37,9 @@ struct BatchInst {
     std::vector<void *> allocs;
     uint64_t bytes = 0;
     LatView view{};
-    double *stage9 = nullptr;   // AoS FLOW staging rows 0..N
-    double *stage5 = nullptr;   // AoS column staging rows 0..N
+    double *stage9 = nullptr;   // AoS FLOW staging rows 0..N (FP64 form: the face fluxes' array, dead between stages)
+    double *stage5 = nullptr;   // AoS column staging rows 0..N (likewise)
+    double row0[9] = {};        // FLOW row 0 as last set (no node: the layout's dummy row)
 };
 
 }  // namespace
@@ -86,13 +87,14 @@ unsigned *slot_flags(cfd_batch *b, int slot) { return b->d_words + 4 + slot; }
 
 uint64_t instance_bytes(int precision, int64_t N)
 {
-    const uint64_t doubles = (22 + 9 + 15) * (uint64_t)N + 14 * (uint64_t)(N + 1);
+    const uint64_t n = (uint64_t)N, doubles = (22 + 9 + 15) * n + 14 * (n + 1);   // with the AoS staging rows
     // mixed: FP32 face/node geometry (12 + 10 + 2), prim32 (9), stage intermediates (40)
-    if (precision == CFD_PREC_MIXED) return doubles * 8 + (12 + 11 + 2 + 9 + 40) * (uint64_t)N * 4;
+    if (precision == CFD_PREC_MIXED) return doubles * 8 + (12 + 11 + 2 + 9 + 40) * n * 4;
     // split: FP32 face metrics (9), node geometry (11), prim32 (9), Q32/R32/V32 (25) and the hi/lo
     // state copy (10); FP64 1/det and Fh (16)
     if (precision == CFD_PREC_SPLIT) return (doubles + 16 * (uint64_t)N) * 8 + (9 + 11 + 9 + 25 + 10) * (uint64_t)N * 4;
-    return (doubles + 65 * (uint64_t)N) * 8;   // stage intermediates (55), unit normals (9), filter width
+    // FP64: stage intermediates (55, the face fluxes' 15 also the staging rows), unit normals (9), filter width
+    return ((22 + 9 + 15) * n + 50 * n + std::max(15 * n, 9 * (n + 1))) * 8;
 }
 
 void drop_graph(cfd_batch *b)
@@ -547,7 +549,8 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     if ((st = ialloc(b, I, 9 * Nz, &m9)) || (st = ialloc(b, I, Nz, &det)) || (st = ialloc(b, I, 9 * Nz, &fm))
         || (st = ialloc(b, I, 3 * Nz, &fdet)) || (st = ialloc(b, I, 9 * Nz, &prim9)) || (st = ialloc(b, I, 5 * Nz, &U0))
         || (st = ialloc(b, I, 5 * Nz, &U1)) || (st = ialloc(b, I, 5 * Nz, &U2))
-        || (st = ialloc(b, I, 9 * (Nz + 1), &I.stage9)) || (st = ialloc(b, I, 5 * (Nz + 1), &I.stage5))) {
+        || (b->precision != CFD_PREC_FP64
+            && ((st = ialloc(b, I, 9 * (Nz + 1), &I.stage9)) || (st = ialloc(b, I, 5 * (Nz + 1), &I.stage5))))) {
         free_instance(I);
         return st;
     }
@@ -606,14 +609,16 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         v.idet64 = idet64;
     } else {
         if ((st = ialloc(b, I, 5 * Nz, &v.Q)) || (st = ialloc(b, I, 15 * Nz, &v.FEG)) || (st = ialloc(b, I, 15 * Nz, &v.V))
-            || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, 15 * Nz, &v.Fh))
+            || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, std::max(15 * Nz, 9 * (Nz + 1)), &v.Fh))
             || (st = ialloc(b, I, 9 * Nz, &kn)) || (st = ialloc(b, I, Nz, &del))) {
             free_instance(I);
             return st;
         }
         v.kn = kn;
         v.del = del;
+        I.stage9 = I.stage5 = v.Fh;
     }
+    std::memcpy(I.row0, host_ptr(S->flow), sizeof I.row0);
     cudaStream_t sm = ctx->stream;
     cudaError_t e = cudaMemcpyAsync(m9, host_ptr(S->m9), 9 * Nz * 8, cudaMemcpyHostToDevice, sm);
     if (e == cudaSuccess) e = cudaMemcpyAsync(det, host_ptr(S->det), Nz * 8, cudaMemcpyHostToDevice, sm);
@@ -621,7 +626,6 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     if (e == cudaSuccess) e = cudaMemcpyAsync(fdet, host_ptr(S->fdet), 3 * Nz * 8, cudaMemcpyHostToDevice, sm);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(I.stage9, host_ptr(S->flow), 9 * (Nz + 1) * 8, cudaMemcpyHostToDevice, sm);
-    if (e == cudaSuccess) e = cudaMemsetAsync(I.stage5, 0, 5 * (Nz + 1) * 8, sm);
     if (e == cudaSuccess) e = cudaMemsetAsync(v.flags, 0, sizeof(unsigned), sm);
     for (double *u : {U0, U1, U2})
         if (e == cudaSuccess) e = cudaMemsetAsync(u, 0, 5 * Nz * 8, sm);
@@ -782,7 +786,8 @@ cfd_status_t cfd_batch_get_flow(cfd_batch_t *b, int32_t slot, cfd_flow_t *host)
     if (b->precision == CFD_PREC_MIXED) mixed_flow_out(I.view, 0, b->ctx->stream);
     if (b->precision == CFD_PREC_SPLIT) split_flow_out(I.view, 0, b->ctx->stream);
     soa_to_aos(b->ctx->stream, I.view.prim9, 9, 9, I.N, I.stage9);
-    cudaError_t e = cudaMemcpyAsync(host, I.stage9, 9 * ((size_t)I.N + 1) * 8, cudaMemcpyDeviceToHost, b->ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(host + 1, I.stage9 + 9, 9 * (size_t)I.N * 8, cudaMemcpyDeviceToHost, b->ctx->stream);
+    std::memcpy(host, I.row0, sizeof I.row0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(b->ctx, e, "cfd_batch_get_flow");
     return CFD_OK;
@@ -797,7 +802,8 @@ cfd_status_t cfd_batch_get_u0(cfd_batch_t *b, int32_t slot, cfd_column_t *host)
         mixed_u_out(I.view, 0, I.stage5, b->ctx->stream);
     else
         soa_to_aos(b->ctx->stream, I.view.U0, 5, 5, I.N, I.stage5);
-    cudaError_t e = cudaMemcpyAsync(host, I.stage5, 5 * ((size_t)I.N + 1) * 8, cudaMemcpyDeviceToHost, b->ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(host + 1, I.stage5 + 5, 5 * (size_t)I.N * 8, cudaMemcpyDeviceToHost, b->ctx->stream);
+    std::memset(host, 0, sizeof *host);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(b->ctx, e, "cfd_batch_get_u0");
     return CFD_OK;
@@ -827,6 +833,7 @@ cfd_status_t cfd_batch_set_flow(cfd_batch_t *b, int32_t slot, const cfd_flow_t *
         e = cudaMemcpyAsync(I.stage9, flow_host, 9 * ((size_t)I.N + 1) * 8, cudaMemcpyHostToDevice, sm);
     if (e == cudaSuccess) e = cudaMemsetAsync(slot_flags(b, slot), 0, sizeof(unsigned), sm);
     if (e != cudaSuccess) return cuda_fail(b->ctx, e, "cfd_batch_set_flow upload");
+    std::memcpy(I.row0, flow_host, sizeof I.row0);
     aos_to_soa(sm, I.stage9, 9, 9, I.N, I.view.prim9);
     if (b->precision == CFD_PREC_MIXED)
         batch_prep_mixed(I.view, sm);
