@@ -74,6 +74,14 @@ struct TileAt {
     int tD, tA, cB;
 };
 
+// The tile of block w of T's grid (gr) laid out in one dimension.
+template <class T>
+__device__ __forceinline__ TileAt tile_of_index(unsigned w, uint3 gr)
+{
+    const unsigned r = w / gr.x;
+    return {(int)(w - r * gr.x) * T::kTile, (int)(r % gr.y) * T::kWide, (int)(r / gr.y)};
+}
+
 template <class T>
 __device__ __forceinline__ TileAt tile_of_block()
 {
@@ -197,5 +205,61 @@ constexpr int tile_smem_floats()
 {
     return 15 * T::kStaged;
 }
+
+// A stage's fluxes in one launch: blocks 0 .. nv - 1 a viscous range each
+// (their chains are the longest), then the face tiles along i, j and k.
+// Ops::visc<LOC>(g, n, q) and Ops::face_tile<T, D>(g, at, smem) of one form.
+struct FluxGrid {
+    unsigned nv, b[2];   // viscous ranges; end of the i tiles, of the j tiles
+    uint3 gr[3];
+};
+using FluxTileI = FaceTile<0, 32>;
+using FluxTileJ = FaceTile<1, 16>;
+using FluxTileK = FaceTile<2, 16>;
+
+inline unsigned flux_grid(const LatView &g, FluxGrid &f)
+{
+    const dim3 d[3] = {FluxTileI::grid(g), FluxTileJ::grid(g), FluxTileK::grid(g)};
+    unsigned n = f.nv = (unsigned)((g.N + kFaceThreads - 1) / kFaceThreads);
+    for (int k = 0; k < 3; ++k) {
+        f.gr[k] = make_uint3(d[k].x, d[k].y, d[k].z);
+        n += d[k].x * d[k].y * d[k].z;
+        if (k < 2) f.b[k] = n;
+    }
+    return n;
+}
+
+template <class Ops, bool LOC>
+__device__ __forceinline__ void flux_block(const LatView &g, int q, const FluxGrid &f, float *smem)
+{
+    const unsigned w = blockIdx.x;
+    if (w < f.nv) {
+        const int n = (int)(w * kFaceThreads + threadIdx.x);
+        if (n < g.N) Ops::template visc<LOC>(g, n, q);
+    } else if (w < f.b[0]) {
+        Ops::template face_tile<FluxTileI, 0>(g, tile_of_index<FluxTileI>(w - f.nv, f.gr[0]), smem);
+    } else if (w < f.b[1]) {
+        Ops::template face_tile<FluxTileJ, 1>(g, tile_of_index<FluxTileJ>(w - f.b[0], f.gr[1]), smem);
+    } else {
+        Ops::template face_tile<FluxTileK, 2>(g, tile_of_index<FluxTileK>(w - f.b[1], f.gr[2]), smem);
+    }
+}
+
+constexpr int flux_smem_floats()
+{
+    constexpr int i = tile_smem_floats<FluxTileI>(), j = tile_smem_floats<FluxTileJ>();
+    return i > j ? i : j;
+}
+
+// Nodes up to which a reduced form's fluxes run in one launch instead of as
+// four kernels on four streams (split form, a stage; four streams against one
+// launch): 17^3 nodes 23.2 and 18.8 us, 24^3 23.0 and 20.8, 33^3 29.2 and
+// 27.5, 46^3 40.6 and 40.3, 64^3 82.6 and 81.3 (mixed 58.6 and 57.4), 256 x
+// 64 x 16 with ghost layers 106 and 113, where each kernel's own registers
+// and the tuned tiles tell.
+#ifndef CFD_ONE_LAUNCH_NODES
+#define CFD_ONE_LAUNCH_NODES 200000
+#endif
+constexpr int kOneLaunchNodes = CFD_ONE_LAUNCH_NODES;
 
 }  // namespace cfd

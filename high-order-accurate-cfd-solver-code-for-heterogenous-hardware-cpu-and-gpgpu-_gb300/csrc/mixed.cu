@@ -109,6 +109,27 @@ void launch_face_tile(const LatView &g, cudaStream_t st, int tile)
     }
 }
 
+struct Fluxes {
+    template <bool LOC>
+    static __device__ __forceinline__ void visc(const LatView &g, int n, int q)
+    {
+        if (g.P.viscous) mx::visc_node<LOC>(g, n, q);
+        else mx::mu_node(g, n, q);
+    }
+    template <class T, int D>
+    static __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *smem)
+    {
+        mx::face_tile<T, D>(g, at, smem);
+    }
+};
+
+template <bool LOC>
+__global__ void __launch_bounds__(kFaceThreads, 7) k_fluxes_m(LatView g, int q, FluxGrid f)
+{
+    __shared__ float smem[flux_smem_floats()];
+    flux_block<Fluxes, LOC>(g, q, f, smem);
+}
+
 // 48 registers: at 128^3 0.115 ms, 0.127 at 64, 0.119 at 40
 #ifndef CFD_MUPD_MIN_BLOCKS
 #define CFD_MUPD_MIN_BLOCKS 5
@@ -243,51 +264,61 @@ int mixed_stage(const StructuredLaunch &S, int jst, double dt, double *Lout, cud
         mark();
     }
     const bool loc = g.loc8 != nullptr;   // lattice with ghost layers and loc codes
-    // The viscous pass and the face passes are independent (the update reads
-    // both): without event timing the viscous pass runs on the side stream,
-    // concurrently with the faces.
-    const bool side = S.side && !ev;
-    cudaStream_t sv = side ? S.side : st;
-    if (side) {
-        cudaEventRecord(S.fork, st);
-        cudaStreamWaitEvent(sv, S.fork, 0);
-    }
-    if (S.P.viscous) {
+    if (!ev && g.N <= kOneLaunchNodes) {
+        FluxGrid f;
+        const unsigned nf = flux_grid(g, f);
         if (loc)
-            k_visc_m<true><<<nb256, 256, 0, sv>>>(g, jst);
+            k_fluxes_m<true><<<nf, kFaceThreads, 0, st>>>(g, jst, f);
         else
-            k_visc_m<false><<<nb256, 256, 0, sv>>>(g, jst);
-        name("viscous");
+            k_fluxes_m<false><<<nf, kFaceThreads, 0, st>>>(g, jst, f);
+        name("fluxes");
     } else {
-        k_mu_m<<<nb256, 256, 0, sv>>>(g, jst);
-        name("mu_only");
+        // The viscous pass and the face passes are independent (the update reads
+        // both): without event timing the viscous pass runs on the side stream,
+        // concurrently with the faces.
+        const bool side = S.side && !ev;
+        cudaStream_t sv = side ? S.side : st;
+        if (side) {
+            cudaEventRecord(S.fork, st);
+            cudaStreamWaitEvent(sv, S.fork, 0);
+        }
+        if (S.P.viscous) {
+            if (loc)
+                k_visc_m<true><<<nb256, 256, 0, sv>>>(g, jst);
+            else
+                k_visc_m<false><<<nb256, 256, 0, sv>>>(g, jst);
+            name("viscous");
+        } else {
+            k_mu_m<<<nb256, 256, 0, sv>>>(g, jst);
+            name("mu_only");
+        }
+        if (side) cudaEventRecord(S.join, sv);
+        mark();
+        // the three face passes write separate fluxes: the j and k passes run on
+        // their own streams, so that no pass waits for the last wave of another
+        const bool fside = side && S.face_side[0] && S.face_side[1];
+        cudaStream_t sj = fside ? S.face_side[0] : st, sk = fside ? S.face_side[1] : st;
+        if (fside) {
+            cudaStreamWaitEvent(sj, S.fork, 0);
+            cudaStreamWaitEvent(sk, S.fork, 0);
+        }
+        launch_face_tile<0>(g, st, S.tile_i);
+        name("face_i");
+        mark();
+        launch_face_tile<1>(g, sj, S.tile_jk);
+        name("face_j");
+        mark();
+        launch_face_tile<2>(g, sk, S.tile_jk);
+        name("face_k");
+        mark();
+        if (fside) {
+            cudaEventRecord(S.face_join[0], sj);
+            cudaEventRecord(S.face_join[1], sk);
+            cudaStreamWaitEvent(st, S.face_join[0], 0);
+            cudaStreamWaitEvent(st, S.face_join[1], 0);
+        }
+        if (side) cudaStreamWaitEvent(st, S.join, 0);
     }
-    if (side) cudaEventRecord(S.join, sv);
-    mark();
-    // the three face passes write separate fluxes: the j and k passes run on
-    // their own streams, so that no pass waits for the last wave of another
-    const bool fside = side && S.face_side[0] && S.face_side[1];
-    cudaStream_t sj = fside ? S.face_side[0] : st, sk = fside ? S.face_side[1] : st;
-    if (fside) {
-        cudaStreamWaitEvent(sj, S.fork, 0);
-        cudaStreamWaitEvent(sk, S.fork, 0);
-    }
-    launch_face_tile<0>(g, st, S.tile_i);
-    name("face_i");
-    mark();
-    launch_face_tile<1>(g, sj, S.tile_jk);
-    name("face_j");
-    mark();
-    launch_face_tile<2>(g, sk, S.tile_jk);
-    name("face_k");
-    mark();
-    if (fside) {
-        cudaEventRecord(S.face_join[0], sj);
-        cudaEventRecord(S.face_join[1], sk);
-        cudaStreamWaitEvent(st, S.face_join[0], 0);
-        cudaStreamWaitEvent(st, S.face_join[1], 0);
-    }
-    if (side) cudaStreamWaitEvent(st, S.join, 0);
     if (loc)
         k_update_m<true><<<nb256, 256, 0, st>>>(g, jst);
     else

@@ -95,6 +95,27 @@ void launch_face_tile_s(const LatView &g, cudaStream_t st, int tile)
     }
 }
 
+struct Fluxes {
+    template <bool LOC>
+    static __device__ __forceinline__ void visc(const LatView &g, int n, int q)
+    {
+        if (g.P.viscous) mx::visc_node<LOC>(sp::hilo_view(g), n, 0);
+        else mx::mu_node(sp::hilo_view(g), n, 0);
+    }
+    template <class T, int D>
+    static __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *smem)
+    {
+        sp::face_tile<T, D>(g, at, smem);
+    }
+};
+
+template <bool LOC>
+__global__ void __launch_bounds__(kFaceThreads, 7) k_fluxes_s(LatView g, int q, FluxGrid f)
+{
+    __shared__ float smem[flux_smem_floats()];
+    flux_block<Fluxes, LOC>(g, q, f, smem);
+}
+
 // 64 registers: at 128^3 0.190 ms, 0.193 at 48 and 40, 0.221 unbounded
 #ifndef CFD_SUPD_MIN_BLOCKS
 #define CFD_SUPD_MIN_BLOCKS 4
@@ -210,47 +231,57 @@ int split_stage(const StructuredLaunch &S, int jst, double dt, double *Lout, cud
         mark();
     }
     const bool loc = g.loc8 != nullptr;
-    const bool side = S.side && !ev;   // viscous pass beside the face passes (not when timing each launch)
-    cudaStream_t sv = side ? S.side : st;
-    if (side) {
-        cudaEventRecord(S.fork, st);
-        cudaStreamWaitEvent(sv, S.fork, 0);
-    }
-    const LatView gh = sp::hilo_view(g);
-    if (S.P.viscous) {
+    if (!ev && g.N <= kOneLaunchNodes) {
+        FluxGrid f;
+        const unsigned nf = flux_grid(g, f);
         if (loc)
-            k_visc_s<true><<<nb256, 256, 0, sv>>>(gh);
+            k_fluxes_s<true><<<nf, kFaceThreads, 0, st>>>(g, jst, f);
         else
-            k_visc_s<false><<<nb256, 256, 0, sv>>>(gh);
-        name("viscous");
+            k_fluxes_s<false><<<nf, kFaceThreads, 0, st>>>(g, jst, f);
+        name("fluxes");
     } else {
-        k_mu_s<<<nb256, 256, 0, sv>>>(gh);
-        name("mu_only");
+        const bool side = S.side && !ev;   // viscous pass beside the face passes (not when timing each launch)
+        cudaStream_t sv = side ? S.side : st;
+        if (side) {
+            cudaEventRecord(S.fork, st);
+            cudaStreamWaitEvent(sv, S.fork, 0);
+        }
+        const LatView gh = sp::hilo_view(g);
+        if (S.P.viscous) {
+            if (loc)
+                k_visc_s<true><<<nb256, 256, 0, sv>>>(gh);
+            else
+                k_visc_s<false><<<nb256, 256, 0, sv>>>(gh);
+            name("viscous");
+        } else {
+            k_mu_s<<<nb256, 256, 0, sv>>>(gh);
+            name("mu_only");
+        }
+        if (side) cudaEventRecord(S.join, sv);
+        mark();
+        const bool fside = side && S.face_side[0] && S.face_side[1];
+        cudaStream_t sj = fside ? S.face_side[0] : st, sk = fside ? S.face_side[1] : st;
+        if (fside) {
+            cudaStreamWaitEvent(sj, S.fork, 0);
+            cudaStreamWaitEvent(sk, S.fork, 0);
+        }
+        launch_face_tile_s<0>(g, st, S.tile_i);
+        name("face_i");
+        mark();
+        launch_face_tile_s<1>(g, sj, S.tile_jk);
+        name("face_j");
+        mark();
+        launch_face_tile_s<2>(g, sk, S.tile_jk);
+        name("face_k");
+        mark();
+        if (fside) {
+            cudaEventRecord(S.face_join[0], sj);
+            cudaEventRecord(S.face_join[1], sk);
+            cudaStreamWaitEvent(st, S.face_join[0], 0);
+            cudaStreamWaitEvent(st, S.face_join[1], 0);
+        }
+        if (side) cudaStreamWaitEvent(st, S.join, 0);
     }
-    if (side) cudaEventRecord(S.join, sv);
-    mark();
-    const bool fside = side && S.face_side[0] && S.face_side[1];
-    cudaStream_t sj = fside ? S.face_side[0] : st, sk = fside ? S.face_side[1] : st;
-    if (fside) {
-        cudaStreamWaitEvent(sj, S.fork, 0);
-        cudaStreamWaitEvent(sk, S.fork, 0);
-    }
-    launch_face_tile_s<0>(g, st, S.tile_i);
-    name("face_i");
-    mark();
-    launch_face_tile_s<1>(g, sj, S.tile_jk);
-    name("face_j");
-    mark();
-    launch_face_tile_s<2>(g, sk, S.tile_jk);
-    name("face_k");
-    mark();
-    if (fside) {
-        cudaEventRecord(S.face_join[0], sj);
-        cudaEventRecord(S.face_join[1], sk);
-        cudaStreamWaitEvent(st, S.face_join[0], 0);
-        cudaStreamWaitEvent(st, S.face_join[1], 0);
-    }
-    if (side) cudaStreamWaitEvent(st, S.join, 0);
     if (loc)
         k_update_s<true><<<nb256, 256, 0, st>>>(g, jst);
     else
