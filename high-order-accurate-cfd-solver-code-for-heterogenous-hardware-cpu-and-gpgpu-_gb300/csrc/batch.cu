@@ -123,16 +123,32 @@ cfd_status_t ialloc(cfd_batch *b, BatchInst &I, size_t count, T **p)
     return CFD_OK;
 }
 
-// The face tiles of direction D of lattice view v (FaceTile<D, tile>::grid).
-template <int D>
-void face_tile_items(const LatView &g, int v, std::vector<BatchItem> &out)
+template <int D, int TILE>
+void face_tile_items(const LatView &g, int v, int kind, std::vector<BatchItem> &out)
 {
-    using T = FaceTile<D, D == 0 ? kBatchTileI : kBatchTileJK>;
+    using T = FaceTile<D, TILE, true>;
     const dim3 gr = T::grid(g);
-    for (unsigned z = 0; z < gr.z; ++z)
-        for (unsigned y = 0; y < gr.y; ++y)
-            for (unsigned x = 0; x < gr.x; ++x)
-                out.push_back(BatchItem{v, D, (int)x * T::kTile, (int)y * T::kWide, (int)z, 0});
+    for (unsigned y = 0; y < gr.y; ++y)
+        for (unsigned x = 0; x < gr.x; ++x)
+            out.push_back(BatchItem{v, kind, (int)x * T::kTile, (int)y * T::kWide, 0, 0});
+}
+
+// The i tiles of lattice view v, of the width that costs least: the number of
+// tiles times what a full one takes (short ones stage short pieces of rows:
+// 1.05 and 1.03 of a wide one's time, from 1.0 / 1.0 to 1.35 / 1.12 tried).
+// Lattices of odd or small extents leave much of a wide tile empty.  A split
+// stage of 18 vortices of 13^3 to 30^3: 78 us, 85 with wide tiles only; 21 of
+// 21^3 to 38^3 181 and 209; 24 of 24^3 to 72^3 752 and 814; mixed 41 and 45,
+// 106 and 119, 473 and 502.
+void i_tiles_of(const LatView &g, int v, std::vector<BatchItem> out[3])
+{
+    auto count = [](dim3 gr) { return (double)gr.x * gr.y; };
+    const double c0 = 1.05 * count(FaceTile<0, kBatchTilesI[0], true>::grid(g)),
+                 c1 = 1.03 * count(FaceTile<0, kBatchTilesI[1], true>::grid(g)),
+                 c2 = count(FaceTile<0, kBatchTilesI[2], true>::grid(g));
+    if (c2 <= c0 && c2 <= c1) face_tile_items<0, kBatchTilesI[2]>(g, v, 2, out[2]);
+    else if (c1 <= c0) face_tile_items<0, kBatchTilesI[1]>(g, v, 1, out[1]);
+    else face_tile_items<0, kBatchTilesI[0]>(g, v, 0, out[0]);
 }
 
 // Nodes per node tile (threads per block of the closing kernel).
@@ -145,7 +161,7 @@ cfd_status_t rebuild(cfd_batch *b)
 {
     std::vector<LatView> views;
     std::vector<BatchTile> tiles;
-    std::vector<BatchItem> faces[3];
+    std::vector<BatchItem> faces[5];   // by kind
     const bool reduced = b->precision != CFD_PREC_FP64;
     const int T = node_tile(b);
     uint64_t nodes = 0;
@@ -157,9 +173,9 @@ cfd_status_t rebuild(cfd_batch *b)
         views.push_back(I.view);
         for (int n0 = 0; n0 < I.N; n0 += T) tiles.push_back(BatchTile{v, n0, std::min(T, I.N - n0), 0});
         if (reduced) {
-            face_tile_items<0>(I.view, v, faces[0]);
-            face_tile_items<1>(I.view, v, faces[1]);
-            face_tile_items<2>(I.view, v, faces[2]);
+            i_tiles_of(I.view, v, faces);
+            face_tile_items<1, kBatchTileJK>(I.view, v, 3, faces[3]);
+            face_tile_items<2, kBatchTileJK>(I.view, v, 4, faces[4]);
         }
         nodes += (uint64_t)I.N;
     }
@@ -202,7 +218,7 @@ cfd_status_t rebuild(cfd_batch *b)
         std::vector<BatchItem> items;
         for (int v = 0; v < (int)views.size(); ++v)
             for (int n0 = 0; n0 < views[v].N; n0 += kFaceThreads)
-                items.push_back(BatchItem{v, 3, n0, std::min(kFaceThreads, views[v].N - n0), 0, 0});
+                items.push_back(BatchItem{v, kBatchVisc, n0, std::min(kFaceThreads, views[v].N - n0), 0, 0});
         for (const auto &f : faces) items.insert(items.end(), f.begin(), f.end());
         if (items.size() > b->items_cap) {
             if (b->d_items) cudaFree(b->d_items);

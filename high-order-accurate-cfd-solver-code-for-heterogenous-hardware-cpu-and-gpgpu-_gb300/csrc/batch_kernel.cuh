@@ -92,9 +92,11 @@ __device__ __forceinline__ int next_item(unsigned *bar)
     return s_w;
 }
 
-// Kind 3: the viscous range of b nodes from node a of one lattice; otherwise a
-// face tile along D = kind (a = first face along D, b = first node across,
-// c = line of the third axis; face_tile.cuh).
+// Kind kBatchVisc: the viscous range of b nodes from node a of one lattice;
+// otherwise a face tile (a = first face along its direction, b = first node
+// of the plane across): kinds 0 to 2 along i of width kBatchTilesI[kind],
+// kinds 3 and 4 along j and k.
+constexpr int kBatchVisc = 5;
 struct BatchItem {
     int inst, kind, a, b, c, pad;
 };
@@ -105,27 +107,32 @@ struct BatchItem {
 // own runs at the registers of the
 // face pass alone (72); in one persistent launch with the viscous and update
 // code it had 80 with spills.  24 vortices of 24^3 to 72^3 (2.7 million
-// nodes), a stage: mixed 0.60 -> 0.50 ms, split 0.81 -> 0.79; one of 24^3,
+// nodes), a stage: mixed 0.60 -> 0.50 ms, split 0.81 -> 0.79 (0.47 and 0.75
+// with FLAT tiles); one of 24^3,
 // viscous, mixed 17.3 -> 15.8 us (18.1 with the viscous ranges in the closing
-// launch).  Tile widths
-// chosen per instance (8, 16 or 32, the least padding) were slower: 0.50
-// and 0.82.
+// launch).
 template <class Ops>
 __global__ void __launch_bounds__(kFaceThreads, Ops::kFaceBlocks)
 k_batch_fluxes(const LatView *__restrict__ views, const BatchItem *__restrict__ items, int jst)
 {
-    __shared__ float smem[Ops::kTileSmemFloats];
+    __shared__ float smem[tile_smem_floats<FaceTile<0, kBatchTilesI[0]>>()];   // the widest staging
     const BatchItem it = items[blockIdx.x];
     const LatView &g = views[it.inst];
     const TileAt at{it.a, it.b, it.c};
-    if (it.kind == 3) {
+    switch (it.kind) {
+    case kBatchVisc: {
         if ((int)threadIdx.x >= it.b) return;
         const int n = it.a + threadIdx.x;
         if (g.P.viscous) Ops::visc(g, n, jst);
         else Ops::mu(g, n, jst);
-    } else if (it.kind == 0) Ops::template face_tile<0>(g, at, smem);
-    else if (it.kind == 1) Ops::template face_tile<1>(g, at, smem);
-    else Ops::template face_tile<2>(g, at, smem);
+        break;
+    }
+    case 0: Ops::template face_tile<0, kBatchTilesI[0]>(g, at, smem); break;
+    case 1: Ops::template face_tile<0, kBatchTilesI[1]>(g, at, smem); break;
+    case 2: Ops::template face_tile<0, kBatchTilesI[2]>(g, at, smem); break;
+    case 3: Ops::template face_tile<1, kBatchTileJK>(g, at, smem); break;
+    default: Ops::template face_tile<2, kBatchTileJK>(g, at, smem); break;
+    }
 }
 
 // The grid barrier and the update of every node tile, in blocks of up to 256

@@ -11,12 +11,12 @@ namespace cfd {
 struct BatchTile;
 struct BatchItem;
 
-// Face-tile shapes of the reduced forms' face launch: faces along i x
-// nodes across for i faces, faces along j or k for j and k faces
-// (kFaceThreads faces per tile).  Shorter i tiles than the single-lattice
-// pass: batched lattices are small (edges 32-96).
-constexpr int kBatchTileI = 32;
-constexpr int kBatchTileJK = 16;
+// Faces along the direction of the reduced forms' face tiles (kFaceThreads
+// faces each, FLAT; face_tile.cuh): along i the width that costs least on an
+// instance's extents (batch.cu i_tiles_of), along j and k always the short
+// one, whose rows across are whole cache lines.
+constexpr int kBatchTilesI[3] = {8, 16, 32};
+constexpr int kBatchTileJK = 8;
 
 struct BatchLaunch {
     const LatView *views;      // device table

@@ -11,17 +11,12 @@
 namespace cfd {
 namespace {
 
-template <int D>
-using BTile = FaceTile<D, D == 0 ? kBatchTileI : kBatchTileJK>;
-
 struct Ops {
     static constexpr int kFaceBlocks = 7;   // as the single lattice's face pass
-    static constexpr int kTileSmemFloats =
-        tile_smem_floats<BTile<0>>() > tile_smem_floats<BTile<1>>() ? tile_smem_floats<BTile<0>>() : tile_smem_floats<BTile<1>>();
-    template <int D>
+    template <int D, int TILE>
     static __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *smem)
     {
-        sp::face_tile<BTile<D>, D>(g, at, smem);
+        sp::face_tile<FaceTile<D, TILE, true>, D>(g, at, smem);
     }
     static __device__ __forceinline__ void prep(const LatView &g, int n, int q) { sp::init_node(g, n, q); }
     // the viscous pass on the hi/lo read copy of the stage's state

@@ -14,8 +14,12 @@ namespace cfd {
 
 constexpr int kFaceThreads = 128;
 
-template <int D, int TILE>
+// FLAT: the nodes across are consecutive nodes of the plane across D (axis A
+// fastest) instead of a piece of one line, so that only the extent along D
+// pads a tile: for the batch's small lattices.
+template <int D, int TILE, bool FLAT = false>
 struct FaceTile {
+    static constexpr bool kFlat = FLAT;
     static constexpr int kTile = TILE;                   // faces along D
     static constexpr int kWide = kFaceThreads / TILE;    // nodes across
     static constexpr int A = D == 0 ? 1 : 0;             // axis across
@@ -48,6 +52,9 @@ struct FaceTile {
     }
     static dim3 grid(const LatView &g)
     {
+        if (FLAT)
+            return dim3((unsigned)((lat_extent_h(g, D) + kTile - 1) / kTile),
+                        (unsigned)((g.N / lat_extent_h(g, D) + kWide - 1) / kWide), 1u);
         return dim3((unsigned)((lat_extent_h(g, D) + kTile - 1) / kTile),
                     (unsigned)((lat_extent_h(g, A) + kWide - 1) / kWide), (unsigned)lat_extent_h(g, B));
     }
@@ -67,8 +74,18 @@ __device__ __forceinline__ int tile_coord(const LatView &g, int d, int c)
     return c < 0 ? 0 : (c >= n ? n - 1 : c);
 }
 
-// The tile at face coordinate tD along D, node tA across (axis A), line cB
-// of axis B: the single-lattice passes take it from blockIdx, the batched
+// The node of plane index m (FLAT tiles) at coordinate cD along D.
+template <int D>
+__device__ __forceinline__ int plane_node(const LatView &g, int m, int cD)
+{
+    if (D == 0) return cD + g.ni * m;
+    if (D == 2) return m + g.ni * g.nj * cD;
+    const int k = (int)((unsigned)m / (unsigned)g.ni);
+    return m - g.ni * k + g.ni * (cD + g.nj * k);
+}
+
+// The tile at face coordinate tD along D, node tA across (axis A, or of the
+// plane), line cB of axis B: the single-lattice passes take it from blockIdx, the batched
 // kernel from its item table.
 struct TileAt {
     int tD, tA, cB;
@@ -117,7 +134,7 @@ __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, fl
 {
     constexpr int S = T::kStaged, R = (S + kFaceThreads - 1) / kFaceThreads;
     const int N = g.N;
-    const int nA = lat_extent(g, T::A);
+    const int nA = T::kFlat ? lat_extent(g, T::A) * lat_extent(g, T::B) : lat_extent(g, T::A);
     int e[R];
     NodeIn in[R];
     float q[R][4], r[R][2];   // Q past rho, the Roe inputs past the velocities
@@ -127,11 +144,17 @@ __device__ __forceinline__ void stage_face_lines(const LatView &g, TileAt at, fl
         if (k == R - 1 && m >= S) break;
         int b, a;
         T::staged(m, b, a);
-        int c[3];
-        c[D] = tile_coord(g, D, at.tD + b - 2);
-        c[T::A] = at.tA + a < nA ? at.tA + a : nA - 1;
-        c[T::B] = at.cB;
-        const int node = c[0] + g.ni * (c[1] + g.nj * c[2]);
+        const int cD = tile_coord(g, D, at.tD + b - 2), cA = at.tA + a < nA ? at.tA + a : nA - 1;
+        int node;
+        if (T::kFlat) {
+            node = plane_node<D>(g, cA, cD);
+        } else {
+            int c[3];
+            c[D] = cD;
+            c[T::A] = cA;
+            c[T::B] = at.cB;
+            node = c[0] + g.ni * (c[1] + g.nj * c[2]);
+        }
         e[k] = T::at(b, a);
         in[k] = lat_node_in<D>(g, node);
 #pragma unroll
@@ -166,6 +189,14 @@ __device__ __forceinline__ bool tile_face(const LatView &g, TileAt at, int &n, i
     T::split(threadIdx.x, t, a);
     int c[3];
     c[D] = at.tD + t;
+    if (T::kFlat) {
+        c[T::A] = c[T::B] = 0;
+        if (c[D] >= lat_extent(g, D) || at.tA + a >= lat_extent(g, T::A) * lat_extent(g, T::B)
+            || !lat_face_needed(g, c[0], c[1], c[2], D))
+            return false;
+        n = plane_node<D>(g, at.tA + a, c[D]);
+        return true;
+    }
     c[T::A] = at.tA + a;
     c[T::B] = at.cB;
     if (c[D] >= lat_extent(g, D) || c[T::A] >= lat_extent(g, T::A) || !lat_face_needed(g, c[0], c[1], c[2], D))
