@@ -387,7 +387,9 @@ class StagedInstance:
 
 class _HostBlocks:
     """Host memory of results that their owner has dropped, kept for the next
-    results of the same size, at most ``limit()`` bytes of it.
+    results, in sizes of powers of two, at most ``limit()`` bytes.
+    One pool serves every batch, so that a new batch's first results do not
+    meet new memory either; trim() gives back what a smaller limit leaves over.
 
     The first write to newly mapped memory costs a page fault per page, eight
     times the copy from the device itself (FLOW of 24 instances, 195 MB: 12.9
@@ -397,7 +399,7 @@ class _HostBlocks:
     class _Lease:
         def __init__(self, pool, mem, shape):
             self.pool, self.mem = pool, mem
-            self.__array_interface__ = dict(mem.__array_interface__, shape=shape, strides=None)
+            self.__array_interface__ = dict(mem.__array_interface__, shape=shape, strides=None)   # mem's first values
 
         def __del__(self):
             self.pool._give_back(self.mem)
@@ -407,13 +409,13 @@ class _HostBlocks:
         self._lock = threading.RLock()   # a finaliser may run inside any of these on the same thread
 
     def array(self, rows: int, cols: int) -> np.ndarray:
-        mem = None
+        size, mem = 1 << (rows * cols - 1).bit_length(), None
         with self._lock:
-            same = self._free.get(rows * cols)
-            if same:
-                mem = same.pop()
+            free = self._free.get(size) or self._free.get(2 * size)
+            if free:
+                mem = free.pop()
                 self._held -= mem.nbytes
-        return np.asarray(self._Lease(self, np.empty(rows * cols) if mem is None else mem, (rows, cols)))
+        return np.asarray(self._Lease(self, np.empty(size) if mem is None else mem, (rows, cols)))
 
     def _give_back(self, mem):
         with self._lock:
@@ -421,9 +423,22 @@ class _HostBlocks:
                 self._free.setdefault(mem.size, []).append(mem)
                 self._held += mem.nbytes
 
-    def clear(self):
+    def trim(self):
         with self._lock:
-            self._free, self._held = {}, 0
+            for size in sorted(self._free, reverse=True):
+                while self._free[size] and self._held > self._limit():
+                    self._held -= self._free[size].pop().nbytes
+
+
+_batches = weakref.WeakSet()
+
+
+def _largest_flow() -> int:
+    """Bytes of the FLOW of the largest open batch's instances, each rounded up."""
+    return 2 * max((sum(tuple(b.rows.values())) for b in tuple(_batches)), default=0) * L.NFLOW * 8
+
+
+_results = _HostBlocks(_largest_flow)
 
 
 class Batch:
@@ -436,9 +451,8 @@ class Batch:
         h = C.c_void_p()
         ctx.check(self.lib.cfd_batch_create(ctx.h, int(precision), int(capacity_bytes), C.byref(h)), "cfd_batch_create")
         self.h = h
-        self.rows = rows = {}
-        # results' host memory: kept up to one FLOW of every instance
-        self._blocks = _HostBlocks(lambda: sum(rows.values()) * L.NFLOW * 8)
+        self.rows = {}
+        _batches.add(self)
         ctx._children.add(self)
 
     @staticmethod
@@ -449,8 +463,8 @@ class Batch:
         if self.h and self.ctx.h:
             self.lib.cfd_batch_destroy(self.h)
         self.h = None
-        self.rows.clear()
-        self._blocks.clear()
+        self.rows = {}
+        _results.trim()
 
     def __del__(self):
         try:
@@ -501,7 +515,7 @@ class Batch:
     def remove(self, slot: int):
         self.ctx.check(self.lib.cfd_batch_remove(self.h, int(slot)), "cfd_batch_remove")
         self.rows.pop(slot, None)
-        self._blocks.clear()
+        _results.trim()
 
     def step(self, nsteps: int = 1):
         self.ctx.check(self.lib.cfd_batch_step(self.h, int(nsteps)), "cfd_batch_step")
@@ -519,12 +533,12 @@ class Batch:
         self.ctx.check(self.lib.cfd_batch_set_hold(self.h, int(slot), 1 if hold else 0), "cfd_batch_set_hold")
 
     def get_flow(self, slot: int) -> np.ndarray:
-        out = self._blocks.array(self.rows[slot], L.NFLOW)
+        out = _results.array(self.rows[slot], L.NFLOW)
         self.ctx.check(self.lib.cfd_batch_get_flow(self.h, int(slot), C.c_void_p(_ptr(out))), "cfd_batch_get_flow")
         return out
 
     def get_u0(self, slot: int) -> np.ndarray:
-        out = self._blocks.array(self.rows[slot], L.NCOL)
+        out = _results.array(self.rows[slot], L.NCOL)
         self.ctx.check(self.lib.cfd_batch_get_u0(self.h, int(slot), C.c_void_p(_ptr(out))), "cfd_batch_get_u0")
         return out
 

@@ -24,15 +24,25 @@ def test_a_block_is_reused_only_after_its_last_view():
     del view
     c = p.array(10, 9)
     assert c.ctypes.data == at
-    assert p.array(10, 5).ctypes.data not in (at, b.ctypes.data)
+    assert p.array(10, 9).ctypes.data not in (at, b.ctypes.data)
+    del c
+    d = p.array(8, 13)                          # 104 of the block's 128 values
+    assert d.ctypes.data == at and d.shape == (8, 13)
+    assert p.array(15, 9).ctypes.data != at     # 135 values: a larger block
 
 
 def test_at_most_the_limit_is_kept():
-    p = _pool(2 * 720)
+    from cfd_gb300 import runtime
+    limit = [2 * 1024]
+    p = runtime._HostBlocks(lambda: limit[0])
     arrays = [p.array(10, 9) for _ in range(5)]
     del arrays
-    assert p._held == 2 * 720
-    p.clear()
+    assert p._held == 2 * 1024
+    limit[0] = 1024
+    p.trim()
+    assert p._held == 1024
+    limit[0] = 0
+    p.trim()
     assert p._held == 0 and p.array(10, 9).shape == (10, 9)
 
 
