@@ -1,6 +1,6 @@
-// batch.cu -- many independent lattices advanced together: one persistent,
-// cooperative launch per RK stage over a tile table of all instances
-// (batch_kernel.cuh), one RK step captured as a CUDA graph, and a tuner that
+// batch.cu -- many independent lattices advanced together: a few launches per
+// RK stage, the last one cooperative, over tables of all instances' tiles
+// (batch_kernel.cuh, batch_fp64.cu), one RK step captured as a CUDA graph, and a tuner that
 // times tile sizes on the live batch (state saved and restored around the
 // trials).  Instances are admitted against a device-memory budget, keep
 // their state resident, and can be added and removed between steps; this is

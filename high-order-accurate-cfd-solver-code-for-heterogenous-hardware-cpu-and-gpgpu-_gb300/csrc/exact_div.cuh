@@ -39,8 +39,7 @@
 // top 53 bits of the integer product of the significands of x and y (no
 // FP64 instruction; the faster choice in kernels with warps to hide its
 // integer latency, 3 or more blocks of 128 per SM), 0 the FP64 product
-// RN(x*y) (kernels at 2 blocks per SM: the drop-in's face kernel, the
-// batched stage, the FP64 face passes at that budget).  A translation unit
+// RN(x*y) (faster at 2 blocks per SM, which no kernel runs at now).  A translation unit
 // sets it before its first include; the two variants live in different
 // inline namespaces, so the host functions of units built with different
 // choices do not collide at link time.  Both give the same bits.

@@ -9,9 +9,9 @@
 // Stage intermediates are FP32 (half the bytes of the FP64 form).
 //
 // Kernels per stage: k_visc_m (radius-2 star), k_face_tile_m<d> x3 (one
-// thread per face, stencil lines staged in shared memory), k_update_m (RK
-// stage + the next stage's U_Q); k_init_m /
-// k_prep_m supply U_Q when no update produced it.  The per-node operations
+// thread per face, stencil lines staged in shared memory), or k_fluxes_m (all
+// four in one launch on small lattices), and k_update_m (RK stage + the next
+// stage's U_Q); k_init_m / k_prep_m supply U_Q when no update produced it.  The per-node operations
 // are in lattice_mixed.cuh.  This file is compiled with FMA contraction on
 // and approximate FP32 division/square root (the mixed form's error budget
 // is 1e-6 relative L2 against the FP64 form).

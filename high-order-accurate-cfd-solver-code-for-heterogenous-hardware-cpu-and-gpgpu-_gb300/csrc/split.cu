@@ -8,7 +8,7 @@
 // star on the hi/lo read copy of the state, FP32, on a side stream),
 // k_face_tile_s<d> x3 (one thread per face, the FP32
 // stencil lines staged in shared memory, the FP64 face flux written to Fh),
-// k_update_s (FP64 flux difference and RK stage + the next stage's U_Q);
+// or k_fluxes_s (all four in one launch on small lattices), and k_update_s (FP64 flux difference and RK stage + the next stage's U_Q);
 // k_init_s / k_prep_s supply U_Q when no update produced it.  Compiled with
 // FMA contraction and approximate FP32 division/square root.
 #include "boundary.h"

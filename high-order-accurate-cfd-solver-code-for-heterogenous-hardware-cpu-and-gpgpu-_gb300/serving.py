@@ -2,8 +2,8 @@
 
 Requests (an initial-value problem on a periodic lattice plus a number of
 SSP-RK3 steps) arrive over time.  The loop keeps every admitted solve's
-state resident in one batch (``runtime.Batch``: one persistent launch per RK
-stage over all instances) and, between steps:
+state resident in one batch (``runtime.Batch``: a few launches per RK stage
+over all instances) and, between steps:
 
 * admits queued requests in arrival order while their device-memory
   footprint fits the batch budget (``cfd_batch_instance_bytes``);

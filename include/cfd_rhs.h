@@ -367,7 +367,7 @@ cfd_status_t cfd_solver_profile_stage(cfd_solver_t *s, int32_t j, double del_t, 
 
 /* ------------------------------------------------ batched lattices ---- */
 /* Many independent periodic lattices of different sizes advanced together:
- * one persistent cooperative kernel launch per RK stage covers every
+ * a few kernel launches per RK stage, the last one cooperative, cover every
  * instance through a tile table, and one RK step is captured as a CUDA
  * graph.  Instances are admitted against a device-memory budget, stay
  * resident, and may be added or removed between steps (the serving loop's
