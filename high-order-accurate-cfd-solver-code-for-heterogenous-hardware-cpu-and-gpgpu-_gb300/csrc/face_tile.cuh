@@ -16,7 +16,7 @@ constexpr int kFaceThreads = 128;
 
 // FLAT: the nodes across are consecutive nodes of the plane across D (axis A
 // fastest) instead of a piece of one line, so that only the extent along D
-// pads a tile: for the batch's small lattices.
+// pads a tile: for small lattices.
 template <int D, int TILE, bool FLAT = false>
 struct FaceTile {
     static constexpr bool kFlat = FLAT;
@@ -244,9 +244,11 @@ struct FluxGrid {
     unsigned nv, b[2];   // viscous ranges; end of the i tiles, of the j tiles
     uint3 gr[3];
 };
-using FluxTileI = FaceTile<0, 32>;
-using FluxTileJ = FaceTile<1, 16>;
-using FluxTileK = FaceTile<2, 16>;
+// Small and odd extents: FLAT tiles of 16 and 8 (split 33^3 24.9 us a stage,
+// 37 x 41 x 19 inviscid 20.7; 27.0 and 22.5 with lines of 32 and 16).
+using FluxTileI = FaceTile<0, 16, true>;
+using FluxTileJ = FaceTile<1, 8, true>;
+using FluxTileK = FaceTile<2, 8, true>;
 
 inline unsigned flux_grid(const LatView &g, FluxGrid &f)
 {
@@ -284,9 +286,9 @@ constexpr int flux_smem_floats()
 
 // Nodes up to which a reduced form's fluxes run in one launch instead of as
 // four kernels on four streams (split form, a stage; four streams against one
-// launch): 17^3 nodes 23.2 and 18.8 us, 24^3 23.0 and 20.8, 33^3 29.2 and
-// 27.5, 46^3 40.6 and 40.3, 64^3 82.6 and 81.3 (mixed 58.6 and 57.4), 256 x
-// 64 x 16 with ghost layers 106 and 113, where each kernel's own registers
+// launch): 17^3 nodes 23.2 and 17.1 us, 24^3 23.0 and 20.7, 33^3 29.2 and
+// 24.9, 46^3 40.6 and 38.0; 64^3 82.6 and 81.3 (with tiles of 32 and 16), 256
+// x 64 x 16 with ghost layers 106 and 113, where each kernel's own registers
 // and the tuned tiles tell.
 #ifndef CFD_ONE_LAUNCH_NODES
 #define CFD_ONE_LAUNCH_NODES 200000

@@ -72,10 +72,10 @@ __global__ void __launch_bounds__(256) k_mu_m(LatView g, int q)
 
 // Faces per tile along D (a block of 128 threads covers kTile x 128/kTile
 // faces; face_tile.cuh), StructuredLaunch::tile_i / tile_jk.  TGV 128^3: i
-// tiles of 16 / 32 / 64 / 128 took 0.097 / 0.093 / 0.091 / 0.090 ms, j/k
-// tiles of 4 / 8 / 16 / 32 took 0.098 / 0.094 / 0.092 / 0.102-0.146 ms; the
-// defaults 64 and 16 keep small lattices' i lines from idling most of a
-// block, and the solver's tuner picks per lattice.
+// tiles of 32 / 64 / 128 take 0.070 / 0.069 / 0.069 ms, j and k tiles of 8 /
+// 16 / 32 0.072 / 0.070-0.073 / 0.083-0.119 ms; the defaults 64 and 16 keep
+// small lattices' i lines from idling most of a block, and the solver's tuner
+// picks per lattice.
 
 // One instance per candidate tile width (face_tile.cuh): faces along i of
 // 32, 64 or 128, along j or k of 8, 16 or 32; the solver times them when it
