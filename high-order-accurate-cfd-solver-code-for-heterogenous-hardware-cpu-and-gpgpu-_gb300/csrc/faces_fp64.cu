@@ -38,17 +38,23 @@ __global__ void __launch_bounds__(128, 6) k_face_base(LatView g, FaceScratch fs,
     if (n < n1) ex::base_node(g, fs, n, blockIdx.y);
 }
 
-// MB: twice the blocks of 128 per SM its registers allow (StructuredLaunch::
-// face_mb): 128, 80 or 64 registers.  TGV 128^3 6.5, 6.3, 6.2 ms; vortex
-// 64^3 1.17, 1.10, 1.09 ms; 53,000 ghosted nodes 0.195, 0.184, 0.182 ms.
+// MB: the blocks of 256 per SM its registers allow (StructuredLaunch::
+// face_mb): 128, 80 or 64 registers.  TGV 128^3 6.5, 6.3, 6.2 ms with blocks
+// of 128; vortex 64^3 1.17, 1.10, 1.09 ms; 53,000 ghosted nodes 0.195, 0.184,
+// 0.182 ms.  Instruction fetch is what costs it most after the FP64 pipe:
+// blocks of 256 instead of 128 at 64 registers 6.18 -> 5.90 ms, with a barrier
+// between the phases 5.78 (vortex 1.00 -> 0.91, 53,000 nodes 0.180 -> 0.170;
+// blocks of 512 6.10, of 128 with barriers 6.07).
+constexpr int kCharThreads = 256;
 template <int MB>
-__global__ void __launch_bounds__(128, 2 * MB) k_face_char(LatView g, FaceScratch fs, int n1, int d0)
+__global__ void __launch_bounds__(kCharThreads, MB) k_face_char(LatView g, FaceScratch fs, int n1, int d0)
 {
     const int n = fs.n0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x;
-    if (n < n1) ex::char_node(g, fs, n, d0 + blockIdx.y, blockIdx.x % 5u);
+    if (n < n1) ex::char_node(g, fs, n, d0 + blockIdx.y, blockIdx.x % 5u, ex::BlockSync{});
 }
 
-__global__ void __launch_bounds__(128, 6) k_face_back(LatView g, FaceScratch fs, int n1)
+// blocks of 256: TGV 128^3 2.00 -> 1.97 ms, vortex 64^3 0.338 -> 0.330 (128); 2.04 with 384
+__global__ void __launch_bounds__(256, 3) k_face_back(LatView g, FaceScratch fs, int n1)
 {
     const int n = fs.n0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x;
     if (n < n1) ex::back_node(g, fs, n, blockIdx.y, blockIdx.x % 5u);
@@ -62,10 +68,10 @@ __global__ void __launch_bounds__(128, 4) k_face_flux(LatView g, FaceScratch fs,
 
 void face_char(const LatView &g, const FaceScratch &fs, int n1, int mb, int d0, int nd, cudaStream_t st)
 {
-    const dim3 grid(5 * blocks_for(n1 - fs.n0, 128), nd);   // the five fields of 128 faces are neighbouring blocks
-    if (mb == 2) k_face_char<2><<<grid, 128, 0, st>>>(g, fs, n1, d0);
-    else if (mb == 3) k_face_char<3><<<grid, 128, 0, st>>>(g, fs, n1, d0);
-    else k_face_char<4><<<grid, 128, 0, st>>>(g, fs, n1, d0);
+    const dim3 grid(5 * blocks_for(n1 - fs.n0, kCharThreads), nd);   // the five fields of 128 faces are neighbouring blocks
+    if (mb == 2) k_face_char<2><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);
+    else if (mb == 3) k_face_char<3><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);
+    else k_face_char<4><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);
 }
 
 }  // namespace
@@ -100,7 +106,7 @@ int fp64_faces(const StructuredLaunch &S, const LatView &g, cudaStream_t st, con
             launches += 6;
         }
         if (one) mark("face_char");
-        k_face_back<<<dim3(5 * nb, 3), 128, 0, st>>>(g, fs, n1);
+        k_face_back<<<dim3(5 * blocks_for(n1 - n0, 256), 3), 256, 0, st>>>(g, fs, n1);
         if (one) mark("face_back");
         k_face_flux<<<dim3(blocks_for(2LL * (n1 - n0), 128), 3), 128, 0, st>>>(g, fs, n1);
         if (one) mark("face_flux");

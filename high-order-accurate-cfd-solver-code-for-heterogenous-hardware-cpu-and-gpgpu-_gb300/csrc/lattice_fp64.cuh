@@ -209,7 +209,9 @@ __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &f
     for (int s = 0; s < FB_N; ++s) col[(size_t)(FS_BASE + s) * fs.ld] = B[s];
 }
 
-__device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q)
+template <class Sync = NoSync>
+__device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q,
+                                          const Sync &sync = Sync())
 {
     const int N = g.N;
     int i, j, k;
@@ -223,7 +225,7 @@ __device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &f
     int s[6];
 #pragma unroll
     for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, d, o - 2);
-    char_pair(L, [&](int o, int c) { return g.Q[c * N + s[o]]; }, g.P.eps, pos, neg);
+    char_pair(L, [&](int o, int c) { return g.Q[c * N + s[o]]; }, g.P.eps, pos, neg, sync);
     col[(FS_POS + q) * ld] = pos;
     col[(FS_NEG + q) * ld] = neg;
 }

@@ -388,7 +388,19 @@ __device__ __forceinline__ WenoConst weno_const(double cm2, double cm1, double c
 #define CFD_US 1
 #endif
 // weno_pair with its products on the integer pipe.
-__device__ __forceinline__ void weno_pair_i(const double c[6], double eps, double &pos, double &neg)
+// Called between the phases of one field's reconstruction: BlockSync keeps
+// the warps of a block within a phase, so that they fetch the same few KB of
+// its 59 KB of code (threads without a face have exited; the others meet
+// every barrier).
+struct NoSync {
+    __device__ __forceinline__ void operator()() const {}
+};
+struct BlockSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <class Sync = NoSync>
+__device__ __forceinline__ void weno_pair_i(const double c[6], double eps, double &pos, double &neg,
+                                            const Sync &sync = Sync())
 {
     using xdiv::scale2;
     const double cm2 = c[0], cm1 = c[1], c0 = c[2], c1 = c[3], c2 = c[4], c3 = c[5];
@@ -416,8 +428,10 @@ __device__ __forceinline__ void weno_pair_i(const double c[6], double eps, doubl
     S[4] = eps + (T[2] + scale2<-2>(S[4]));
     S[5] = eps + (T[3] + scale2<-2>(S[5]));
     xi::sq_n(S);
+    sync();
     double w[6] = {1.0 / 16.0, 5.0 / 8.0, 5.0 / 16.0, 5.0 / 16.0, 5.0 / 8.0, 1.0 / 16.0};
     xi::div_n(w, S);
+    sync();
     double a[3] = {w[5], w[4], w[3]}, b[3] = {w[2], w[1], w[0]};
     Over<true>(a[0] + a[1] + a[2]).all(a);
     Over<true>(b[0] + b[1] + b[2]).all(b);
@@ -433,9 +447,11 @@ __device__ __forceinline__ void weno_pair_i(const double c[6], double eps, doubl
 // One characteristic field of a face: row L of the left eigenvectors times
 // the six stencil points (point(o, c): component c of point o, left-2 ..
 // right+2), and the WENO5 pair.
-template <class Point>
-__device__ __forceinline__ void char_pair(const double L[5], const Point &point, double eps, double &pos, double &neg)
+template <class Point, class Sync = NoSync>
+__device__ __forceinline__ void char_pair(const double L[5], const Point &point, double eps, double &pos, double &neg,
+                                          const Sync &sync = Sync())
 {
+    sync();
     double cv[6];
     xi::Fac f[5];
 #pragma unroll
@@ -449,7 +465,8 @@ __device__ __forceinline__ void char_pair(const double L[5], const Point &point,
         xi::mul_n(f, p, r);
         cv[o] = r[0] + r[1] + r[2] + r[3] + r[4];
     }
-    weno_pair_i(cv, eps, pos, neg);
+    sync();
+    weno_pair_i(cv, eps, pos, neg, sync);
 }
 
 // One side's contravariant flux x det_f (Weno.cl:2291-2507, 2585-2728) and
