@@ -401,7 +401,9 @@ __global__ void __launch_bounds__(128, 6) k_row_base(const int *__restrict__ gri
     for (int c = 0; c < 3; ++c) col[(RF_KN + c) * ld] = kn[c];
 }
 
-__global__ void __launch_bounds__(128, 8) k_row_char(const double *__restrict__ Q, double eps, RowRound R)
+// blocks of 256 whose warps keep to one phase (faces_fp64.cu k_face_char): Weno
+// on 96^3 rows 4.77 -> 4.70 ms
+__global__ void __launch_bounds__(256, 4) k_row_char(const double *__restrict__ Q, double eps, RowRound R)
 {
     const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;
     if (gid >= R.r1) return;
@@ -412,12 +414,13 @@ __global__ void __launch_bounds__(128, 8) k_row_char(const double *__restrict__ 
     if (st[0] < 0) return;
     double L[5], pos, neg;
     ex::left_row(q, [&](int s) { return col[(RF_BASE + s) * ld]; }, [&](int c) { return col[(RF_KN + c) * ld]; }, L);
-    ex::char_pair(L, [&](int o, int c) { return Q[5 * (size_t)st[o] + c]; }, eps, pos, neg);
+    ex::char_pair(L, [&](int o, int c) { return Q[5 * (size_t)st[o] + c]; }, eps, pos, neg,
+                  ex::BlockSync{});
     col[(RF_POS + q) * ld] = pos;
     col[(RF_NEG + q) * ld] = neg;
 }
 
-__global__ void __launch_bounds__(128, 6) k_row_back(const double *__restrict__ F, const double *__restrict__ E,
+__global__ void __launch_bounds__(256, 3) k_row_back(const double *__restrict__ F, const double *__restrict__ E,
                                                      const double *__restrict__ G, RowRound R)
 {
     const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;
@@ -704,10 +707,10 @@ void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, 
         const int round = (int)row_round(ld);
         for (int r0 = 0; r0 < n_items; r0 += round) {
             const RowRound R{face_scratch + 30 * ld, r0, std::min(n_items, r0 + round), round};
-            const unsigned n = blocks_for(R.r1 - r0, 128);
+            const unsigned n = blocks_for(R.r1 - r0, 128), n2 = blocks_for(R.r1 - r0, 256);
             k_row_base<<<dim3(n, 3), 128, 0, st>>>(grid, metric, roe, n_rows, R);
-            k_row_char<<<dim3(5 * n, 3), 128, 0, st>>>(Q, P.eps, R);
-            k_row_back<<<dim3(5 * n, 3), 128, 0, st>>>(F, E, G, R);
+            k_row_char<<<dim3(5 * n2, 3), 256, 0, st>>>(Q, P.eps, R);
+            k_row_back<<<dim3(5 * n2, 3), 256, 0, st>>>(F, E, G, R);
             k_row_flux<<<dim3(blocks_for(2LL * (R.r1 - r0), 128), 3), 128, 0, st>>>(
                 deter, grid, metric, roe, n_items, n_rows, Fp, Fm, stamp, gen, ld, R);
         }

@@ -15,8 +15,8 @@
 // SM).  The hand-over between the kernels (kFaceScratch doubles per face)
 // costs 0.7 KB per face of L2 and HBM traffic, which the FP64-bound kernels
 // hide.  TGV 128^3, all three directions: 16.1 ms with one kernel per
-// direction and only the divisions on the integer pipe; 10.2 ms here
-// (base 0.30, char 6.20, back 2.01, flux 1.70; the FP64 pipe is busy 65 to
+// direction and only the divisions on the integer pipe; 9.8 ms here
+// (base 0.30, char 5.78, back 1.97, flux 1.70; the FP64 pipe is busy 65 to
 // 80 % of the time, with branch-free groups and an instruction footprint
 // that stays near the instruction cache's size as the remaining limits).
 #include "internal.h"
