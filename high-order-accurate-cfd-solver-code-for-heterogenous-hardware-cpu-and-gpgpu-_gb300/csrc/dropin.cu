@@ -229,8 +229,12 @@ __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, do
 // callers without the scratch.  TGV 96^3, both kernels: 1.00 ms at 3 or 4
 // blocks per SM, 1.19 at 5; in one kernel 1.17 at 3, 1.38 at 4 (3 KB of spill
 // loads per thread).
+// The integer form in blocks of 256, which share its long code better: 0.73
+// -> 0.69 ms for both kernels.
+template <bool I>
+constexpr int kViscousThreads = I ? 256 : 128;
 template <bool NODE, bool I>
-__global__ void __launch_bounds__(128, 4) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
+__global__ void __launch_bounds__(kViscousThreads<I>, 512 / kViscousThreads<I>) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
                                                  double *__restrict__ E, double *__restrict__ G,
                                                  double *__restrict__ Fv, double *__restrict__ Ev,
                                                  double *__restrict__ Gv, const int *__restrict__ grid,
@@ -670,7 +674,8 @@ int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, d
     if (scratch && scratch_rows >= n_items) {
         const bool fp = n_items <= kPlainNodes;
         (fp ? k_node_flux<false> : k_node_flux<true>)<<<nb, 128, 0, st>>>(F, E, G, metric, det, flow, n_items, P.les, scratch);
-        (fp ? k_viscous<false, false> : k_viscous<false, true>)<<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
+        const int T = fp ? kViscousThreads<false> : kViscousThreads<true>;
+        (fp ? k_viscous<false, false> : k_viscous<false, true>)<<<blocks_for(n_items, T), T, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
                                              scratch);
         return 2;
     }

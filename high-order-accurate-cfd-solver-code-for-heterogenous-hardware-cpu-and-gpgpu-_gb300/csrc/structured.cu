@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(128, 6) k_prep(LatView g, int q)
 }
 
 // Blocks of 256 share the integer form's long code better (128^3 1.45 -> 1.33
-// ms); the plain form's lattices are too small to fill the SMs with them
+// ms; 1.44 with barriers between its loops' passes); the plain form's lattices are too small to fill the SMs with them
 // (53,000 nodes 0.059 -> 0.073).
 template <bool I>
 constexpr int kViscThreads = I ? 256 : 128;
