@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(256, 4) k_batch_char(const LatView *__restrict
 {
     const int w = blockIdx.x / 5u;
     const BatchTile t = tiles[t0 + w];
-    if ((int)threadIdx.x < t.count)
-        ex::char_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u, ex::BlockSync{});
+    ex::char_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u,
+                  (int)threadIdx.x < t.count, ex::BlockSync{});
 }
 
 __global__ void __launch_bounds__(256, 3) k_batch_back(const LatView *__restrict__ views,

@@ -410,16 +410,19 @@ __global__ void __launch_bounds__(128, 6) k_row_base(const int *__restrict__ gri
 __global__ void __launch_bounds__(256, 4) k_row_char(const double *__restrict__ Q, double eps, RowRound R)
 {
     const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;
-    if (gid >= R.r1) return;
     double *col = row_column(R, gid, d);
     const size_t ld = R.ld;
-    int st[6];
-    stencil_rows(col, ld, st);
-    if (st[0] < 0) return;
-    double L[5], pos, neg;
-    ex::left_row(q, [&](int s) { return col[(RF_BASE + s) * ld]; }, [&](int c) { return col[(RF_KN + c) * ld]; }, L);
-    ex::char_pair(L, [&](int o, int c) { return Q[5 * (size_t)st[o] + c]; }, eps, pos, neg,
-                  ex::BlockSync{});
+    int st[6] = {-1, -1, -1, -1, -1, -1};
+    if (gid < R.r1) stencil_rows(col, ld, st);
+    const bool face = st[0] >= 0;   // the other threads only meet the barriers
+    double pos, neg;
+    ex::char_pair(
+        face,
+        [&](double (&L)[5]) {
+            ex::left_row(q, [&](int s) { return col[(RF_BASE + s) * ld]; }, [&](int c) { return col[(RF_KN + c) * ld]; }, L);
+        },
+        [&](int o, int c) { return Q[5 * (size_t)st[o] + c]; }, eps, pos, neg, ex::BlockSync{});
+    if (!face) return;
     col[(RF_POS + q) * ld] = pos;
     col[(RF_NEG + q) * ld] = neg;
 }

@@ -50,7 +50,7 @@ template <int MB>
 __global__ void __launch_bounds__(kCharThreads, MB) k_face_char(LatView g, FaceScratch fs, int n1, int d0)
 {
     const int n = fs.n0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x;
-    if (n < n1) ex::char_node(g, fs, n, d0 + blockIdx.y, blockIdx.x % 5u, ex::BlockSync{});
+    ex::char_node(g, fs, n, d0 + blockIdx.y, blockIdx.x % 5u, n < n1, ex::BlockSync{});
 }
 
 // blocks of 256: TGV 128^3 2.00 -> 1.97 ms, vortex 64^3 0.338 -> 0.330 (128); 2.04 with 384

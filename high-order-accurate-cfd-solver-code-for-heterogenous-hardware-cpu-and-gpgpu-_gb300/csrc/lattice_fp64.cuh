@@ -209,23 +209,29 @@ __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &f
     for (int s = 0; s < FB_N; ++s) col[(size_t)(FS_BASE + s) * fs.ld] = B[s];
 }
 
+// Every thread of the block calls it when Sync is the block's barrier; those
+// past the range of nodes with active = false.
 template <class Sync = NoSync>
-__device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q,
+__device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q, bool active,
                                           const Sync &sync = Sync())
 {
     const int N = g.N;
     int i, j, k;
-    if (!face_at(g, n, d, i, j, k)) return;
+    const bool face = active && face_at(g, n, d, i, j, k);
     double *col = face_column(fs, n, d);
     const double *kn = g.kn + (size_t)d * 3 * N + n;
     const size_t ld = fs.ld;
-    double L[5];
-    left_row(q, [&](int s) { return col[(FS_BASE + s) * ld]; }, [&](int c) { return kn[(size_t)c * N]; }, L);
-    double pos, neg;
     int s[6];
+    double pos, neg;
+    char_pair(
+        face,
+        [&](double (&L)[5]) {
+            left_row(q, [&](int e) { return col[(FS_BASE + e) * ld]; }, [&](int c) { return kn[(size_t)c * N]; }, L);
 #pragma unroll
-    for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, d, o - 2);
-    char_pair(L, [&](int o, int c) { return g.Q[c * N + s[o]]; }, g.P.eps, pos, neg, sync);
+            for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, d, o - 2);
+        },
+        [&](int o, int c) { return g.Q[c * N + s[o]]; }, g.P.eps, pos, neg, sync);
+    if (!face) return;
     col[(FS_POS + q) * ld] = pos;
     col[(FS_NEG + q) * ld] = neg;
 }

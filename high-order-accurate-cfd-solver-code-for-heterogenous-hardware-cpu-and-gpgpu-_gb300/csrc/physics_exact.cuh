@@ -381,58 +381,68 @@ __device__ __forceinline__ WenoConst weno_const(double cm2, double cm1, double c
     return w;
 }
 
-#ifndef CFD_UP
-#define CFD_UP 6
-#endif
-#ifndef CFD_US
-#define CFD_US 1
-#endif
-// weno_pair with its products on the integer pipe.
-// Called between the phases of one field's reconstruction: BlockSync keeps
+// Called between the phases of one field's reconstruction.  BlockSync keeps
 // the warps of a block within a phase, so that they fetch the same few KB of
-// its 59 KB of code (threads without a face have exited; the others meet
-// every barrier).
+// its 59 KB of code.  It is a barrier of the whole block: every thread meets
+// every one of them, those without a face (`face` false: past the range, or
+// a node whose face is not needed) included; only what lies between is theirs
+// to skip.
 struct NoSync {
     __device__ __forceinline__ void operator()() const {}
 };
 struct BlockSync {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
+
+// weno_pair with its products on the integer pipe, from the six projected
+// points c, two barriers between its three phases.
 template <class Sync = NoSync>
-__device__ __forceinline__ void weno_pair_i(const double c[6], double eps, double &pos, double &neg,
+__device__ __forceinline__ void weno_pair_i(bool face, const double c[6], double eps, double &pos, double &neg,
                                             const Sync &sync = Sync())
 {
     using xdiv::scale2;
-    const double cm2 = c[0], cm1 = c[1], c0 = c[2], c1 = c[3], c2 = c[4], c3 = c[5];
-    const WenoConst kc = weno_const(cm2, cm1, c0, c1, c2, c3);
-    const double p0 = kc.f1 - kc.v2 + kc.h3;
-    const double p1 = kc.h0 + kc.q1 - scale2<-3>(c2);
-    const double p2 = -scale2<-3>(cm1) + kc.q0 + kc.h1;
-    const double m2 = kc.hm2 - kc.vm1 + kc.f0;
-    const double b0 = kc.b0, b1 = kc.b1;   // 3 c0, 3 c1
-    double T[4] = {cm2 - scale2<1>(cm1) + c0, cm1 - scale2<1>(c0) + c1, c0 - scale2<1>(c1) + c2,
-                   c1 - scale2<1>(c2) + c3};
-    xi::sq_n(T);
-    {
-        const xi::Fac k = xi::fac(13.0 / 12.0);
-        const xi::Fac a[4] = {k, k, k, k}, b[4] = {xi::fac(T[0]), xi::fac(T[1]), xi::fac(T[2]), xi::fac(T[3])};
-        xi::mul_n(a, b, T);
+    double p0, p1, p2, m2, S[6];
+    if (face) {   // the candidates and the weights' denominators
+        const double cm2 = c[0], cm1 = c[1], c0 = c[2], c1 = c[3], c2 = c[4], c3 = c[5];
+        const WenoConst kc = weno_const(cm2, cm1, c0, c1, c2, c3);
+        p0 = kc.f1 - kc.v2 + kc.h3;
+        p1 = kc.h0 + kc.q1 - scale2<-3>(c2);
+        p2 = -scale2<-3>(cm1) + kc.q0 + kc.h1;
+        m2 = kc.hm2 - kc.vm1 + kc.f0;
+        const double b0 = kc.b0, b1 = kc.b1;   // 3 c0, 3 c1
+        double T[4] = {cm2 - scale2<1>(cm1) + c0, cm1 - scale2<1>(c0) + c1, c0 - scale2<1>(c1) + c2,
+                       c1 - scale2<1>(c2) + c3};
+        xi::sq_n(T);
+        {
+            const xi::Fac k = xi::fac(13.0 / 12.0);
+            const xi::Fac a[4] = {k, k, k, k}, b[4] = {xi::fac(T[0]), xi::fac(T[1]), xi::fac(T[2]), xi::fac(T[3])};
+            xi::mul_n(a, b, T);
+        }
+        S[0] = cm2 - scale2<2>(cm1) + b0;
+        S[1] = cm1 - c1;
+        S[2] = b0 - scale2<2>(c1) + c2;
+        S[3] = cm1 - scale2<2>(c0) + b1;
+        S[4] = c0 - c2;
+        S[5] = b1 - scale2<2>(c2) + c3;
+        xi::sq_n(S);
+        S[0] = eps + (T[0] + scale2<-2>(S[0]));
+        S[1] = eps + (T[1] + scale2<-2>(S[1]));
+        S[2] = eps + (T[2] + scale2<-2>(S[2]));
+        S[3] = eps + (T[1] + scale2<-2>(S[3]));
+        S[4] = eps + (T[2] + scale2<-2>(S[4]));
+        S[5] = eps + (T[3] + scale2<-2>(S[5]));
+        xi::sq_n(S);
     }
-    double S[6] = {cm2 - scale2<2>(cm1) + b0, cm1 - c1, b0 - scale2<2>(c1) + c2,
-                   cm1 - scale2<2>(c0) + b1, c0 - c2, b1 - scale2<2>(c2) + c3};
-    xi::sq_n(S);
-    S[0] = eps + (T[0] + scale2<-2>(S[0]));
-    S[1] = eps + (T[1] + scale2<-2>(S[1]));
-    S[2] = eps + (T[2] + scale2<-2>(S[2]));
-    S[3] = eps + (T[1] + scale2<-2>(S[3]));
-    S[4] = eps + (T[2] + scale2<-2>(S[4]));
-    S[5] = eps + (T[3] + scale2<-2>(S[5]));
-    xi::sq_n(S);
     sync();
-    double w[6] = {1.0 / 16.0, 5.0 / 8.0, 5.0 / 16.0, 5.0 / 16.0, 5.0 / 8.0, 1.0 / 16.0};
-    xi::div_n(w, S);
+    if (face) {   // the weights, in place of their denominators
+        double w[6] = {1.0 / 16.0, 5.0 / 8.0, 5.0 / 16.0, 5.0 / 16.0, 5.0 / 8.0, 1.0 / 16.0};
+        xi::div_n(w, S);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) S[k] = w[k];
+    }
     sync();
-    double a[3] = {w[5], w[4], w[3]}, b[3] = {w[2], w[1], w[0]};
+    if (!face) return;   // no barrier follows
+    double a[3] = {S[5], S[4], S[3]}, b[3] = {S[2], S[1], S[0]};
     Over<true>(a[0] + a[1] + a[2]).all(a);
     Over<true>(b[0] + b[1] + b[2]).all(b);
     const xi::Fac f[6] = {xi::fac(a[0]), xi::fac(a[1]), xi::fac(a[2]), xi::fac(b[0]), xi::fac(b[1]), xi::fac(b[2])};
@@ -444,29 +454,37 @@ __device__ __forceinline__ void weno_pair_i(const double c[6], double eps, doubl
     neg = r[3] + r[4] + r[5];
 }
 
-// One characteristic field of a face: row L of the left eigenvectors times
-// the six stencil points (point(o, c): component c of point o, left-2 ..
-// right+2), and the WENO5 pair.
-template <class Point, class Sync = NoSync>
-__device__ __forceinline__ void char_pair(const double L[5], const Point &point, double eps, double &pos, double &neg,
-                                          const Sync &sync = Sync())
+// One characteristic field of a face: row L of the left eigenvectors (left(L)
+// forms it) times the six stencil points (point(o, c): component c of point
+// o, left-2 .. right+2), and the WENO5 pair.  With a BlockSync every thread
+// of the block calls it, face or not; without a face neither left nor point
+// is called and pos and neg are not set.
+template <class Left, class Point, class Sync = NoSync>
+__device__ __forceinline__ void char_pair(bool face, const Left &left, const Point &point, double eps, double &pos,
+                                          double &neg, const Sync &sync = Sync())
 {
-    sync();
-    double cv[6];
     xi::Fac f[5];
+    if (face) {
+        double L[5];
+        left(L);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) f[c] = xi::fac(L[c]);
-#pragma unroll
-    for (int o = 0; o < 6; ++o) {
-        xi::Fac p[5];
-        double r[5];
-#pragma unroll
-        for (int c = 0; c < 5; ++c) p[c] = xi::fac(point(o, c));
-        xi::mul_n(f, p, r);
-        cv[o] = r[0] + r[1] + r[2] + r[3] + r[4];
+        for (int c = 0; c < 5; ++c) f[c] = xi::fac(L[c]);
     }
     sync();
-    weno_pair_i(cv, eps, pos, neg, sync);
+    double cv[6];
+    if (face) {
+#pragma unroll
+        for (int o = 0; o < 6; ++o) {
+            xi::Fac p[5];
+            double r[5];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) p[c] = xi::fac(point(o, c));
+            xi::mul_n(f, p, r);
+            cv[o] = r[0] + r[1] + r[2] + r[3] + r[4];
+        }
+    }
+    sync();
+    weno_pair_i(face, cv, eps, pos, neg, sync);
 }
 
 // One side's contravariant flux x det_f (Weno.cl:2291-2507, 2585-2728) and
