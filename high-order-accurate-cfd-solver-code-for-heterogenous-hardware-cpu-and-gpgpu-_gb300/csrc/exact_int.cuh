@@ -83,6 +83,15 @@ CFD_XI_HD uint32_t funnel_l(uint32_t lo, uint32_t hi, uint32_t s)
 #endif
 }
 
+// The host's seeds of the reciprocal and the reciprocal root; a check may put
+// worse ones in their place, as far off as the device's may be.
+#ifndef CFD_XI_HOST_RCP
+#define CFD_XI_HOST_RCP(m) (1.0f / (m))
+#endif
+#ifndef CFD_XI_HOST_RSQRT
+#define CFD_XI_HOST_RSQRT(m) ((float)(1.0 / std::sqrt((double)(m))))
+#endif
+
 constexpr uint32_t kMark = 0x60000000u;
 
 // Nonzero for the high word of an operand outside [2^-255, 2^257) (biased
@@ -240,9 +249,10 @@ CFD_XI_HD double small_or(uint32_t mark, uint32_t hi, uint32_t lo, double x, dou
 // A divisor b = +-B 2^(e - 1075) (B its 53-bit significand, beta = B / 2^52
 // in [1, 2)) with Y, an approximation of 2^64 / beta that Y <= 2^64 / beta
 // < Y + 4 (for beta = 1: Y = 2^64 - 1).  A float reciprocal of B's top 24
-// bits, at most 1 - 2^-24, seeds it: r = S 2^-24 with eps = 1 - beta r
-// = E / 2^76 exactly, E = 2^76 - S B, and |eps| < 2^-21.4 (the seed within
-// 2^-23, the dropped bits of B within 2^-23), so |E| < 2^54.6 and its low
+// bits, clamped to [1/2, 1 - 2^-24], seeds it: r = S 2^-24 with eps = 1 -
+// beta r = E / 2^76 exactly, E = 2^76 - S B, and |eps| < 2^-21.4 (the seed
+// within 2^-23, which for a divisor just below 2 may be under 1/2; the dropped
+// bits of B within 2^-23), so |E| < 2^54.6 and its low
 // 64 bits are E.  Then 2^64 / beta = S 2^40 (1 + eps + eps^2 + ...) and
 //   Y = S 2^40 + floor(S (E + floor(E^2 / 2^76)) / 2^36) - 2:
 // the terms left out are below 2^-64.2 / (1 - eps) relative, under one unit
@@ -257,10 +267,10 @@ CFD_XI_HD float seed_rcp(float m)
 {
 #if defined(__CUDA_ARCH__)
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));   // within one ulp
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));   // within 2^-23 for m in [1, 2)
     return r;
 #else
-    return 1.0f / m;
+    return CFD_XI_HOST_RCP(m);
 #endif
 }
 
@@ -269,12 +279,13 @@ CFD_XI_HD Divisor divisor(double b)
     const uint32_t bh = hi32(b), bl = lo32(b);
     const uint32_t mb = ((bh << 3) & 0x7fffffu) | (bl >> 29) | 0x3f800000u;
 #if defined(__CUDA_ARCH__)
-    const uint32_t rb = __float_as_uint(fminf(seed_rcp(__uint_as_float(mb)), 0.99999994f));
+    const uint32_t rb = __float_as_uint(fmaxf(fminf(seed_rcp(__uint_as_float(mb)), 0.99999994f), 0.5f));
 #else
     float m, r;
     std::memcpy(&m, &mb, 4);
     r = seed_rcp(m);
     r = r < 0.99999994f ? r : 0.99999994f;
+    r = r > 0.5f ? r : 0.5f;
     uint32_t rb;
     std::memcpy(&rb, &r, 4);
 #endif
@@ -417,7 +428,7 @@ CFD_XI_HD float seed_rsqrt(float m)
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
     return r;
 #else
-    return (float)(1.0 / std::sqrt((double)m));
+    return CFD_XI_HOST_RSQRT(m);
 #endif
 }
 
