@@ -408,13 +408,21 @@ class _HostBlocks:
         self._limit, self._held, self._free = limit, 0, {}
         self._lock = threading.RLock()   # a finaliser may run inside any of these on the same thread
 
+    def _take(self, size):
+        """A free block of `size` values or None; the lock is held."""
+        try:
+            mem = self._free[size].pop()
+        except (KeyError, IndexError):
+            return None
+        self._held -= mem.nbytes
+        return mem
+
     def array(self, rows: int, cols: int) -> np.ndarray:
-        size, mem = 1 << (rows * cols - 1).bit_length(), None
+        size = 1 << (rows * cols - 1).bit_length()
         with self._lock:
-            free = self._free.get(size) or self._free.get(2 * size)
-            if free:
-                mem = free.pop()
-                self._held -= mem.nbytes
+            mem = self._take(size)
+            if mem is None:
+                mem = self._take(2 * size)
         return np.asarray(self._Lease(self, np.empty(size) if mem is None else mem, (rows, cols)))
 
     def _give_back(self, mem):
@@ -426,19 +434,32 @@ class _HostBlocks:
     def trim(self):
         with self._lock:
             for size in sorted(self._free, reverse=True):
-                while self._free[size] and self._held > self._limit():
-                    self._held -= self._free[size].pop().nbytes
+                while self._held > self._limit() and self._take(size) is not None:
+                    pass
 
 
-_batches = weakref.WeakSet()
+class _OpenFlows:
+    """Bytes of FLOW of each open batch's instances, counted by the batches as
+    they add, remove and close, on any thread.  Calling it gives what the
+    results pool may hold: the largest batch's, each result rounded up."""
+
+    def __init__(self):
+        self._bytes, self._lock = {}, threading.RLock()
+
+    def count(self, batch, rows: int):
+        with self._lock:
+            if rows:
+                self._bytes[id(batch)] = rows * L.NFLOW * 8
+            else:
+                self._bytes.pop(id(batch), None)
+
+    def __call__(self) -> int:
+        with self._lock:
+            return 2 * max(tuple(self._bytes.values()), default=0)
 
 
-def _largest_flow() -> int:
-    """Bytes of the FLOW of the largest open batch's instances, each rounded up."""
-    return 2 * max((sum(tuple(b.rows.values())) for b in tuple(_batches)), default=0) * L.NFLOW * 8
-
-
-_results = _HostBlocks(_largest_flow)
+_open_flows = _OpenFlows()
+_results = _HostBlocks(_open_flows)
 
 
 def _result(rows: int, cols: int) -> np.ndarray:
@@ -458,7 +479,6 @@ class Batch:
         ctx.check(self.lib.cfd_batch_create(ctx.h, int(precision), int(capacity_bytes), C.byref(h)), "cfd_batch_create")
         self.h = h
         self.rows = {}
-        _batches.add(self)
         ctx._children.add(self)
 
     @staticmethod
@@ -470,6 +490,7 @@ class Batch:
             self.lib.cfd_batch_destroy(self.h)
         self.h = None
         self.rows = {}
+        _open_flows.count(self, 0)
         _results.trim()
 
     def __del__(self):
@@ -487,8 +508,12 @@ class Batch:
         slot = C.c_int32()
         self.ctx.check(self.lib.cfd_batch_add(self.h, C.byref(geom), C.byref(pr), C.c_void_p(_ptr(f)),
                                               float(case.dt if dt is None else dt), C.byref(slot)), "cfd_batch_add")
-        self.rows[slot.value] = case.g_node + 1
-        return slot.value
+        return self._admitted(slot.value, case.g_node + 1)
+
+    def _admitted(self, slot: int, rows: int) -> int:
+        self.rows[slot] = rows
+        _open_flows.count(self, sum(self.rows.values()))
+        return slot
 
     @staticmethod
     def stage(case, flow=None, dt=None, params=None) -> "StagedInstance":
@@ -515,12 +540,12 @@ class Batch:
         h = staged.take()
         slot = C.c_int32()
         self.ctx.check(self.lib.cfd_batch_add_staged(self.h, h, C.byref(slot)), "cfd_batch_add_staged")
-        self.rows[slot.value] = staged.rows
-        return slot.value
+        return self._admitted(slot.value, staged.rows)
 
     def remove(self, slot: int):
         self.ctx.check(self.lib.cfd_batch_remove(self.h, int(slot)), "cfd_batch_remove")
         self.rows.pop(slot, None)
+        _open_flows.count(self, sum(self.rows.values()))
         _results.trim()
 
     def step(self, nsteps: int = 1):
