@@ -421,8 +421,6 @@ class _HostBlocks:
         size = 1 << (rows * cols - 1).bit_length()
         with self._lock:
             mem = self._take(size)
-            if mem is None:
-                mem = self._take(2 * size)
         return np.asarray(self._Lease(self, np.empty(size) if mem is None else mem, (rows, cols)))
 
     def _give_back(self, mem):
@@ -564,6 +562,11 @@ class Batch:
         self.ctx.check(self.lib.cfd_batch_set_hold(self.h, int(slot), 1 if hold else 0), "cfd_batch_set_hold")
 
     def get_flow(self, slot: int) -> np.ndarray:
+        """FLOW rows 0..g_node.  From 1 MB the array is a writable view of
+        pooled memory (of the next power of two; nothing beyond the rows is
+        touched) that the caller holds until its last view is dropped: it does
+        not own its data, so ndarray.resize() refuses to grow it; copy() gives
+        an array that does.  get_u0 alike."""
         out = _result(self.rows[slot], L.NFLOW)
         self.ctx.check(self.lib.cfd_batch_get_flow(self.h, int(slot), C.c_void_p(_ptr(out))), "cfd_batch_get_flow")
         return out

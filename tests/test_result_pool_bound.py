@@ -1,11 +1,13 @@
 """The byte bound of the result pool while batches come and go on other
-threads."""
+threads, and the size of the block behind a result."""
 from __future__ import annotations
 
 import sys
 import threading
 import time
 import types
+
+import numpy as np
 
 
 class _FakeLib:
@@ -85,3 +87,16 @@ def test_the_bound_follows_the_largest_open_batch(pkg):
     assert runtime._results._limit() == 0
     a.close()
 
+
+def test_a_result_never_sits_on_a_block_twice_the_next_power_of_two(pkg):
+    from cfd_gb300 import runtime
+    p = runtime._HostBlocks(lambda: 1 << 20)
+    large = p.array(20, 9)                      # 180 values: a block of 256
+    at = large.ctypes.data
+    del large
+    small = p.array(10, 9)                      # 90 values: one of 128, not the free 256
+    assert small.ctypes.data != at and small.base.mem.size == 128
+    assert small.flags.writeable and not small.flags.owndata
+    grown = small.copy()
+    grown.resize((11, 9))                       # a copy owns its data
+    assert np.array_equal(grown[:10], small)
