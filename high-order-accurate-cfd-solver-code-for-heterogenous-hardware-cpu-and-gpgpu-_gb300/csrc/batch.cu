@@ -910,6 +910,8 @@ cfd_status_t cfd_batch_tune(cfd_batch_t *b, int32_t steps_per_trial)
     size_t total = 0;
     for (auto &a : arrays) total += a.second;
     if (total == 0) return CFD_OK;
+    if (b->dirty && (st = rebuild(b)) != CFD_OK) return st;
+    if (b->ntiles == 0) return CFD_OK;   // every instance is held: nothing to time
     char *backup = nullptr;
     cudaError_t e = cudaMalloc(&backup, total);
     if (e != cudaSuccess) return cuda_fail(b->ctx, e, "cfd_batch_tune backup");
