@@ -205,15 +205,21 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
 // -------------------------------------------------------------- Viscous --
 // Viscous.cl:23-643.
 // The inviscid node fluxes and the filter width of every row (their own
-// kernel: beside the viscous fluxes they would spill).
+// kernel: beside the viscous fluxes they would spill) but those k_viscous
+// skips.
 template <bool I>
 __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, double *__restrict__ E,
-                                                      double *__restrict__ G, const double *__restrict__ metric,
+                                                      double *__restrict__ G, const int *__restrict__ grid,
+                                                      const double *__restrict__ metric,
                                                       const double *__restrict__ det, const double *__restrict__ flow,
-                                                      int n_items, int les, double *__restrict__ width)
+                                                      int n_items, int n_rows, int les, double *__restrict__ width)
 {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= n_items) return;
+    {
+        int idx[3][7];
+        if (!gather_star(grid, gid, n_rows, idx)) return;
+    }
     const double D = det[gid];
     const double *m = metric + 63 * (size_t)gid;
     const double *fr = flow + 9 * (size_t)gid;
@@ -676,7 +682,8 @@ int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, d
     const unsigned nb = blocks_for(n_items, 128);
     if (scratch && scratch_rows >= n_items) {
         const bool fp = n_items <= kPlainNodes;
-        (fp ? k_node_flux<false> : k_node_flux<true>)<<<nb, 128, 0, st>>>(F, E, G, metric, det, flow, n_items, P.les, scratch);
+        (fp ? k_node_flux<false> : k_node_flux<true>)<<<nb, 128, 0, st>>>(F, E, G, grid, metric, det, flow, n_items,
+                                                                         n_rows, P.les, scratch);
         const int T = fp ? kViscousThreads<false> : kViscousThreads<true>;
         (fp ? k_viscous<false, false> : k_viscous<false, true>)<<<blocks_for(n_items, T), T, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
                                              scratch);
