@@ -376,8 +376,7 @@ cfd_status_t cfd_viscous(cfd_ctx_t *ctx, cfd_column_t *U_C, cfd_column_t *F_C, c
     ctx->launches += launch_viscous(ctx->stream, make_phys(params), (const double *)a[0].dev, (double *)a[1].dev,
                                     (double *)a[2].dev, (double *)a[3].dev, (double *)a[4].dev, (double *)a[5].dev,
                                     (double *)a[6].dev, (const int *)a[7].dev, (const double *)a[8].dev,
-                                    (const double *)a[9].dev, (double *)a[10].dev, n_items, ctx->n_rows, ctx->d_flags,
-                                    ctx->face_reuse ? ctx->d_face : nullptr, ctx->face_rows) - 1;
+                                    (const double *)a[9].dev, (double *)a[10].dev, n_items, ctx->n_rows, ctx->d_flags) - 1;
     return stage_out(ctx, a, 11, after_launch(ctx, "cfd_viscous launch"));
 }
 
@@ -449,7 +448,7 @@ cfd_status_t cfd_rk3_step(cfd_ctx_t *ctx, double Mach, double del_t, const cfd_d
             n += launch_uq(ctx->stream, U[j], Q, grid, dd, flow, roe, g_node + 1, ctx->n_rows, ctx->d_flags, face,
                            ctx->face_rows);
             n += launch_viscous(ctx->stream, P, U[j], F_, E_, G_, Fv_, Ev_, Gv_, grid, met, dd, flow, g_node + 1,
-                                ctx->n_rows, ctx->d_flags, face, ctx->face_rows);
+                                ctx->n_rows, ctx->d_flags);
             launch_weno(ctx->stream, P, j, Mach, del_t, dt_, dd, U[0], U[1], U[2], grid, Q, met, roe, Fv_, Ev_, Gv_,
                         F_, E_, G_, flow, sd_node + 1, ctx->n_rows, ctx->d_flags, nullptr, face, ctx->face_rows,
                         next_face_gen(ctx->face_gen));

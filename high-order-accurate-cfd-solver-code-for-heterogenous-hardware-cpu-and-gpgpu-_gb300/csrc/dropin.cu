@@ -205,14 +205,17 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
 // -------------------------------------------------------------- Viscous --
 // Viscous.cl:23-643.
 // The inviscid node fluxes and the filter width of every row (their own
-// kernel: beside the viscous fluxes they would spill) but those k_viscous
-// skips.
+// kernel: beside the viscous fluxes they would spill; in one: TGV 96^3 1.17 ms
+// at 3 blocks per SM, 1.38 at 4, with 3 KB of spill loads per thread) but
+// those k_viscous skips.  The width waits in component 0 of the row's own Fv,
+// which k_viscous writes after reading it: no memory but the call's outputs,
+// so calls on different streams share nothing.
 template <bool I>
 __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, double *__restrict__ E,
-                                                      double *__restrict__ G, const int *__restrict__ grid,
-                                                      const double *__restrict__ metric,
+                                                      double *__restrict__ G, double *__restrict__ Fv,
+                                                      const int *__restrict__ grid, const double *__restrict__ metric,
                                                       const double *__restrict__ det, const double *__restrict__ flow,
-                                                      int n_items, int n_rows, int les, double *__restrict__ width)
+                                                      int n_items, int n_rows, int les)
 {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= n_items) return;
@@ -227,26 +230,20 @@ __global__ void __launch_bounds__(128, 6) k_node_flux(double *__restrict__ F, do
     double Qn[5], H;
     ex::node_flux<I>(prim, [&](int k) { return m[k]; }, D,
                   [&](int e, int c, double f) { (e == 0 ? F : (e == 1 ? E : G))[5 * (size_t)gid + c] = f; }, Qn, H);
-    if (les) width[gid] = ex::filter_width(D);
+    if (les) Fv[5 * (size_t)gid] = ex::filter_width(D);
 }
 
-// NODE = false: the inviscid node fluxes and the filter width come from
-// k_node_flux (width: one double per row); true: all in one kernel, for
-// callers without the scratch.  TGV 96^3, both kernels: 1.00 ms at 3 or 4
-// blocks per SM, 1.19 at 5; in one kernel 1.17 at 3, 1.38 at 4 (3 KB of spill
-// loads per thread).
-// The integer form in blocks of 256, which share its long code better: 0.73
-// -> 0.69 ms for both kernels.
+// After k_node_flux.  TGV 96^3, both kernels: 1.00 ms at 3 or 4 blocks of 128
+// per SM, 1.19 at 5.  The integer form in blocks of 256, which share its long
+// code better: 0.73 -> 0.69 ms for both kernels (0.72 with the check of the
+// neighbour chain in both).
 template <bool I>
 constexpr int kViscousThreads = I ? 256 : 128;
-template <bool NODE, bool I>
-__global__ void __launch_bounds__(kViscousThreads<I>, 512 / kViscousThreads<I>) k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ F,
-                                                 double *__restrict__ E, double *__restrict__ G,
-                                                 double *__restrict__ Fv, double *__restrict__ Ev,
-                                                 double *__restrict__ Gv, const int *__restrict__ grid,
-                                                 const double *__restrict__ metric, const double *__restrict__ det,
-                                                 double *__restrict__ flow, int n_items, int n_rows, unsigned *flags,
-                                                 const double *__restrict__ width)
+template <bool I>
+__global__ void __launch_bounds__(kViscousThreads<I>, 512 / kViscousThreads<I>)
+k_viscous(Phys P, const double *__restrict__ U, double *__restrict__ Fv, double *__restrict__ Ev,
+          double *__restrict__ Gv, const int *__restrict__ grid, const double *__restrict__ metric,
+          const double *__restrict__ det, double *__restrict__ flow, int n_items, int n_rows, unsigned *flags)
 {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= n_items) return;
@@ -262,11 +259,6 @@ __global__ void __launch_bounds__(kViscousThreads<I>, 512 / kViscousThreads<I>) 
     const double *fr = flow + 9 * (size_t)gid;
     const double prim[5] = {fr[FRHO], fr[FU], fr[FV], fr[FW], fr[FP]};
     auto metric_at = [&](int k) { return m[k]; };
-    if (NODE) {
-        double Qn[5], H;
-        ex::node_flux<I>(prim, metric_at, D,
-                      [&](int e, int c, double f) { (e == 0 ? F : (e == 1 ? E : G))[5 * (size_t)gid + c] = f; }, Qn, H);
-    }
     double mu;
     {
         // the star is walked again for each direction (it is cached by now):
@@ -295,7 +287,7 @@ __global__ void __launch_bounds__(kViscousThreads<I>, 512 / kViscousThreads<I>) 
                          *up = U + 5 * (size_t)grid_nb(grid, gid, plus_slot(d));
             KS[d] = P.les && P.les != 2 ? ex::ks_root(Ui[c], Ui[0], um[c], um[0], up[c], up[0]) : 0.0;
         }
-        ex::viscous_node<I>(dU, Ui, metric_at, D, NODE ? ex::filter_width(D) : width[gid], prim, KS, P,
+        ex::viscous_node<I>(dU, Ui, metric_at, D, P.les ? Fv[5 * (size_t)gid] : 0.0, prim, KS, P,
                          [&](int e, int c, double f) {
                              (e == 0 ? Fv : (e == 1 ? Ev : Gv))[5 * (size_t)gid + c] = P.viscous ? f : 0.0;
                          },
@@ -677,21 +669,15 @@ int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const doub
 
 int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
                     double *Ev, double *Gv, const int *grid, const double *metric, const double *det, double *flow,
-                    int n_items, int n_rows, unsigned *flags, double *scratch, long long scratch_rows)
+                    int n_items, int n_rows, unsigned *flags)
 {
-    const unsigned nb = blocks_for(n_items, 128);
-    if (scratch && scratch_rows >= n_items) {
-        const bool fp = n_items <= kPlainNodes;
-        (fp ? k_node_flux<false> : k_node_flux<true>)<<<nb, 128, 0, st>>>(F, E, G, grid, metric, det, flow, n_items,
-                                                                         n_rows, P.les, scratch);
-        const int T = fp ? kViscousThreads<false> : kViscousThreads<true>;
-        (fp ? k_viscous<false, false> : k_viscous<false, true>)<<<blocks_for(n_items, T), T, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
-                                             scratch);
-        return 2;
-    }
-    k_viscous<true, false><<<nb, 128, 0, st>>>(P, U, F, E, G, Fv, Ev, Gv, grid, metric, det, flow, n_items, n_rows, flags,
-                                        nullptr);
-    return 1;
+    const bool fp = n_items <= kPlainNodes;
+    const int T = fp ? kViscousThreads<false> : kViscousThreads<true>;
+    (fp ? k_node_flux<false> : k_node_flux<true>)<<<blocks_for(n_items, 128), 128, 0, st>>>(
+        F, E, G, Fv, grid, metric, det, flow, n_items, n_rows, P.les);
+    (fp ? k_viscous<false> : k_viscous<true>)<<<blocks_for(n_items, T), T, 0, st>>>(P, U, Fv, Ev, Gv, grid, metric, det,
+                                                                                    flow, n_items, n_rows, flags);
+    return 2;
 }
 
 // Grid of k_weno_minus: two resident blocks of 128 per SM, at most one

@@ -93,10 +93,10 @@ cfd_status_t stage_out(cfd_ctx *ctx, const BufArg *a, int n, cfd_status_t launch
 // kernels launched (2 or 1).
 int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
               double *roe, int n_items, int n_rows, unsigned *flags, double *node_scratch, long long scratch_rows);
-// Viscous; the scratch as for launch_uq.  Returns the kernels launched.
+// Viscous.  Returns the kernels launched.
 int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
                     double *Ev, double *Gv, const int *grid, const double *metric, const double *det, double *flow,
-                    int n_items, int n_rows, unsigned *flags, double *scratch, long long scratch_rows);
+                    int n_items, int n_rows, unsigned *flags);
 void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, const double *deter,
                  const double *det, double *U0, double *U1, double *U2, const int *grid, const double *Q,
                  const double *metric, const double *roe, const double *Fv, const double *Ev, const double *Gv,

@@ -336,7 +336,7 @@ cfd_status_t run_stage(cfd_solver *s, int j, double dt, bool want_L)
         const int nu = launch_uq(ctx->stream, Uj, s->Q, s->grid, s->det, s->flow, s->roe, s->g_node + 1, s->n_rows,
                                  ctx->d_flags, s->face, s->n_rows);
         const int nv = launch_viscous(ctx->stream, s->P, Uj, s->F, s->E, s->G, s->Fv, s->Ev, s->Gv, s->grid, s->metric,
-                                      s->det, s->flow, s->g_node + 1, s->n_rows, ctx->d_flags, s->face, s->n_rows);
+                                      s->det, s->flow, s->g_node + 1, s->n_rows, ctx->d_flags);
         launch_weno(ctx->stream, s->P, j, s->P.mach, dt, s->deter, s->det, s->U[0], s->U[1], s->U[2], s->grid, s->Q,
                     s->metric, s->roe, s->Fv, s->Ev, s->Gv, s->F, s->E, s->G, s->flow, s->sd_node + 1, s->n_rows,
                     ctx->d_flags, want_L ? s->L : nullptr, s->face, s->n_rows, next_face_gen(s->face_gen));
@@ -633,7 +633,7 @@ cfd_status_t cfd_solver_profile_stage(cfd_solver_t *s, int32_t j, double del_t, 
                                  s->ctx->d_flags, s->face, s->n_rows);
         cudaEventRecord(ev[1], stream);
         const int nv = launch_viscous(stream, s->P, Uj, s->F, s->E, s->G, s->Fv, s->Ev, s->Gv, s->grid, s->metric,
-                                      s->det, s->flow, s->g_node + 1, s->n_rows, s->ctx->d_flags, s->face, s->n_rows);
+                                      s->det, s->flow, s->g_node + 1, s->n_rows, s->ctx->d_flags);
         cudaEventRecord(ev[2], stream);
         launch_weno(stream, s->P, j, s->P.mach, del_t, s->deter, s->det, s->U[0], s->U[1], s->U[2], s->grid, s->Q,
                     s->metric, s->roe, s->Fv, s->Ev, s->Gv, s->F, s->E, s->G, s->flow, s->sd_node + 1, s->n_rows,

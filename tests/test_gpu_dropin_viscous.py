@@ -1,5 +1,5 @@
 """cfd_viscous around its two launches: rows whose neighbour chain leaves the
-table are skipped whole."""
+table are skipped whole, and no memory but the call's own is used."""
 from __future__ import annotations
 
 import numpy as np
@@ -46,3 +46,33 @@ def test_rows_with_a_bad_chain_are_left_as_they_were(ctx, reuse):
         ctx.set_face_reuse(True)
         for p in dev.values():
             ctx.free(p)
+
+
+@pytest.mark.parametrize("les", [0, 1, 2])
+def test_the_scratch_of_the_other_kernels_is_not_used(ctx, les):
+    """The face scratch belongs to cfd_uq and cfd_weno, which may run for
+    another table on another stream: with and without it cfd_viscous makes
+    the same two launches and the same bits."""
+    import dataclasses
+
+    from cfd_gb300 import cases
+    c = cases.taylor_green(shape=(9, 8, 7))
+    c = dataclasses.replace(c, params=dataclasses.replace(c.params, les=les))
+    out, launches = [], []
+    for reuse in (True, False):
+        ctx.set_face_reuse(reuse)
+        a = copy_arrays(c.arrays)
+        dev = ctx.upload_case(a)
+        try:
+            ctx.uq(dev["U0"], dev["Q"], dev["grid"], dev["det"], dev["flow"], dev["roe"], c.g_node + 1)
+            n = ctx.launch_count
+            _viscous(ctx, dev, c, c.g_node + 1)
+            launches.append(ctx.launch_count - n)
+            out.append([ctx.download(dev, k, a[k]) for k in OUT + ("flow",)])
+        finally:
+            ctx.set_face_reuse(True)
+            for p in dev.values():
+                ctx.free(p)
+    assert launches == [2, 2]
+    for a, b in zip(*out):
+        assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
