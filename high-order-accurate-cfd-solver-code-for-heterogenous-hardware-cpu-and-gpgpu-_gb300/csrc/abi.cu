@@ -220,7 +220,7 @@ cfd_status_t cfd_ctx_destroy(cfd_ctx_t *ctx)
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->d_flags) cudaFree(ctx->d_flags);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
-    if (ctx->d_face) cudaFree(ctx->d_face);
+    row_scratch_free(ctx->scratch);
     for (auto &m : ctx->mirrors) cudaFree(m.second.first);
     delete ctx;
     return CFD_OK;
@@ -257,28 +257,15 @@ cfd_status_t cfd_ctx_set_rows(cfd_ctx_t *ctx, int32_t n_rows)
 {
     if (!ctx || n_rows <= 0) return fail(ctx, CFD_EINVAL, "n_rows must be positive");
     ctx->n_rows = n_rows;
-    // cfd_weno's face scratch; without it (no memory) cfd_weno evaluates
-    // both faces per row, with the same results
-    if (ctx->face_rows < n_rows) {
+    // the face scratch of cfd_uq and cfd_weno; without it (no memory for 252
+    // bytes per row and the smallest round) they evaluate every row by
+    // itself, with the same results
+    if (ctx->scratch.rows < n_rows) {
         cfd_status_t s = use_device(ctx);
         if (s != CFD_OK) return s;
-        if (ctx->d_face) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(ctx->d_face);
-        }
-        ctx->d_face = nullptr;
-        ctx->face_rows = 0;
-        void *buf = nullptr;
-        if (cudaMalloc(&buf, face_scratch_bytes(n_rows)) == cudaSuccess) {
-            double *f = static_cast<double *>(buf);
-            if (cudaMemset(face_stamps(f, n_rows), 0, (size_t)n_rows * 3 * sizeof(unsigned)) == cudaSuccess) {
-                ctx->d_face = f;
-                ctx->face_rows = n_rows;
-            } else {
-                cudaFree(buf);
-            }
-        }
-        cudaGetLastError();   // a failed allocation only disables the sharing
+        if (ctx->scratch.face) cudaStreamSynchronize(ctx->stream);
+        row_scratch_free(ctx->scratch);
+        row_scratch_alloc(ctx->scratch, n_rows);
     }
     return CFD_OK;
 }
@@ -337,6 +324,8 @@ cfd_status_t cfd_buffer_read(cfd_ctx_t *ctx, void *dst, const void *src, size_t 
     return CFD_OK;
 }
 
+static RowScratch scratch_of(const cfd_ctx_t *ctx) { return ctx->face_reuse ? ctx->scratch : RowScratch(); }
+
 static cfd_status_t check_launch_args(cfd_ctx_t *ctx, int32_t n_items, const char *who)
 {
     if (!ctx) return CFD_EINVAL;
@@ -357,8 +346,7 @@ cfd_status_t cfd_uq(cfd_ctx_t *ctx, cfd_column_t *U_C, cfd_column_t *Q_C, const 
     if ((s = stage_in(ctx, a, 6, "cfd_uq")) != CFD_OK) return s;
     ctx->launches += launch_uq(ctx->stream, (double *)a[0].dev, (double *)a[1].dev, (const int *)a[2].dev,
                                (const double *)a[3].dev, (const double *)a[4].dev, (double *)a[5].dev, n_items,
-                               ctx->n_rows, ctx->d_flags, ctx->face_reuse ? ctx->d_face : nullptr,
-                               ctx->face_rows) - 1;
+                               ctx->n_rows, ctx->d_flags, scratch_of(ctx)) - 1;
     return stage_out(ctx, a, 6, after_launch(ctx, "cfd_uq launch"));
 }
 
@@ -400,15 +388,15 @@ cfd_status_t cfd_weno(cfd_ctx_t *ctx, int32_t j, double Mach, double del_t, cons
     if ((s = stage_in(ctx, a, 16, "cfd_weno")) != CFD_OK) return s;
     BufArg l[] = {{L_out, 40, true}};
     if (L_out && (s = stage_in(ctx, l, 1, "cfd_weno")) != CFD_OK) return s;
-    double *const face = ctx->face_reuse ? ctx->d_face : nullptr;
+    const RowScratch face = scratch_of(ctx);
     launch_weno(ctx->stream, make_phys(params), j, Mach, del_t, (const double *)a[0].dev, (const double *)a[1].dev,
                 (double *)a[2].dev, (double *)a[3].dev, (double *)a[4].dev, (const int *)a[5].dev,
                 (const double *)a[6].dev, (const double *)a[7].dev, (const double *)a[8].dev,
                 (const double *)a[9].dev, (const double *)a[10].dev, (const double *)a[11].dev,
                 (const double *)a[12].dev, (const double *)a[13].dev, (const double *)a[14].dev, (double *)a[15].dev,
-                n_items, ctx->n_rows, ctx->d_flags, L_out ? (double *)l[0].dev : nullptr, face, ctx->face_rows,
+                n_items, ctx->n_rows, ctx->d_flags, L_out ? (double *)l[0].dev : nullptr, face,
                 next_face_gen(ctx->face_gen));
-    ctx->launches += weno_launches(face, ctx->face_rows, n_items) - 1;
+    ctx->launches += weno_launches(face, n_items) - 1;
     s = stage_out(ctx, a, 16, after_launch(ctx, "cfd_weno launch"));
     return L_out ? stage_out(ctx, l, 1, s) : s;
 }
@@ -435,7 +423,7 @@ cfd_status_t cfd_rk3_step(cfd_ctx_t *ctx, double Mach, double del_t, const cfd_d
                   {FLOW, 72, true}};
     if ((s = stage_in(ctx, a, 16, "cfd_rk3_step")) != CFD_OK) return s;
     const Phys P = make_phys(params);
-    double *const face = ctx->face_reuse ? ctx->d_face : nullptr;
+    const RowScratch face = scratch_of(ctx);
     double *U[3] = {(double *)a[2].dev, (double *)a[3].dev, (double *)a[4].dev};
     const int *grid = (const int *)a[5].dev;
     const double *dt_ = (const double *)a[0].dev, *dd = (const double *)a[1].dev, *met = (const double *)a[7].dev;
@@ -445,14 +433,13 @@ cfd_status_t cfd_rk3_step(cfd_ctx_t *ctx, double Mach, double del_t, const cfd_d
     uint64_t n = 0;
     for (int step = 0; step < nsteps; ++step)
         for (int j = 0; j < 3; ++j) {   // Solver.cpp:365-658, j passed per stage
-            n += launch_uq(ctx->stream, U[j], Q, grid, dd, flow, roe, g_node + 1, ctx->n_rows, ctx->d_flags, face,
-                           ctx->face_rows);
+            n += launch_uq(ctx->stream, U[j], Q, grid, dd, flow, roe, g_node + 1, ctx->n_rows, ctx->d_flags, face);
             n += launch_viscous(ctx->stream, P, U[j], F_, E_, G_, Fv_, Ev_, Gv_, grid, met, dd, flow, g_node + 1,
                                 ctx->n_rows, ctx->d_flags);
             launch_weno(ctx->stream, P, j, Mach, del_t, dt_, dd, U[0], U[1], U[2], grid, Q, met, roe, Fv_, Ev_, Gv_,
-                        F_, E_, G_, flow, sd_node + 1, ctx->n_rows, ctx->d_flags, nullptr, face, ctx->face_rows,
+                        F_, E_, G_, flow, sd_node + 1, ctx->n_rows, ctx->d_flags, nullptr, face,
                         next_face_gen(ctx->face_gen));
-            n += weno_launches(face, ctx->face_rows, sd_node + 1);
+            n += weno_launches(face, sd_node + 1);
             if (bc) {
                 bc_apply_aos(ctx->stream, bc->dev, flow, Mach);
                 n += bc->dev.launches();

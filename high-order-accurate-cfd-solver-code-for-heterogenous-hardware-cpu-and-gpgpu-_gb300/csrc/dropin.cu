@@ -654,13 +654,36 @@ __global__ void __launch_bounds__(128, REUSE ? 5 : 1) k_weno(Phys P, int j, doub
         atomicOr(flags, CFD_FLAG_NONFINITE);
 }
 
-int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
-              double *roe, int n_items, int n_rows, unsigned *flags, double *node_scratch, long long scratch_rows)
+cudaError_t row_scratch_alloc(RowScratch &S, long long rows)
 {
-    if (node_scratch && scratch_rows >= n_rows) {   // 5 of the 30 doubles per row
-        k_uq_node<<<blocks_for(n_rows, 128), 128, 0, st>>>(flow, n_rows, node_scratch);
+    RowScratch n;
+    n.rows = rows;
+    n.round = std::min(rows, kRowRound);
+    cudaError_t e = cudaMalloc((void **)&n.face, row_face_bytes(rows));
+    if (e == cudaSuccess) e = cudaMemset(n.stamps(), 0, (size_t)rows * 3 * sizeof(unsigned));
+    if (e == cudaSuccess) e = round_alloc(n.round, std::min(rows, kLeastRound), row_round_bytes, (void **)&n.col);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        row_scratch_free(n);
+    }
+    S = n;
+    return e;
+}
+
+void row_scratch_free(RowScratch &S)
+{
+    if (S.face) cudaFree(S.face);
+    if (S.col) cudaFree(S.col);
+    S = RowScratch();
+}
+
+int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
+              double *roe, int n_items, int n_rows, unsigned *flags, const RowScratch &scratch)
+{
+    if (scratch.serves(n_rows)) {
+        k_uq_node<<<blocks_for(n_rows, 128), 128, 0, st>>>(flow, n_rows, scratch.face);
         k_uq<true><<<blocks_for(n_items, 128), 128, 0, st>>>(U, Q, grid, det, flow, roe, n_items, n_rows, flags,
-                                                             node_scratch);
+                                                             scratch.face);
         return 2;
     }
     k_uq<false><<<blocks_for(n_items, 128), 128, 0, st>>>(U, Q, grid, det, flow, roe, n_items, n_rows, flags, nullptr);
@@ -698,16 +721,16 @@ void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, 
                  const double *det, double *U0, double *U1, double *U2, const int *grid, const double *Q,
                  const double *metric, const double *roe, const double *Fv, const double *Ev, const double *Gv,
                  const double *F, const double *E, const double *G, double *flow, int n_items, int n_rows,
-                 unsigned *flags, double *L_out, double *face_scratch, long long scratch_rows, unsigned gen)
+                 unsigned *flags, double *L_out, const RowScratch &scratch, unsigned gen)
 {
     const unsigned nb = blocks_for(n_items, 128);
-    if (face_scratch && scratch_rows >= n_items) {
-        const long long ld = scratch_rows;
-        double *Fp = face_scratch, *Fm = face_scratch + 15 * ld;
-        unsigned *stamp = face_stamps(face_scratch, ld);
-        const int round = (int)row_round(ld);
+    if (scratch.serves(n_items)) {
+        const long long ld = scratch.rows;
+        double *Fp = scratch.face, *Fm = scratch.face + 15 * ld;
+        unsigned *stamp = scratch.stamps();
+        const int round = (int)scratch.round;
         for (int r0 = 0; r0 < n_items; r0 += round) {
-            const RowRound R{face_scratch + 30 * ld, r0, std::min(n_items, r0 + round), round};
+            const RowRound R{scratch.col, r0, std::min(n_items, r0 + round), round};
             const unsigned n = blocks_for(R.r1 - r0, 128), n2 = blocks_for(R.r1 - r0, 256);
             k_row_base<<<dim3(n, 3), 128, 0, st>>>(grid, metric, roe, n_rows, R);
             k_row_char<<<dim3(5 * n2, 3), 256, 0, st>>>(Q, P.eps, R);

@@ -12,6 +12,7 @@
 
 #include "cfd_rhs.h"
 #include "physics.cuh"
+#include "rounds.h"
 
 // Device error-flag bits (one 32-bit word per context, or per instance in
 // the batched solver).
@@ -31,10 +32,7 @@ struct cfd_ctx {
     unsigned *h_flags = nullptr;   // pinned mirror
     uint64_t launches = 0;
     std::string last_error;
-    // cfd_weno's face scratch (30 doubles per row and one round's, allocated by
-    // cfd_ctx_set_rows; null: each row evaluates both faces itself)
-    double *d_face = nullptr;   // face_scratch_bytes(face_rows)
-    long long face_rows = 0;
+    cfd::RowScratch scratch;   // of cfd_uq and cfd_weno, allocated by cfd_ctx_set_rows
     unsigned face_gen = 0;
     bool face_reuse = true;
     // device mirrors of host buffers handed to the kernel entry points:
@@ -88,11 +86,11 @@ cfd_status_t stage_in(cfd_ctx *ctx, BufArg *a, int n, const char *who);
 cfd_status_t stage_out(cfd_ctx *ctx, const BufArg *a, int n, cfd_status_t launch_status);
 
 // Drop-in kernel launchers (dropin.cu).  All pointers are device pointers.
-// U_Q; with a scratch of >= n_rows rows (30 doubles each, cfd_weno's face
-// scratch) it first computes sqrt(rho) and its products once per row.  Returns the
-// kernels launched (2 or 1).
+// U_Q; with a scratch that serves n_rows rows it first computes sqrt(rho) and
+// its products once per row (5 of the 30 doubles of a row's faces).  Returns
+// the kernels launched (2 or 1).
 int launch_uq(cudaStream_t st, double *U, double *Q, const int *grid, const double *det, const double *flow,
-              double *roe, int n_items, int n_rows, unsigned *flags, double *node_scratch, long long scratch_rows);
+              double *roe, int n_items, int n_rows, unsigned *flags, const RowScratch &scratch);
 // Viscous.  Returns the kernels launched.
 int launch_viscous(cudaStream_t st, const Phys &P, const double *U, double *F, double *E, double *G, double *Fv,
                     double *Ev, double *Gv, const int *grid, const double *metric, const double *det, double *flow,
@@ -101,36 +99,18 @@ void launch_weno(cudaStream_t st, const Phys &P, int j, double mach, double dt, 
                  const double *det, double *U0, double *U1, double *U2, const int *grid, const double *Q,
                  const double *metric, const double *roe, const double *Fv, const double *Ev, const double *Gv,
                  const double *F, const double *E, const double *G, double *flow, int n_items, int n_rows,
-                 unsigned *flags, double *L_out, double *face_scratch, long long scratch_rows, unsigned gen);
-// Face scratch of launch_weno for `rows` rows: +1/2 faces [3][5][rows] and
-// -1/2 faces [3][5][rows] (doubles), the face kernels' own scratch for one
-// round of rows, then generation stamps [3][rows] (unsigned, zero when
-// allocated).  gen: a value new to the scratch on every call
-// (next_face_gen).
-constexpr long long kRowRound = 1 << 18;   // rows of one round of the face kernels: 302 MB, some 25 waves of blocks
-constexpr int kRowFace = 48;               // doubles of one row's face along one direction
-inline long long row_round(long long rows) { return rows < kRowRound ? rows : kRowRound; }
-inline size_t face_scratch_doubles(long long rows) { return (size_t)rows * 30 + (size_t)row_round(rows) * 3 * kRowFace; }
-inline size_t face_scratch_bytes(long long rows)
-{
-    return face_scratch_doubles(rows) * sizeof(double) + (size_t)rows * 3 * sizeof(unsigned);
-}
-inline unsigned *face_stamps(double *scratch, long long rows)
-{
-    return reinterpret_cast<unsigned *>(scratch + face_scratch_doubles(rows));
-}
+                 unsigned *flags, double *L_out, const RowScratch &scratch, unsigned gen);
+// gen of launch_weno: a value new to the scratch's stamps on every call.
 inline unsigned next_face_gen(unsigned &g)
 {
     g = g + 1 == 0 ? 1 : g + 1;
     return g;
 }
 // Kernels one launch_weno issues: four face kernels per round, the unstamped
-// faces and the update with a face scratch of >= n_items rows, else 1.
-inline int weno_launches(const double *face_scratch, long long scratch_rows, int n_items)
+// faces and the update with a scratch that serves n_items rows, else 1.
+inline int weno_launches(const RowScratch &S, int n_items)
 {
-    if (!face_scratch || scratch_rows < n_items) return 1;
-    const long long round = row_round(scratch_rows);
-    return (int)(4 * ((n_items + round - 1) / round) + 2);
+    return S.serves(n_items) ? (int)(4 * ((n_items + S.round - 1) / S.round) + 2) : 1;
 }
 
 }  // namespace cfd

@@ -43,7 +43,7 @@ struct cfd_solver {
     double *U[3] = {nullptr, nullptr, nullptr};
     double *Q = nullptr, *F = nullptr, *E = nullptr, *G = nullptr, *Fv = nullptr, *Ev = nullptr, *Gv = nullptr;
     double *roe = nullptr, *L = nullptr;
-    double *face = nullptr;     // gather path: the Weno pass's face scratch (face_scratch_bytes(n_rows))
+    cfd::RowScratch face;       // gather path: the U_Q and Weno passes' scratch
     unsigned face_gen = 0;
     // structured path
     cfd::StructuredLaunch S{};
@@ -97,9 +97,10 @@ cfd_status_t create_gather(cfd_solver *s, const cfd_geometry_t *g)
     double **c5[] = {&s->Q, &s->F, &s->E, &s->G, &s->Fv, &s->Ev, &s->Gv, &s->L};
     for (double **p : c5)
         if ((st = dalloc_t(s, R * 5, p))) return st;
-    if ((st = dalloc_t(s, R * 36, &s->roe)) || (st = dalloc(s, face_scratch_bytes((long long)R), (void **)&s->face)))
-        return st;
-    cudaMemsetAsync(face_stamps(s->face, (long long)R), 0, R * 3 * sizeof(unsigned), s->ctx->stream);
+    if ((st = dalloc_t(s, R * 36, &s->roe))) return st;
+    if (const cudaError_t fe = row_scratch_alloc(s->face, (long long)R); fe != cudaSuccess)
+        return cuda_fail(s->ctx, fe, "cudaMalloc (solver)");
+    s->bytes += row_face_bytes((long long)R) + row_round_bytes(s->face.round);
     for (int q = 0; q < 3; ++q) cudaMemsetAsync(s->U[q], 0, R * 5 * sizeof(double), s->ctx->stream);
     for (double **p : c5) cudaMemsetAsync(*p, 0, R * 5 * sizeof(double), s->ctx->stream);
     cudaMemsetAsync(s->roe, 0, R * 36 * sizeof(double), s->ctx->stream);
@@ -334,13 +335,13 @@ cfd_status_t run_stage(cfd_solver *s, int j, double dt, bool want_L)
     } else {
         double *Uj = s->U[j];
         const int nu = launch_uq(ctx->stream, Uj, s->Q, s->grid, s->det, s->flow, s->roe, s->g_node + 1, s->n_rows,
-                                 ctx->d_flags, s->face, s->n_rows);
+                                 ctx->d_flags, s->face);
         const int nv = launch_viscous(ctx->stream, s->P, Uj, s->F, s->E, s->G, s->Fv, s->Ev, s->Gv, s->grid, s->metric,
                                       s->det, s->flow, s->g_node + 1, s->n_rows, ctx->d_flags);
         launch_weno(ctx->stream, s->P, j, s->P.mach, dt, s->deter, s->det, s->U[0], s->U[1], s->U[2], s->grid, s->Q,
                     s->metric, s->roe, s->Fv, s->Ev, s->Gv, s->F, s->E, s->G, s->flow, s->sd_node + 1, s->n_rows,
-                    ctx->d_flags, want_L ? s->L : nullptr, s->face, s->n_rows, next_face_gen(s->face_gen));
-        ctx->launches += nu + nv + weno_launches(s->face, s->n_rows, s->sd_node + 1);
+                    ctx->d_flags, want_L ? s->L : nullptr, s->face, next_face_gen(s->face_gen));
+        ctx->launches += nu + nv + weno_launches(s->face, s->sd_node + 1);
         if (s->has_bc) {
             bc_apply_aos(ctx->stream, s->bc, s->flow, s->P.mach);
             ctx->launches += s->bc.launches();
@@ -438,6 +439,7 @@ cfd_status_t cfd_solver_destroy(cfd_solver_t *s)
         if (s->S.face_join[f]) cudaEventDestroy(s->S.face_join[f]);
     }
     bc_free(s->bc);
+    row_scratch_free(s->face);
     for (void *p : s->allocs) cudaFree(p);
     delete s;
     return CFD_OK;
@@ -630,20 +632,20 @@ cfd_status_t cfd_solver_profile_stage(cfd_solver_t *s, int32_t j, double del_t, 
         cudaEventRecord(ev[0], stream);
         double *Uj = s->U[j];
         const int nu = launch_uq(stream, Uj, s->Q, s->grid, s->det, s->flow, s->roe, s->g_node + 1, s->n_rows,
-                                 s->ctx->d_flags, s->face, s->n_rows);
+                                 s->ctx->d_flags, s->face);
         cudaEventRecord(ev[1], stream);
         const int nv = launch_viscous(stream, s->P, Uj, s->F, s->E, s->G, s->Fv, s->Ev, s->Gv, s->grid, s->metric,
                                       s->det, s->flow, s->g_node + 1, s->n_rows, s->ctx->d_flags);
         cudaEventRecord(ev[2], stream);
         launch_weno(stream, s->P, j, s->P.mach, del_t, s->deter, s->det, s->U[0], s->U[1], s->U[2], s->grid, s->Q,
                     s->metric, s->roe, s->Fv, s->Ev, s->Gv, s->F, s->E, s->G, s->flow, s->sd_node + 1, s->n_rows,
-                    s->ctx->d_flags, nullptr, s->face, s->n_rows, next_face_gen(s->face_gen));
+                    s->ctx->d_flags, nullptr, s->face, next_face_gen(s->face_gen));
         cudaEventRecord(ev[3], stream);
         snames[0] = "uq";
         snames[1] = "viscous";
         snames[2] = "weno";
         // uq: per-row pass + Roe kernel; weno: plus faces + update
-        s->ctx->launches += (nu - 1) + (nv - 1) + weno_launches(s->face, s->n_rows, s->sd_node + 1) - 1;
+        s->ctx->launches += (nu - 1) + (nv - 1) + weno_launches(s->face, s->sd_node + 1) - 1;
     }
     s->ctx->launches += nk;
     if (s->has_bc) {   // the boundary routine as one timed entry
