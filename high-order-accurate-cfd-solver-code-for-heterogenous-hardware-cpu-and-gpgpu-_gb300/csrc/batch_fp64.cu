@@ -105,30 +105,23 @@ k_batch_close(const LatView *__restrict__ views, const BatchTile *__restrict__ t
 cudaError_t batch_stage_fp64(const BatchLaunch &b, int j)
 {
     const int T = b.threads, ld = b.round_tiles * T;
-    k_batch_visc<<<b.ntiles, T, 0, b.stream>>>(b.views, b.tiles, j);
+    cudaError_t e = cudaSuccess;
+    auto launch = [&](auto kernel, dim3 grid, auto... args) {
+        if (e == cudaSuccess) e = batch_launch(kernel, grid, T, b.stream, false, b.views, b.tiles, args...);
+    };
+    launch(k_batch_visc, b.ntiles, j);
     int t0 = 0;
     for (;; t0 += b.round_tiles) {
         const int nt = b.ntiles - t0 < b.round_tiles ? b.ntiles - t0 : b.round_tiles;
-        k_batch_base<<<dim3(nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
-        k_batch_char<<<dim3(5 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
-        k_batch_back<<<dim3(5 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+        launch(k_batch_base, dim3(nt, 3), t0, b.scratch, ld);
+        launch(k_batch_char, dim3(5 * nt, 3), t0, b.scratch, ld);
+        launch(k_batch_back, dim3(5 * nt, 3), t0, b.scratch, ld);
         if (t0 + nt == b.ntiles) break;   // the closing launch takes this round's fluxes
-        k_batch_flux<<<dim3(2 * nt, 3), T, 0, b.stream>>>(b.views, b.tiles, t0, b.scratch, ld);
+        launch(k_batch_flux, dim3(2 * nt, 3), t0, b.scratch, ld);
     }
-    const cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(b.blocks);
-    cfg.blockDim = dim3(T);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = b.stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_batch_close, b.views, b.tiles, b.ntiles, t0, j, b.scratch, ld, b.bar, b.gflags,
-                              b.limit_ns);
+    return batch_launch(k_batch_close, b.blocks, T, b.stream, true, b.views, b.tiles, b.ntiles, t0, j, b.scratch, ld, b.bar,
+                        b.gflags, b.limit_ns);
 }
 
 int batch_launches_fp64(int ntiles, int round_tiles)

@@ -157,21 +157,10 @@ k_batch_close_reduced(const LatView *__restrict__ views, const BatchTile *__rest
 template <class Ops>
 cudaError_t batch_stage_reduced(const BatchLaunch &b, int j)
 {
-    k_batch_fluxes<Ops><<<b.nitems, kFaceThreads, 0, b.stream>>>(b.views, b.items, j);
-    const cudaError_t e = cudaPeekAtLastError();
+    const cudaError_t e = batch_launch(k_batch_fluxes<Ops>, b.nitems, kFaceThreads, b.stream, false, b.views, b.items, j);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(b.blocks);
-    cfg.blockDim = dim3(b.threads);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = b.stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_batch_close_reduced<Ops>, b.views, b.tiles, b.ntiles, j, b.bar,
-                              b.gflags, b.limit_ns);
+    return batch_launch(k_batch_close_reduced<Ops>, b.blocks, b.threads, b.stream, true, b.views, b.tiles, b.ntiles, j, b.bar,
+                        b.gflags, b.limit_ns);
 }
 
 template <class Ops>

@@ -37,6 +37,23 @@ struct BatchLaunch {
     int round_tiles = 0;
 };
 
+// Launches a kernel and returns the launch's own error: an error that other
+// code left pending on this thread is neither taken for it nor cleared.
+template <class... P, class... A>
+cudaError_t batch_launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t stream, bool cooperative, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cooperative ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Nodes whose faces one round of the FP64 form's face kernels takes at most
 // (1.06 GB of scratch).
 constexpr int kBatchRound = 1 << 20;
