@@ -47,8 +47,11 @@ struct cfd_solver {
     unsigned face_gen = 0;
     // structured path
     cfd::StructuredLaunch S{};
-    double *stage9 = nullptr;   // AoS staging, rows 0..N, 9 doubles
-    double *stage5 = nullptr;   // AoS staging, rows 0..N, 5 doubles
+    // AoS staging, rows 0..N of 9 and of 5 doubles (FP64 form: the face
+    // fluxes' array, dead between stages), and FLOW row 0 as last set (no
+    // node: the layout's dummy row; row 0 of the others is zero)
+    double *stage9 = nullptr, *stage5 = nullptr;
+    double row0[9] = {};
     double *Lsoa = nullptr;
     // mixed form: the U slot holding the current state (-1: the uploaded FP64
     // FLOW is current) and the stage whose U_Q outputs are ready (-1: none)
@@ -130,9 +133,9 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
     double *m9, *det, *fm, *fdet;
     cfd_status_t st;
     if ((st = dalloc_t(s, 9 * N, &m9)) || (st = dalloc_t(s, N, &det)) || (st = dalloc_t(s, 9 * N, &fm))
-        || (st = dalloc_t(s, 3 * N, &fdet)) || (st = dalloc_t(s, 9 * N, &S.prim9))
-        || (st = dalloc_t(s, 9 * (N + 1), &s->stage9)) || (st = dalloc_t(s, 5 * (N + 1), &s->stage5))
-        || (st = dalloc_t(s, 5 * N, &s->Lsoa)))
+        || (st = dalloc_t(s, 3 * N, &fdet)) || (st = dalloc_t(s, 9 * N, &S.prim9)) || (st = dalloc_t(s, 5 * N, &s->Lsoa)))
+        return st;
+    if (s->mixed && ((st = dalloc_t(s, 9 * (N + 1), &s->stage9)) || (st = dalloc_t(s, 5 * (N + 1), &s->stage5))))
         return st;
     for (int q = 0; q < 3; ++q)
         if ((st = dalloc_t(s, 5 * N, &S.U[q]))) return st;
@@ -153,17 +156,14 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
             return st;
         cudaMemsetAsync(S.V32, 0, 15 * N * sizeof(float), S.stream);
     } else {          // FP64 stage intermediates
-        const size_t fs_ld = N < kFaceRound ? N : kFaceRound;
         if ((st = dalloc_t(s, 5 * N, &S.Q)) || (st = dalloc_t(s, 15 * N, &S.FEG)) || (st = dalloc_t(s, 15 * N, &S.V))
-            || (st = dalloc_t(s, 5 * N, &S.sh)) || (st = dalloc_t(s, 15 * N, &S.Fh))
-            || (st = dalloc_t(s, 9 * N, &S.kn)) || (st = dalloc_t(s, N, &S.del)) || (st = dalloc_t(s, 3 * (size_t)kFaceScratch * fs_ld, &S.fs)))
+            || (st = dalloc_t(s, 5 * N, &S.sh)) || (st = dalloc_t(s, std::max(15 * N, 9 * (N + 1)), &S.Fh))
+            || (st = dalloc_t(s, 9 * N, &S.kn)) || (st = dalloc_t(s, N, &S.del)))
             return st;
-        S.fs_ld = (int)fs_ld;
+        s->stage9 = s->stage5 = S.Fh;
         cudaMemsetAsync(S.V, 0, 15 * N * sizeof(double), S.stream);
     }
     for (int q = 0; q < 3; ++q) cudaMemsetAsync(S.U[q], 0, 5 * N * sizeof(double), S.stream);
-    cudaMemsetAsync(s->stage5, 0, 5 * (N + 1) * sizeof(double), S.stream);
-    cudaMemsetAsync(s->stage9, 0, 9 * (N + 1) * sizeof(double), S.stream);
     // geometry AoS -> SoA on the host (one-off)
     HostDoubles h, hd, hf, hfd;
     lattice_geometry_soa(g, s->map, h, hd, hf, hfd);
@@ -216,6 +216,15 @@ cfd_status_t create_structured(cfd_solver *s, const cfd_geometry_t *g)
         }
     }
     if (!s->mixed) {
+        // the face pass's scratch, last: as many nodes a round as what is
+        // left allows
+        long long round = std::min((long long)N, (long long)kFaceRound);
+        const auto bytes = [](long long nodes) { return (size_t)nodes * 3 * kFaceScratch * sizeof(double); };
+        const cudaError_t e = round_alloc(round, std::min(round, kLeastRound), bytes, (void **)&S.fs);
+        if (e != cudaSuccess) return cuda_fail(s->ctx, e, "cudaMalloc (solver)");
+        s->allocs.push_back(S.fs);
+        s->bytes += bytes(round);
+        S.fs_ld = (int)round;
         fp64_geometry(S);
         s->ctx->launches += 1;
     }
@@ -306,6 +315,21 @@ cfd_status_t tune_face_tiles(cfd_solver *s)
     std::lock_guard<std::mutex> lock(g_tile_mutex);
     g_tile_cache[key] = {ti, tjk};
     return CFD_OK;
+}
+
+constexpr double kZeroRow[9] = {};
+
+// Rows 0..g_node of `comps` doubles from src to the host; row 0 from row0
+// where that is given (src then holds the nodes alone).  Waits for them.
+cfd_status_t rows_out(cfd_solver *s, void *host, const double *src, int comps, const double *row0, const char *what)
+{
+    const size_t first = row0 ? (size_t)comps : 0;
+    cudaError_t e = cudaMemcpyAsync((double *)host + first, src + first,
+                                    ((size_t)s->n_rows * comps - first) * sizeof(double), cudaMemcpyDeviceToHost,
+                                    s->ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(s->ctx, e, what);
+    if (row0) std::memcpy(host, row0, comps * sizeof(double));
+    return drain(s->ctx);
 }
 
 // where stage j's U_Q comes from (mixed form; the FP64 form always preps)
@@ -532,6 +556,7 @@ cfd_status_t cfd_solver_set_flow(cfd_solver_t *s, const cfd_flow_t *flow_host)
         s->S.stream = s->ctx->stream;
         s->prep_ready = -1;
         s->cur_slot = -1;
+        std::memcpy(s->row0, flow_host, sizeof s->row0);
         st = upload(s, s->stage9, flow_host, R * sizeof(cfd_flow_t));
         if (st == CFD_OK) aos_to_soa(s->ctx->stream, s->stage9, 9, 9, N, s->S.prim9, s->S.row_of);
     }
@@ -544,8 +569,7 @@ cfd_status_t cfd_solver_get_flow(cfd_solver_t *s, cfd_flow_t *flow_host)
     if (!s || !flow_host) return CFD_EINVAL;
     cfd_status_t st = use_device(s->ctx);
     if (st != CFD_OK) return st;
-    const size_t R = (size_t)s->n_rows;
-    const double *src = s->flow;
+    const double *src = s->flow, *row0 = nullptr;
     if (s->path == CFD_PATH_STRUCTURED) {
         s->S.stream = s->ctx->stream;
         if (s->mixed && s->cur_slot >= 0) {   // FP64 FLOW of the current state
@@ -557,10 +581,9 @@ cfd_status_t cfd_solver_get_flow(cfd_solver_t *s, cfd_flow_t *flow_host)
         }
         soa_to_aos(s->ctx->stream, s->S.prim9, 9, 9, (long long)s->ni * s->nj * s->nk, s->stage9, s->S.row_of);
         src = s->stage9;
+        row0 = s->row0;
     }
-    cudaError_t e = cudaMemcpyAsync(flow_host, src, R * sizeof(cfd_flow_t), cudaMemcpyDeviceToHost, s->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(s->ctx, e, "cudaMemcpyAsync D2H (flow)");
-    return drain(s->ctx);
+    return rows_out(s, flow_host, src, 9, row0, "cudaMemcpyAsync D2H (flow)");
 }
 
 cfd_status_t cfd_solver_get_u0(cfd_solver_t *s, cfd_column_t *u0_host)
@@ -568,18 +591,16 @@ cfd_status_t cfd_solver_get_u0(cfd_solver_t *s, cfd_column_t *u0_host)
     if (!s || !u0_host) return CFD_EINVAL;
     cfd_status_t st = use_device(s->ctx);
     if (st != CFD_OK) return st;
-    const size_t R = (size_t)s->n_rows;
-    const double *src = s->U[0];
+    const double *src = s->U[0], *row0 = nullptr;
     if (s->path == CFD_PATH_STRUCTURED) {
         if (s->form == CFD_PREC_MIXED)
             mixed_u_out(make_view(s->S, 0.0, nullptr), 0, s->stage5, s->ctx->stream);
         else
             soa_to_aos(s->ctx->stream, s->S.U[0], 5, 5, (long long)s->ni * s->nj * s->nk, s->stage5, s->S.row_of);
         src = s->stage5;
+        row0 = kZeroRow;
     }
-    cudaError_t e = cudaMemcpyAsync(u0_host, src, R * sizeof(cfd_column_t), cudaMemcpyDeviceToHost, s->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(s->ctx, e, "cudaMemcpyAsync D2H (U0)");
-    return drain(s->ctx);
+    return rows_out(s, u0_host, src, 5, row0, "cudaMemcpyAsync D2H (U0)");
 }
 
 cfd_status_t cfd_solver_step(cfd_solver_t *s, double del_t, int32_t nsteps)
@@ -601,14 +622,13 @@ cfd_status_t cfd_solver_stage(cfd_solver_t *s, int32_t j, double del_t, cfd_colu
     if (st != CFD_OK) return st;
     if ((st = run_stage(s, j, del_t, L_host != nullptr)) != CFD_OK) return st;
     if (L_host) {
-        const size_t R = (size_t)s->n_rows;
-        const double *src = s->L;
+        const double *src = s->L, *row0 = nullptr;
         if (s->path == CFD_PATH_STRUCTURED) {
             soa_to_aos(s->ctx->stream, s->Lsoa, 5, 5, (long long)s->ni * s->nj * s->nk, s->stage5, s->S.row_of);
             src = s->stage5;
+            row0 = kZeroRow;
         }
-        cudaError_t e = cudaMemcpyAsync(L_host, src, R * sizeof(cfd_column_t), cudaMemcpyDeviceToHost, s->ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(s->ctx, e, "cudaMemcpyAsync D2H (L)");
+        return rows_out(s, L_host, src, 5, row0, "cudaMemcpyAsync D2H (L)");
     }
     return drain(s->ctx);
 }

@@ -75,3 +75,22 @@ def test_drop_in_kernels(ctx):
         own.close()
     for x, y in zip(*out):
         assert np.array_equal(x.view(np.uint64), y.view(np.uint64))
+
+
+@pytest.mark.parametrize("maker", ["periodic", "walls"])
+def test_structured_fp64_solver(ctx, maker):
+    """The solver's arrays take 116 doubles per node; 117, as much as before
+    the face pass had scratch, are enough."""
+    from cfd_gb300 import cases, runtime
+    c = cases.taylor_green(n=64) if maker == "periodic" else cases.channel(ni=64, nj=58, nk=60)
+    n = c.g_node
+    s = runtime.Solver(ctx, c)
+    assert s.info().path == "structured"
+    assert s.info().device_bytes <= 8 * n * (117 + 126) + 8 * n      # index and loc codes
+    want = _advance(s, c)
+    assert np.array_equal(want[0], c.arrays["flow"][0])              # the dummy row as it was set
+    with free_memory(8 * n * 117 + 6 * n + SLACK):
+        s = runtime.Solver(ctx, c)
+        assert s.info().device_bytes < 8 * n * (117 + 126 // 2)
+        got = _advance(s, c)
+    assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
