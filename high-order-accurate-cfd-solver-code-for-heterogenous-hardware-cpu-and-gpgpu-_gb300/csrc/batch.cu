@@ -35,7 +35,7 @@ struct BatchInst {
     cfd_params_t prm{};
     double dt = 0.0;
     std::vector<void *> allocs;
-    uint64_t bytes = 0;
+    uint64_t bytes = 0;         // its own arrays
     LatView view{};
     double *stage9 = nullptr;   // AoS FLOW staging rows 0..N (FP64 form: the face fluxes' array, dead between stages)
     double *stage5 = nullptr;   // AoS column staging rows 0..N (likewise)
@@ -47,7 +47,8 @@ struct BatchInst {
 struct cfd_batch {
     cfd_ctx *ctx = nullptr;
     int precision = CFD_PREC_FP64;
-    uint64_t capacity = 0, used = 0;
+    uint64_t capacity = 0, used = 0;      // used: instance_bytes of every instance
+    uint64_t own = 0;                     // their own arrays; the rest of `used` is the face scratch's
     std::vector<BatchInst> slots;
     LatView *d_views = nullptr;
     size_t views_cap = 0;
@@ -60,7 +61,7 @@ struct cfd_batch {
     size_t items_cap = 0;
     int nitems = 0;
     double *d_scratch = nullptr;          // FP64 form: face scratch of round_tiles tiles
-    size_t scratch_cap = 0;               // doubles
+    size_t scratch_cap = 0;               // bytes
     int round_tiles = 0;
     int n_views = 0;
     unsigned *d_words = nullptr;          // [0..1] barrier, [2] batch flags, [3] phase-A work counter, [4..] per-slot flags
@@ -93,9 +94,16 @@ uint64_t instance_bytes(int precision, int64_t N)
     // split: FP32 face metrics (9), node geometry (11), prim32 (9), Q32/R32/V32 (25) and the hi/lo
     // state copy (10); FP64 1/det and Fh (16)
     if (precision == CFD_PREC_SPLIT) return (doubles + 16 * (uint64_t)N) * 8 + (9 + 11 + 9 + 25 + 10) * (uint64_t)N * 4;
-    // FP64: stage intermediates (55, the face fluxes' 15 also the staging rows), unit normals (9), filter width
-    return ((22 + 9 + 15) * n + 50 * n + std::max(15 * n, 9 * (n + 1))) * 8;
+    // FP64: stage intermediates (55, the face fluxes' 15 also the staging
+    // rows), filter width; and ten doubles per node towards the face scratch,
+    // so that a budget filled to the last instance still has rounds of a
+    // fourteenth of the batch
+    return (doubles + 52 * n) * 8;
 }
+
+// Bytes of the budget that the FP64 form's face scratch may take: what the
+// instances' own arrays leave.
+uint64_t scratch_budget(const cfd_batch *b) { return b->capacity > b->own ? b->capacity - b->own : 0; }
 
 void drop_graph(cfd_batch *b)
 {
@@ -104,6 +112,18 @@ void drop_graph(cfd_batch *b)
     b->gexec = nullptr;
     b->graph = nullptr;
     b->graph_ok = false;
+}
+
+// Gives the FP64 form's face scratch back (queued steps may still use it).
+void release_scratch(cfd_batch *b)
+{
+    if (!b->d_scratch) return;
+    cudaStreamSynchronize(b->ctx->stream);
+    drop_graph(b);   // its launches hold the address
+    cudaFree(b->d_scratch);
+    b->d_scratch = nullptr;
+    b->scratch_cap = 0;
+    b->dirty = true;
 }
 
 void free_instance(BatchInst &I)
@@ -234,24 +254,20 @@ cfd_status_t rebuild(cfd_batch *b)
     }
     if (b->precision == CFD_PREC_FP64 && b->ntiles > 0) {
         // scratch for one round of tiles: kBatchRound nodes, or as many as
-        // there is memory for
-        int round = std::min(b->ntiles, std::max(1, kBatchRound / T));
-        for (;; round = (round + 1) / 2) {
-            const size_t need = 3 * (size_t)kFaceScratch * (size_t)round * (size_t)T;
-            if (need <= b->scratch_cap) break;
-            if (b->d_scratch) cudaFree(b->d_scratch);
-            b->d_scratch = nullptr;
-            b->scratch_cap = 0;
-            e = cudaMalloc(&b->d_scratch, need * sizeof(double));
-            if (e == cudaSuccess) {
-                b->scratch_cap = need;
-                break;
-            }
-            b->d_scratch = nullptr;
-            if (e != cudaErrorMemoryAllocation || round == 1) return cuda_fail(b->ctx, e, "batch face scratch");
-            cudaGetLastError();
+        // the budget and the memory leave, one tile at least
+        const auto bytes = [T](long long tiles) { return 3 * (size_t)kFaceScratchNormals * (size_t)tiles * (size_t)T * sizeof(double); };
+        const uint64_t budget = scratch_budget(b);
+        long long round = std::min<long long>(b->ntiles, std::max(1, kBatchRound / T));
+        round = std::max<long long>(1, std::min<long long>(round, (long long)(budget / bytes(1))));
+        if (bytes(round) > b->scratch_cap || b->scratch_cap > std::max<uint64_t>(budget, bytes(1))) {
+            release_scratch(b);
+            void *p = nullptr;
+            e = round_alloc(round, 1, bytes, &p);
+            if (e != cudaSuccess) return cuda_fail(b->ctx, e, "batch face scratch");
+            b->d_scratch = (double *)p;
+            b->scratch_cap = bytes(round);
         }
-        b->round_tiles = round;
+        b->round_tiles = (int)round;
     }
     drop_graph(b);
     b->dirty = false;
@@ -540,6 +556,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     const int N = S->N;
     const uint64_t need = instance_bytes(b->precision, N);
     if (b->used + need > b->capacity) return fail(ctx, CFD_ENOMEM, "cfd_batch_add: device-memory budget exhausted");
+    if (b->own + need + b->scratch_cap > b->capacity) release_scratch(b);   // the next step takes what is left then
     int slot = -1;
     for (size_t s = 0; s < b->slots.size(); ++s)
         if (!b->slots[s].active) {
@@ -594,7 +611,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     v.U2 = U2;
     v.flags = slot_flags(b, slot);
     v.Lout = nullptr;
-    double *kn = nullptr, *del = nullptr;
+    double *del = nullptr;
     if (b->precision == CFD_PREC_MIXED) {
         float *fm32, *fdet32, *node32, *idet32;
         if ((st = ialloc(b, I, 9 * Nz, &fm32)) || (st = ialloc(b, I, 3 * Nz, &fdet32))
@@ -626,11 +643,10 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
     } else {
         if ((st = ialloc(b, I, 5 * Nz, &v.Q)) || (st = ialloc(b, I, 15 * Nz, &v.FEG)) || (st = ialloc(b, I, 15 * Nz, &v.V))
             || (st = ialloc(b, I, 5 * Nz, &v.sh)) || (st = ialloc(b, I, std::max(15 * Nz, 9 * (Nz + 1)), &v.Fh))
-            || (st = ialloc(b, I, 9 * Nz, &kn)) || (st = ialloc(b, I, Nz, &del))) {
+            || (st = ialloc(b, I, Nz, &del))) {
             free_instance(I);
             return st;
         }
-        v.kn = kn;
         v.del = del;
         I.stage9 = I.stage5 = v.Fh;
     }
@@ -684,7 +700,7 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         split_geometry(S);
         batch_prep_split(v, sm);
     } else {
-        fp64_geometry(v, kn, del, sm);
+        fp64_geometry(v, nullptr, del, sm);
         batch_prep_fp64(v, sm);
     }
     ctx->launches += b->precision == CFD_PREC_MIXED   ? 2 + kMixedGeometryLaunches
@@ -697,7 +713,8 @@ cfd_status_t cfd_batch_add_staged(cfd_batch_t *b, cfd_batch_staged_t *staged, in
         return cuda_fail(ctx, e, "cfd_batch_add prep");
     }
     I.active = true;
-    b->used += I.bytes;
+    b->used += need;
+    b->own += I.bytes;
     b->dirty = true;
     *slot_out = slot;
     return CFD_OK;
@@ -708,9 +725,11 @@ cfd_status_t cfd_batch_remove(cfd_batch_t *b, int32_t slot)
     if (!b || slot < 0 || slot >= (int)b->slots.size() || !b->slots[slot].active) return CFD_EINVAL;
     use_device(b->ctx);
     cudaStreamSynchronize(b->ctx->stream);
-    b->used -= b->slots[slot].bytes;
+    b->used -= instance_bytes(b->precision, b->slots[slot].N);
+    b->own -= b->slots[slot].bytes;
     free_instance(b->slots[slot]);
     b->dirty = true;
+    if (b->own == 0) release_scratch(b);
     return CFD_OK;
 }
 

@@ -9,7 +9,10 @@
 // One persistent launch for the whole stage needed 250 registers (8 warps
 // per SM), too few to hide the integer chains of the products and quotients.
 // The face scratch is the batch's, kept between steps, for at most
-// kBatchRound nodes; a larger batch runs its faces in rounds of tiles.
+// kBatchRound nodes and within what the instances leave of the budget; a
+// larger batch runs its faces in rounds of tiles.  The unit normals are formed
+// into it by each stage instead of kept per instance, so that a budget filled
+// to the last instance still has rounds of a fourteenth of the batch.
 // 8 vortices (24^3-48^3, 384,631 nodes), one step with FLOW in and out:
 // 13.9 ms as one persistent launch per stage, 11.8 with the integer products
 // in it, 8.7 ms here.
@@ -49,7 +52,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_base(const LatView *__restrict
     const int w = blockIdx.x;
     const BatchTile t = tiles[t0 + w];
     if ((int)threadIdx.x < t.count)
-        ex::base_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y);
+        ex::base_node<true>(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(256, 4) k_batch_char(const LatView *__restrict__ views,
@@ -57,7 +60,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_char(const LatView *__restrict
 {
     const int w = blockIdx.x / 5u;
     const BatchTile t = tiles[t0 + w];
-    ex::char_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u,
+    ex::char_node<true>(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u,
                   (int)threadIdx.x < t.count, ex::BlockSync{});
 }
 
@@ -67,7 +70,7 @@ __global__ void __launch_bounds__(256, 3) k_batch_back(const LatView *__restrict
     const int w = blockIdx.x / 5u;
     const BatchTile t = tiles[t0 + w];
     if ((int)threadIdx.x < t.count)
-        ex::back_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u);
+        ex::back_node<true>(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + threadIdx.x, blockIdx.y, blockIdx.x % 5u);
 }
 
 // Half h of tile w's faces along d, two lanes per face.
@@ -77,7 +80,7 @@ __device__ __forceinline__ void flux_half(const LatView *__restrict__ views, con
     const BatchTile t = tiles[t0 + w];
     const int k = h * (int)(blockDim.x / 2) + (int)(threadIdx.x / 2);
     const bool in = k < t.count;
-    ex::flux_node(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + (in ? k : 0), d, in);
+    ex::flux_node<true>(views[t.inst], tile_scratch(p, t, w, ld), t.n0 + (in ? k : 0), d, in);
 }
 
 __global__ void __launch_bounds__(256, 2) k_batch_flux(const LatView *__restrict__ views,

@@ -31,7 +31,7 @@ struct BatchLaunch {
     // reduced forms: viscous ranges and face tiles
     const BatchItem *items = nullptr;
     int nitems = 0;
-    // FP64 form: the face kernels' scratch, [3][kFaceScratch] columns of
+    // FP64 form: the face kernels' scratch, [3][kFaceScratchNormals] columns of
     // round_tiles tiles
     double *scratch = nullptr;
     int round_tiles = 0;
@@ -55,7 +55,7 @@ cudaError_t batch_launch(void (*kernel)(P...), dim3 grid, int threads, cudaStrea
 }
 
 // Nodes whose faces one round of the FP64 form's face kernels takes at most
-// (1.06 GB of scratch).
+// (1.13 GB of scratch).
 constexpr int kBatchRound = 1 << 20;
 
 // One RK stage j (its last or only launch cooperative).  Returns the launch

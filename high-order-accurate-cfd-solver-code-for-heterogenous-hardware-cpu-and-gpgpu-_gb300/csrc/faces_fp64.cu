@@ -84,7 +84,7 @@ void fp64_geometry(const StructuredLaunch &S)
 
 void fp64_geometry(const LatView &g, double *kn, double *del, cudaStream_t st)
 {
-    k_geometry<<<dim3(blocks_for(g.N, 128), 3), 128, 0, st>>>(g, kn, del);
+    k_geometry<<<dim3(blocks_for(g.N, 128), kn ? 3 : 1), 128, 0, st>>>(g, kn, del);
 }
 
 int fp64_faces(const StructuredLaunch &S, const LatView &g, cudaStream_t st, const std::function<void(const char *)> &mark)

@@ -37,7 +37,7 @@ struct LatView {
     double *U0, *U1, *U2;
     // FP64 stage intermediates
     double *Q, *FEG, *V, *sh, *Fh;
-    const double *kn;          // [9][N] unit normals of the faces
+    const double *kn;          // [9][N] unit normals of the faces (null: in the face scratch)
     const double *del;         // [N] 1 / det^(1/3) (null: evaluated where it is used)
     // FP32 stage intermediates (mixed form)
     float *Q32, *R32, *V32, *Fh32;
@@ -68,7 +68,9 @@ struct FaceScratch {
     double *p;
     int n0, ld;
 };
-constexpr int kFaceScratch = 42;   // doubles per node and direction
+// doubles per node and direction: with the unit normals in an array of their
+// own (LatView::kn), and with them formed by each stage and kept here
+constexpr int kFaceScratch = 42, kFaceScratchNormals = 45;
 
 __device__ __forceinline__ bool lat_locdir(const LatView &g, int d) { return g.loc8 && ((g.locdirs >> d) & 1); }
 

@@ -173,12 +173,29 @@ __device__ __forceinline__ void face_node(const LatView &g, int n)
 // flux (flux_node).  What they hand on stays in a scratch of kFaceScratch
 // doubles per face and direction.
 enum { FS_BASE = 0, FS_POS = FB_N, FS_NEG = FS_POS + 5, FS_CA = FS_NEG + 5, FS_CB = FS_CA + 5, FS_QP = FS_CB + 5,
-       FS_QN = FS_QP + 5, FS_N = FS_QN + 5 };
+       FS_QN = FS_QP + 5, FS_KN = FS_QN + 5 };
+static_assert(FS_KN == kFaceScratch && FS_KN + 3 == kFaceScratchNormals, "face scratch");
 
-// the scratch column of node n, direction d: element s at [s * ld]
+// The unit normal of a face, component c at [c * ld].
+struct FaceNormal {
+    const double *p;
+    size_t ld;
+    __device__ __forceinline__ double operator()(int c) const { return p[c * ld]; }
+};
+
+// The scratch column of node n, direction d: element s at [s * ld].  KN: the
+// normals are in it.
+template <bool KN>
 __device__ __forceinline__ double *face_column(const FaceScratch &fs, int n, int d)
 {
-    return fs.p + (size_t)d * FS_N * fs.ld + (n - fs.n0);
+    return fs.p + (size_t)d * (KN ? kFaceScratchNormals : kFaceScratch) * fs.ld + (n - fs.n0);
+}
+
+template <bool KN>
+__device__ __forceinline__ FaceNormal face_normal_at(const LatView &g, const FaceScratch &fs, const double *col, int n, int d)
+{
+    if (KN) return {col + (size_t)FS_KN * fs.ld, (size_t)fs.ld};
+    return {g.kn + (size_t)d * 3 * g.N + n, (size_t)g.N};
 }
 
 __device__ __forceinline__ bool face_at(const LatView &g, int n, int d, int &i, int &j, int &k)
@@ -187,6 +204,7 @@ __device__ __forceinline__ bool face_at(const LatView &g, int n, int d, int &i, 
     return lat_face_needed(g, i, j, k, d);
 }
 
+template <bool KN = false>
 __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &fs, int n, int d)
 {
     const int N = g.N;
@@ -202,8 +220,16 @@ __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &f
     Over<true>(sb + si).all(x);
 #pragma unroll
     for (int c = 0; c < 4; ++c) r[c] = x[c];
-    const double kn[3] = {g.kn[(d * 3 + 0) * N + n], g.kn[(d * 3 + 1) * N + n], g.kn[(d * 3 + 2) * N + n]};
-    double B[FB_N], *col = face_column(fs, n, d);
+    double B[FB_N], kn[3], *col = face_column<KN>(fs, n, d);
+    if (KN) {
+        face_normal(g.fm[(d * 3 + 0) * N + n], g.fm[(d * 3 + 1) * N + n], g.fm[(d * 3 + 2) * N + n], kn);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) col[(size_t)(FS_KN + c) * fs.ld] = kn[c];
+    } else {
+        const FaceNormal k = face_normal_at<KN>(g, fs, col, n, d);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) kn[c] = k(c);
+    }
     face_base(r, kn, B);
 #pragma unroll
     for (int s = 0; s < FB_N; ++s) col[(size_t)(FS_BASE + s) * fs.ld] = B[s];
@@ -211,22 +237,22 @@ __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &f
 
 // Every thread of the block calls it when Sync is the block's barrier; those
 // past the range of nodes with active = false.
-template <class Sync = NoSync>
+template <bool KN = false, class Sync = NoSync>
 __device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &fs, int n, int d, int q, bool active,
                                           const Sync &sync = Sync())
 {
     const int N = g.N;
     int i, j, k;
     const bool face = active && face_at(g, n, d, i, j, k);
-    double *col = face_column(fs, n, d);
-    const double *kn = g.kn + (size_t)d * 3 * N + n;
+    double *col = face_column<KN>(fs, n, d);
+    const FaceNormal kn = face_normal_at<KN>(g, fs, col, n, d);
     const size_t ld = fs.ld;
     int s[6];
     double pos, neg;
     char_pair(
         face,
         [&](double (&L)[5]) {
-            left_row(q, [&](int e) { return col[(FS_BASE + e) * ld]; }, [&](int c) { return kn[(size_t)c * N]; }, L);
+            left_row(q, [&](int e) { return col[(FS_BASE + e) * ld]; }, kn, L);
 #pragma unroll
             for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, d, o - 2);
         },
@@ -236,16 +262,16 @@ __device__ __forceinline__ void char_node(const LatView &g, const FaceScratch &f
     col[(FS_NEG + q) * ld] = neg;
 }
 
+template <bool KN = false>
 __device__ __forceinline__ void back_node(const LatView &g, const FaceScratch &fs, int n, int d, int q)
 {
     const int N = g.N;
     int i, j, k;
     if (!face_at(g, n, d, i, j, k)) return;
-    double *col = face_column(fs, n, d);
-    const double *kn = g.kn + (size_t)d * 3 * N + n;
+    double *col = face_column<KN>(fs, n, d);
     const size_t ld = fs.ld;
     double qp, qn;
-    back_pair(q, [&](int s) { return col[(FS_BASE + s) * ld]; }, [&](int c) { return kn[(size_t)c * N]; },
+    back_pair(q, [&](int s) { return col[(FS_BASE + s) * ld]; }, face_normal_at<KN>(g, fs, col, n, d),
               [&](int s) { return col[(FS_POS + s) * ld]; }, [&](int s) { return col[(FS_NEG + s) * ld]; }, qp, qn);
     col[(FS_QP + q) * ld] = qp;
     col[(FS_QN + q) * ld] = qn;
@@ -260,13 +286,14 @@ __device__ __forceinline__ void back_node(const LatView &g, const FaceScratch &f
 
 // lanes 2m and 2m + 1 of a warp: the pos and neg side of one face; lanes
 // without a face take part with a face they do not store
+template <bool KN = false>
 __device__ __forceinline__ void flux_node(const LatView &g, const FaceScratch &fs, int n, int d, bool active)
 {
     const int N = g.N;
     int i, j, k;
     const bool face = active && face_at(g, n, d, i, j, k);
     const int side = threadIdx.x & 1;
-    const double *col = face_column(fs, n, d);
+    const double *col = face_column<KN>(fs, n, d);
     const size_t ld = fs.ld;
     double q[5] = {1.0, 0.0, 0.0, 0.0, 2.5}, m[3] = {1.0, 0.0, 0.0}, det = 1.0, Fhat[5];
     if (face) {
@@ -284,11 +311,13 @@ __device__ __forceinline__ void flux_node(const LatView &g, const FaceScratch &f
 }
 
 // What the face and viscous kernels take from the geometry alone, once per
-// solver: the unit normals of the faces along d and the filter width.
+// solver: the unit normals of the faces along d (kn null: none) and the
+// filter width.
 __device__ __forceinline__ void geometry_node(const LatView &g, double *kn, double *del, int n, int d)
 {
     const int N = g.N;
     if (d == 0) del[n] = filter_width(g.det[n]);
+    if (!kn) return;
     double k[3];
     face_normal(g.fm[(d * 3 + 0) * N + n], g.fm[(d * 3 + 1) * N + n], g.fm[(d * 3 + 2) * N + n], k);
 #pragma unroll
