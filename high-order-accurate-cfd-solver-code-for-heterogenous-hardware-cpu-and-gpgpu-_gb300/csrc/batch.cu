@@ -150,7 +150,7 @@ void face_tile_items(const LatView &g, int v, int kind, std::vector<BatchItem> &
     const dim3 gr = T::grid(g);
     for (unsigned y = 0; y < gr.y; ++y)
         for (unsigned x = 0; x < gr.x; ++x)
-            out.push_back(BatchItem{v, kind, (int)x * T::kTile, (int)y * T::kWide, 0, 0});
+            out.push_back(BatchItem{v, kind, (int)x * T::kTile, (int)y * T::kWide});
 }
 
 // The i tiles of lattice view v, of the width that costs least: the number of
@@ -238,7 +238,7 @@ cfd_status_t rebuild(cfd_batch *b)
         std::vector<BatchItem> items;
         for (int v = 0; v < (int)views.size(); ++v)
             for (int n0 = 0; n0 < views[v].N; n0 += kFaceThreads)
-                items.push_back(BatchItem{v, kBatchVisc, n0, std::min(kFaceThreads, views[v].N - n0), 0, 0});
+                items.push_back(BatchItem{v, kBatchVisc, n0, std::min(kFaceThreads, views[v].N - n0)});
         for (const auto &f : faces) items.insert(items.end(), f.begin(), f.end());
         if (items.size() > b->items_cap) {
             if (b->d_items) cudaFree(b->d_items);

@@ -98,7 +98,7 @@ __device__ __forceinline__ int next_item(unsigned *bar)
 // kinds 3 and 4 along j and k.
 constexpr int kBatchVisc = 5;
 struct BatchItem {
-    int inst, kind, a, b, c, pad;
+    int inst, kind, a, b;
 };
 
 // The fluxes of every instance: the viscous ranges first (their chains are
@@ -118,7 +118,7 @@ k_batch_fluxes(const LatView *__restrict__ views, const BatchItem *__restrict__ 
     __shared__ float smem[tile_smem_floats<FaceTile<0, kBatchTilesI[0]>>()];   // the widest staging
     const BatchItem it = items[blockIdx.x];
     const LatView &g = views[it.inst];
-    const TileAt at{it.a, it.b, it.c};
+    const TileAt at{it.a, it.b, 0};
     switch (it.kind) {
     case kBatchVisc: {
         if ((int)threadIdx.x >= it.b) return;

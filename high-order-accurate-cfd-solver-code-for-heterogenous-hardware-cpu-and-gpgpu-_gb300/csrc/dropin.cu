@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128) k_uq(double *__restrict__ U, double *__re
             const double *sn = sh + 5 * (size_t)nr, *sg = sh + 5 * (size_t)gid;
             const double sb = sn[0];
             double x[4] = {sn[1] + sg[1], sn[2] + sg[2], sn[3] + sg[3], sn[4] + sg[4]};
-            ex::Over<true>(sb + si).all(x);
+            ex::Over(sb + si).all(x);
 #pragma unroll
             for (int c = 0; c < 4; ++c) ra[c] = x[c];
             ra[4] = xi::mul(sb, si);

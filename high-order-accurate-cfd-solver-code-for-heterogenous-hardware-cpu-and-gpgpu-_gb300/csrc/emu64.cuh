@@ -171,35 +171,5 @@ __device__ __forceinline__ double sub(double a, double b) { return add(a, f64(u6
 // a * b (exact_int.cuh).
 __device__ __forceinline__ double mul(double a, double b) { return xi::mul(a, b); }
 
-// A binary64 value whose +, - and * run on the integer pipe (the routines
-// above; the same bits as the FP64 instructions).  An expression over Dbl
-// reads and evaluates exactly like the same expression over double: the
-// same operations in the same order, double constants converted exactly.
-struct Dbl {
-    double v;
-    Dbl() = default;
-    __host__ __device__ __forceinline__ constexpr Dbl(double x) : v(x) {}
-};
-__device__ __forceinline__ Dbl operator+(Dbl a, Dbl b) { return Dbl(add(a.v, b.v)); }
-__device__ __forceinline__ Dbl operator-(Dbl a, Dbl b) { return Dbl(sub(a.v, b.v)); }
-__device__ __forceinline__ Dbl operator*(Dbl a, Dbl b) { return Dbl(mul(a.v, b.v)); }
-__device__ __forceinline__ Dbl operator-(Dbl a) { return Dbl(f64(u64(a.v) ^ kSign)); }
-
-// Products on the integer pipe, sums on the FP64 pipe.
-struct DblM {
-    double v;
-    DblM() = default;
-    __host__ __device__ __forceinline__ constexpr DblM(double x) : v(x) {}
-};
-__device__ __forceinline__ DblM operator+(DblM a, DblM b) { return DblM(__dadd_rn(a.v, b.v)); }
-__device__ __forceinline__ DblM operator-(DblM a, DblM b) { return DblM(__dsub_rn(a.v, b.v)); }
-__device__ __forceinline__ DblM operator*(DblM a, DblM b) { return DblM(mul(a.v, b.v)); }
-__device__ __forceinline__ DblM operator-(DblM a) { return DblM(f64(u64(a.v) ^ kSign)); }
-
-// The double held by a value of any of the three types.
-__device__ __forceinline__ double val(double x) { return x; }
-__device__ __forceinline__ double val(Dbl x) { return x.v; }
-__device__ __forceinline__ double val(DblM x) { return x.v; }
-
 }  // namespace emu
 }  // namespace cfd

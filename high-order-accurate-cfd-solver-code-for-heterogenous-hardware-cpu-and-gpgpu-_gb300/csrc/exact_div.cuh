@@ -23,7 +23,9 @@
 // full division sequence.  quotient_int goes further on a part whose FP64
 // rate is a small fraction of its integer rate: only q0 on the FP64 pipe,
 // its rounding decided from the exact integer remainder of the significands
-// (the default of div()).
+// (the default of div()).  The kernels take scale2 from here and their
+// quotients from exact_int.cuh; div, rcp and pow2_over are the forms for code
+// without its groups, which cfd_probe_emu64 runs against the device.
 #pragma once
 
 #include <cstdint>
@@ -39,7 +41,7 @@
 // top 53 bits of the integer product of the significands of x and y (no
 // FP64 instruction; the faster choice in kernels with warps to hide its
 // integer latency, 3 or more blocks of 128 per SM), 0 the FP64 product
-// RN(x*y) (faster at 2 blocks per SM, which no kernel runs at now).  A translation unit
+// RN(x*y) (faster at 2 blocks per SM).  A translation unit
 // sets it before its first include; the two variants live in different
 // inline namespaces, so the host functions of units built with different
 // choices do not collide at link time.  Both give the same bits.

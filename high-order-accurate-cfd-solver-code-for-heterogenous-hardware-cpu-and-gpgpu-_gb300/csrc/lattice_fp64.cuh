@@ -126,48 +126,8 @@ __device__ __forceinline__ void mu_node(const LatView &g, int n, int q)
     g.prim9[LF_MU * N + n] = mu_of<true>(Ui, g.P);
 }
 
-// Face n+1/2 along D: Roe average of the two nodes, LLF face flux and the
-// 6th-order correction (Weno.cl:336-3058 for that face, once).  SD: shared
-// reciprocals for divisions by one divisor (physics_exact.cuh Over).
-template <int D, bool SD = true>
-__device__ __forceinline__ void face_node(const LatView &g, int n)
-{
-    const int N = g.N;
-    int i, j, k;
-    lat_ijk(g, n, i, j, k);
-    if (!lat_face_needed(g, i, j, k, D)) return;
-    int s[6];
-#pragma unroll
-    for (int o = 0; o < 6; ++o) s[o] = lat_step(g, i, j, k, D, o - 2);
-    double pts[6][5];
-#pragma unroll
-    for (int o = 0; o < 6; ++o)
-#pragma unroll
-        for (int c = 0; c < 5; ++c) pts[o][c] = g.Q[c * N + s[o]];
-    double r[5];
-    {
-        const int l = s[2], rr = s[3];   // node (left) and its +D neighbour
-        const double sb = g.sh[rr], si = g.sh[l];
-        r[4] = sb * si;
-        const Over<SD> den(sb + si);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) r[c] = den(g.sh[(1 + c) * N + rr] + g.sh[(1 + c) * N + l]);
-    }
-    double Fhat[5];
-    face_flux<SD>(pts, g.fm[(D * 3 + 0) * N + n], g.fm[(D * 3 + 1) * N + n], g.fm[(D * 3 + 2) * N + n], g.fdet[D * N + n],
-              r, g.P.eps, Fhat);
-    const double *NF = g.FEG + (size_t)D * 5 * N;
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-        double f[6];
-#pragma unroll
-        for (int o = 0; o < 6; ++o) f[o] = NF[c * N + s[o]];
-        g.Fh[(D * 5 + c) * N + n] = corrected(Fhat[c], f);
-    }
-}
-
-// Face n+1/2 along d in four kernels (physics_exact.cuh), over the faces of
-// a range of nodes: the Roe average and its scalars (base_node), one thread
+// Face n+1/2 along d (Weno.cl:336-3058 for that face, once) in four kernels
+// (physics_exact.cuh), over the faces of a range of nodes: the Roe average and its scalars (base_node), one thread
 // per characteristic field and correction component (char_node), one per
 // component of the face states (back_node), two lanes per face for the LLF
 // flux (flux_node).  What they hand on stays in a scratch of kFaceScratch
@@ -217,7 +177,7 @@ __device__ __forceinline__ void base_node(const LatView &g, const FaceScratch &f
     r[4] = sb * si;
 #pragma unroll
     for (int c = 0; c < 4; ++c) x[c] = g.sh[(1 + c) * N + rr] + g.sh[(1 + c) * N + n];
-    Over<true>(sb + si).all(x);
+    Over(sb + si).all(x);
 #pragma unroll
     for (int c = 0; c < 4; ++c) r[c] = x[c];
     double B[FB_N], kn[3], *col = face_column<KN>(fs, n, d);

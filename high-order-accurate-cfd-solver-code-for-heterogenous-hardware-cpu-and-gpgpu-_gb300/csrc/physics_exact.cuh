@@ -9,12 +9,11 @@
 // algebraic rewriting) and the translation units that include this header
 // are compiled with --fmad=false.  With IEEE-correct division and square
 // root on the GPU this reproduces the reference's results to the last bit
-// except where libm functions differ (cbrt).  Divisions that share a divisor
-// use one reciprocal and an exactly checked correction (exact_div.cuh,
-// `Over`), and the reciprocals, the corrections and the single divisions
-// decide their rounding from exact integer remainders: the same bits as the
-// division, with most of the work moved from the FP64 pipe (two operations
-// per clock per SM on GB300) to the integer pipes.
+// except where libm functions differ (cbrt).  The products, quotients and
+// roots run on the integer pipe (exact_int.cuh; divisions that share a
+// divisor share its reciprocal, `Over`), which decides their rounding
+// exactly: the same bits, with most of the work moved from the FP64 pipe (two
+// operations per clock per SM on GB300).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -29,15 +28,9 @@ namespace ex {
 
 __device__ __forceinline__ double sq(double x) { return x * x; }
 
-// Division of several numerators by one divisor b: Over<true>(b)(x) == x / b,
-// bit for bit, with the reciprocal computed once (exact_div.cuh);
-// Over<false> divides each numerator (the same bits; faster where the
-// kernel's occupancy hides the division latency, e.g. the batched form).
-template <bool SHARED>
-struct Over;
-
-template <>
-struct Over<true> {
+// Division of several numerators by one divisor b: Over(b)(x) == x / b, bit
+// for bit, with the reciprocal computed once (exact_int.cuh).
+struct Over {
     xi::Divisor d;
     __device__ __forceinline__ explicit Over(double divisor) : d(xi::divisor(divisor)) {}
     // with Y of xi::Divisor given as a double's bits (y of reciprocal())
@@ -59,13 +52,6 @@ struct Over<true> {
     }
 };
 
-template <>
-struct Over<false> {
-    double b;
-    __device__ __forceinline__ explicit Over(double divisor) : b(divisor) {}
-    __device__ __forceinline__ double operator()(double x) const { return x / b; }
-};
-
 // a / b with the same bits (exact_int.cuh).
 __device__ __forceinline__ double dv(double a, double b) { return xi::divide(a, b); }
 
@@ -76,12 +62,11 @@ __device__ __forceinline__ double enthalpy(double rho, double u, double v, doubl
 }
 
 // U_Q.cl:60-109 for one face: {u, v, w, h, rho}; (sb,...) the neighbour.
-template <bool SD = true>
 __device__ __forceinline__ void roe(double sb, double ub, double vb, double wb, double hb, double si, double ui,
                                     double vi, double wi, double hi, double r[5])
 {
     r[4] = sb * si;
-    const Over<SD> d(sb + si);
+    const Over d(sb + si);
     r[0] = d(sb * ub + si * ui);
     r[1] = d(sb * vb + si * vi);
     r[2] = d(sb * wb + si * wi);
@@ -89,7 +74,6 @@ __device__ __forceinline__ void roe(double sb, double ub, double vb, double wb, 
 }
 
 // WENO5 pair, Weno.cl:1056-1280; c[0..5] = left-2 .. right+2.
-template <bool SD = true>
 __device__ __forceinline__ void weno_pair(const double cc[6], double eps, double &pos, double &neg)
 {
     const double *c = cc + 2;   // c[0] = left node of the face
@@ -114,7 +98,7 @@ __device__ __forceinline__ void weno_pair(const double cc[6], double eps, double
     const double wm0 = dv(5.0 / 16.0, sq(eps + (ISm0)));
     const double wm1 = dv(5.0 / 8.0, sq(eps + (ISm1)));
     const double wm2 = dv(1.0 / 16.0, sq(eps + (ISm2)));
-    const Over<SD> sp(wp0 + wp1 + wp2), sm(wm0 + wm1 + wm2);
+    const Over sp(wp0 + wp1 + wp2), sm(wm0 + wm1 + wm2);
     const double Wp0 = sp(wp0), Wp1 = sp(wp1), Wp2 = sp(wp2);
     const double Wm0 = sm(wm0), Wm1 = sm(wm1), Wm2 = sm(wm2);
     pos = Wp0 * p0 + Wp1 * p1 + Wp2 * p2;
@@ -128,10 +112,9 @@ struct StateQuot {
     double k1, k2, k3, e12, e13, e23, v1, v2, v3, v4;
 };
 
-template <bool SD = true>
 __device__ __forceinline__ StateQuot state_quot(const double q[5])
 {
-    const Over<true> d(q[0]);
+    const Over d(q[0]);
     double a[6] = {q[1] * q[1], q[2] * q[2], q[3] * q[3], q[1] * q[2], q[1] * q[3], q[2] * q[3]};
     double b[4] = {q[1], q[2], q[3], q[4]};
     d.all(a);
@@ -174,14 +157,13 @@ __device__ __forceinline__ double lambda5(const double q[5], const StateQuot &t,
 // face metric and Roe state r = {u,v,w,h,rho}, projection of the six stencil
 // points pts (left-2 .. right+2), WENO5, back-projection, contravariant
 // fluxes x face det, lambda_5 LLF.
-template <bool SD = true>
 __device__ __forceinline__ void face_flux(const double pts[6][5], double mx, double my, double mz, double DET_F,
                                           const double r[5], double eps, double Fhat[5])
 {
     const double ru = r[0], rv = r[1], rw = r[2], rh = r[3], rrho = r[4];
     const double kk = sqrt(mx * mx + my * my + mz * mz);
     const double a = sqrt(0.4 * (rh - xdiv::scale2<-1>(ru * ru + rv * rv + rw * rw)));
-    const Over<SD> dk(kk);
+    const Over dk(kk);
     const double kx = dk(mx), ky = dk(my), kz = dk(mz);
     const double theta = kx * ru + ky * rv + kz * rw;
     const double phi_sq = 0.5 * 0.4 * (ru * ru + rv * rv + rw * rw);
@@ -189,7 +171,7 @@ __device__ __forceinline__ void face_flux(const double pts[6][5], double mx, dou
     const double beta = dv(1.0, sqrt(2.0) * rrho * a);
     double cpos[5], cneg[5];
     {
-        const Over<SD> da(a * a), dr(rrho);
+        const Over da(a * a), dr(rrho);
         const double f = da(phi_sq);
         const double Lm[5][5] = {
             {kx * (1.0 - f) - dr(kz * rv - ky * rw), da(kx * 0.4 * ru), da(kx * 0.4 * rv) + dr(kz),
@@ -209,12 +191,12 @@ __device__ __forceinline__ void face_flux(const double pts[6][5], double mx, dou
             for (int o = 0; o < 6; ++o)
                 cv[o] = Lm[q][0] * pts[o][0] + Lm[q][1] * pts[o][1] + Lm[q][2] * pts[o][2] + Lm[q][3] * pts[o][3]
                         + Lm[q][4] * pts[o][4];
-            weno_pair<SD>(cv, eps, cpos[q], cneg[q]);
+            weno_pair(cv, eps, cpos[q], cneg[q]);
         }
     }
     double qp[5], qn[5];
     {
-        const Over<SD> d4(0.4);
+        const Over d4(0.4);
         const double R[5][5] = {
             {kx, ky, kz, alpha, alpha},
             {kx * ru, ky * ru - kz * rrho, kz * ru + ky * rrho, alpha * (ru + kx * a), alpha * (ru - kx * a)},
@@ -231,7 +213,7 @@ __device__ __forceinline__ void face_flux(const double pts[6][5], double mx, dou
                     + R[q][4] * (cneg[4]);
         }
     }
-    const StateQuot tp = state_quot<SD>(qp), tn = state_quot<SD>(qn);
+    const StateQuot tp = state_quot(qp), tn = state_quot(qn);
     const double lp = lambda5(qp, tp, mx, my, mz);
     const double ln = lambda5(qn, tn, mx, my, mz);
     double al = __longlong_as_double(0x7ff8000000000000ULL);   // NaN when neither branch holds (NaN input)
@@ -262,7 +244,7 @@ enum { FB_U, FB_V, FB_W, FB_R, FB_A, FB_TH, FB_PHI, FB_OMF, FB_ALPHA, FB_BETA, F
 // Unit normal of a face metric (Weno.cl:337-348).
 __device__ __forceinline__ void face_normal(double mx, double my, double mz, double k[3])
 {
-    const Over<true> dk(sqrt(mx * mx + my * my + mz * mz));
+    const Over dk(sqrt(mx * mx + my * my + mz * mz));
     double q[3] = {mx, my, mz};
     dk.all(q);
     k[0] = q[0];
@@ -277,7 +259,7 @@ __device__ __forceinline__ void face_base(const double r[5], const double k[3], 
     const double q2 = ru * ru + rv * rv + rw * rw;
     const double a = xi::root(0.4 * (rh - xdiv::scale2<-1>(q2)));
     const double phi_sq = 0.5 * 0.4 * q2;
-    const Over<true> da(a * a), dr(rrho);
+    const Over da(a * a), dr(rrho);
     B[FB_U] = ru;
     B[FB_V] = rv;
     B[FB_W] = rw;
@@ -308,7 +290,7 @@ __device__ __forceinline__ void left_row(int q, const Base &base, const Normal &
         const double kc = kn(q), kq = kn(n), km = kn(m);
         const double rc = base(FB_U + q), rq = base(FB_U + n), rm = base(FB_U + m);
         const double a = base(FB_A);
-        const Over<true> da(a * a, base(FB_YA2)), dr(base(FB_R), base(FB_YR));
+        const Over da(a * a, base(FB_YA2)), dr(base(FB_R), base(FB_YR));
         const double kc4 = kc * 0.4;
         double x[4] = {kc4 * rc, kc4 * rq, kc4 * rm, kc4}, y[3] = {km * rq - kq * rm, km, kq};
         da.all(x);
@@ -443,8 +425,8 @@ __device__ __forceinline__ void weno_pair_i(bool face, const double c[6], double
     sync();
     if (!face) return;   // no barrier follows
     double a[3] = {S[5], S[4], S[3]}, b[3] = {S[2], S[1], S[0]};
-    Over<true>(a[0] + a[1] + a[2]).all(a);
-    Over<true>(b[0] + b[1] + b[2]).all(b);
+    Over(a[0] + a[1] + a[2]).all(a);
+    Over(b[0] + b[1] + b[2]).all(b);
     const xi::Fac f[6] = {xi::fac(a[0]), xi::fac(a[1]), xi::fac(a[2]), xi::fac(b[0]), xi::fac(b[1]), xi::fac(b[2])};
     const xi::Fac f1 = xi::fac(p1), f2 = xi::fac(p2);
     const xi::Fac v[6] = {xi::fac(p0), f1, f2, f1, f2, xi::fac(m2)};
@@ -498,7 +480,7 @@ __device__ __forceinline__ void side_flux(const double q[5], double mx, double m
         const xi::Fac u[7] = {q1, q2, q3, q1, q1, q2, q0}, v[7] = {q1, q2, q3, q2, q3, q3, q0};
         double r[7];
         xi::mul_n(u, v, r);
-        const Over<true> d(q[0]);
+        const Over d(q[0]);
         const double k = dv(r[0] + r[1] + r[2], xdiv::scale2<1>(r[6]));
 #pragma unroll
         for (int i = 0; i < 6; ++i) a[i] = r[i];
@@ -592,7 +574,7 @@ __device__ __forceinline__ void back_pair(int q, const Base &base, const Normal 
             e[1] = t[1];
             e[2] = t[2];
             e[3] = phi + y[0];
-            Over<true>(0.4).all(e);
+            Over(0.4).all(e);
         }
         {
             const xi::Fac u[6] = {fkz, fky, fkx, fkz, fky, fkx}, v[6] = {fv, fw, fw, fu, fu, fv};
@@ -817,8 +799,8 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
         double s[4] = {Ui[0], Ui[1], Ui[2], Ui[3]};
         squares<I>(s);
         double x[5] = {1.0, Ui[1], Ui[2], Ui[3], Ui[4]}, y[7] = {Ui[1], Ui[2], Ui[3], Ui[4], s[1], s[2], s[3]};
-        Over<true>(Ui[0]).all(x);   // r0, v1, v2, v3, U4 / U0
-        Over<true>(s[0]).all(y);    // a1 .. a4, U1^2, U2^2, U3^2 over U0^2
+        Over(Ui[0]).all(x);   // r0, v1, v2, v3, U4 / U0
+        Over(s[0]).all(y);    // a1 .. a4, U1^2, U2^2, U3^2 over U0^2
         d_temp = product<I>(P.c_temp, x[4] - scale2<-1>(y[4] + y[5] + y[6]));
 #pragma unroll 1
         for (int d = 0; d < 3; ++d) {
@@ -927,7 +909,7 @@ __device__ __forceinline__ void viscous_node(const Deriv &dU, const double Ui[5]
                 double R[3] = {dm, dm, dm};
                 const double by[3] = {K[0], K[1], K[2]};
                 xi::div_n(R, by);
-                Over<true>(C_T).all(R);
+                Over(C_T).all(R);
                 const double one[3] = {1.0 + R[0], 1.0 + R[1], 1.0 + R[2]};
                 xi::div_n(c, one);
             }
@@ -1033,7 +1015,7 @@ __device__ __forceinline__ double mu_of(const double Ui[5], const Phys &P)
     double s[4] = {Ui[0], Ui[1], Ui[2], Ui[3]};
     squares<I>(s);
     double y[3] = {s[1], s[2], s[3]};
-    Over<true>(s[0]).all(y);
+    Over(s[0]).all(y);
     const double d_temp = product<I>(P.c_temp, dv(Ui[4], Ui[0]) - xdiv::scale2<-1>(y[0] + y[1] + y[2]));
     const double sd = xi::root(d_temp);
     return product<I>(product<I>(product<I>(sd, sd), sd), dv(P.st1, d_temp + P.st));
@@ -1064,7 +1046,7 @@ __device__ __forceinline__ void rk_and_primitives(int j, double del_t, double ma
     } else {
         double t[5], s[5], r[5], z[5] = {U0[0], U0[1], U0[2], U0[3], U0[4]};
         const double y[5] = {U2[0], U2[1], U2[2], U2[3], U2[4]};
-        Over<true>(3.0).all(z);
+        Over(3.0).all(z);
         scaled<I>(del_t, l5, t);
         scaled<I>(2.0 / 3.0, y, s);
         scaled<I>(2.0 / 3.0, t, r);
@@ -1077,7 +1059,7 @@ __device__ __forceinline__ void rk_and_primitives(int j, double del_t, double ma
         scaled<I>(dv(1.0, det), un, fu);
     }
     rho = fu[0];
-    const Over<true> d0(fu[0]);   // u, v, w, e, p / rho and 1.4 p / rho share the divisor
+    const Over d0(fu[0]);   // u, v, w, e, p / rho and 1.4 p / rho share the divisor
     double q[4] = {fu[1], fu[2], fu[3], fu[4]};
     d0.all(q);
     u = q[0];
