@@ -292,14 +292,12 @@ __device__ __forceinline__ void face_tile(const LatView &g, TileAt at, float *sm
     const int N = g.N;
     int n, t, a;
     const bool face = tile_face<T, D>(g, at, n, t, a);
-    float m[3] = {0.f, 0.f, 0.f}, det_f = 0.f;   // loaded while the staging waits
-    if (face) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) m[c] = lat_ldg(g.fm32 + (size_t)(D * 3 + c) * N, 4u * n);
-        det_f = lat_ldg(g.fdet32 + (size_t)D * N, 4u * n);
-    }
     stage_face_lines<T, D>(g, at, sQ, sR, sF);
     if (!face) return;
+    float m[3];   // loaded here: before the staging it costs registers (a direction along k 0.072 -> 0.082 ms)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) m[c] = lat_ldg(g.fm32 + (size_t)(D * 3 + c) * N, 4u * n);
+    const float det_f = lat_ldg(g.fdet32 + (size_t)D * N, 4u * n);
     float2 P[3][5];
     float r[5];
     tile_stencil<T>(sQ, sR, t, a, P, r);
