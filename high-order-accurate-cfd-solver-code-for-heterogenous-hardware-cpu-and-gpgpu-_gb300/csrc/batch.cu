@@ -255,6 +255,7 @@ cfd_status_t rebuild(cfd_batch *b)
     if (b->precision == CFD_PREC_FP64 && b->ntiles > 0) {
         // scratch for one round of tiles: kBatchRound nodes, or as many as
         // the budget and the memory leave, one tile at least
+        static_assert(3ull * kFaceScratchNormals * 8 * kBatchRound / 10000000 == 113, "cfd_rhs.h states the size");
         const auto bytes = [T](long long tiles) { return 3 * (size_t)kFaceScratchNormals * (size_t)tiles * (size_t)T * sizeof(double); };
         const uint64_t budget = scratch_budget(b);
         long long round = std::min<long long>(b->ntiles, std::max(1, kBatchRound / T));

@@ -132,8 +132,8 @@ void bc_apply_split(cudaStream_t st, const BcDevice &bc, const LatView &g, int q
 // Target m of one entry of the routine on a lattice state held in a
 // precision form's own representation: m = 0 the boundary node, m = 1..3
 // its ghosts (face codes; node rules have only m = 0, mirror passes only
-// m = 1..3).  The same rules on (rho, u, v, w, p), the fields the next stage
-// reads (U_Q.cl takes rho, u, v, w, p of FLOW): outlet copies the first
+// m = 1..3).  The routine's rules for the fields the next stage reads (U_Q.cl
+// takes rho, u, v, w, p of FLOW), on the state U they form: outlet copies the first
 // inward node into the node and its ghosts, inlet writes the free stream
 // (Flow_Initialisation.cpp:35-48), boundary mirrors inward node m into
 // ghost m, wall sets zero velocity at the node and mirrors with the velocity

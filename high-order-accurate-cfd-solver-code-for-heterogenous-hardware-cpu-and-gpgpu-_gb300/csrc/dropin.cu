@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(128, 6) k_row_base(const int *__restrict__ gri
 }
 
 // blocks of 256 whose warps keep to one phase (faces_fp64.cu k_face_char): Weno
-// on 96^3 rows 4.77 -> 4.70 ms
+// on 96^3 rows 4.77 -> 4.74 ms
 __global__ void __launch_bounds__(256, 4) k_row_char(const double *__restrict__ Q, double eps, RowRound R)
 {
     const int gid = R.r0 + (blockIdx.x / 5u) * blockDim.x + threadIdx.x, d = blockIdx.y, q = blockIdx.x % 5u;

@@ -15,8 +15,8 @@
 // SM).  The hand-over between the kernels (kFaceScratch doubles per face)
 // costs 0.7 KB per face of L2 and HBM traffic, which the FP64-bound kernels
 // hide.  TGV 128^3, all three directions: 16.1 ms with one kernel per
-// direction and only the divisions on the integer pipe; 9.8 ms here
-// (base 0.30, char 5.78, back 1.97, flux 1.70; the FP64 pipe is busy 65 to
+// direction and only the divisions on the integer pipe; 9.9 ms here
+// (base 0.30, char 5.88, back 1.97, flux 1.70; the FP64 pipe is busy 65 to
 // 80 % of the time, with branch-free groups and an instruction footprint
 // that stays near the instruction cache's size as the remaining limits).
 #include "internal.h"
@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(128, 6) k_face_base(LatView g, FaceScratch fs,
 // 0.182 ms.  Instruction fetch is what costs it most after the FP64 pipe:
 // blocks of 256 instead of 128 at 64 registers 6.18 -> 5.90 ms, with a barrier
 // between the phases 5.78 (vortex 1.00 -> 0.91, 53,000 nodes 0.180 -> 0.170;
-// blocks of 512 6.10, of 128 with barriers 6.07).
+// blocks of 512 6.10, of 128 with barriers 6.07), and 5.88 with the threads
+// that have no face meeting it too, as it has to be.
 constexpr int kCharThreads = 256;
 template <int MB>
 __global__ void __launch_bounds__(kCharThreads, MB) k_face_char(LatView g, FaceScratch fs, int n1, int d0)
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(128, 4) k_face_flux(LatView g, FaceScratch fs,
 
 void face_char(const LatView &g, const FaceScratch &fs, int n1, int mb, int d0, int nd, cudaStream_t st)
 {
-    const dim3 grid(5 * blocks_for(n1 - fs.n0, kCharThreads), nd);   // the five fields of 128 faces are neighbouring blocks
+    const dim3 grid(5 * blocks_for(n1 - fs.n0, kCharThreads), nd);   // the five fields of 256 faces are neighbouring blocks
     if (mb == 2) k_face_char<2><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);
     else if (mb == 3) k_face_char<3><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);
     else k_face_char<4><<<grid, kCharThreads, 0, st>>>(g, fs, n1, d0);

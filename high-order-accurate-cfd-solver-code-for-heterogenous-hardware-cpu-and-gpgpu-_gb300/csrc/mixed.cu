@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) k_mu_m(LatView g, int q)
     if (n < g.N) mx::mu_node(g, n, q);
 }
 
-// 72 registers, no spills: a direction at 128^3 0.070 ms; 0.073 at 64
+// 72 registers, no spills: a direction at 128^3 0.071 ms; 0.074 at 64
 // registers, 0.072 at 77, 0.078 at 94.
 #ifndef CFD_MFACE_MIN_BLOCKS
 #define CFD_MFACE_MIN_BLOCKS 7

@@ -31,9 +31,10 @@ __device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(frcp(a.x),
 // WENO5 on both lanes (neg, pos) in differences: the face value less a node's
 // value, from the lane's one-sided differences away from the node next to the
 // face on its own side: d3 (second to third node), d2 (first to second) and
-// (-p, p) (across the face); the fourth is -swap(d2).  The candidates (15/8,-5/4,3/8 | 3/8,3/4,-1/8 | -1/8,3/4,3/8)
-// less the own node's value, the linear weights 1 : 10 : 5 folded into them and
-// w_k = d_k/(eps+IS_k)^2 with IS and eps over 13/12 (eps here is 12/13 of
+// (-p, p) (across the face); the fourth is -swap(d2).  The candidates
+// (15/8,-5/4,3/8 | 3/8,3/4,-1/8 | -1/8,3/4,3/8) less the own node's value, the
+// linear weights 1 : 10 : 5 folded into them and w_k = d_k/(eps+IS_k)^2 with
+// IS and eps over 13/12 (eps here is 12/13 of
 // the scheme's), which the quotient does not see: 30 paired operations
 // where the same reconstruction of five values takes 47, and its rounding
 // scales with the variation across the stencil.

@@ -38,6 +38,7 @@ constexpr long long kLeastRound = 4096;   // rows or nodes of a round at least (
 // scratch for one round of rows, [3][kRowFace][round].
 constexpr int kRowFace = 48;               // doubles of one row's face along one direction
 constexpr long long kRowRound = 1 << 18;   // rows of a round at most: 302 MB, some 25 waves of blocks
+static_assert(3 * kRowFace * 8 == 1152, "cfd_rhs.h states the bytes per row of a round");
 struct RowScratch {
     double *face = nullptr;   // null: none, each row evaluates both faces itself
     double *col = nullptr;

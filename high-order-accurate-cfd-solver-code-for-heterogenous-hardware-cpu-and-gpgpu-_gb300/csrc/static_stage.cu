@@ -37,6 +37,7 @@ namespace {
 constexpr size_t kPerNode = 22 + 9 + 15 + 5 + 15 + 15 + 5 + 9 + 1 + 3 * kFaceScratch + 15 + 5;   // 242
 constexpr size_t kFlagDoubles = 32;                                    // 256 B for the error word
 constexpr size_t kScratchDoubles = (size_t)CFD_STATIC_MAX_NODES * kPerNode + kFlagDoubles;
+static_assert(kScratchDoubles * 8 / 1000000 == 63, "cfd_rhs.h states the size");
 
 static __device__ __align__(256) double g_stage_scratch[kScratchDoubles];
 

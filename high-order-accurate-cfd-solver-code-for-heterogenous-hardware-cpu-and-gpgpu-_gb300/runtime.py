@@ -103,8 +103,8 @@ class Context:
         self.check(self.lib.cfd_ctx_set_rows(self.h, int(n_rows)), "cfd_ctx_set_rows")
 
     def set_face_reuse(self, on: bool):
-        """cfd_weno: share each interior face between its two rows (default)
-        or evaluate both faces at every row as the reference does."""
+        """cfd_uq and cfd_weno: share each interior face between its two rows
+        (default) or evaluate both faces at every row as the reference does."""
         self.check(self.lib.cfd_ctx_set_face_reuse(self.h, 1 if on else 0), "cfd_ctx_set_face_reuse")
 
     def set_async(self, on: bool):
@@ -591,8 +591,9 @@ class Batch:
         self.ctx.check(self.lib.cfd_batch_set_wait_limit(self.h, int(limit_ns)), "cfd_batch_set_wait_limit")
 
     def set_tiling(self, tile_nodes: int = 0, max_blocks: int = 0, use_graph: bool = True):
-        """tile_nodes: 64/128/256 (1-D tiles), abi.BATCH_FACE_TILES (shared-memory
-        face tiles, mixed and split batches), 0 keeps the current choice."""
+        """tile_nodes: 32/64/128/256 nodes per tile, abi.BATCH_FACE_TILES (128;
+        mixed and split batches), 0 keeps the current choice; max_blocks: of
+        the closing launch."""
         self.ctx.check(self.lib.cfd_batch_set_tiling(self.h, int(tile_nodes), int(max_blocks), 1 if use_graph else 0),
                        "cfd_batch_set_tiling")
 

@@ -182,8 +182,11 @@ cfd_status_t cfd_ctx_set_rows(cfd_ctx_t *ctx, int32_t n_rows);
  * inputs (Weno.cl:336-3058 evaluates both at every row), and cfd_uq computes
  * sqrt(rho) and H once per row instead of once per row and neighbour
  * (U_Q.cl:60-109); the results are the same bits.  on = 0 evaluates
- * everything per row, as the reference does.  Needs 252 bytes per row,
- * allocated by cfd_ctx_set_rows. */
+ * everything per row, as the reference does.  Needs 252 bytes per row and
+ * 1,152 bytes per row of a round, allocated by cfd_ctx_set_rows: a round is
+ * all rows up to 2^18 (302 MB), less where memory is short.  Both calls use
+ * that memory, so those of one context must not overlap on different streams;
+ * cfd_viscous uses no memory but its arguments. */
 cfd_status_t cfd_ctx_set_face_reuse(cfd_ctx_t *ctx, int on);
 /* Kernels this context launched since creation (for accounting). */
 uint64_t cfd_ctx_launch_count(const cfd_ctx_t *ctx);
@@ -377,18 +380,22 @@ typedef struct cfd_batch cfd_batch_t;
 typedef struct {
     int32_t n_active;          /* instances in the batch                      */
     int32_t tile_nodes;        /* nodes per tile = threads per block          */
-    int32_t blocks;            /* persistent grid size                        */
+    int32_t blocks;            /* grid of a stage's closing launch            */
     int32_t graph;             /* 1 when steps replay a captured CUDA graph   */
     int32_t precision;         /* cfd_precision_t of the whole batch          */
     int32_t n_held;            /* instances held out of cfd_batch_step        */
     uint64_t nodes_total;
-    uint64_t device_bytes;     /* admitted instance memory                    */
+    uint64_t device_bytes;     /* admitted: cfd_batch_instance_bytes of each  */
     uint64_t capacity_bytes;   /* admission budget                            */
-    int32_t face_tiles;        /* 1: phase A in shared-memory face tiles      */
+    int32_t face_tiles;        /* 1: CFD_BATCH_FACE_TILES is set (below)      */
     int32_t reserved;
 } cfd_batch_info_t;
 
-/* capacity_bytes = 0: 85 % of the device memory free at creation. */
+/* capacity_bytes = 0: 85 % of the device memory free at creation.  The FP64
+ * form also works through a scratch of up to 1.13 GB, which takes what the
+ * instances' own arrays leave of the budget (102 of 112 doubles per node are
+ * theirs): a budget filled to the last instance runs its faces in rounds of a
+ * fourteenth of the batch, a tenth slower. */
 cfd_status_t cfd_batch_create(cfd_ctx_t *ctx, int32_t precision, uint64_t capacity_bytes, cfd_batch_t **batch);
 cfd_status_t cfd_batch_destroy(cfd_batch_t *b);
 /* Device bytes one instance of `nodes` lattice nodes takes (admission). */
@@ -440,8 +447,10 @@ cfd_status_t cfd_batch_slot_status(cfd_batch_t *b, int32_t slot);
  * error flags.  Waits for queued steps first.  This is the recovery path
  * after a barrier timeout and the restore path of a checkpoint. */
 cfd_status_t cfd_batch_set_flow(cfd_batch_t *b, int32_t slot, const cfd_flow_t *flow_host);
-/* Deadline of the persistent kernel's grid barrier in nanoseconds (< 0: the
- * default, 5 s + 50 ns per batched node).  A block that waits longer gives up
+/* Deadline of the closing launch's grid barrier in nanoseconds (< 0: the
+ * default, 5 s + 50 ns per batched node; in the reduced forms the barrier
+ * orders nothing and is there for this deadline alone).  A block that waits
+ * longer gives up
  * and skips the rest of that stage; the step reports CFD_ETIMEOUT once (the
  * reference exits the process on any kernel failure, Solver.cpp:378-381)
  * and every instance it was advancing is marked interrupted: its state is
@@ -449,18 +458,17 @@ cfd_status_t cfd_batch_set_flow(cfd_batch_t *b, int32_t slot, const cfd_flow_t *
  * (CFD_ETIMEOUT) until cfd_batch_set_flow restores it or it is removed.
  * Instances that were held are not affected. */
 cfd_status_t cfd_batch_set_wait_limit(cfd_batch_t *b, int64_t limit_ns);
-/* tile_nodes in {32, 64, 128, 256}: phase A of a stage works on 1-D tiles of
- * that many nodes, each face evaluated from its own stencil gathers;
- * CFD_BATCH_FACE_TILES (mixed and split batches): phase A works on the
- * viscous ranges and on 2-D face tiles whose stencil lines a block of 128
- * threads stages in shared memory (32 faces along i x 4, or 16 along j or k
- * x 8); 0 keeps the current choice.  max_blocks (0 = occupancy limit),
- * use_graph 0/1. */
+/* tile_nodes in {32, 64, 128, 256}: nodes per tile, that is threads per block,
+ * of the FP64 form's launches and of the reduced forms' closing launch (their
+ * fluxes always run on face tiles of 128, whose stencil lines a block stages
+ * in shared memory); CFD_BATCH_FACE_TILES (mixed and split batches): the same
+ * as 128; 0 keeps the current choice.  max_blocks: blocks of the closing
+ * launch at most (0 = occupancy limit).  use_graph 0/1.  Every choice gives
+ * the same bits. */
 #define CFD_BATCH_FACE_TILES 1
 cfd_status_t cfd_batch_set_tiling(cfd_batch_t *b, int32_t tile_nodes, int32_t max_blocks, int32_t use_graph);
-/* Times each tiling (1-D tiles of 32, 64, 128, 256 nodes and, for the mixed and
- * split batches, the face tiles) on the live batch (state saved and
- * restored) and keeps the fastest. */
+/* Times tiles of 32, 64, 128 and 256 nodes on the live batch (state saved
+ * and restored) and keeps the fastest; nothing where every instance is held. */
 cfd_status_t cfd_batch_tune(cfd_batch_t *b, int32_t steps_per_trial);
 cfd_status_t cfd_batch_info(const cfd_batch_t *b, cfd_batch_info_t *info);
 
@@ -521,7 +529,7 @@ cfd_status_t cfd_probe_emu64(cfd_ctx_t *ctx, int64_t n_per_class, uint64_t seed,
  * only handed buffers): one SSP-RK3 stage j on a periodic ni x nj x nk
  * lattice, the same kernels as the resident solver's structured path, with
  * every intermediate kept in a library-owned device array sized for
- * CFD_STATIC_MAX_NODES nodes (about 27 MB per GPU that loads the library,
+ * CFD_STATIC_MAX_NODES nodes (about 63 MB per GPU that loads the library,
  * held until the process exits).  The caller passes the reference-layout
  * device buffers, rows 1..ni*nj*nk in lattice order (i fastest); det, deter
  * and metric are read; FLOW, U_j, the U the stage advances and L_out (may be
