@@ -359,8 +359,9 @@ cfd_status_t cfd_rk3_step(cfd_ctx_t *ctx, double Mach, double del_t, const cfd_d
 cfd_status_t cfd_solver_set_boundary(cfd_solver_t *s, const cfd_bc_t *bc);
 
 /* One stage j of the host loop with a CUDA event around every kernel
- * launch; out[i] receives each launch's name and device time.  The stage
- * advances the state like cfd_solver_stage. */
+ * launch; out[i] receives each launch's name and device time (the launches of
+ * a pass that runs in rounds, of a drop-in call or of the boundary routine
+ * are one entry).  The stage advances the state like cfd_solver_stage. */
 typedef struct {
     char name[24];
     double ms;
